@@ -6,11 +6,17 @@
 // the header (a few hundred bytes of text) is scanned on the host and the vertex block goes to
 // the device as it is in the file; one kernel then turns each vertex into a record.
 //
-// Kernel layout: a CTA owns 128 consecutive vertices.  It copies their bytes (128 × stride)
-// into shared memory with coalesced 4-byte loads, so a field at any byte offset is one or two
-// shared words joined by a funnel shift (strides need not be multiples of 4).  Each thread
-// builds its record in registers and stores it into a dense shared row; one cp.async.bulk
-// store then writes the CTA's records (128 × 224 B or 128 × 128 B) to global memory.
+// Kernel layout: a CTA owns 128 consecutive vertices.  It copies their bytes (128 × stride) into
+// shared memory, by 16-byte cp.async where the block is 16-byte aligned (any 128 vertices then
+// start on such a boundary), else by coalesced 4-byte loads; each thread builds its record in
+// registers, and the records take the vertices' place in shared memory on their way out (FP32
+// records by one cp.async.bulk store, half records by coalesced 16-byte stores).
+//
+// What bounds it: HBM.  A record's values are defined in double (gs_convert.cuh), and in double the
+// kernel took 783 us for 1M degree-3 vertices into FP32 records, all of it on the double pipe
+// (about 300 operations a vertex at two per clock and SM).  Worked out in pairs of floats, with the
+// double path kept for the vertices whose rounding the pairs do not settle (gs_convert_fast.cuh;
+// about 0.1 % of covariances), the same bits take 87 us: 472 MB at 5.4 TB/s, 80 % of a plain copy.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -19,6 +25,7 @@
 
 #include <cuda_bf16.h>
 
+#include "gs_convert_fast.cuh"
 #include "gs_internal.h"
 
 namespace gs {
@@ -220,144 +227,246 @@ struct PlyParams {
     gs_ply_layout L;
     const uint8_t *vertices;
     uint8_t *records;
+    uint32_t wide;  // vertices 16-byte aligned: whole CTAs stage by 16-byte copies
 };
-
-// The float at byte b of the staged words (b need not be a multiple of 4).
-__device__ __forceinline__ float staged_f32(const uint32_t *s, uint32_t b) {
-    const uint32_t w = b >> 2, sh = (b & 3u) * 8u;
-    uint32_t v = s[w];
-    if (sh) v = __funnelshift_r(v, s[w + 1], sh);
-    return __uint_as_float(v);
-}
 
 __device__ __forceinline__ uint32_t f16_bits(float x) { return (uint32_t)__half_as_ushort(__float2half_rn(x)); }
 __device__ __forceinline__ uint32_t bf16_bits(float x) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
 
+// 2^(j/32), j = 0..31, as pairs of floats (exp_certain), copied to shared memory by each CTA.
+__constant__ Two c_exp_table[GS_EXP_TABLE_SIZE] = GS_EXP_TABLE;
+
+// A vertex's fields in the staged bytes.  ALIGNED: the vertex starts on a word, every field lies
+// on a word, and f_rest is one ascending run, so a field is one shared load at a constant distance
+// from a base; otherwise a field is one or two words joined by a funnel shift.
+template <bool ALIGNED>
+struct StagedVertex {
+    const gs_ply_layout &L;
+    const uint32_t *s;
+    uint32_t base;  // byte of the vertex in the staged words
+
+    __device__ __forceinline__ float at(int32_t off) const {
+        const uint32_t b = base + (uint32_t)off, w = b >> 2;
+        if constexpr (ALIGNED) return __uint_as_float(s[w]);
+        const uint32_t sh = (b & 3u) * 8u;
+        uint32_t v = s[w];
+        if (sh) v = __funnelshift_r(v, s[w + 1], sh);
+        return __uint_as_float(v);
+    }
+
+    // SH coefficient k of channel c: f_rest is channel-major (K coefficients of R, then G, then B)
+    __device__ __forceinline__ float sh(uint32_t K, uint32_t k, uint32_t c) const {
+        if (k >= K) return 0.0f;
+        if constexpr (ALIGNED) return __uint_as_float(s[((base + (uint32_t)L.f_rest[0]) >> 2) + c * K + k]);
+        return at(L.f_rest[c * K + k]);
+    }
+};
+
+// The double path of the colour (rgb = 0.5 + SH_C0·f_dc and a = sigmoid(opacity), to 8 bits), of
+// a scale and of a rotation: taken where the float path is not certain of its rounding.
+__device__ __noinline__ uint32_t ply_unorm8_dc(float dc) { return unorm8_rne(0.5 + kShC0 * (double)dc); }
+__device__ __noinline__ uint32_t ply_unorm8_opacity(float op) { return unorm8_rne(1.0 / (1.0 + exp(-(double)op))); }
+__device__ __noinline__ float ply_scale(float s) { return (float)exp((double)s); }
+__device__ __noinline__ float4 ply_rot(float x, float y, float z, float w) {
+    const double q[4] = {x, y, z, w};
+    const double nrm = sqrt(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
+    return make_float4((float)(q[0] / nrm), (float)(q[1] / nrm), (float)(q[2] / nrm), (float)(q[3] / nrm));
+}
+struct Cov3d {
+    float v[6];
+};
+__device__ __noinline__ Cov3d ply_cov3d(float4 r, float s0, float s1, float s2) {
+    const float rot[4] = {r.x, r.y, r.z, r.w}, scale[3] = {s0, s1, s2};
+    Cov3d c;
+    cov3d_from_rot_scale(rot, scale, c.v);
+    return c;
+}
+
+// Half records leave through rows padded to 144 bytes (dense 128-byte rows would put a
+// quarter-warp's 16-byte stores on one bank).
 template <uint32_t FMT>
+constexpr uint32_t kPlyRowBytes = (FMT == GS_FORMAT_FP32) ? 224u : 144u;
+
+// Tiles ahead of its own whose vertex bytes a CTA asks L2 for (as the preprocess does).
+constexpr uint32_t kPlyPrefetchTiles = 152 * 4;
+
+template <uint32_t FMT, bool ALIGNED>
 __global__ void __launch_bounds__(kPlyThreads) ply_convert_kernel(const __grid_constant__ PlyParams P) {
     constexpr uint32_t REC = (FMT == GS_FORMAT_FP32) ? 224u : 128u;
+    constexpr uint32_t ROW16 = kPlyRowBytes<FMT> / 16;
+    // The staged vertex words, and after all threads hold their records in registers, the rows of
+    // the records in the same bytes: half the shared memory, so more CTAs an SM.
     extern __shared__ __align__(16) uint8_t smem[];
-    uint4 *s_out = reinterpret_cast<uint4 *>(smem);                      // kPlyThreads × REC
-    uint32_t *s_in = reinterpret_cast<uint32_t *>(smem + kPlyThreads * REC);  // staged vertex words
+    uint32_t *s_in = reinterpret_cast<uint32_t *>(smem);
+    uint4 *s_out = reinterpret_cast<uint4 *>(smem);
+    __shared__ Two s_table[GS_EXP_TABLE_SIZE];
     const gs_ply_layout &L = P.L;
     const uint32_t tid = threadIdx.x;
     const uint64_t first = (uint64_t)blockIdx.x * kPlyThreads;
     const uint32_t cnt = (uint32_t)min((uint64_t)kPlyThreads, (uint64_t)L.count - first);
+    const bool wide = P.wide && cnt == kPlyThreads;  // 128 × stride bytes from a 16-byte boundary
+    if (tid < GS_EXP_TABLE_SIZE) s_table[tid] = c_exp_table[tid];
 
-    // ---- stage the CTA's vertex bytes [b0, b1) as the words that cover them ----
-    const uint64_t total = (uint64_t)L.count * L.stride;
+    // ---- stage the CTA's vertex bytes [b0, b1) ----
     const uint64_t b0 = first * L.stride, b1 = (first + cnt) * L.stride;
-    const uint64_t w0 = b0 >> 2, w1 = (b1 + 3) >> 2;
-    const uint32_t nw = (uint32_t)(w1 - w0);
-    const uint32_t *v32 = reinterpret_cast<const uint32_t *>(P.vertices);
-    const uint64_t whole = total >> 2;  // words lying wholly inside the vertex block
-    for (uint32_t k = tid; k < nw; k += kPlyThreads) {
-        const uint64_t w = w0 + k;
-        uint32_t v;
-        if (w < whole) {
-            v = __ldcs(v32 + w);
-        } else {  // the block's last, partial word: only its bytes below `total`
-            v = 0;
-            for (uint32_t j = 0; j < 4; ++j)
-                if (w * 4 + j < total) v |= (uint32_t)P.vertices[w * 4 + j] << (8 * j);
+    const uint64_t w0 = b0 >> 2;
+    if (wide) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(P.vertices + b0);
+        const uint32_t chunks = kPlyThreads * L.stride / 16u;
+        for (uint32_t q = tid; q < chunks; q += kPlyThreads) cp_async16(smem + 16u * q, src + q);
+        const uint64_t ahead = first + (uint64_t)kPlyPrefetchTiles * kPlyThreads;
+        if (tid == 0 && ahead + kPlyThreads <= L.count)
+            prefetch_l2_bulk(P.vertices + ahead * L.stride, kPlyThreads * L.stride);
+        cp_async_wait_all();
+    } else {
+        // the words that cover the bytes; a block's last, partial word is read bytewise
+        const uint64_t total = (uint64_t)L.count * L.stride, w1 = (b1 + 3) >> 2, whole = total >> 2;
+        const uint32_t nw = (uint32_t)(w1 - w0);
+        const uint32_t *v32 = reinterpret_cast<const uint32_t *>(P.vertices);
+        for (uint32_t k = tid; k < nw; k += kPlyThreads) {
+            const uint64_t w = w0 + k;
+            uint32_t v;
+            if (w < whole) {
+                v = __ldcs(v32 + w);
+            } else {
+                v = 0;
+                for (uint32_t j = 0; j < 4; ++j)
+                    if (w * 4 + j < total) v |= (uint32_t)P.vertices[w * 4 + j] << (8 * j);
+            }
+            s_in[k] = v;
         }
-        s_in[k] = v;
     }
     __syncthreads();
 
+    uint32_t rec[REC / 4];  // the record, in words
     if (tid < cnt) {
-        const uint32_t base = (uint32_t)((first + tid) * L.stride - (w0 << 2));
-        auto rd = [&](int32_t off) { return staged_f32(s_in, base + (uint32_t)off); };
-        // colour: rgb = 0.5 + SH_C0·f_dc and a = sigmoid(opacity), to 8 bits
+        const StagedVertex<ALIGNED> V{L, s_in, (uint32_t)((first + tid) * L.stride - (w0 << 2))};
+        // colour: floats within 1e-4 of 255·channel settle all but the halfway cases
         uint32_t color = 0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) color |= unorm8_rne(0.5 + kShC0 * (double)rd(L.f_dc[c])) << (8 * c);
-        color |= unorm8_rne(1.0 / (1.0 + exp(-(double)rd(L.opacity)))) << 24;
+        for (int c = 0; c < 3; ++c) {
+            const float dc = V.at(L.f_dc[c]);
+            uint32_t u;
+            if (!unorm8_certain(fmaf(dc, (float)(255.0 * kShC0), 127.5f), 1e-4f, &u)) u = ply_unorm8_dc(dc);
+            color |= u << (8 * c);
+        }
+        {
+            const float op = V.at(L.opacity);
+            uint32_t u;
+            if (!unorm8_certain(255.0f / (1.0f + expf(-op)), 1e-4f, &u)) u = ply_unorm8_opacity(op);
+            color |= u << 24;
+        }
         float scale[3], rot[4];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) scale[k] = (float)exp((double)rd(L.scale[k]));
-        {
-            const double q[4] = {rd(L.rot[1]), rd(L.rot[2]), rd(L.rot[3]), rd(L.rot[0])};  // x, y, z, w
-            const double nrm = sqrt(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) rot[k] = (float)(q[k] / nrm);
+        for (int k = 0; k < 3; ++k) {
+            const float s = V.at(L.scale[k]);
+            if (!exp_certain(s, s_table, &scale[k])) scale[k] = ply_scale(s);
         }
-        // SH: f_rest is channel-major (K coefficients of R, then G, then B); sh[3k + c]
-        const uint32_t K = L.sh_rest;
-        auto sh = [&](int k, int c) { return (uint32_t)k < K ? rd(L.f_rest[c * K + k]) : 0.0f; };
-        uint4 *row = s_out + tid * (REC / 16);
-        if constexpr (FMT == GS_FORMAT_FP32) {
-            uint32_t w[56];
-            w[0] = __float_as_uint(rd(L.pos[0]));
-            w[1] = __float_as_uint(rd(L.pos[1]));
-            w[2] = __float_as_uint(rd(L.pos[2]));
-            w[3] = color;
-#pragma unroll
-            for (int k = 0; k < 15; ++k)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) w[4 + 3 * k + c] = __float_as_uint(sh(k, c));
-            float cov[6];
-            cov3d_from_rot_scale(rot, scale, cov);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) w[49 + k] = __float_as_uint(cov[k]);
-            w[55] = 0u;
-#pragma unroll
-            for (int k = 0; k < 14; ++k) row[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-        } else {
-            uint32_t h[64];  // the record as 16-bit units
-#pragma unroll
-            for (int k = 0; k < 64; ++k) h[k] = 0u;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const uint32_t b = __float_as_uint(rd(L.pos[k]));
-                h[2 * k] = b & 0xFFFFu;
-                h[2 * k + 1] = b >> 16;
+        {
+            const float q[4] = {V.at(L.rot[1]), V.at(L.rot[2]), V.at(L.rot[3]), V.at(L.rot[0])};  // x, y, z, w
+            if (!unit_quat_certain(q, [](float s) { return rsqrtf(s); }, rot)) {
+                const float4 r = ply_rot(q[0], q[1], q[2], q[3]);
+                rot[0] = r.x;
+                rot[1] = r.y;
+                rot[2] = r.z;
+                rot[3] = r.w;
             }
-            h[6] = color & 0xFFFFu;
-            h[7] = color >> 16;
+        }
+        const uint32_t K = L.sh_rest;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) h[8 + k] = f16_bits(rot[k]);
+        for (int k = 0; k < 3; ++k) rec[k] = __float_as_uint(V.at(L.pos[k]));
+        rec[3] = color;
+        if constexpr (FMT == GS_FORMAT_FP32) {
+            float cov[6];
+            if (!cov3d_certain(rot, scale, cov)) {
+                const Cov3d c = ply_cov3d(make_float4(rot[0], rot[1], rot[2], rot[3]), scale[0], scale[1], scale[2]);
 #pragma unroll
-            for (int k = 0; k < 3; ++k) h[12 + k] = f16_bits(scale[k]);
+                for (int k = 0; k < 6; ++k) cov[k] = c.v[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) rec[49 + k] = __float_as_uint(cov[k]);
+            rec[55] = 0u;
 #pragma unroll
             for (int k = 0; k < 15; ++k)
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    h[15 + 3 * k + c] = (FMT == GS_FORMAT_HALF_SH_FP16) ? f16_bits(sh(k, c)) : bf16_bits(sh(k, c));
+                for (int c = 0; c < 3; ++c) rec[4 + 3 * k + c] = __float_as_uint(V.sh(K, k, c));
+        } else {
+            // 16-bit units from byte 16: rot, scale, SH, padding
+            rec[4] = f16_bits(rot[0]) | (f16_bits(rot[1]) << 16);
+            rec[5] = f16_bits(rot[2]) | (f16_bits(rot[3]) << 16);
+            rec[6] = f16_bits(scale[0]) | (f16_bits(scale[1]) << 16);
+            rec[7] = f16_bits(scale[2]);
+            auto sh16 = [&](int i) {  // unit i of the SH run
+                const float v = V.sh(K, i / 3, i % 3);
+                return (FMT == GS_FORMAT_HALF_SH_FP16) ? f16_bits(v) : bf16_bits(v);
+            };
+            rec[7] |= sh16(0) << 16;
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                row[k] = make_uint4(h[8 * k] | (h[8 * k + 1] << 16), h[8 * k + 2] | (h[8 * k + 3] << 16),
-                                    h[8 * k + 4] | (h[8 * k + 5] << 16), h[8 * k + 6] | (h[8 * k + 7] << 16));
+            for (int i = 1; i < 45; i += 2) rec[8 + i / 2] = sh16(i) | (sh16(i + 1) << 16);
+            rec[30] = rec[31] = 0u;
         }
     }
-
-    // ---- one bulk store of the CTA's records (generic-proxy writes made visible to it first) ----
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-        const uint32_t src = (uint32_t)__cvta_generic_to_shared(s_out);
-        uint8_t *dst = P.records + first * REC;
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src),
-                     "r"(cnt * REC)
-                     : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncthreads();  // every vertex is in registers: the rows may take its place
+    if (tid < cnt) {
+        uint4 *row = s_out + tid * ROW16;
+#pragma unroll
+        for (uint32_t k = 0; k < REC / 16; ++k)
+            row[k] = make_uint4(rec[4 * k], rec[4 * k + 1], rec[4 * k + 2], rec[4 * k + 3]);
+    }
+    uint8_t *dst = P.records + first * REC;
+    if constexpr (FMT == GS_FORMAT_FP32) {
+        // one bulk store of the CTA's records (generic-proxy writes made visible to it first)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (tid == 0) {
+            const uint32_t src = (uint32_t)__cvta_generic_to_shared(s_out);
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src),
+                         "r"(cnt * REC)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
+    } else {
+        __syncthreads();
+        constexpr uint32_t C16 = REC / 16;
+        uint4 *d16 = reinterpret_cast<uint4 *>(dst);
+        for (uint32_t q = tid; q < cnt * C16; q += kPlyThreads) d16[q] = s_out[(q / C16) * ROW16 + q % C16];
     }
 }
 
-template <uint32_t FMT>
+// Whether every field of a vertex lies on a word and f_rest is one ascending run of floats.
+static bool ply_layout_aligned(const gs_ply_layout &L) {
+    uint32_t low = L.stride;
+    for (int k = 0; k < 3; ++k) low |= (uint32_t)(L.pos[k] | L.f_dc[k] | L.scale[k]);
+    for (int k = 0; k < 4; ++k) low |= (uint32_t)L.rot[k];
+    low |= (uint32_t)L.opacity;
+    for (uint32_t k = 0; k < 3 * L.sh_rest; ++k) {
+        low |= (uint32_t)L.f_rest[k];
+        if (L.f_rest[k] != L.f_rest[0] + 4 * (int32_t)k) return false;
+    }
+    return (low & 3u) == 0;
+}
+
+template <uint32_t FMT, bool ALIGNED>
 cudaError_t launch_ply_fmt(const PlyParams &P, cudaStream_t st) {
-    constexpr uint32_t REC = (FMT == GS_FORMAT_FP32) ? 224u : 128u;
-    const size_t smem = kPlyThreads * REC + align_up((size_t)kPlyThreads * P.L.stride + 8, 16);
-    cudaError_t e = cudaFuncSetAttribute(ply_convert_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kPlyThreads * REC + align_up((size_t)kPlyThreads * kPlyMaxStride + 8, 16)));
+    auto smem_of = [](uint32_t stride) {
+        const size_t in = align_up((size_t)kPlyThreads * stride + 8, 16), out = kPlyThreads * kPlyRowBytes<FMT>;
+        return in > out ? in : out;
+    };
+    cudaError_t e = cudaFuncSetAttribute(ply_convert_kernel<FMT, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem_of(kPlyMaxStride));
     if (e != cudaSuccess) return e;
     const uint32_t grid = (P.L.count + kPlyThreads - 1) / kPlyThreads;
-    ply_convert_kernel<FMT><<<grid, kPlyThreads, smem, st>>>(P);
+    ply_convert_kernel<FMT, ALIGNED><<<grid, kPlyThreads, smem_of(P.L.stride), st>>>(P);
     count_launches(1);
     return cudaGetLastError();
+}
+
+template <uint32_t FMT>
+cudaError_t launch_ply_layout(const PlyParams &P, cudaStream_t st) {
+    return ply_layout_aligned(P.L) ? launch_ply_fmt<FMT, true>(P, st) : launch_ply_fmt<FMT, false>(P, st);
 }
 
 cudaError_t launch_ply_convert(const void *vertices, const gs_ply_layout &L, uint32_t format, void *records,
@@ -367,13 +476,14 @@ cudaError_t launch_ply_convert(const void *vertices, const gs_ply_layout &L, uin
     P.L = L;
     P.vertices = static_cast<const uint8_t *>(vertices);
     P.records = static_cast<uint8_t *>(records);
+    P.wide = (uintptr_t)vertices % 16 == 0 ? 1u : 0u;
     switch (format) {
         case GS_FORMAT_FP32:
-            return launch_ply_fmt<GS_FORMAT_FP32>(P, st);
+            return launch_ply_layout<GS_FORMAT_FP32>(P, st);
         case GS_FORMAT_HALF_SH_FP16:
-            return launch_ply_fmt<GS_FORMAT_HALF_SH_FP16>(P, st);
+            return launch_ply_layout<GS_FORMAT_HALF_SH_FP16>(P, st);
         default:
-            return launch_ply_fmt<GS_FORMAT_HALF_SH_BF16>(P, st);
+            return launch_ply_layout<GS_FORMAT_HALF_SH_BF16>(P, st);
     }
 }
 

@@ -428,13 +428,6 @@ __device__ __forceinline__ bool gaussian_selected(const uint32_t *selection, uin
 }
 
 // ---- global -> shared staging: 16-byte cp.async chunks, or a bulk copy on an mbarrier -----
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
