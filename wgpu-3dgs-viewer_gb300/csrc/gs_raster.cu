@@ -540,6 +540,14 @@ __global__ void tile_ranges_kernel(const uint2 *__restrict__ pairs, const Ctrl *
 // The tile sort keeps its own control block; fold its status bits into the raster's.
 __global__ void merge_status_kernel(Ctrl *dst, const Ctrl *src) { dst->status |= src->status; }
 
+// exp(x) on [-9, 0] by the SFU: what __expf computes, without its handling of denormal arguments
+// and results (an argument that small flushes to 0, whose exp is the same 1).
+__device__ __forceinline__ float exp_sfu(float x) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(x, 1.4426950408889634f)));
+    return e;
+}
+
 // One fragment of a staged splat at the pixel centre (pxc, pyc) (render.wesl:143-181):
 // false when discarded or when it cannot change the pixel, else its alpha.
 template <uint32_t MODE, bool PORTABLE_EXP>
@@ -556,7 +564,7 @@ __device__ __forceinline__ bool fragment(const float4 a, const float4 b, float p
         const float r2 = fmaf(qx, qx, __fmul_rn(qy, qy));
         if (!(r2 <= a.z)) return false;
         if constexpr (MODE == GS_DISPLAY_SPLAT) {
-            const float e = PORTABLE_EXP ? exp_portable(-r2) : __expf(-r2);
+            const float e = PORTABLE_EXP ? exp_portable(-r2) : exp_sfu(-r2);
             *alpha = __fmul_rn(a.w, e);
         } else {
             *alpha = (r2 > outline2) ? 1.0f : a.w;
@@ -569,44 +577,78 @@ __device__ __forceinline__ bool fragment(const float4 a, const float4 b, float p
 __device__ __forceinline__ float blend8(float d, float om, float s_alpha) { return rintf(fmaf(d, om, s_alpha)); }
 
 struct RasterShared {
-    float4 a[kRasterThreads];    // cx, cy, r² limit, alpha
-    float4 b[kRasterThreads];    // q (or the point half sides)
-    float4 c[kRasterThreads];    // s255.rgb
-    float4 box[kRasterThreads];  // fragment box in pixel-centre coordinates
-    float2 inv[kRasterThreads];  // 1 / |Q·(7, 0)|², 1 / |Q·(0, 3)|² (the block edges in quad space)
+    float4 raw[kRasterThreads * 3];  // the next chunk's splats, thread t's own at 3t
+    float4 a[kRasterThreads];        // cx, cy, r² limit, alpha
+    float4 b[kRasterThreads];        // q (or the point half sides)
+    float4 c[kRasterThreads];        // s255.rgb
+    float4 box[kRasterThreads];      // fragment box in pixel-centre coordinates
+    float2 inv[kRasterThreads];      // 1 / |Q·(7, 0)|², 1 / |Q·(0, 3)|² (the block edges in quad space)
     uint8_t list[kRasterThreads / 32][kRasterThreads];
     uint32_t kmin;
 };
 
-// Stage list entries [rel0, rel0 + cnt) of the tile (cnt <= 256), one per thread.
-template <uint32_t MODE>
-__device__ __forceinline__ void stage_chunk(RasterShared &S, const gs_splat *__restrict__ sorted,
-                                            const uint2 *__restrict__ pairs, uint32_t first, uint32_t cnt,
-                                            float std2, uint32_t max_splats) {
-    const uint32_t tid = threadIdx.x;
-    if (tid < cnt) {
-        const uint32_t k = pairs[first + tid].y;
-        float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
-        if (k < max_splats) {  // ranks come from the tile sort; false only after a timeout
-            const float4 *src = reinterpret_cast<const float4 *>(sorted + k);
-            a = __ldg(src);
-            b = __ldg(src + 1);
-            c = __ldg(src + 2);
-        }
-        // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
-        const float lim =
-            (MODE == GS_DISPLAY_SPLAT) ? splat_r2_bound(c.w, splat_colour_reach(c.x, c.y, c.z), std2) : std2;
-        S.a[tid] = make_float4(a.x, a.y, lim, c.w);
-        S.b[tid] = b;
-        S.c[tid] = c;
-        S.box[tid] = make_float4(a.x - a.z, a.x + a.z, a.y - a.w, a.y + a.w);
-        if constexpr (MODE != GS_DISPLAY_POINT) {
-            const float e1x = b.x * kBlockSpanX, e1y = b.z * kBlockSpanX;
-            const float e2x = b.y * kBlockSpanY, e2y = b.w * kBlockSpanY;
-            S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
+// The tile's list entries, a chunk of 256 at a time, one entry per thread.  The splats of the
+// chunk after the staged one are in flight (cp.async into the thread's own part of `raw`) and the
+// pair of the chunk after that is in a register, so neither of the two dependent global loads of
+// an entry is waited for while the warps blend.
+struct ChunkSource {
+    const gs_splat *__restrict__ splats;
+    const uint2 *__restrict__ pairs;  // the tile's own list
+    uint32_t max_splats;
+    uint32_t value;  // pair value of the chunk after the one in flight
+
+    __device__ __forceinline__ uint32_t pair_value(uint32_t base, uint32_t cnt) const {
+        return threadIdx.x < cnt ? pairs[base + threadIdx.x].y : 0xFFFFFFFFu;
+    }
+
+    __device__ __forceinline__ void fetch(RasterShared &S, uint32_t k) const {
+        float4 *dst = S.raw + 3u * threadIdx.x;
+        if (k < max_splats) {  // pair values come from the tile sort; else no entry, or a timeout
+            const float4 *src = reinterpret_cast<const float4 *>(splats + k);
+            cp_async16(dst, src);
+            cp_async16(dst + 1, src + 1);
+            cp_async16(dst + 2, src + 2);
+        } else {
+            dst[0] = make_float4(0.0f, 0.0f, -1.0f, -1.0f);
+            dst[1] = dst[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-}
+
+    // Start a walk: [base, base + cnt) goes into flight, [next, next + next_cnt) is the chunk after.
+    __device__ __forceinline__ void begin(RasterShared &S, uint32_t base, uint32_t cnt, uint32_t next,
+                                          uint32_t next_cnt) {
+        fetch(S, pair_value(base, cnt));
+        value = pair_value(next, next_cnt);
+    }
+
+    // Stage the chunk in flight (cnt entries), then put the next one (if more) in flight and read the
+    // pairs [after, after + after_cnt).  The caller puts a barrier on either side.
+    template <uint32_t MODE>
+    __device__ __forceinline__ void stage(RasterShared &S, uint32_t cnt, float std2, bool more, uint32_t after,
+                                          uint32_t after_cnt) {
+        const uint32_t tid = threadIdx.x;
+        cp_async_wait_all();
+        if (tid < cnt) {
+            const float4 a = S.raw[3u * tid], b = S.raw[3u * tid + 1u], c = S.raw[3u * tid + 2u];
+            // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
+            const float lim =
+                (MODE == GS_DISPLAY_SPLAT) ? splat_r2_bound(c.w, splat_colour_reach(c.x, c.y, c.z), std2) : std2;
+            S.a[tid] = make_float4(a.x, a.y, lim, c.w);
+            S.b[tid] = b;
+            S.c[tid] = c;
+            S.box[tid] = make_float4(a.x - a.z, a.x + a.z, a.y - a.w, a.y + a.w);
+            if constexpr (MODE != GS_DISPLAY_POINT) {
+                const float e1x = b.x * kBlockSpanX, e1y = b.z * kBlockSpanX;
+                const float e2x = b.y * kBlockSpanY, e2y = b.w * kBlockSpanY;
+                S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
+            }
+        }
+        if (more) {
+            fetch(S, value);
+            value = pair_value(after, after_cnt);
+        }
+    }
+};
 
 // Whether the fragment ellipse {p : |Q·(p - c)|² <= lim} of a staged splat meets the rectangle
 // of pixel centres [bx0, bx0 + 7] x [by0, by0 + 3] of a warp's block.  With c outside the
@@ -668,16 +710,38 @@ __device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t cnt,
     return nl;
 }
 
+// A pixel of a warp's block whose transmittance stands for its quarter of the block.
+__device__ __forceinline__ float sample_x(uint32_t q) { return (q & 1u) ? 6.0f : 1.0f; }
+__device__ __forceinline__ float sample_y(uint32_t q) { return (q & 2u) ? 3.0f : 0.0f; }
+
+// Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats: three
+// quarters of it (768 by default: 668, 408 and 1962 us at 6M / 1080p, 1M / 1080p and 3M / 4K, against
+// 683, 412, 2084 at 1024 and 669, 425, 1937 at 512).  Ellipses end sooner, as outlines are opaque and
+// interiors keep their full alpha: a quarter (256: the frame of 700k at 1600x900 387 us, against 388
+// at 384, 414 at 768 and 392 at 128).
+template <uint32_t MODE>
+__device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
+    return MODE == GS_DISPLAY_ELLIPSE ? suffix_min / 4u : suffix_min - suffix_min / 4u;
+}
+
 // K4.  One CTA per 16x16 tile; each warp owns an 8x4 pixel block, each thread one pixel.
+// Points are opaque: each pixel takes the nearest point that covers it, found front to back.
 // Short tile lists are blended back to front in one pass.  Long ones use an exact early-out:
-//   A. walk the list front to back (nearest first) until the pixel's transmittance drops
-//      below `eps`, at list position k;
+//   A. walk the list front to back (nearest first) until the transmittance of four sample pixels
+//      of the warp's block drops below `eps`, at list position k.  The lanes take 8 splats x 4
+//      samples at a time: k only says where to start, so no pixel's own walk is needed;
 //   B. blend positions k.. back to front twice, from destination 0 and from 255.  The blend
 //      with 8-bit rounding is monotone in the destination, so the two results bound the
 //      result of every history before k; when they meet, that is the exact pixel.  A pixel
 //      whose bounds do not meet restarts B from k - (n - k) (k = 0 starts from the cleared
 //      value, which is exact).
 // Every pixel therefore ends bit-identical to the full back-to-front pass.
+//
+// Bound: instruction issue (no memory system near its limit), so time follows the warp iterations
+// of the list loops and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K:
+// 935, 514 and 2614 us with a walk A of every pixel over compacted lists and each chunk's loads
+// waited for; 668, 408 and 1937 us with the sampled walk, the loads a chunk ahead and the SFU exp
+// without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 59 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT>
 __device__ __forceinline__ void raster_tile(
     RasterShared &S, const gs_splat *__restrict__ sorted, const uint2 *__restrict__ pairs,
@@ -694,18 +758,51 @@ __device__ __forceinline__ void raster_tile(
         if (threadIdx.x == 0) atomicOr(&pctrl->status, kStatusBounds);
         range = make_uint2(0u, 0u);
     }
-    const uint32_t s0 = range.x, n = range.y - range.x;
+    const uint32_t n = range.y - range.x;
     const uint32_t wx0 = tx * GS_TILE + (warp & 1u) * 8u, wy0 = ty * GS_TILE + (warp >> 1) * 4u;
     const uint32_t px = wx0 + (lane & 7u), py = wy0 + (lane >> 3);
     const float pxc = (float)px + 0.5f, pyc = (float)py + 0.5f;
     const float bx0 = (float)wx0 + 0.5f, bx1 = (float)wx0 + 7.5f;
     const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 3.5f;
     float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f;
+    ChunkSource src{sorted, pairs + range.x, max_splats, 0u};
+    constexpr uint32_t C = kRasterThreads;
+    // the chunk before list position `end` (for walks from the end of the list)
+    auto below = [](uint32_t end) { return end > C ? end - C : 0u; };
 
-    if (n < suffix_min) {
-        for (uint32_t base = 0; base < n; base += kRasterThreads) {
-            const uint32_t cnt = min(kRasterThreads, n - base);
-            stage_chunk<MODE>(S, sorted, pairs, s0 + base, cnt, std2, max_splats);
+    if constexpr (MODE == GS_DISPLAY_POINT) {
+        // alpha is 1: blending a fragment replaces the pixel, whatever lies behind it
+        bool found = px >= W || py >= H;
+        uint32_t base = below(n), cnt = n - base;
+        src.begin(S, base, cnt, below(base), base - below(base));
+        for (uint32_t end = n; end > 0;) {
+            src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+            __syncthreads();
+            if (__any_sync(0xFFFFFFFFu, !found)) {
+                const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
+                for (int i = (int)nl - 1; i >= 0; --i) {
+                    if (__all_sync(0xFFFFFFFFu, found)) break;
+                    const uint32_t j = S.list[warp][i];
+                    float al;
+                    if (!found && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) {
+                        const float4 c = S.c[j];
+                        d0 = blend8(0.0f, 0.0f, c.x);
+                        d1 = blend8(0.0f, 0.0f, c.y);
+                        d2 = blend8(0.0f, 0.0f, c.z);
+                        found = true;
+                    }
+                }
+            }
+            if (__syncthreads_and(found)) break;
+            end = base;
+            base = below(end);
+            cnt = end - base;
+        }
+    } else if (n < early_out_min<MODE>(suffix_min)) {
+        if (n > 0) src.begin(S, 0, min(C, n), C, n > C ? min(C, n - C) : 0u);
+        for (uint32_t base = 0; base < n; base += C) {
+            const uint32_t cnt = min(C, n - base), after = base + 2u * C;
+            src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
             __syncthreads();
             const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
             for (uint32_t i = 0; i < nl; ++i) {
@@ -723,41 +820,44 @@ __device__ __forceinline__ void raster_tile(
             __syncthreads();
         }
     } else {
-        // ---- A: front-to-back transmittance to find the start position k ----
-        float T = 1.0f;
+        // ---- A: front-to-back transmittance of the samples to find the start position k ----
         uint32_t k = 0;
-        bool found = false;
-        for (uint32_t end = n; end > 0;) {
-            const uint32_t base = end > kRasterThreads ? end - kRasterThreads : 0u;
-            const uint32_t cnt = end - base;
-            stage_chunk<MODE>(S, sorted, pairs, s0 + base, cnt, std2, max_splats);
-            __syncthreads();
-            if (__any_sync(0xFFFFFFFFu, !found)) {
-                const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
-                for (int i = (int)nl - 1; i >= 0; --i) {
-                    if (__all_sync(0xFFFFFFFFu, found)) break;
-                    const uint32_t j = S.list[warp][i];
-                    float al;
-                    if (COUNT && !found) ++n_eval;
-                    if (!found && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) {
-                        if (COUNT) ++n_alpha, ++n_trans;
-                        T = __fmul_rn(T, __fsub_rn(1.0f, al));
-                        if (T < eps) {
-                            found = true;
-                            k = base + j;
+        {
+            const float sxc = bx0 + sample_x(lane & 3u), syc = by0 + sample_y(lane & 3u);
+            float T = 1.0f;  // this lane's share of its sample's transmittance
+            bool found = false;
+            uint32_t base = below(n), cnt = n - base;
+            src.begin(S, base, cnt, below(base), base - below(base));
+            for (uint32_t end = n; end > 0;) {
+                src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+                __syncthreads();
+                for (int top = (int)cnt; top > 0 && !found; top -= 32) {
+#pragma unroll
+                    for (int it = 0; it < 4; ++it) {
+                        const int j = top - 1 - it * 8 - (int)(lane >> 2);
+                        float al;
+                        if (COUNT && j >= 0) ++n_eval;
+                        if (j >= 0 && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], sxc, syc, outline2, &al)) {
+                            if (COUNT) ++n_alpha, ++n_trans;
+                            T = __fmul_rn(T, __fsub_rn(1.0f, al));
                         }
                     }
+                    float t = T;  // the product over the sample's eight lanes
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
+                    if (__all_sync(0xFFFFFFFFu, t < eps)) {
+                        found = true;
+                        k = base + (uint32_t)max(top - 32, 0);
+                    }
                 }
+                if (__syncthreads_and(found)) break;
+                end = base;
+                base = below(end);
+                cnt = end - base;
             }
-            if (__syncthreads_and(found)) break;
-            end = base;
         }
-        if (!found) k = 0;
-        // The bounds argument holds from any start position, so a warp starts all its pixels at
-        // the smallest k among them: lanes share issue slots, the earlier start costs the warp
-        // nothing, and it makes the bounds more likely to meet on the first pass.
-        k = __reduce_min_sync(0xFFFFFFFFu, k);
-        // ---- B: bounded back-to-front passes from k ----
+        // ---- B: bounded back-to-front passes from k (the same for all pixels of a warp) ----
         bool active = true;
         float h0 = 0.0f, h1 = 0.0f, h2 = 0.0f;
         for (;;) {
@@ -773,13 +873,15 @@ __device__ __forceinline__ void raster_tile(
                 d0 = d1 = d2 = 0.0f;
                 h0 = h1 = h2 = top;
             }
-            for (uint32_t base = kmin / kRasterThreads * kRasterThreads; base < n; base += kRasterThreads) {
-                const uint32_t cnt = min(kRasterThreads, n - base);
+            const uint32_t start = kmin / C * C;
+            src.begin(S, start, min(C, n - start), start + C, start + C < n ? min(C, n - start - C) : 0u);
+            for (uint32_t base = start; base < n; base += C) {
+                const uint32_t cnt = min(C, n - base), after = base + 2u * C;
                 __syncthreads();
-                stage_chunk<MODE>(S, sorted, pairs, s0 + base, cnt, std2, max_splats);
+                src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
                 __syncthreads();
                 // k is uniform across the warp: a warp whose suffix starts past this chunk skips it
-                const bool inside = active && k < base + kRasterThreads;  // chunk holds suffix entries
+                const bool inside = active && k < base + C;  // chunk holds suffix entries
                 if (__any_sync(0xFFFFFFFFu, inside)) {
                     const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
                     // Bounds that have met stay equal (same inputs, same operations), so once
