@@ -1321,7 +1321,7 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
                     else
                         err = launch_raster(&seg, 1, raster_mode(uh[i]), views[i].target, views[i].width, views[i].height,
                                             views[i].pitch, v.max_pairs, v.raster_scratch.ptr, mv->frame.exact_exp, vs,
-                                            &b->tuning);
+                                            &b->tuning, tile_base[n]);
                 }
             }
         }

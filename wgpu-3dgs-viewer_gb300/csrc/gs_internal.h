@@ -163,10 +163,11 @@ struct RasterSegment {
 };
 size_t raster_scratch_bytes(uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 // exact_exp: 1 = the portable exp (bit-identical with the CPU oracle), 0 = the SFU exp.
+// tiles_at_once: tiles of all views that are rendered side by side with this one (0: it is alone).
 cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const RasterMode &u,
                           uint8_t *target, uint32_t width, uint32_t height, uint32_t pitch,
                           uint32_t max_pairs, void *scratch, int exact_exp, cudaStream_t st,
-                          const Tuning *tuning = nullptr);
+                          const Tuning *tuning = nullptr, uint32_t tiles_at_once = 0);
 // Scratch control block of a raster call (status, pair counts).
 const Ctrl *raster_ctrl(const void *scratch);
 

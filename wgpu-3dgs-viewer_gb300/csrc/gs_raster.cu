@@ -53,6 +53,17 @@ constexpr uint32_t kEmitBlocks = 152 * 8;
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = 256 * kScanItems;
 
+// CTAs of a kernel that the current device holds at once (0 when it cannot be told).
+template <class K>
+static uint32_t resident_ctas(K kernel, uint32_t threads, size_t smem) {
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)threads, smem) != cudaSuccess)
+        return 0;
+    return (uint32_t)sms * (uint32_t)per_sm;
+}
+
 static uint32_t bits_for(uint32_t v) {
     uint32_t b = 1;
     while (b < 32 && (v >> b) != 0) ++b;
@@ -548,27 +559,35 @@ __device__ __forceinline__ float exp_sfu(float x) {
     return e;
 }
 
-// One fragment of a staged splat at the pixel centre (pxc, pyc) (render.wesl:143-181):
-// false when discarded or when it cannot change the pixel, else its alpha.
+// Squared quad offset of the pixel centre (pxc, pyc) from a staged splat, and the alpha there
+// (render.wesl:143-181).
+__device__ __forceinline__ float fragment_r2(const float4 a, const float4 b, float pxc, float pyc) {
+    const float dx = __fsub_rn(pxc, a.x), dy = __fsub_rn(pyc, a.y);
+    const float qx = fmaf(b.x, dx, __fmul_rn(b.y, dy));
+    const float qy = fmaf(b.z, dx, __fmul_rn(b.w, dy));
+    return fmaf(qx, qx, __fmul_rn(qy, qy));
+}
+
+template <uint32_t MODE, bool PORTABLE_EXP>
+__device__ __forceinline__ float fragment_alpha(const float4 a, float r2, float outline2) {
+    if constexpr (MODE == GS_DISPLAY_SPLAT) return __fmul_rn(a.w, PORTABLE_EXP ? exp_portable(-r2) : exp_sfu(-r2));
+    return (r2 > outline2) ? 1.0f : a.w;
+}
+
+// One fragment of a staged splat at the pixel centre: false when discarded or when it cannot change
+// the pixel, else its alpha.
 template <uint32_t MODE, bool PORTABLE_EXP>
 __device__ __forceinline__ bool fragment(const float4 a, const float4 b, float pxc, float pyc, float outline2,
                                          float *alpha) {
-    const float dx = __fsub_rn(pxc, a.x), dy = __fsub_rn(pyc, a.y);
     if constexpr (MODE == GS_DISPLAY_POINT) {
+        const float dx = __fsub_rn(pxc, a.x), dy = __fsub_rn(pyc, a.y);
         if (!(dx >= -b.x && dx < b.x && dy >= -b.y && dy < b.y)) return false;
         *alpha = 1.0f;
         return true;
     } else {
-        const float qx = fmaf(b.x, dx, __fmul_rn(b.y, dy));
-        const float qy = fmaf(b.z, dx, __fmul_rn(b.w, dy));
-        const float r2 = fmaf(qx, qx, __fmul_rn(qy, qy));
+        const float r2 = fragment_r2(a, b, pxc, pyc);
         if (!(r2 <= a.z)) return false;
-        if constexpr (MODE == GS_DISPLAY_SPLAT) {
-            const float e = PORTABLE_EXP ? exp_portable(-r2) : exp_sfu(-r2);
-            *alpha = __fmul_rn(a.w, e);
-        } else {
-            *alpha = (r2 > outline2) ? 1.0f : a.w;
-        }
+        *alpha = fragment_alpha<MODE, PORTABLE_EXP>(a, r2, outline2);
         return true;
     }
 }
@@ -621,32 +640,52 @@ struct ChunkSource {
         value = pair_value(next, next_cnt);
     }
 
+    // A splat into the thread's staged entry.
+    template <uint32_t MODE>
+    static __device__ __forceinline__ void put(RasterShared &S, const float4 a, const float4 b, const float4 c,
+                                               float std2) {
+        const uint32_t tid = threadIdx.x;
+        // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
+        const float lim =
+            (MODE == GS_DISPLAY_SPLAT) ? splat_r2_bound(c.w, splat_colour_reach(c.x, c.y, c.z), std2) : std2;
+        S.a[tid] = make_float4(a.x, a.y, lim, c.w);
+        S.b[tid] = b;
+        S.c[tid] = c;
+        S.box[tid] = make_float4(a.x - a.z, a.x + a.z, a.y - a.w, a.y + a.w);
+        if constexpr (MODE != GS_DISPLAY_POINT) {
+            const float e1x = b.x * kBlockSpanX, e1y = b.z * kBlockSpanX;
+            const float e2x = b.y * kBlockSpanY, e2y = b.w * kBlockSpanY;
+            S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
+        }
+    }
+
     // Stage the chunk in flight (cnt entries), then put the next one (if more) in flight and read the
     // pairs [after, after + after_cnt).  The caller puts a barrier on either side.
     template <uint32_t MODE>
     __device__ __forceinline__ void stage(RasterShared &S, uint32_t cnt, float std2, bool more, uint32_t after,
                                           uint32_t after_cnt) {
-        const uint32_t tid = threadIdx.x;
+        const float4 *raw = S.raw + 3u * threadIdx.x;
         cp_async_wait_all();
-        if (tid < cnt) {
-            const float4 a = S.raw[3u * tid], b = S.raw[3u * tid + 1u], c = S.raw[3u * tid + 2u];
-            // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
-            const float lim =
-                (MODE == GS_DISPLAY_SPLAT) ? splat_r2_bound(c.w, splat_colour_reach(c.x, c.y, c.z), std2) : std2;
-            S.a[tid] = make_float4(a.x, a.y, lim, c.w);
-            S.b[tid] = b;
-            S.c[tid] = c;
-            S.box[tid] = make_float4(a.x - a.z, a.x + a.z, a.y - a.w, a.y + a.w);
-            if constexpr (MODE != GS_DISPLAY_POINT) {
-                const float e1x = b.x * kBlockSpanX, e1y = b.z * kBlockSpanX;
-                const float e2x = b.y * kBlockSpanY, e2y = b.w * kBlockSpanY;
-                S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
-            }
-        }
+        if (threadIdx.x < cnt) put<MODE>(S, raw[0], raw[1], raw[2], std2);
         if (more) {
             fetch(S, value);
             value = pair_value(after, after_cnt);
         }
+    }
+
+    // Stage a list that is one chunk, straight from memory.
+    template <uint32_t MODE>
+    __device__ __forceinline__ void stage_only(RasterShared &S, uint32_t n, float std2) const {
+        if (threadIdx.x >= n) return;
+        const uint32_t k = pairs[threadIdx.x].y;
+        float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
+        if (k < max_splats) {
+            const float4 *s = reinterpret_cast<const float4 *>(splats + k);
+            a = __ldg(s);
+            b = __ldg(s + 1);
+            c = __ldg(s + 2);
+        }
+        put<MODE>(S, a, b, c, std2);
     }
 };
 
@@ -686,18 +725,18 @@ __device__ __forceinline__ bool ellipse_meets_block(const float4 a, const float4
     return m;
 }
 
-// The calling warp's list of staged entries whose fragments can reach its pixel block, in draw
-// order: the fragment box, then (splat and ellipse modes) the ellipse itself must meet the block.
+// The calling warp's list of staged entries from jmin on whose fragments can reach its pixel block, in
+// draw order: the fragment box, then (splat and ellipse modes) the ellipse itself must meet the block.
 template <uint32_t MODE>
-__device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t cnt, float bx0, float bx1, float by0,
-                                                  float by1) {
+__device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t jmin, uint32_t cnt, float bx0, float bx1,
+                                                  float by0, float by1) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
     uint32_t nl = 0;
-    for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
+    for (uint32_t j0 = jmin & ~31u; j0 < cnt; j0 += 32) {
         const uint32_t j = j0 + lane;
         bool hit = false;
-        if (j < cnt) {
+        if (j >= jmin && j < cnt) {
             const float4 box = S.box[j];
             hit = !(box.y < bx0 || box.x > bx1 || box.w < by0 || box.z > by1);
             if (MODE != GS_DISPLAY_POINT && hit) hit = ellipse_meets_block(S.a[j], S.b[j], S.inv[j], bx0, bx1, by0, by1);
@@ -714,11 +753,60 @@ __device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t cnt,
 __device__ __forceinline__ float sample_x(uint32_t q) { return (q & 1u) ? 6.0f : 1.0f; }
 __device__ __forceinline__ float sample_y(uint32_t q) { return (q & 2u) ? 3.0f : 0.0f; }
 
+// Blends the warp's list entries [0, nl) onto the pixel (d), and with BOTH onto the upper bound (h)
+// as well, for lanes with `on`.  UNROLL 1: one entry after another, skipping what the fragment test
+// skips; the fewest instructions.  UNROLL 4: four entries are evaluated side by side and a missed one
+// blends with alpha 0, which leaves the pixel as it is; more instructions, but the warp waits for one
+// chain of loads, exp and test where it waited for four.
+template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, bool BOTH, uint32_t UNROLL>
+__device__ __forceinline__ void blend_list(const RasterShared &S, uint32_t nl, bool on, float pxc, float pyc,
+                                           float outline2, float d[3], float h[3], uint32_t &n_eval, uint32_t &n_alpha,
+                                           uint32_t &n_blend) {
+    const uint32_t warp = threadIdx.x >> 5;
+    auto blend = [&](const float4 c, float al) {
+        const float om = __fsub_rn(1.0f, al);
+        const float s[3] = {__fmul_rn(c.x, al), __fmul_rn(c.y, al), __fmul_rn(c.z, al)};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            d[q] = blend8(d[q], om, s[q]);
+            if (BOTH) h[q] = blend8(h[q], om, s[q]);
+        }
+    };
+    if constexpr (UNROLL == 1) {
+        for (uint32_t i = 0; i < nl; ++i) {
+            const uint32_t j = S.list[warp][i];
+            float al;
+            if (!on) continue;
+            if (COUNT) ++n_eval;
+            if (!fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) continue;
+            if (COUNT) ++n_alpha, n_blend += BOTH ? 2 : 1;
+            blend(S.c[j], al);
+        }
+    } else {
+        for (uint32_t i = 0; i < nl; i += UNROLL) {
+            float al[UNROLL];
+            float4 c[UNROLL];
+#pragma unroll
+            for (uint32_t u = 0; u < UNROLL; ++u) {
+                const uint32_t j = S.list[warp][min(i + u, nl - 1u)];
+                const float4 a = S.a[j], b = S.b[j];
+                const float r2 = fragment_r2(a, b, pxc, pyc);
+                const float v = fragment_alpha<MODE, PORTABLE_EXP>(a, r2, outline2);
+                al[u] = (r2 <= a.z && on && i + u < nl) ? v : 0.0f;
+                c[u] = S.c[j];
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < UNROLL; ++u) blend(c[u], al[u]);
+        }
+    }
+}
+
 // Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats: three
 // quarters of it (768 by default: 668, 408 and 1962 us at 6M / 1080p, 1M / 1080p and 3M / 4K, against
 // 683, 412, 2084 at 1024 and 669, 425, 1937 at 512).  Ellipses end sooner, as outlines are opaque and
 // interiors keep their full alpha: a quarter (256: the frame of 700k at 1600x900 387 us, against 388
 // at 384, 414 at 768 and 392 at 128).
+constexpr float kWalkCourse = 0.9f;
 template <uint32_t MODE>
 __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
     return MODE == GS_DISPLAY_ELLIPSE ? suffix_min / 4u : suffix_min - suffix_min / 4u;
@@ -740,9 +828,9 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // Bound: instruction issue (no memory system near its limit), so time follows the warp iterations
 // of the list loops and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K:
 // 935, 514 and 2614 us with a walk A of every pixel over compacted lists and each chunk's loads
-// waited for; 668, 408 and 1937 us with the sampled walk, the loads a chunk ahead and the SFU exp
-// without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 59 us.
-template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT>
+// waited for; 635, 396 and 1882 us with the sampled walk, the loads a chunk ahead and the SFU exp
+// without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
+template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL>
 __device__ __forceinline__ void raster_tile(
     RasterShared &S, const gs_splat *__restrict__ sorted, const uint2 *__restrict__ pairs,
     const uint2 *__restrict__ ranges, uint8_t *__restrict__ target, uint32_t W, uint32_t H, uint32_t pitch,
@@ -764,7 +852,7 @@ __device__ __forceinline__ void raster_tile(
     const float pxc = (float)px + 0.5f, pyc = (float)py + 0.5f;
     const float bx0 = (float)wx0 + 0.5f, bx1 = (float)wx0 + 7.5f;
     const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 3.5f;
-    float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f;
+    float d[3] = {0.0f, 0.0f, 0.0f};
     ChunkSource src{sorted, pairs + range.x, max_splats, 0u};
     constexpr uint32_t C = kRasterThreads;
     // the chunk before list position `end` (for walks from the end of the list)
@@ -774,21 +862,24 @@ __device__ __forceinline__ void raster_tile(
         // alpha is 1: blending a fragment replaces the pixel, whatever lies behind it
         bool found = px >= W || py >= H;
         uint32_t base = below(n), cnt = n - base;
-        src.begin(S, base, cnt, below(base), base - below(base));
+        if (n > C) src.begin(S, base, cnt, below(base), base - below(base));
         for (uint32_t end = n; end > 0;) {
-            src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+            if (n > C)
+                src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+            else
+                src.stage_only<MODE>(S, n, std2);
             __syncthreads();
             if (__any_sync(0xFFFFFFFFu, !found)) {
-                const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
+                const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
                 for (int i = (int)nl - 1; i >= 0; --i) {
                     if (__all_sync(0xFFFFFFFFu, found)) break;
                     const uint32_t j = S.list[warp][i];
                     float al;
                     if (!found && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) {
                         const float4 c = S.c[j];
-                        d0 = blend8(0.0f, 0.0f, c.x);
-                        d1 = blend8(0.0f, 0.0f, c.y);
-                        d2 = blend8(0.0f, 0.0f, c.z);
+                        d[0] = blend8(0.0f, 0.0f, c.x);
+                        d[1] = blend8(0.0f, 0.0f, c.y);
+                        d[2] = blend8(0.0f, 0.0f, c.z);
                         found = true;
                     }
                 }
@@ -798,25 +889,23 @@ __device__ __forceinline__ void raster_tile(
             base = below(end);
             cnt = end - base;
         }
+    } else if (n <= C && n < early_out_min<MODE>(suffix_min)) {
+        if (n > 0) {
+            src.stage_only<MODE>(S, n, std2);
+            __syncthreads();
+            const uint32_t nl = compact_chunk<MODE>(S, 0, n, bx0, bx1, by0, by1);
+            blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, true, pxc, pyc, outline2, d, d, n_eval, n_alpha,
+                                                                 n_blend);
+        }
     } else if (n < early_out_min<MODE>(suffix_min)) {
-        if (n > 0) src.begin(S, 0, min(C, n), C, n > C ? min(C, n - C) : 0u);
+        src.begin(S, 0, C, C, min(C, n - C));
         for (uint32_t base = 0; base < n; base += C) {
             const uint32_t cnt = min(C, n - base), after = base + 2u * C;
             src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
             __syncthreads();
-            const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
-            for (uint32_t i = 0; i < nl; ++i) {
-                const uint32_t j = S.list[warp][i];
-                float al;
-                if (COUNT) ++n_eval;
-                if (!fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) continue;
-                if (COUNT) ++n_alpha, ++n_blend;
-                const float4 c = S.c[j];
-                const float om = __fsub_rn(1.0f, al);
-                d0 = blend8(d0, om, __fmul_rn(c.x, al));
-                d1 = blend8(d1, om, __fmul_rn(c.y, al));
-                d2 = blend8(d2, om, __fmul_rn(c.z, al));
-            }
+            const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
+            blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, true, pxc, pyc, outline2, d, d, n_eval, n_alpha,
+                                                                 n_blend);
             __syncthreads();
         }
     } else {
@@ -839,6 +928,9 @@ __device__ __forceinline__ void raster_tile(
                         if (COUNT && j >= 0) ++n_eval;
                         if (j >= 0 && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], sxc, syc, outline2, &al)) {
                             if (COUNT) ++n_alpha, ++n_trans;
+                            // an ellipse's outline is opaque where the sample lies, not where the
+                            // block's other pixels do
+                            if (MODE == GS_DISPLAY_ELLIPSE) al = S.a[j].w;
                             T = __fmul_rn(T, __fsub_rn(1.0f, al));
                         }
                     }
@@ -851,6 +943,18 @@ __device__ __forceinline__ void raster_tile(
                         k = base + (uint32_t)max(top - 32, 0);
                     }
                 }
+                // A walk that will end in the far part of the list saves nothing: B costs more per
+                // entry than one blend of the whole list.  T falls about evenly per entry, so from a
+                // quarter of the list on it must be on course for eps (to the power kWalkCourse of
+                // the share walked).
+                if (!found && 4u * (n - base) >= n) {
+                    float t = T;
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
+                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
+                    const float course = __powf(eps, kWalkCourse * (float)(n - base) / (float)n);
+                    found = __any_sync(0xFFFFFFFFu, !(t < course));  // k = 0
+                }
                 if (__syncthreads_and(found)) break;
                 end = base;
                 base = below(end);
@@ -859,7 +963,8 @@ __device__ __forceinline__ void raster_tile(
         }
         // ---- B: bounded back-to-front passes from k (the same for all pixels of a warp) ----
         bool active = true;
-        float h0 = 0.0f, h1 = 0.0f, h2 = 0.0f;
+        float h[3] = {0.0f, 0.0f, 0.0f};
+        auto met = [&]() { return d[0] == h[0] && d[1] == h[1] && d[2] == h[2]; };
         for (;;) {
             if (tid == 0) S.kmin = 0xFFFFFFFFu;
             __syncthreads();
@@ -869,9 +974,8 @@ __device__ __forceinline__ void raster_tile(
             const uint32_t kmin = S.kmin;
             if (kmin == 0xFFFFFFFFu) break;
             if (active) {
-                const float top = (k == 0) ? 0.0f : 255.0f;
-                d0 = d1 = d2 = 0.0f;
-                h0 = h1 = h2 = top;
+                d[0] = d[1] = d[2] = 0.0f;
+                h[0] = h[1] = h[2] = (k == 0) ? 0.0f : 255.0f;
             }
             const uint32_t start = kmin / C * C;
             src.begin(S, start, min(C, n - start), start + C, start + C < n ? min(C, n - start - C) : 0u);
@@ -880,56 +984,27 @@ __device__ __forceinline__ void raster_tile(
                 __syncthreads();
                 src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
                 __syncthreads();
-                // k is uniform across the warp: a warp whose suffix starts past this chunk skips it
-                const bool inside = active && k < base + C;  // chunk holds suffix entries
-                if (__any_sync(0xFFFFFFFFu, inside)) {
-                    const uint32_t nl = compact_chunk<MODE>(S, cnt, bx0, bx1, by0, by1);
+                // wmin is the warp's k: a warp whose suffix starts past this chunk skips it
+                if (wmin < base + C) {
+                    const uint32_t nl = compact_chunk<MODE>(S, wmin > base ? wmin - base : 0u, cnt, bx0, bx1, by0, by1);
                     // Bounds that have met stay equal (same inputs, same operations), so once
                     // every started lane of the warp has met, one chain per channel suffices.
-                    const bool met = d0 == h0 && d1 == h1 && d2 == h2;
-                    if (__all_sync(0xFFFFFFFFu, !inside || (met && base >= k))) {
-                        for (uint32_t i = 0; i < nl; ++i) {
-                            const uint32_t j = S.list[warp][i];
-                            float al;
-                            if (!inside) continue;
-                            if (COUNT) ++n_eval;
-                            if (!fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) continue;
-                            if (COUNT) ++n_alpha, ++n_blend;
-                            const float4 c = S.c[j];
-                            const float om = __fsub_rn(1.0f, al);
-                            d0 = blend8(d0, om, __fmul_rn(c.x, al));
-                            d1 = blend8(d1, om, __fmul_rn(c.y, al));
-                            d2 = blend8(d2, om, __fmul_rn(c.z, al));
-                        }
-                        if (inside) {
-                            h0 = d0;
-                            h1 = d1;
-                            h2 = d2;
+                    if (__all_sync(0xFFFFFFFFu, !active || met())) {
+                        blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, active, pxc, pyc, outline2, d, h,
+                                                                             n_eval, n_alpha, n_blend);
+                        if (active) {
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) h[q] = d[q];
                         }
                     } else {
-                        for (uint32_t i = 0; i < nl; ++i) {
-                            const uint32_t j = S.list[warp][i];
-                            float al;
-                            if (!active || base + j < k) continue;
-                            if (COUNT) ++n_eval;
-                            if (!fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) continue;
-                            if (COUNT) ++n_alpha, n_blend += 2;
-                            const float4 c = S.c[j];
-                            const float om = __fsub_rn(1.0f, al);
-                            const float s0a = __fmul_rn(c.x, al), s1a = __fmul_rn(c.y, al), s2a = __fmul_rn(c.z, al);
-                            d0 = blend8(d0, om, s0a);
-                            d1 = blend8(d1, om, s1a);
-                            d2 = blend8(d2, om, s2a);
-                            h0 = blend8(h0, om, s0a);
-                            h1 = blend8(h1, om, s1a);
-                            h2 = blend8(h2, om, s2a);
-                        }
+                        blend_list<MODE, PORTABLE_EXP, COUNT, true, UNROLL>(S, nl, active, pxc, pyc, outline2, d, h,
+                                                                            n_eval, n_alpha, n_blend);
                     }
                 }
             }
             __syncthreads();
             if (active) {
-                if (d0 == h0 && d1 == h1 && d2 == h2) {
+                if (met()) {
                     active = false;
                 } else {
                     const uint32_t suffix = n - k;
@@ -939,7 +1014,7 @@ __device__ __forceinline__ void raster_tile(
         }
     }
     if (px < W && py < H) {
-        const uint32_t rgba = (uint32_t)d0 | ((uint32_t)d1 << 8) | ((uint32_t)d2 << 16) | 0xFF000000u;
+        const uint32_t rgba = (uint32_t)d[0] | ((uint32_t)d[1] << 8) | ((uint32_t)d[2] << 16) | 0xFF000000u;
         *reinterpret_cast<uint32_t *>(target + (size_t)py * pitch + (size_t)px * 4u) = rgba;
     }
     if constexpr (COUNT) {
@@ -953,14 +1028,17 @@ __device__ __forceinline__ void raster_tile(
 }
 
 
-template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT>
-__global__ void __launch_bounds__(kRasterThreads, 6) raster_kernel(const RasterJob J, float std2, float outline2,
+// FEW: a grid of few tiles (at most kFewTiles), whose time is that of its longest lists, not of the
+// instructions of all: blend_list four entries at a time, in up to 64 registers a thread (4 CTAs an SM;
+// 3 and 5 CTAs take 48 and 55 us for 100k at 640x360, and 4 CTAs 49 us, against 70 us without FEW).
+template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, bool FEW>
+__global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(const RasterJob J, float std2, float outline2,
                                                                 uint32_t suffix_min, float eps,
                                                                 unsigned long long *counters) {
     __shared__ RasterShared S;
-    raster_tile<MODE, PORTABLE_EXP, COUNT>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch, J.tiles_x,
-                                           std2, outline2, J.max_splats, suffix_min, eps, counters, J.ctrl,
-                                           J.order ? J.order[blockIdx.x] : blockIdx.x);
+    raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch,
+                                                          J.tiles_x, std2, outline2, J.max_splats, suffix_min, eps,
+                                                          counters, J.ctrl, J.order ? J.order[blockIdx.x] : blockIdx.x);
 }
 
 // One grid over the tiles of several views (a batch): CTA b rasterises tile b - tile_base[v] of
@@ -979,7 +1057,7 @@ __global__ void __launch_bounds__(kRasterThreads, 6) raster_views_kernel(const R
     }
     const RasterJob &J = jobs[lo];
     const uint32_t b = blockIdx.x - tile_base[lo];
-    raster_tile<MODE, PORTABLE_EXP, false>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch, J.tiles_x,
+    raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch, J.tiles_x,
                                            std2, outline2, J.max_splats, suffix_min, eps, nullptr, J.ctrl,
                                            J.order ? J.order[b] : b);
 }
@@ -996,20 +1074,33 @@ cudaError_t raster_counters(unsigned long long out[4], bool reset) {
     return e;
 }
 
+template <uint32_t MODE, bool EXACT, bool COUNT, bool FEW>
+static void launch_raster_tiles(const RasterJob &J, float std2, float outline2, cudaStream_t st, const Tuning &t,
+                                unsigned long long *counts) {
+    raster_kernel<MODE, EXACT, COUNT, FEW><<<J.ntiles, kRasterThreads, 0, st>>>(J, std2, outline2, t.suffix_min, t.eps,
+                                                                                counts);
+}
+
+// Grids of up to four resident waves of the FEW kernel take it: 1456 tiles (1.4M splats at 892x401)
+// 588 -> 544 us a frame, 1881 tiles 271 -> 245 us, 130 tiles with long lists 2453 -> 1997 us; beyond,
+// the instructions count: 4836 tiles 169 -> 174 us, 3645 tiles of points 350 -> 356 us.  Views of a
+// batch overlap, so the tiles of all of them count.
+constexpr uint32_t kFewTiles = 152 * 4 * 4;
+
 template <uint32_t MODE>
-static void launch_raster_mode(const RasterJob &J, uint32_t ntiles, float std2, float outline2, int exact,
+static void launch_raster_mode(const RasterJob &J, uint32_t tiles_at_once, float std2, float outline2, int exact,
                                cudaStream_t st, const Tuning &t) {
-    if (exact) {
-        raster_kernel<MODE, true, false><<<ntiles, kRasterThreads, 0, st>>>(J, std2, outline2, t.suffix_min, t.eps,
-                                                                            nullptr);
-    } else if (MODE == GS_DISPLAY_SPLAT && prof_counting()) {
+    const bool few = tiles_at_once <= kFewTiles;
+    if (MODE == GS_DISPLAY_SPLAT && !exact && prof_counting()) {
         unsigned long long *counts = nullptr;
         cudaGetSymbolAddress((void **)&counts, g_raster_counts);
-        raster_kernel<GS_DISPLAY_SPLAT, false, true><<<ntiles, kRasterThreads, 0, st>>>(J, std2, outline2,
-                                                                                       t.suffix_min, t.eps, counts);
+        launch_raster_tiles<GS_DISPLAY_SPLAT, false, true, false>(J, std2, outline2, st, t, counts);
+    } else if (exact) {
+        few ? launch_raster_tiles<MODE, true, false, true>(J, std2, outline2, st, t, nullptr)
+            : launch_raster_tiles<MODE, true, false, false>(J, std2, outline2, st, t, nullptr);
     } else {
-        raster_kernel<MODE, false, false><<<ntiles, kRasterThreads, 0, st>>>(J, std2, outline2, t.suffix_min, t.eps,
-                                                                             nullptr);
+        few ? launch_raster_tiles<MODE, false, false, true>(J, std2, outline2, st, t, nullptr)
+            : launch_raster_tiles<MODE, false, false, false>(J, std2, outline2, st, t, nullptr);
     }
 }
 
@@ -1100,19 +1191,9 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
     // wave (at most kEmitBlocks, the per-CTA count area) keeps a second, late wave from
     // doubling the kernel's span.
     const size_t emit_smem = L.counts ? (size_t)L.ntiles * 4u : 4u * 256u * 4u;
-    uint32_t emit_wave = kEmitBlocks;
-    {
-        int dev = 0, sms = 0, per_sm = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-            (L.counts ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bin_emit_kernel<true>, kBinThreads, emit_smem)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bin_emit_kernel<false>, kBinThreads,
-                                                                       emit_smem)) == cudaSuccess &&
-            sms > 0 && per_sm > 0) {
-            const uint32_t wave = (uint32_t)sms * (uint32_t)per_sm;
-            if (wave < emit_wave) emit_wave = wave;
-        }
-    }
+    uint32_t emit_wave = L.counts ? resident_ctas(bin_emit_kernel<true>, kBinThreads, emit_smem)
+                                  : resident_ctas(bin_emit_kernel<false>, kBinThreads, emit_smem);
+    if (emit_wave == 0 || emit_wave > kEmitBlocks) emit_wave = kEmitBlocks;
     uint32_t rank_offset = 0;
     bool cleared = false;
     prof_mark(kProfBin, true, st);
@@ -1229,12 +1310,13 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
 
 cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint8_t *target,
                           uint32_t W, uint32_t H, uint32_t pitch, uint32_t max_pairs, void *scratch, int exact_exp,
-                          cudaStream_t st, const Tuning *tuning) {
+                          cudaStream_t st, const Tuning *tuning, uint32_t tiles_at_once) {
     const Tuning tn = tuning ? *tuning : default_tuning();
     cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
     if (e != cudaSuccess) return e;
     const RasterJob J = raster_job(segs, nseg, target, W, H, pitch, max_pairs, scratch);
     if (J.ntiles == 0) return cudaSuccess;
+    const uint32_t at_once = tiles_at_once > J.ntiles ? tiles_at_once : J.ntiles;
     const float std2 = u.std_dev * u.std_dev;
     const float o = u.std_dev - 0.1f;
     const float outline2 = o * o;
@@ -1242,13 +1324,13 @@ cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const Raster
     count_launches(1);
     switch (u.display_mode) {
         case GS_DISPLAY_SPLAT:
-            launch_raster_mode<GS_DISPLAY_SPLAT>(J, J.ntiles, std2, outline2, exact_exp, st, tn);
+            launch_raster_mode<GS_DISPLAY_SPLAT>(J, at_once, std2, outline2, exact_exp, st, tn);
             break;
         case GS_DISPLAY_ELLIPSE:
-            launch_raster_mode<GS_DISPLAY_ELLIPSE>(J, J.ntiles, std2, outline2, exact_exp, st, tn);
+            launch_raster_mode<GS_DISPLAY_ELLIPSE>(J, at_once, std2, outline2, exact_exp, st, tn);
             break;
         default:
-            launch_raster_mode<GS_DISPLAY_POINT>(J, J.ntiles, std2, outline2, exact_exp, st, tn);
+            launch_raster_mode<GS_DISPLAY_POINT>(J, at_once, std2, outline2, exact_exp, st, tn);
             break;
     }
     prof_mark(kProfRaster, false, st);
