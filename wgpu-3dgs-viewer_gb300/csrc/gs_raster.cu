@@ -861,33 +861,38 @@ __device__ __forceinline__ void raster_tile(
     if constexpr (MODE == GS_DISPLAY_POINT) {
         // alpha is 1: blending a fragment replaces the pixel, whatever lies behind it
         bool found = px >= W || py >= H;
-        uint32_t base = below(n), cnt = n - base;
-        if (n > C) src.begin(S, base, cnt, below(base), base - below(base));
-        for (uint32_t end = n; end > 0;) {
-            if (n > C)
-                src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
-            else
-                src.stage_only<MODE>(S, n, std2);
-            __syncthreads();
-            if (__any_sync(0xFFFFFFFFu, !found)) {
-                const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
-                for (int i = (int)nl - 1; i >= 0; --i) {
-                    if (__all_sync(0xFFFFFFFFu, found)) break;
-                    const uint32_t j = S.list[warp][i];
-                    float al;
-                    if (!found && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) {
-                        const float4 c = S.c[j];
-                        d[0] = blend8(0.0f, 0.0f, c.x);
-                        d[1] = blend8(0.0f, 0.0f, c.y);
-                        d[2] = blend8(0.0f, 0.0f, c.z);
-                        found = true;
-                    }
+        auto nearest = [&](uint32_t cnt) {
+            const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
+            for (int i = (int)nl - 1; i >= 0; --i) {
+                const uint32_t j = S.list[warp][i];
+                float al;
+                if (!found && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pxc, pyc, outline2, &al)) {
+                    const float4 c = S.c[j];
+                    d[0] = blend8(0.0f, 0.0f, c.x);
+                    d[1] = blend8(0.0f, 0.0f, c.y);
+                    d[2] = blend8(0.0f, 0.0f, c.z);
+                    found = true;
                 }
+                if (__all_sync(0xFFFFFFFFu, found)) break;
             }
-            if (__syncthreads_and(found)) break;
-            end = base;
-            base = below(end);
-            cnt = end - base;
+        };
+        if (n <= C) {
+            if (n > 0) {
+                src.stage_only<MODE>(S, n, std2);
+                __syncthreads();
+                nearest(n);
+            }
+        } else {
+            uint32_t base = n - C;
+            src.begin(S, base, C, below(base), base - below(base));
+            for (uint32_t end = n; end > 0;) {
+                src.stage<MODE>(S, end - base, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+                __syncthreads();
+                if (__any_sync(0xFFFFFFFFu, !found)) nearest(end - base);
+                if (__syncthreads_and(found)) break;
+                end = base;
+                base = below(end);
+            }
         }
     } else if (n <= C && n < early_out_min<MODE>(suffix_min)) {
         if (n > 0) {

@@ -567,8 +567,249 @@ static cudaError_t ensure_sort_smem() {
     return cudaSuccess;
 }
 
+// ---- small sorts: every pass in one launch of one cluster --------------------------------------
+// Up to kClusterMaxPairs pairs are sorted by a single thread-block cluster: CTA c holds positions
+// [c K, (c + 1) K) in registers (K = 1024 ROWS), each pass ranks them as sort_pass_block does, the
+// CTAs exchange their digit counts through distributed shared memory, and every pair goes straight
+// to its place in the shared memory of the CTA that owns it.  Two cluster barriers a pass take the
+// place of a launch, a look-back and a trip through global memory, and the digit histogram kernel
+// falls away, as a pass counts what it holds.
+constexpr uint32_t kClusterThreads = 1024;
+constexpr uint32_t kClusterWarps = kClusterThreads / 32;
+constexpr uint32_t kClusterMaxCtas = 16;
+
+template <uint32_t ROWS>
+struct ClusterShared {
+    uint2 kv[kClusterThreads * ROWS];
+    uint32_t whist[kClusterWarps][256];
+    uint32_t cnt[kClusterMaxCtas][256];
+    uint32_t part[4][256];
+    uint32_t base[256];
+    uint32_t tmp[kClusterWarps];
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+// Every CTA of the cluster arrives; shared-memory writes before it, local and remote, are visible
+// after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared address `p` of this CTA, in CTA `cta` of the cluster.
+__device__ __forceinline__ uint32_t remote_smem(const void *p, uint32_t cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+    return r;
+}
+
+template <uint32_t ROWS>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    sort_cluster_kernel(uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, const uint32_t *count,
+                        uint32_t max_count, const PassSplit sp, Ctrl *ctrl) {
+    constexpr uint32_t K = kClusterThreads * ROWS;
+    extern __shared__ __align__(16) uint8_t cluster_smem[];
+    ClusterShared<ROWS> &S = *reinterpret_cast<ClusterShared<ROWS> *>(cluster_smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = lanemask_lt();
+    const uint32_t me = cluster_rank(), ctas = cluster_size();
+    if (me == 0 && tid == 0) ctrl->status = 0u;  // of the call; no flag is waited for here
+    const uint32_t n = load_count(count, max_count);
+    const bool some = me * K < n;  // this CTA holds pairs
+    const uint32_t at0 = warp * (32u * ROWS) + lane;
+
+    uint32_t k[ROWS], v[ROWS], r[ROWS];
+#pragma unroll
+    for (uint32_t i = 0; i < ROWS; ++i) {
+        const uint32_t pos = me * K + at0 + 32u * i;
+        const bool ok = pos < n;  // padding keys (all ones, last) stay behind every pair
+        k[i] = ok ? keys[pos] : 0xFFFFFFFFu;
+        v[i] = ok ? vals[pos] : 0u;
+    }
+    cluster_sync();  // every CTA has started: its shared memory may be written
+    for (uint32_t p = 0; p < sp.n; ++p) {
+        const uint32_t shift = sp.shift[p], bits = sp.bits[p], dmask = (1u << bits) - 1u;
+        for (uint32_t q = tid; q < kClusterWarps * 256u; q += kClusterThreads) (&S.whist[0][0])[q] = 0u;
+        __syncthreads();
+        if (some) {
+#pragma unroll
+            for (uint32_t i = 0; i < ROWS; ++i) {
+                const uint32_t d = (k[i] >> shift) & dmask;
+                uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+                for (uint32_t b = 0; b < 8; ++b) {
+                    if (b >= bits) break;
+                    const uint32_t bit = (d >> b) & 1u;
+                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, bit);
+                    peers &= bit ? bal : ~bal;
+                }
+                const uint32_t rank = __popc(peers & lt);
+                const uint32_t pre = S.whist[warp][d];
+                __syncwarp();
+                if (rank == 0) S.whist[warp][d] = pre + __popc(peers);
+                __syncwarp();
+                r[i] = pre + rank;
+            }
+        }
+        __syncthreads();
+        // Digit d of warps 8q .. 8q + 7 (q = tid / 256): exclusive offsets over the warps, the CTA's count
+        const uint32_t d = tid & 255u, q = tid >> 8;
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) {
+            c[w] = S.whist[8u * q + w][d];
+            sum += c[w];
+        }
+        S.part[q][d] = sum;
+        __syncthreads();
+        uint32_t run = 0, total = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t x = S.part[j][d];
+            if (j < q) run += x;
+            total += x;
+        }
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) {
+            S.whist[8u * q + w][d] = run;
+            run += c[w];
+        }
+        for (uint32_t j = q; j < ctas; j += 4)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote_smem(&S.cnt[me][d], j)), "r"(total) : "memory");
+        cluster_sync();  // also: every CTA holds its pairs in registers, so kv is free
+        uint32_t all = 0, before = 0;
+        if (tid < 256u) {
+            for (uint32_t j = 0; j < ctas; ++j) {
+                const uint32_t x = S.cnt[j][d];
+                if (j < me) before += x;
+                all += x;
+            }
+        }
+        uint32_t every;
+        const uint32_t first = block_scan_excl<kClusterWarps>(all, S.tmp, &every);
+        if (tid < 256u) S.base[d] = first + before;
+        __syncthreads();
+        if (some) {
+#pragma unroll
+            for (uint32_t i = 0; i < ROWS; ++i) {
+                const uint32_t dd = (k[i] >> shift) & dmask;
+                const uint32_t pos = S.base[dd] + S.whist[warp][dd] + r[i];  // below the pairs of all CTAs
+                const uint32_t cta = pos / K;
+                asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(remote_smem(&S.kv[pos - cta * K], cta)),
+                             "r"(k[i]), "r"(v[i])
+                             : "memory");
+            }
+        }
+        cluster_sync();
+        if (some) {
+#pragma unroll
+            for (uint32_t i = 0; i < ROWS; ++i) {
+                const uint2 kv = S.kv[at0 + 32u * i];
+                k[i] = kv.x;
+                v[i] = kv.y;
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < ROWS; ++i) {
+        const uint32_t pos = me * K + at0 + 32u * i;
+        if (pos < n) {
+            keys[pos] = k[i];
+            vals[pos] = v[i];
+        }
+    }
+}
+
+// Largest cluster of sort_cluster_kernel<ROWS> that the current device can hold (0: none).
+template <uint32_t ROWS>
+static uint32_t cluster_ctas_supported() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> cached[kDevices];  // 1 + the answer
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+    int known = cached[dev].load(std::memory_order_acquire);
+    if (known) return (uint32_t)(known - 1);
+    auto *fn = sort_cluster_kernel<ROWS>;
+    uint32_t best = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterShared<ROWS>)) == cudaSuccess &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        for (uint32_t ctas = kClusterMaxCtas; ctas >= 1 && !best; ctas /= 2) {
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = ctas;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(ctas);
+            cfg.blockDim = dim3(kClusterThreads);
+            cfg.dynamicSmemBytes = sizeof(ClusterShared<ROWS>);
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0) best = ctas;
+        }
+    }
+    cudaGetLastError();  // an unsupported size is not the caller's error
+    cached[dev].store((int)best + 1, std::memory_order_release);
+    return best;
+}
+
+// Launches the sort on one cluster where `max_count` fits ROWS rows; false: not this size.
+template <uint32_t ROWS>
+static bool launch_cluster_rows(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
+                                const PassSplit &sp, Ctrl *ctrl, cudaStream_t st, cudaError_t *err) {
+    constexpr uint32_t K = kClusterThreads * ROWS;
+    const uint32_t ctas = (max_count + K - 1) / K;
+    if (ctas == 0 || ctas > cluster_ctas_supported<ROWS>()) return false;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ctas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = sizeof(ClusterShared<ROWS>);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    *err = cudaLaunchKernelEx(&cfg, sort_cluster_kernel<ROWS>, keys, vals, count, max_count, sp, ctrl);
+    count_launches(1);
+    return true;
+}
+
+// The fewest rows that fit: fewer rows a thread and more CTAs are faster throughout (16384 pairs: 24.5,
+// 25.0, 29.2 and 41.4 us at 1, 2, 4 and 8 rows).  Against the histogram and pass kernels: 5,000 pairs 63.9 ->
+// 18.8 us, 30,000 72.9 -> 29.1, 65,536 74.2 -> 37.3, 131,072 72.3 -> 58.2; at 12 rows (196,608 pairs) they
+// are the faster ones, 78.0 against 80.3.
+// Eight rows take an SM's whole register file for most of a frame's sort, which is a loss where other
+// views could run beside it (`overlapped`; 10 views of 93k: 554 -> 582 us a batch with them).
+static bool launch_sort_cluster(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
+                                uint32_t key_bits, bool overlapped, Ctrl *ctrl, cudaStream_t st, cudaError_t *err) {
+    const PassSplit sp = even_split(key_bits);
+    return launch_cluster_rows<1>(keys, vals, max_count, count, sp, ctrl, st, err) ||
+           launch_cluster_rows<2>(keys, vals, max_count, count, sp, ctrl, st, err) ||
+           launch_cluster_rows<4>(keys, vals, max_count, count, sp, ctrl, st, err) ||
+           (!overlapped && launch_cluster_rows<8>(keys, vals, max_count, count, sp, ctrl, st, err));
+}
+
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
-                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning) {
+                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning,
+                        bool overlapped) {
+    // One cluster where the pairs fit (the bounded-wait hook stalls look-backs, which it has none of).
+    if (wait_config().stall_tile == kNoStall) {
+        cudaError_t e = cudaSuccess;
+        prof_mark(prof_stage, true, st);
+        const bool done = launch_sort_cluster(keys, vals, max_count, count, key_bits, overlapped,
+                                              reinterpret_cast<Ctrl *>(scratch), st, &e);
+        if (done) prof_mark(prof_stage, false, st);
+        if (done) return e == cudaSuccess ? cudaGetLastError() : e;
+    }
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const Tuning tn = tuning ? *tuning : default_tuning();
     const uint32_t db = tn.sort_digit_bits < kMinDigitBits   ? kMinDigitBits
