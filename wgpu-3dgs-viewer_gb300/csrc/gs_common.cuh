@@ -106,6 +106,18 @@ __device__ __forceinline__ void ctrl_reset(Ctrl *ctrl, int mode, Ctrl *owner, ui
         for (uint32_t k = t; k < 4 * 256; k += blockDim.x) (&ctrl->hist[0][0])[k] = 0u;
 }
 
+// Starts a raster call that waits for no flag (one thread): status and pair counts.  The call lays
+// out `arena_words` of arena, so payload may lie past them when it is over: what lies there is not
+// known to be clean any more, and a later call that reads flags clears it.
+__device__ __forceinline__ void ctrl_reset_flagless(Ctrl *ctrl, uint32_t arena_words) {
+    ctrl->status = 0u;
+    ctrl->count = 0u;
+    ctrl->total = 0u;
+    ctrl->pair_base = 0u;
+    ctrl->seg_total = 0u;
+    if (ctrl->clean > arena_words) ctrl->clean = arena_words;
+}
+
 // The arena words this call must clear (set by the owner's mode-1 reset), cleared by every CTA
 // of a grid that runs before any look-back of the call (grid-stride, 16-byte stores).
 __device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena) {

@@ -50,6 +50,9 @@ struct RasterLayout {
 constexpr uint32_t kCountTiles = 8192;
 constexpr uint32_t kEmitBlocks = 152 * 8;
 
+// Ranks a direct frame can have: a bit each in shared memory (RasterShared::raw).
+constexpr uint32_t kDirectMaxRanks = 3u * 16u * kRasterThreads * 8u;
+
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = 256 * kScanItems;
 
@@ -146,21 +149,41 @@ Tuning default_tuning() {
     return t;
 }
 
+// A tile rectangle in one word: bytes x0, y0, 127 - x1, 127 - y1 of its first and last tile, in units of
+// 2^shift tiles so that a target has at most 128 of them each way.  With a tile's own bytes (x, y,
+// 127 - x, 127 - y), each below 128, the rectangle can hold the tile when no byte of the difference
+// borrows: one subtraction under guard bits.  (With shift 0 it does hold it.)
+constexpr uint32_t kRectGuard = 0x80808080u, kEmptyRect = 0x7F7F7F7Fu;
+__device__ __forceinline__ uint32_t pack_rect(uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, uint32_t shift) {
+    return (x0 >> shift) | ((y0 >> shift) << 8) | ((127u - (x1 >> shift)) << 16) | ((127u - (y1 >> shift)) << 24);
+}
+__device__ __forceinline__ bool rect_may_hold(uint32_t rect, uint32_t tile) {
+    return (((tile | kRectGuard) - rect) & kRectGuard) == kRectGuard;
+}
+
 // K3a: per draw rank, the splat's tile rectangle, the corner tiles its footprint misses, and
 // its tile count.  With `binfo` (one view of one model, its preprocess having stored each
 // visible splat's tiles) the rank gathers that 16-byte record; otherwise it gathers the 48-byte
 // splat and works the tiles out here.  Several models first copy their splats into draw order.
 // The first segment's launch (arena non-null) also clears the flag-arena words the call must
 // clear, before the scan and the tile sort read any flag.
+// With `rects` (and no counts) the ranks are scanned by raster_direct_kernel up to the capacity: each
+// gets its rectangle in one word, an empty one where there is no splat or no tile is kept; the first
+// segment's launch (reset non-null) starts the call's control block.
 __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     const gs_splat *__restrict__ splats, const uint4 *__restrict__ binfo, const uint32_t *__restrict__ sorted_index,
     const uint32_t *count, uint32_t max_count, uint32_t rank_offset, gs_splat *__restrict__ sorted_out, int direct,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *__restrict__ info,
-    uint32_t *__restrict__ counts, const Ctrl *owner, uint64_t *arena) {
+    uint32_t *__restrict__ counts, const Ctrl *owner, uint64_t *arena, uint32_t *__restrict__ rects,
+    uint32_t rect_shift, Ctrl *reset, uint32_t arena_words) {
     if (arena) arena_clear(owner, arena);
+    if (reset && blockIdx.x == 0 && threadIdx.x == 0) ctrl_reset_flagless(reset, arena_words);
     const uint32_t n = count ? min(*count, max_count) : max_count;
     const uint32_t k = blockIdx.x * kBinThreads + threadIdx.x;
-    if (k >= n) return;
+    if (k >= n) {
+        if (rects && k < max_count) rects[k] = kEmptyRect;
+        return;
+    }
     // Indices come from the depth sort; the bound check only matters if that sort timed out.
     const uint32_t gi = sorted_index[k];
     uint4 t = make_uint4(0u, 0u, 0u, 0u);  // x0 | y0 << 16, w | h << 16, mask, count
@@ -182,8 +205,11 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
             t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
         }
     }
+    if (counts) counts[k] = t.w;
+    else rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
+                                    (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
+                        : kEmptyRect;
     info[k] = make_uint4(t.x, t.y, t.z, direct ? gi : rank_offset + k);
-    counts[k] = t.w;
 }
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
@@ -832,28 +858,20 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL>
 __device__ __forceinline__ void raster_tile(
-    RasterShared &S, const gs_splat *__restrict__ sorted, const uint2 *__restrict__ pairs,
-    const uint2 *__restrict__ ranges, uint8_t *__restrict__ target, uint32_t W, uint32_t H, uint32_t pitch,
-    uint32_t tiles_x, float std2, float outline2, uint32_t max_splats, uint32_t suffix_min, float eps,
-    unsigned long long *counters, Ctrl *pctrl, uint32_t tile) {
+    RasterShared &S, const RasterJob &J, const uint2 *__restrict__ list, uint32_t n, float std2, float outline2,
+    uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
     // Work tallies of the counting variant (profiling only): fragment evaluations, alphas,
     // channel-triple blends and transmittance updates.
     uint32_t n_eval = 0, n_alpha = 0, n_blend = 0, n_trans = 0;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
-    uint2 range = ranges[tile];
-    if (range.y < range.x || range.y > pctrl->count) {
-        if (threadIdx.x == 0) atomicOr(&pctrl->status, kStatusBounds);
-        range = make_uint2(0u, 0u);
-    }
-    const uint32_t n = range.y - range.x;
+    const uint32_t W = J.W, H = J.H, tx = tile % J.tiles_x, ty = tile / J.tiles_x;
     const uint32_t wx0 = tx * GS_TILE + (warp & 1u) * 8u, wy0 = ty * GS_TILE + (warp >> 1) * 4u;
     const uint32_t px = wx0 + (lane & 7u), py = wy0 + (lane >> 3);
     const float pxc = (float)px + 0.5f, pyc = (float)py + 0.5f;
     const float bx0 = (float)wx0 + 0.5f, bx1 = (float)wx0 + 7.5f;
     const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 3.5f;
     float d[3] = {0.0f, 0.0f, 0.0f};
-    ChunkSource src{sorted, pairs + range.x, max_splats, 0u};
+    ChunkSource src{J.splats, list, J.max_splats, 0u};
     constexpr uint32_t C = kRasterThreads;
     // the chunk before list position `end` (for walks from the end of the list)
     auto below = [](uint32_t end) { return end > C ? end - C : 0u; };
@@ -1020,7 +1038,7 @@ __device__ __forceinline__ void raster_tile(
     }
     if (px < W && py < H) {
         const uint32_t rgba = (uint32_t)d[0] | ((uint32_t)d[1] << 8) | ((uint32_t)d[2] << 16) | 0xFF000000u;
-        *reinterpret_cast<uint32_t *>(target + (size_t)py * pitch + (size_t)px * 4u) = rgba;
+        *reinterpret_cast<uint32_t *>(J.target + (size_t)py * J.pitch + (size_t)px * 4u) = rgba;
     }
     if constexpr (COUNT) {
         const uint32_t v[4] = {n_eval, n_alpha, n_blend, n_trans};
@@ -1033,6 +1051,15 @@ __device__ __forceinline__ void raster_tile(
 }
 
 
+// The tile's run of the tile-sorted pairs; empty (and reported) when a scan that gave up left it
+// outside the list.
+__device__ __forceinline__ uint2 tile_range(const RasterJob &J, uint32_t tile) {
+    const uint2 range = J.ranges[tile];
+    if (range.y >= range.x && range.y <= J.ctrl->count) return range;
+    if (threadIdx.x == 0) atomicOr(&J.ctrl->status, kStatusBounds);
+    return make_uint2(0u, 0u);
+}
+
 // FEW: a grid of few tiles (at most kFewTiles), whose time is that of its longest lists, not of the
 // instructions of all: blend_list four entries at a time, in up to 64 registers a thread (4 CTAs an SM;
 // 3 and 5 CTAs take 48 and 55 us for 100k at 640x360, and 4 CTAs 49 us, against 70 us without FEW).
@@ -1041,9 +1068,89 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(con
                                                                 uint32_t suffix_min, float eps,
                                                                 unsigned long long *counters) {
     __shared__ RasterShared S;
-    raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch,
-                                                          J.tiles_x, std2, outline2, J.max_splats, suffix_min, eps,
-                                                          counters, J.ctrl, J.order ? J.order[blockIdx.x] : blockIdx.x);
+    const uint32_t tile = J.order ? J.order[blockIdx.x] : blockIdx.x;
+    const uint2 r = tile_range(J, tile);
+    raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J, J.pairs + r.x, r.y - r.x, std2, outline2, suffix_min, eps,
+                                                          counters, tile);
+}
+
+// A frame of few splats and tiles without the binning's scan, emission and tile sort: each tile's CTA
+// goes through the rectangles of all ranks (draw order), marks those that hold its tile in one bit
+// each, and writes its own list of pairs behind those of the CTAs before it.  The scan is bound by L2
+// (4 bytes a rank and tile; 16-byte records took 166 us for a frame of 47.5k ranks and 825 tiles, the
+// words 102 us), the lists by the latency of a thread's few tile records.
+template <uint32_t MODE, bool PORTABLE_EXP, bool FEW>
+__global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
+    raster_direct_kernel(const RasterJob J, const uint32_t *__restrict__ rects, const uint4 *__restrict__ info,
+                         uint32_t ranks, uint32_t shift, uint2 *__restrict__ pairs, uint32_t max_pairs, float std2,
+                         float outline2, uint32_t suffix_min, float eps) {
+    __shared__ RasterShared S;
+    __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;
+    uint32_t *hits = reinterpret_cast<uint32_t *>(S.raw);  // bit r of word q: rank 32 q + r holds the tile
+    static_assert(sizeof(S.raw) * 8 >= kDirectMaxRanks, "a bit per rank");
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
+    const uint32_t tx = tile % J.tiles_x, ty = tile / J.tiles_x, words = (ranks + 31u) / 32u;
+    const uint32_t here = pack_rect(tx, ty, tx, ty, shift);
+    constexpr uint32_t STEP = kRasterThreads / 32u;
+    for (uint32_t q0 = warp; q0 < words; q0 += 8u * STEP) {
+        uint32_t r[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            const uint32_t k = 32u * (q0 + u * STEP) + lane;
+            r[u] = k < ranks ? rects[k] : kEmptyRect;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            const uint32_t q = q0 + u * STEP;
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, rect_may_hold(r[u], here));
+            if (lane == 0 && q < words) hits[q] = m;
+        }
+    }
+    __syncthreads();
+    // thread t owns the words [t per, (t + 1) per): their places in the list by a block scan
+    const uint32_t per = (words + kRasterThreads - 1u) / kRasterThreads;
+    const uint32_t first = min(words, tid * per), last = min(words, first + per);
+    uint32_t sum = 0;
+    for (uint32_t q = first; q < last; ++q) {
+        const uint32_t found = hits[q];
+        uint32_t kept = found;
+        for (uint32_t m = found; m; m &= m - 1u) {
+            const uint32_t r = __ffs(m) - 1u;
+            const uint4 in = info[32u * q + r];  // x0 | y0 << 16, w | h << 16, kept tiles (0: all), value
+            const uint32_t dx = tx - (in.x & 0xFFFFu), dy = ty - (in.x >> 16), w = in.y & 0xFFFFu;
+            if (!(dx < w && dy < (in.y >> 16)) || (in.z != 0u && !((in.z >> (dy * w + dx)) & 1u))) kept &= ~(1u << r);
+        }
+        if (kept != found) hits[q] = kept;
+        sum += __popc(kept);
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, n = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kRasterThreads / 32u; ++w) {
+        if (w < warp) before += s_warp[w];
+        n += s_warp[w];
+    }
+    if (tid == 0) s_base = n ? atomicAdd(&J.ctrl->total, n) : 0u;
+    __syncthreads();
+    uint32_t base = s_base;
+    if (base > max_pairs || n > max_pairs - base) {  // the list is full: reported, the tile stays empty
+        if (tid == 0) atomicOr(&J.ctrl->status, kStatusCapacity);
+        base = n = 0;
+    } else {
+        uint32_t at = base + before + incl - sum;
+        for (uint32_t q = first; q < last; ++q)
+            for (uint32_t m = hits[q]; m; m &= m - 1u) pairs[at++] = make_uint2(tile, info[32u * q + __ffs(m) - 1u].w);
+    }
+    __syncthreads();
+    raster_tile<MODE, PORTABLE_EXP, false, FEW ? 4u : 1u>(S, J, pairs + base, n, std2, outline2, suffix_min, eps, nullptr,
+                                                          tile);
 }
 
 // One grid over the tiles of several views (a batch): CTA b rasterises tile b - tile_base[v] of
@@ -1061,10 +1168,10 @@ __global__ void __launch_bounds__(kRasterThreads, 6) raster_views_kernel(const R
         else hi = mid - 1;
     }
     const RasterJob &J = jobs[lo];
-    const uint32_t b = blockIdx.x - tile_base[lo];
-    raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J.splats, J.pairs, J.ranges, J.target, J.W, J.H, J.pitch, J.tiles_x,
-                                           std2, outline2, J.max_splats, suffix_min, eps, nullptr, J.ctrl,
-                                           J.order ? J.order[b] : b);
+    const uint32_t b = blockIdx.x - tile_base[lo], tile = J.order ? J.order[b] : b;
+    const uint2 r = tile_range(J, tile);
+    raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J, J.pairs + r.x, r.y - r.x, std2, outline2, suffix_min, eps, nullptr,
+                                               tile);
 }
 
 // Work tallies of the counting raster variant (profiling only).
@@ -1216,7 +1323,7 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(g.splats, binfo, g.sorted_index, g.count, g.max_count,
                                                          rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y,
                                                          u.display_mode, u.std_dev * u.std_dev, L.info, L.offsets,
-                                                         L.ctrl, cleared ? nullptr : L.flags);
+                                                         L.ctrl, cleared ? nullptr : L.flags, nullptr, 0, nullptr, 0);
         cleared = true;
         const uint32_t scan_blocks = (g.max_count + kScanTile - 1) / kScanTile;
         bin_scan_kernel<<<scan_blocks, 256, 0, st>>>(L.offsets, g.count, g.max_count, L.ctrl, L.flags);
@@ -1313,15 +1420,85 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
     return launch_binning_ranges(segs, nseg, W, H, max_pairs, scratch, st);
 }
 
+// Frames of up to kDirectWork ranks x tiles take raster_direct_kernel: its CTAs read every rank's word,
+// where the binning's eight launches and the two of the tile sort cost about 50 us whatever the frame.
+// 5k splats x 240 tiles (1.2e6): 95 -> 45 us a frame; 47.5k x 825 (3.9e7): 132 -> 102; 38.9k x 2272
+// (8.8e7): 128 -> 125; 68.4k x 1400 (9.6e7): 157 -> 167; 28.6k x 5292 (1.5e8): 135 -> 161.  Views of a
+// batch overlap, so the tiles of all of them count (10 views of 11.6k, 4e8 so counted: 234 -> 440).
+constexpr uint64_t kDirectWork = 60'000'000;
+static bool direct_raster(uint32_t ranks, uint32_t tiles_at_once) {
+    return ranks > 0 && ranks <= kDirectMaxRanks && (uint64_t)ranks * tiles_at_once <= kDirectWork;
+}
+
+template <uint32_t MODE>
+static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift,
+                               uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
+    const bool few = tiles_at_once <= kFewTiles;
+    auto go = [&](auto kernel) {
+        kernel<<<J.ntiles, kRasterThreads, 0, st>>>(J, L.offsets, L.info, ranks, shift, L.pairs, max_pairs, std2, outline2,
+                                                    t.suffix_min, t.eps);
+    };
+    if (exact) few ? go(raster_direct_kernel<MODE, true, true>) : go(raster_direct_kernel<MODE, true, false>);
+    else few ? go(raster_direct_kernel<MODE, false, true>) : go(raster_direct_kernel<MODE, false, false>);
+}
+
+// Tile records of every rank, then the tiles (see raster_direct_kernel).
+static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg, uint32_t ranks, const RasterMode &u,
+                                        const RasterJob &J, uint32_t max_pairs, void *scratch, uint32_t tiles_at_once,
+                                        int exact_exp, cudaStream_t st, const Tuning &tn) {
+    const RasterLayout L = raster_layout(scratch, ranks, J.W, J.H, max_pairs);
+    const float std2 = u.std_dev * u.std_dev, o = u.std_dev - 0.1f, outline2 = o * o;
+    const int direct = nseg == 1 ? 1 : 0;
+    uint32_t rank_offset = 0, shift = 0;
+    while (((L.tiles_x - 1u) >> shift) > 127u || ((L.tiles_y - 1u) >> shift) > 127u) ++shift;
+    bool started = false;
+    prof_mark(kProfBin, true, st);
+    for (uint32_t s = 0; s < nseg; ++s) {
+        const RasterSegment &g = segs[s];
+        const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
+        if (blocks == 0) continue;
+        const uint4 *binfo = direct && g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
+        bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(g.splats, binfo, g.sorted_index, g.count, g.max_count, rank_offset,
+                                                         L.sorted, direct, L.tiles_x, L.tiles_y, u.display_mode, std2,
+                                                         L.info + rank_offset, nullptr, nullptr, nullptr,
+                                                         L.offsets + rank_offset, shift, started ? nullptr : L.ctrl,
+                                                         L.arena_words);
+        count_launches(1);
+        started = true;
+        rank_offset += g.max_count;
+    }
+    prof_mark(kProfBin, false, st);
+    prof_mark(kProfRaster, true, st);
+    switch (u.display_mode) {
+        case GS_DISPLAY_SPLAT:
+            launch_direct_mode<GS_DISPLAY_SPLAT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            break;
+        case GS_DISPLAY_ELLIPSE:
+            launch_direct_mode<GS_DISPLAY_ELLIPSE>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            break;
+        default:
+            launch_direct_mode<GS_DISPLAY_POINT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            break;
+    }
+    count_launches(1);
+    prof_mark(kProfRaster, false, st);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint8_t *target,
                           uint32_t W, uint32_t H, uint32_t pitch, uint32_t max_pairs, void *scratch, int exact_exp,
                           cudaStream_t st, const Tuning *tuning, uint32_t tiles_at_once) {
     const Tuning tn = tuning ? *tuning : default_tuning();
-    cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
-    if (e != cudaSuccess) return e;
     const RasterJob J = raster_job(segs, nseg, target, W, H, pitch, max_pairs, scratch);
     if (J.ntiles == 0) return cudaSuccess;
     const uint32_t at_once = tiles_at_once > J.ntiles ? tiles_at_once : J.ntiles;
+    uint32_t ranks = 0;
+    for (uint32_t s = 0; s < nseg; ++s) ranks += segs[s].max_count;
+    // (the counting rasteriser and the bounded-wait hook know the general path only)
+    if (direct_raster(ranks, at_once) && !prof_counting() && wait_config().stall_tile == kNoStall)
+        return launch_raster_direct(segs, nseg, ranks, u, J, max_pairs, scratch, at_once, exact_exp, st, tn);
+    cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
+    if (e != cudaSuccess) return e;
     const float std2 = u.std_dev * u.std_dev;
     const float o = u.std_dev - 0.1f;
     const float outline2 = o * o;
