@@ -1247,6 +1247,11 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
         }
         b->chunks = (uint32_t)chunks.size();
         const PreView *pv_dev = reinterpret_cast<const PreView *>(b->views_dev.ptr);
+        // With one rasteriser grid, the views' tile sorts run as one segmented sort (one launch per
+        // pass over all views' pairs: keys (view, tile) with depth order kept inside each tile)
+        // when every target fits two tile-sort passes; else each view sorts its own pairs.
+        bool segmented = b->tuning.raster_grid != 0;
+        for (uint32_t i = 0; i < n && segmented; ++i) segmented = tile_sort_segmentable(views[i].width, views[i].height);
         // One rasteriser grid over every view's tiles: the views' raster jobs (pointers into
         // their scratch) and the prefix of their tile counts, known before any launch.
         std::vector<RasterJob> jobs(n);
@@ -1256,18 +1261,13 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
             uint32_t *ind = reinterpret_cast<uint32_t *>(v.control.ptr);
             const RasterSegment seg{(const gs_splat *)v.splats.ptr, (const uint32_t *)v.indices.ptr, ind + 1, ms[i]->n};
             jobs[i] = raster_job(&seg, 1, views[i].target, views[i].width, views[i].height, views[i].pitch, v.max_pairs,
-                                 v.raster_scratch.ptr);
+                                 v.raster_scratch.ptr, segmented);
             tile_base[i + 1] = tile_base[i] + jobs[i].ntiles;
         }
         GS_CUDA(b->jobs_dev.ensure((size_t)n * sizeof(RasterJob)));
         GS_CUDA(cudaMemcpy(b->jobs_dev.ptr, jobs.data(), (size_t)n * sizeof(RasterJob), cudaMemcpyHostToDevice));
         GS_CUDA(b->tile_base_dev.ensure((size_t)(n + 1) * 4));
         GS_CUDA(cudaMemcpy(b->tile_base_dev.ptr, tile_base.data(), (size_t)(n + 1) * 4, cudaMemcpyHostToDevice));
-        // With one rasteriser grid, the views' tile sorts run as one segmented sort (one launch per
-        // pass over all views' pairs: keys (view, tile) with depth order kept inside each tile)
-        // when every target fits two tile-sort passes; else each view sorts its own pairs.
-        bool segmented = b->tuning.raster_grid != 0;
-        for (uint32_t i = 0; i < n && segmented; ++i) segmented = tile_sort_segmentable(views[i].width, views[i].height);
         std::vector<SortSegment> sort_segs(segmented ? n : 0);
         std::vector<uint32_t> sort_base(n + 1, 0u);
         if (segmented) {
@@ -1314,7 +1314,7 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
                     // display mode and std dev, which are part of the shape key (frame.gt).
                     if (segmented)
                         err = launch_binning_front(&seg, 1, raster_mode(uh[i]), views[i].width, views[i].height,
-                                                   v.max_pairs, v.raster_scratch.ptr, vs);
+                                                   v.max_pairs, v.raster_scratch.ptr, vs, true);
                     else if (b->tuning.raster_grid)
                         err = launch_binning(&seg, 1, raster_mode(uh[i]), views[i].width, views[i].height, v.max_pairs,
                                              v.raster_scratch.ptr, vs);

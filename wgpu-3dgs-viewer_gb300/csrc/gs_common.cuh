@@ -49,8 +49,7 @@ struct Ctrl {
     uint32_t ticket[8];
     uint32_t count;       // preprocess: V; raster: tile pairs kept
     uint32_t total;       // raster: tile pairs wanted (saturating)
-    uint32_t pair_base;   // raster: running pair offset across segments
-    uint32_t seg_total;   // raster: pairs of the segment being binned
+    uint32_t unused[2];
     uint32_t serial;      // area owner: last epoch handed out in the area
     uint32_t clean;       // area owner: leading arena words holding only zeros or flag words
     uint32_t clear_lo;    // area owner: arena words [clear_lo, clear_hi) to clear in this call
@@ -62,15 +61,14 @@ struct Ctrl {
 };
 static_assert(sizeof(Ctrl) % 16 == 0, "Ctrl must keep 16-byte alignment of what follows");
 
-// Resets a control block (one CTA): mode 1 = a new stage call (epoch, status, tickets, counters,
-// histograms, wait configuration); mode 0 = a new segment inside a call (epoch and tickets 0..1
-// only).  The epoch comes from `owner`, the block holding the area's serial counter (the block
-// itself for a single-stage area).  `arena_words` (owner, mode 1 only): words of the flag arena
-// this call uses, or kKeepArena when this call runs no clearing kernel.
-__device__ __forceinline__ void ctrl_reset(Ctrl *ctrl, int mode, Ctrl *owner, uint32_t arena_words, WaitCfg cfg) {
+// Resets a control block for a new stage call (one CTA): epoch, status, tickets, counters,
+// histograms, wait configuration.  The epoch comes from `owner`, the block holding the area's serial
+// counter (the block itself for a single-stage area).  `arena_words` (owner only): words of the flag
+// arena this call uses, or kKeepArena when this call runs no clearing kernel.
+__device__ __forceinline__ void ctrl_reset(Ctrl *ctrl, Ctrl *owner, uint32_t arena_words, WaitCfg cfg) {
     const uint32_t t = threadIdx.x;
     if (t == 0) {
-        if (ctrl == owner && mode == 1) {
+        if (ctrl == owner) {
             if (owner->serial >= kSerialRestart) {
                 owner->serial = 0u;
                 owner->clean = 0u;  // flags of the old serial range may match new epochs
@@ -89,21 +87,14 @@ __device__ __forceinline__ void ctrl_reset(Ctrl *ctrl, int mode, Ctrl *owner, ui
         const uint32_t e = owner->serial + 1u;
         owner->serial = e;
         ctrl->epoch = e;
-        ctrl->ticket[0] = 0u;
-        ctrl->ticket[1] = 0u;
-        if (mode == 1) {
-            ctrl->status = 0u;
-            for (int k = 1; k < 8; ++k) ctrl->ticket[k] = 0u;
-            ctrl->count = 0u;
-            ctrl->total = 0u;
-            ctrl->pair_base = 0u;
-            ctrl->seg_total = 0u;
-            ctrl->spin_limit = cfg.spin_limit;
-            ctrl->stall_tile = cfg.stall_tile;
-        }
+        ctrl->status = 0u;
+        for (int k = 0; k < 8; ++k) ctrl->ticket[k] = 0u;
+        ctrl->count = 0u;
+        ctrl->total = 0u;
+        ctrl->spin_limit = cfg.spin_limit;
+        ctrl->stall_tile = cfg.stall_tile;
     }
-    if (mode == 1)
-        for (uint32_t k = t; k < 4 * 256; k += blockDim.x) (&ctrl->hist[0][0])[k] = 0u;
+    for (uint32_t k = t; k < 4 * 256; k += blockDim.x) (&ctrl->hist[0][0])[k] = 0u;
 }
 
 // Starts a raster call that waits for no flag (one thread): status and pair counts.  The call lays
@@ -113,12 +104,10 @@ __device__ __forceinline__ void ctrl_reset_flagless(Ctrl *ctrl, uint32_t arena_w
     ctrl->status = 0u;
     ctrl->count = 0u;
     ctrl->total = 0u;
-    ctrl->pair_base = 0u;
-    ctrl->seg_total = 0u;
     if (ctrl->clean > arena_words) ctrl->clean = arena_words;
 }
 
-// The arena words this call must clear (set by the owner's mode-1 reset), cleared by every CTA
+// The arena words this call must clear (set by the owner's reset), cleared by every CTA
 // of a grid that runs before any look-back of the call (grid-stride, 16-byte stores).
 __device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena) {
     const uint32_t lo = owner->clear_lo, hi = owner->clear_hi;

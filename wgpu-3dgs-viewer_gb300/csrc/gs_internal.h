@@ -27,10 +27,9 @@ void count_launches(uint32_t n);
 // Records `message` as the calling thread's gs_last_error() and returns `status`.
 gs_status set_error(gs_status status, const char *message);
 
-// Resets a control block (see ctrl_reset): owner = the block holding the area's epoch counter
-// and arena mark (nullptr: the block itself); arena_words = the flag-arena words of this call
-// for the owner's mode-1 reset, kKeepArena when no clearing kernel runs in the call.
-__global__ void ctrl_init_kernel(Ctrl *ctrl, int mode, Ctrl *owner, uint32_t arena_words, WaitCfg cfg);
+// Resets the control block of a single-stage area (see ctrl_reset): arena_words = the flag-arena words
+// of this call, kKeepArena when no clearing kernel runs in the call.
+__global__ void ctrl_init_kernel(Ctrl *ctrl, uint32_t arena_words, WaitCfg cfg);
 
 // Look-back configuration every stage launch carries (the poll bound, and the stalled tile of
 // the bounded-wait test hook gs_debug_set_wait_fault).
@@ -113,12 +112,10 @@ PassSplit even_split_max(uint32_t key_bits, uint32_t max_digit);
 __host__ __device__ inline uint32_t hist_stride(uint32_t npasses) { return npasses <= 4 ? 256u : 1024u / npasses; }
 
 // Packed (uint2 {key, value}) in-place sort for internal pair lists whose digit histograms
-// (split by even_split) the producer accumulated into the control block `ctrl` after
-// sort_pairs_begin(): as counts, or (hist_scanned) already as exclusive digit offsets.  Its
+// (split by tile_split) the producer accumulated into the control block `ctrl`: as counts, or (hist_scanned) already as exclusive digit offsets.  Its
 // look-back flags (sort_pairs_flag_words of them) lie in the flag arena of the area whose
 // control block `owner` is; `alt` holds max_count pairs.
 size_t sort_pairs_flag_words(uint32_t max_count, uint32_t key_bits);
-cudaError_t sort_pairs_begin(Ctrl *ctrl, Ctrl *owner, cudaStream_t st);
 // The split of a tile-pair sort (producers of its digit histograms must use the same one).
 PassSplit tile_split(uint32_t key_bits);
 
@@ -142,6 +139,12 @@ cudaError_t launch_sort_segments(const SortSegment *segs_dev, const uint32_t *bl
                                  uint32_t total_blocks, cudaStream_t st);
 cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *count, uint32_t key_bits, Ctrl *ctrl,
                               uint64_t *flags, uint2 *alt, cudaStream_t st, bool hist_scanned);
+
+// The tile sort on compact items, in two passes (key_bits <= 16): items hold the tile's high digit
+// (tile >> tile_split.bits[0]) above value_bits bits of value, `low` the low digits; the digit offsets
+// in `ctrl` are exclusive.  The sorted values end up in `items`.
+cudaError_t launch_sort_items(uint32_t *items, const uint8_t *low, uint32_t *alt, uint32_t max_count, const uint32_t *count,
+                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st);
 
 // ---- K3 binning + K4 raster (gs_raster.cu) ----
 // The only frame uniforms binning and rasterisation read: camera, model and SH fields never
@@ -177,19 +180,23 @@ const Ctrl *raster_ctrl(const void *scratch);
 // can be known (and uploaded for a multi-view grid) before any launch.
 struct RasterJob {
     const gs_splat *splats;
-    const uint2 *pairs;
+    const uint32_t *values;  // pair values in tile and draw order, value i at values[i << value_shift]
+    uint32_t value_shift;
     const uint2 *ranges;
     const uint32_t *order;  // launch order of the tiles (null: tile = CTA index)
     uint8_t *target;
     uint32_t W, H, pitch, tiles_x, max_splats, ntiles;
     Ctrl *ctrl;
+    const Ctrl *sort_ctrl;  // tile sort: its status joins the raster's
 };
+// segmented: the view's pairs are sorted by launch_sort_segments, which keeps whole pairs.
 RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, uint32_t width, uint32_t height,
-                     uint32_t pitch, uint32_t max_pairs, void *scratch);
+                     uint32_t pitch, uint32_t max_pairs, void *scratch, bool segmented = false);
 // Binning of one view up to its tile sort (tile rectangles, count scan, pair emission, per-tile
-// counts and ranges or the sort's digit histograms).
+// counts and ranges or the sort's digit histograms).  segmented: as in raster_job.
 cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint32_t width,
-                                 uint32_t height, uint32_t max_pairs, void *scratch, cudaStream_t st);
+                                 uint32_t height, uint32_t max_pairs, void *scratch, cudaStream_t st,
+                                 bool segmented = false);
 // The view's tile sort as a segment of a segmented sort (pointer arithmetic on its scratch), and
 // whether its target is small enough for one (two tile-sort passes: at most 65536 tiles).
 SortSegment tile_sort_segment(const RasterSegment *segs, uint32_t nseg, uint32_t width, uint32_t height,

@@ -754,7 +754,7 @@ __global__ void preprocess_empty_kernel(uint32_t *indirect, uint32_t *dispatch, 
 // lie where a flag is read: its arena is never cleared (kKeepArena).
 __global__ void ctrl_init_views_kernel(const PreView *views, uint32_t nviews, Ctrl *group, WaitCfg cfg) {
     Ctrl *c = blockIdx.x < nviews ? views[blockIdx.x].ctrl : group;
-    ctrl_reset(c, 1, c, kKeepArena, cfg);
+    ctrl_reset(c, c, kKeepArena, cfg);
 }
 
 __global__ void preprocess_views_empty_kernel(const PreView *views, uint32_t nviews) {
@@ -841,7 +841,7 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
                               const gs_frame_uniforms *u_dev, uint4 *binfo) {
     Ctrl *ctrl = reinterpret_cast<Ctrl *>(scratch);
     uint64_t *flags = reinterpret_cast<uint64_t *>((uint8_t *)scratch + align_up(sizeof(Ctrl), 256));
-    ctrl_init_kernel<<<1, 256, 0, st>>>(ctrl, 1, nullptr, kKeepArena, wait_config());
+    ctrl_init_kernel<<<1, 256, 0, st>>>(ctrl, kKeepArena, wait_config());
     count_launches(1);
     if (n == 0) {
         preprocess_empty_kernel<<<1, 1, 0, st>>>(indirect, dispatch, ctrl);

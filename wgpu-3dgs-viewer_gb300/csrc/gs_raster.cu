@@ -4,10 +4,10 @@
 // BlendState::ALPHA_BLENDING onto a Rgba8Unorm target cleared to opaque black
 // (src/renderer.rs:162-195, 284-308; src/shader/render.wesl:46-56, 75-181).  This file
 // restates that per pixel:
-//   * K3 walks the depth-sorted splats, gathers each splat record into draw order, counts the
-//     16x16 tiles its fragment box touches, scans the counts (block scan + decoupled
-//     look-back) and emits (tile, draw-rank) pairs; a stable 8-bit-digit radix sort by tile
-//     then groups the pairs per tile with draw order kept inside each tile.
+//   * K3 walks the depth-sorted splats, counts the 16x16 tiles each one's footprint touches, scans the
+//     counts (block scan + decoupled look-back) and emits (tile, value) pairs; a stable radix sort
+//     by tile then groups the values per tile with draw order kept inside each tile.  Frames of few
+//     splats and tiles skip the scan, the pairs and their sort (raster_direct_kernel).
 //   * K4 runs one CTA per tile; each thread owns one pixel and walks the tile's splats in
 //     draw order (far to near), staged 256 at a time in shared memory.  For every fragment
 //     it evaluates the interpolated quad offset q, the discard test, the alpha of the display
@@ -15,6 +15,7 @@
 //     every fragment: d' = round(d·(1-α) + s·α) in units of 1/255.
 // Fragments whose alpha cannot move an 8-bit channel (see splat_r2_bound) lie outside the splat's
 // fragment box and are never visited; skipping them leaves every pixel bit-identical.
+#include <algorithm>
 #include <cstdlib>
 
 #include "gs_internal.h"
@@ -42,6 +43,9 @@ struct RasterLayout {
     uint32_t *order;     // tiles by descending pair count: the rasteriser's launch order (counting path)
     uint2 *sort_alt;     // the tile sort's ping-pong buffer, capacity max_pairs
     uint32_t tiles_x, tiles_y, ntiles, key_bits;
+    uint32_t value_bits;  // compact items (see launch_sort_items): bits of a pair value; 0: whole pairs
+    uint32_t *items() const { return reinterpret_cast<uint32_t *>(pairs); }
+    uint8_t *low(uint32_t max_pairs) const { return reinterpret_cast<uint8_t *>(pairs) + (size_t)max_pairs * 4; }
 };
 
 // Up to kCountTiles tiles (1080p has 8160), the emit kernel counts pairs per tile in shared
@@ -120,6 +124,9 @@ static RasterLayout raster_layout(void *scratch, uint32_t max_splats, uint32_t w
         p += align_up((size_t)kEmitBlocks * L.ntiles * 4, 256);
     }
     L.sort_alt = reinterpret_cast<uint2 *>(p);
+    // The counting path's tiles take two digits; their high digit leaves 26 bits or more for a value.
+    const uint32_t bits = bits_for(max_splats);
+    L.value_bits = L.counts && bits < 32 && tile_split(L.key_bits).bits[1] + bits <= 32 ? bits : 0u;
     return L;
 }
 
@@ -181,7 +188,9 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     const uint32_t n = count ? min(*count, max_count) : max_count;
     const uint32_t k = blockIdx.x * kBinThreads + threadIdx.x;
     if (k >= n) {
-        if (rects && k < max_count) rects[k] = kEmptyRect;
+        if (k >= max_count) return;
+        if (rects) rects[k] = kEmptyRect;
+        else if (!direct) counts[k] = 0u;  // several models: the scan covers every segment's capacity
         return;
     }
     // Indices come from the depth sort; the bound check only matters if that sort timed out.
@@ -213,9 +222,10 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
 }
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
-// the last tile records the segment's total.
+// the last tile records the pairs wanted and kept, and a list overflow.
 __global__ void __launch_bounds__(256) bin_scan_kernel(uint32_t *__restrict__ data, const uint32_t *count,
-                                                       uint32_t max_count, Ctrl *ctrl, uint64_t *flags) {
+                                                       uint32_t max_count, uint32_t max_pairs, Ctrl *ctrl,
+                                                       uint64_t *flags) {
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_tile, s_epoch, s_prefix, s_limit, s_stall;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -274,7 +284,11 @@ __global__ void __launch_bounds__(256) bin_scan_kernel(uint32_t *__restrict__ da
             const uint32_t sat = incl > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)incl;
             if (tile > 0) publish_flag(flags + tile, tile, s_stall, pack_flag(epoch, kFlagPrefix, sat));
             s_prefix = prefix;
-            if (tile == ntiles - 1) ctrl->seg_total = sat;
+            if (tile == ntiles - 1) {
+                ctrl->total = sat;
+                ctrl->count = min(sat, max_pairs);
+                if (sat > max_pairs) atomicOr(&ctrl->status, kStatusCapacity);
+            }
         }
     }
     __syncthreads();
@@ -316,101 +330,138 @@ __device__ __forceinline__ uint32_t kept_tile_place(uint32_t m, uint32_t w, uint
 }
 
 // K3c: every splat writes its (tile, value) pairs at its scanned offset, its kept tiles in
-// row-major order.  The 32 ranks of a warp own one contiguous run of pairs, and the warp writes
-// that run together: pair r of the run goes to lane r mod 32, which finds its splat by binary
-// search over the warp's exclusive count prefix and its tile from the pair's place in the
-// splat's rectangle (its kept tiles skip the dropped corners).  Stores are consecutive, every
-// lane has a pair in every round but the last, and one large splat is spread over the warp like
-// any other.  Also accumulates the tile counts (or the tile-key digit histograms of the tile
-// sort) in shared memory: each CTA loops over chunks of 256 ranks (grid-stride) and hands its
-// shared bins on once.
-template <bool COUNTS>
+// row-major order.  A warp takes an equal share of the pairs, not of the ranks: the nearest splats of
+// a close-up cover thousands of tiles each and lie next to one another in draw order (400k splats at
+// 1366x768 from inside the scene: 97 us by ranks, 16 by pairs).  It finds its first rank by a 32-way
+// search of the offsets, then goes through windows of 32 ranks: pair r of a window goes to lane r mod
+// 32, which finds its splat by binary search over the warp's exclusive count prefix and its tile from
+// the pair's place in the splat's rectangle (its kept tiles skip the dropped corners).  Stores are
+// consecutive.  Also accumulates the tile counts (or the tile-key digit histograms of the tile sort) in
+// shared memory; each CTA hands its shared bins on once.
+// COUNTS: one counter per tile, else the digit histograms; COMPACT: items and low digits, else pairs.
+constexpr uint32_t kEmitMin = 96;  // pairs of a warp's share at least (its search costs about 3 us)
+
+template <bool COUNTS, bool COMPACT>
 __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
     const uint4 *__restrict__ info, const uint32_t *__restrict__ offsets, const uint32_t *count, uint32_t max_count,
-    uint2 *__restrict__ pairs, uint32_t max_pairs, uint32_t tiles_x, uint32_t ntiles, const Ctrl *ctrl,
+    uint2 *__restrict__ pairs, uint32_t max_pairs, uint32_t value_bits, uint32_t tiles_x, uint32_t ntiles, Ctrl *ctrl,
     Ctrl *sort_ctrl, const PassSplit split, uint32_t *__restrict__ blockcounts) {
-    // COUNTS: one counter per tile; else the tile-key digit histograms of the tile sort
     extern __shared__ uint32_t s_bins[];
     const uint32_t nbins = COUNTS ? ntiles : 4u * 256u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
     const uint32_t n = count ? min(*count, max_count) : max_count;
+    const uint32_t total = ctrl->total;
+    // a scan that gave up leaves offsets nothing can be found by (status already set): emit nothing
+    const bool sound = !(*(volatile uint32_t *)&ctrl->status & kStatusTimeout);
     for (uint32_t i = tid; i < nbins; i += kBinThreads) s_bins[i] = 0u;
     __syncthreads();
-    const uint32_t seg_total = ctrl->seg_total;
-    const uint64_t pair_base = ctrl->pair_base;
-    auto emit = [&](uint32_t t, uint32_t value, uint64_t at) {
+    uint32_t *items = reinterpret_cast<uint32_t *>(pairs);
+    uint8_t *low = reinterpret_cast<uint8_t *>(pairs) + (size_t)max_pairs * 4u;
+    const uint32_t low_bits = split.bits[0], low_mask = (1u << low_bits) - 1u;
+    auto emit = [&](uint32_t t, uint32_t value, uint32_t at) {
         if (at < max_pairs) {
-            pairs[at] = make_uint2(t, value);
+            if constexpr (COMPACT) {
+                items[at] = ((t >> low_bits) << value_bits) | value;
+                low[at] = (uint8_t)(t & low_mask);
+            } else {
+                pairs[at] = make_uint2(t, value);
+            }
             if constexpr (COUNTS) {
                 if (t < ntiles) atomicAdd(&s_bins[t], 1u);
-                else atomicOr(&const_cast<Ctrl *>(ctrl)->status, kStatusBounds);
+                else atomicOr(&ctrl->status, kStatusBounds);
             } else {
                 for (uint32_t p = 0; p < split.n; ++p)
                     atomicAdd(&s_bins[p * 256u + ((t >> split.shift[p]) & ((1u << split.bits[p]) - 1u))], 1u);
             }
         }
     };
-    for (uint32_t k0 = blockIdx.x * kBinThreads; k0 < n; k0 += gridDim.x * kBinThreads) {
-        const uint32_t k = k0 + tid;
-        uint4 in = make_uint4(0u, 0u, 0u, 0u);
-        uint32_t cnt = 0;
-        uint64_t o = 0;
-        if (k < n) {
-            in = info[k];
-            const uint32_t off = offsets[k];
-            const uint32_t next = (k + 1 < n) ? offsets[k + 1] : seg_total;
-            cnt = next - off;
-            o = pair_base + off;
-            // A count beyond the splat's tile rectangle can only come from a scan whose
-            // look-back gave up (status already set): emit nothing for it.
-            if (next < off || cnt > (in.y & 0xFFFFu) * (in.y >> 16)) {
-                if (cnt) atomicOr(&const_cast<Ctrl *>(ctrl)->status, kStatusBounds);
-                cnt = 0;
+    const uint32_t warps = gridDim.x * (kBinThreads / 32u), w = blockIdx.x * (kBinThreads / 32u) + (tid >> 5);
+    const uint32_t share = max(kEmitMin, (uint32_t)(((uint64_t)total + warps - 1u) / warps));
+    const uint64_t first = (uint64_t)w * share;
+    if (sound && n > 0 && first < total) {
+        const uint32_t q0 = (uint32_t)first, q1 = (uint32_t)min((uint64_t)total, first + share);
+        // the last rank from lo on whose offset is at or before q (offsets[lo] is): the one that holds
+        // pair q, as ranks without pairs share the next one's offset
+        auto rank_of = [&](uint32_t q, uint32_t lo) {
+            uint32_t hi = n;
+            while (hi - lo > 1u) {
+                const uint32_t step = (hi - lo + 31u) / 32u, at = lo + lane * step;
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, at < hi && offsets[at] <= q);
+                lo += (m ? 31u - __clz(m) : 0u) * step;
+                hi = min(hi, lo + step);
             }
-        }
-        // warp-exclusive prefix of the counts: this lane's pairs are [excl, excl + cnt) of the run
-        uint32_t incl = cnt;
-#pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= d) incl += y;
-        }
-        const uint32_t excl = incl - cnt, run = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        // a lane's rectangle: x0 | y0 << 16, width, kept-tile mask, value, 1 / width
-        const uint32_t w = in.y & 0xFFFFu;
-        const float inv_w = w ? 1.0f / (float)w : 0.0f;
-        for (uint32_t r0 = 0; r0 < run; r0 += 32) {
-            const uint32_t r = r0 + lane;
-            // the largest lane whose run starts at or before r (a lane with no pairs shares its
-            // start with the next lane, so the search lands on a lane that has pairs)
-            uint32_t src = 0;
-#pragma unroll
-            for (uint32_t step = 16; step >= 1; step >>= 1) {
-                const uint32_t e = __shfl_sync(0xFFFFFFFFu, excl, src + step);
-                if (e <= r) src += step;
+            return lo;
+        };
+        uint32_t empty = 0;  // windows without pairs in a row
+        for (uint32_t k0 = rank_of(q0, 0); k0 < n; k0 += 32u) {
+            const uint32_t k = k0 + lane;
+            uint4 in = make_uint4(0u, 0u, 0u, 0u);
+            uint32_t from = q1, to = q1, off = q1;  // this rank's pairs of the warp's share
+            if (k < n) {
+                in = info[k];
+                off = offsets[k];
+                const uint32_t next = (k + 1 < n) ? offsets[k + 1] : total;
+                // A count beyond the splat's tile rectangle can only come from a bad scan: emit nothing for it.
+                if (next >= off && next - off <= (in.y & 0xFFFFu) * (in.y >> 16)) {
+                    from = min(max(off, q0), q1);
+                    to = min(max(next, q0), q1);
+                } else {
+                    atomicOr(&ctrl->status, kStatusBounds);
+                }
             }
-            const uint32_t sx = __shfl_sync(0xFFFFFFFFu, in.x, src), swh = __shfl_sync(0xFFFFFFFFu, in.y, src);
-            const uint32_t sw = swh & 0xFFFFu;  // in.y: w | h << 16
-            const uint32_t smask = __shfl_sync(0xFFFFFFFFu, in.z, src), sval = __shfl_sync(0xFFFFFFFFu, in.w, src);
-            const float sinv = __shfl_sync(0xFFFFFFFFu, inv_w, src);
-            const uint32_t sex = __shfl_sync(0xFFFFFFFFu, excl, src);
-            const uint32_t olo = __shfl_sync(0xFFFFFFFFu, (uint32_t)o, src);
-            const uint32_t ohi = __shfl_sync(0xFFFFFFFFu, (uint32_t)(o >> 32), src);
-            if (r < run) {
-                const uint32_t local = r - sex;
-                // in.z: tiles kept of a rectangle of at most 16 (bit ty·w + tx); 0 = all of it
-                const uint32_t pos = smask ? kept_tile_place(smask, sw, swh >> 16, local) : local;
-                // row = floor(pos / w), exact in float: pos < 2^24 and the error of 1/w is
-                // far below the 1/w gap between pos/w and the next integer
-                const uint32_t ty = (uint32_t)(((float)pos + 0.5f) * sinv), tx = pos - ty * sw;
-                const uint64_t at = (((uint64_t)ohi << 32) | olo) + local;
-                emit(((sx >> 16) + ty) * tiles_x + (sx & 0xFFFFu) + tx, sval, at);
+            const bool more = __shfl_sync(0xFFFFFFFFu, to, 31) < q1;
+            const uint32_t cnt = to - from;
+            // warp-exclusive prefix of the counts: this lane's pairs are [excl, excl + cnt) of the run
+            uint32_t incl = cnt;
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            const uint32_t excl = incl - cnt, run = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            // a lane's rectangle: x0 | y0 << 16, width, kept-tile mask, value, 1 / width
+            const uint32_t iw = in.y & 0xFFFFu;
+            const float inv_w = iw ? 1.0f / (float)iw : 0.0f;
+            for (uint32_t r0 = 0; r0 < run; r0 += 32) {
+                const uint32_t r = r0 + lane;
+                // the largest lane whose run starts at or before r (a lane with no pairs shares its
+                // start with the next lane, so the search lands on a lane that has pairs)
+                uint32_t src = 0;
+#pragma unroll
+                for (uint32_t step = 16; step >= 1; step >>= 1) {
+                    const uint32_t e = __shfl_sync(0xFFFFFFFFu, excl, src + step);
+                    if (e <= r) src += step;
+                }
+                const uint32_t sx = __shfl_sync(0xFFFFFFFFu, in.x, src), swh = __shfl_sync(0xFFFFFFFFu, in.y, src);
+                const uint32_t sw = swh & 0xFFFFu;  // in.y: w | h << 16
+                const uint32_t smask = __shfl_sync(0xFFFFFFFFu, in.z, src), sval = __shfl_sync(0xFFFFFFFFu, in.w, src);
+                const float sinv = __shfl_sync(0xFFFFFFFFu, inv_w, src);
+                const uint32_t at = __shfl_sync(0xFFFFFFFFu, from - excl, src) + r;
+                const uint32_t soff = __shfl_sync(0xFFFFFFFFu, off, src);
+                if (r < run) {
+                    const uint32_t local = at - soff;  // place among the splat's kept tiles
+                    // in.z: tiles kept of a rectangle of at most 16 (bit ty·w + tx); 0 = all of it
+                    const uint32_t pos = smask ? kept_tile_place(smask, sw, swh >> 16, local) : local;
+                    // row = floor(pos / w), exact in float: pos < 2^24 and the error of 1/w is
+                    // far below the 1/w gap between pos/w and the next integer
+                    const uint32_t ty = (uint32_t)(((float)pos + 0.5f) * sinv), tx = pos - ty * sw;
+                    emit(((sx >> 16) + ty) * tiles_x + (sx & 0xFFFFu) + tx, sval, at);
+                }
+            }
+            if (!more) break;
+            // a long stretch of ranks without pairs (another model's unused capacity, splats outside the
+            // target) is passed over by another search
+            empty = run ? 0u : empty + 1u;
+            if (empty == 4u) {
+                empty = 0;
+                const uint32_t here = __shfl_sync(0xFFFFFFFFu, to, 31), at = k0 + 31u;
+                k0 = max(k0, rank_of(here, at) - 32u);  // at + 1 <= the rank found, or no rank is left
             }
         }
     }
     __syncthreads();
     if constexpr (COUNTS) {
-        // every CTA of the grid writes its slice (zeros when it had no ranks): plain stores,
+        // every CTA of the grid writes its slice (zeros when it had no pairs): plain stores,
         // summed per tile by tile_count_kernel
         uint32_t *dst = blockcounts + (size_t)blockIdx.x * ntiles;
         for (uint32_t t = tid; t < ntiles; t += kBinThreads) dst[t] = s_bins[t];
@@ -420,6 +471,18 @@ __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
             if (v) atomicAdd(&sort_ctrl->hist[p][tid], v);
         }
     }
+}
+
+// Starts a raster call: its control block and the tile sort's (CTA 0), the tile counts cleared by the
+// other CTAs.
+__global__ void __launch_bounds__(256) raster_init_kernel(Ctrl *ctrl, Ctrl *sort_ctrl, uint32_t arena_words, WaitCfg cfg,
+                                                          uint32_t *counts, uint32_t ntiles) {
+    if (blockIdx.x == 0) {
+        ctrl_reset(ctrl, ctrl, arena_words, cfg);
+        ctrl_reset(sort_ctrl, ctrl, kKeepArena, cfg);
+        return;
+    }
+    for (uint32_t t = (blockIdx.x - 1u) * 1024u + threadIdx.x, e = min(ntiles, blockIdx.x * 1024u); t < e; t += 256u) counts[t] = 0u;
 }
 
 // Per-tile pair counts of one segment (the sum over the emit CTAs), added to the running
@@ -450,33 +513,40 @@ __device__ __forceinline__ uint32_t order_class(uint32_t c) {
     return 1u + 2u * lg + (lg > 0 ? (c >> (lg - 1u)) & 1u : 0u);
 }
 
-// [start, end) of every tile from the per-tile counts (exclusive scan; one CTA, 8 tiles a
-// thread), the tile sort's digit offsets (exclusive scans of the digit histograms, which are sums
-// of those counts), and the rasteriser's
-// launch order: tiles by descending size class (a counting sort), so the longest lists start
-// first and the grid does not end on a few long tiles that started late.  The order inside a
-// class is whatever the shared atomics give; it only schedules CTAs, every tile's pixels are
-// the same in any order.
+// [start, end) of every tile from the per-tile counts (exclusive scan; one CTA, 8 consecutive tiles a
+// thread), the tile sort's exclusive digit offsets, and the rasteriser's launch order: tiles by
+// descending size class (a counting sort), so the longest lists start first and the grid does not end
+// on a few long tiles that started late.  The order inside a class is whatever the shared atomics give;
+// it only schedules CTAs, every tile's pixels are the same in any order.
+// One SM's load and store slots bound it, so all global traffic is coalesced through shared memory; the
+// high digit's offsets are the scan's values at its first tiles, the low digit's counts strided sums, a
+// class takes one atomic a warp, and the class starts one warp's scan (10.7 us at 8160 tiles against 14.5
+// with strided accesses, an atomic per tile and digit and a serial walk over the classes).
+constexpr uint32_t kScanTilesMax = 8192;
+static_assert(kCountTiles <= kScanTilesMax, "8 tiles a thread");
 __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restrict__ counts, uint32_t ntiles,
                                                          uint2 *__restrict__ ranges, uint32_t *__restrict__ order,
                                                          Ctrl *sort_ctrl, const PassSplit split) {
-    __shared__ uint32_t s_w[32];
-    __shared__ uint32_t s_h[4][256];
-    __shared__ uint32_t s_cls[kOrderClasses];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    (&s_h[0][0])[tid] = 0u;
-    if (tid < kOrderClasses) s_cls[tid] = 0u;
+    __shared__ __align__(16) uint32_t s_v[kScanTilesMax + 4];
+    __shared__ uint32_t s_w[32], s_low[1024], s_lw[10], s_cls[96];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = lanemask_lt();
+    if (tid < 96u) s_cls[tid] = 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        const uint32_t t = tid + 1024u * j;
+        s_v[t] = t < ntiles ? counts[t] : 0u;
+    }
     __syncthreads();
     const uint32_t base = tid * 8u;
     uint32_t v[8], sum = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < 8; ++j) {
-        v[j] = base + j < ntiles ? counts[base + j] : 0u;
-        sum += v[j];
-        if (base + j < ntiles) atomicAdd(&s_cls[order_class(v[j])], 1u);
-        if (v[j])
-            for (uint32_t p = 0; p < split.n; ++p)
-                atomicAdd(&s_h[p][((base + j) >> split.shift[p]) & ((1u << split.bits[p]) - 1u)], v[j]);
+    for (uint32_t j = 0; j < 8; j += 4) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(&s_v[base + j]);
+        v[j] = x.x;
+        v[j + 1] = x.y;
+        v[j + 2] = x.z;
+        v[j + 3] = x.w;
+        sum += (x.x + x.y) + (x.z + x.w);
     }
     uint32_t inc = sum;
 #pragma unroll
@@ -486,6 +556,22 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restr
     }
     if (lane == 31) s_w[warp] = inc;
     __syncthreads();
+    // a tile's place in its class: the warp's tiles of the class together
+    uint32_t place[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        const bool in = base + j < ntiles;
+        const uint32_t cls = in ? order_class(v[j]) : kOrderClasses;  // past the tiles: a class of its own
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
+        uint32_t at = 0;
+        if ((peers & lt) == 0u) at = atomicAdd(&s_cls[cls], (uint32_t)__popc(peers));
+        place[j] = __shfl_sync(0xFFFFFFFFu, at, __ffs(peers) - 1) + __popc(peers & lt);
+    }
+    // low digit: thread (part, d) sums every parts-th of the digit's tiles
+    const uint32_t lows = 1u << split.bits[0], parts = 1024u / lows, d = tid & (lows - 1u), part = tid >> split.bits[0];
+    uint32_t low = 0;
+    for (uint32_t t = part * lows + d; t < ntiles; t += 1024u) low += s_v[t];
+    s_low[tid] = low;
     if (warp == 0) {
         uint32_t x = s_w[lane], xi = x;
 #pragma unroll
@@ -495,52 +581,69 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restr
         }
         s_w[lane] = xi - x;  // exclusive over warps
     }
-    if (tid == 32) {  // first position of each size class, largest class first
-        uint32_t at = 0;
-        for (int c = (int)kOrderClasses - 1; c >= 0; --c) {
-            const uint32_t k = s_cls[c];
-            s_cls[c] = at;
-            at += k;
+    __syncthreads();
+    if (warp == 1) {  // first place of each size class, largest class first: lane l takes classes 65 - 3l ..
+        uint32_t c[3], s = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) {
+            const int k = (int)kOrderClasses - 1 - 3 * (int)lane - (int)j;
+            c[j] = k >= 0 ? s_cls[k] : 0u;
+            s += c[j];
+        }
+        uint32_t xi = s;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, xi, o);
+            if (lane >= o) xi += y;
+        }
+        uint32_t at = xi - s;
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) {
+            const int k = (int)kOrderClasses - 1 - 3 * (int)lane - (int)j;
+            if (k >= 0) s_cls[k] = at;
+            at += c[j];
         }
     }
+    uint32_t before = 0;  // low digits' exclusive offsets: warps 2 to 9, a digit a thread
+    if (warp >= 2 && warp < 10) {
+        const uint32_t q = tid - 64u;
+        uint32_t x = 0;
+        if (q < lows)
+            for (uint32_t p = 0; p < parts; ++p) x += s_low[p * lows + q];
+        uint32_t xi = x;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, xi, o);
+            if (lane >= o) xi += y;
+        }
+        before = xi - x;
+        if (lane == 31) s_lw[warp] = xi;
+    }
     __syncthreads();
+    if (warp >= 2 && warp < 10 && tid - 64u < lows) {
+        for (uint32_t w = 2; w < warp; ++w) before += s_lw[w];
+        sort_ctrl->hist[0][tid - 64u] = before;
+    }
     uint32_t run = s_w[warp] + inc - sum;
+    // the starts take the counts' place (everybody is past reading them), then the order the starts'
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) {
-        if (base + j < ntiles) {
-            ranges[base + j] = make_uint2(run, run + v[j]);
-            order[atomicAdd(&s_cls[order_class(v[j])], 1u)] = base + j;
-        }
+        const uint32_t t = base + j;
+        s_v[t] = run;
+        // the first tile of a high digit: the pairs before it
+        if (t < ntiles && (t & (lows - 1u)) == 0u) sort_ctrl->hist[1][t >> split.shift[1]] = run;
+        place[j] += t < ntiles ? s_cls[order_class(v[j])] : 0u;
         run += v[j];
     }
-    // the tile sort's digit offsets: per pass (256 threads each), the exclusive scan of its counts
-    __shared__ uint32_t s_hw[32];
-    const uint32_t p = tid >> 8, d = tid & 255u;
-    const uint32_t hv = s_h[p][d];
-    uint32_t hx = hv;
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, hx, o);
-        if (lane >= o) hx += y;
-    }
-    if (lane == 31) s_hw[warp] = hx;
+    if (tid == 1023u) s_v[kScanTilesMax] = run;
     __syncthreads();
-    uint32_t hpre = 0;
-    for (uint32_t w = p * 8u; w < warp; ++w) hpre += s_hw[w];
-    if (p < split.n) sort_ctrl->hist[p][d] = hpre + hx - hv;
-}
-
-// K3d: advance the running pair base past a segment; flags a tile-pair list overflow.
-__global__ void bin_advance_kernel(Ctrl *ctrl, const uint32_t *count, uint32_t max_count, uint32_t max_pairs) {
-    const uint32_t n = count ? min(*count, max_count) : max_count;
-    const uint64_t seg = n ? ctrl->seg_total : 0u;
-    const uint64_t want = (uint64_t)ctrl->total + seg;
-    const uint32_t sat = want > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)want;
-    const uint32_t kept = sat > max_pairs ? max_pairs : sat;
-    if (sat > max_pairs) ctrl->status |= kStatusCapacity;
-    ctrl->total = sat;
-    ctrl->count = kept;
-    ctrl->pair_base = kept;
+    for (uint32_t t = tid; t < ntiles; t += 1024u) ranges[t] = make_uint2(s_v[t], s_v[t + 1]);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j)
+        if (base + j < ntiles) s_v[place[j]] = base + j;
+    __syncthreads();
+    for (uint32_t t = tid; t < ntiles; t += 1024u) order[t] = s_v[t];
 }
 
 // [start, end) of every tile's run in the tile-sorted pairs; each thread checks four
@@ -573,9 +676,6 @@ __global__ void tile_ranges_kernel(const uint2 *__restrict__ pairs, const Ctrl *
         }
     }
 }
-
-// The tile sort keeps its own control block; fold its status bits into the raster's.
-__global__ void merge_status_kernel(Ctrl *dst, const Ctrl *src) { dst->status |= src->status; }
 
 // exp(x) on [-9, 0] by the SFU: what __expf computes, without its handling of denormal arguments
 // and results (an argument that small flushes to 0, whose exp is the same 1).
@@ -638,12 +738,12 @@ struct RasterShared {
 // an entry is waited for while the warps blend.
 struct ChunkSource {
     const gs_splat *__restrict__ splats;
-    const uint2 *__restrict__ pairs;  // the tile's own list
-    uint32_t max_splats;
+    const uint32_t *__restrict__ values;  // the tile's own list (RasterJob::values)
+    uint32_t value_shift, max_splats;
     uint32_t value;  // pair value of the chunk after the one in flight
 
     __device__ __forceinline__ uint32_t pair_value(uint32_t base, uint32_t cnt) const {
-        return threadIdx.x < cnt ? pairs[base + threadIdx.x].y : 0xFFFFFFFFu;
+        return threadIdx.x < cnt ? values[(size_t)(base + threadIdx.x) << value_shift] : 0xFFFFFFFFu;
     }
 
     __device__ __forceinline__ void fetch(RasterShared &S, uint32_t k) const {
@@ -703,7 +803,7 @@ struct ChunkSource {
     template <uint32_t MODE>
     __device__ __forceinline__ void stage_only(RasterShared &S, uint32_t n, float std2) const {
         if (threadIdx.x >= n) return;
-        const uint32_t k = pairs[threadIdx.x].y;
+        const uint32_t k = pair_value(0, n);
         float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
         if (k < max_splats) {
             const float4 *s = reinterpret_cast<const float4 *>(splats + k);
@@ -858,7 +958,7 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL>
 __device__ __forceinline__ void raster_tile(
-    RasterShared &S, const RasterJob &J, const uint2 *__restrict__ list, uint32_t n, float std2, float outline2,
+    RasterShared &S, const RasterJob &J, const uint32_t *__restrict__ list, uint32_t list_shift, uint32_t n, float std2, float outline2,
     uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
     // Work tallies of the counting variant (profiling only): fragment evaluations, alphas,
     // channel-triple blends and transmittance updates.
@@ -871,7 +971,7 @@ __device__ __forceinline__ void raster_tile(
     const float bx0 = (float)wx0 + 0.5f, bx1 = (float)wx0 + 7.5f;
     const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 3.5f;
     float d[3] = {0.0f, 0.0f, 0.0f};
-    ChunkSource src{J.splats, list, J.max_splats, 0u};
+    ChunkSource src{J.splats, list, list_shift, J.max_splats, 0u};
     constexpr uint32_t C = kRasterThreads;
     // the chunk before list position `end` (for walks from the end of the list)
     auto below = [](uint32_t end) { return end > C ? end - C : 0u; };
@@ -1051,6 +1151,12 @@ __device__ __forceinline__ void raster_tile(
 }
 
 
+// The tile sort keeps its own control block: one thread of a view's rasteriser folds its status into the
+// raster's.
+__device__ __forceinline__ void merge_status(const RasterJob &J) {
+    if (const uint32_t s = J.sort_ctrl->status) atomicOr(&J.ctrl->status, s);
+}
+
 // The tile's run of the tile-sorted pairs; empty (and reported) when a scan that gave up left it
 // outside the list.
 __device__ __forceinline__ uint2 tile_range(const RasterJob &J, uint32_t tile) {
@@ -1068,9 +1174,11 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(con
                                                                 uint32_t suffix_min, float eps,
                                                                 unsigned long long *counters) {
     __shared__ RasterShared S;
+    if (blockIdx.x == 0 && threadIdx.x == 0) merge_status(J);
     const uint32_t tile = J.order ? J.order[blockIdx.x] : blockIdx.x;
     const uint2 r = tile_range(J, tile);
-    raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J, J.pairs + r.x, r.y - r.x, std2, outline2, suffix_min, eps,
+    raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J, J.values + ((size_t)r.x << J.value_shift), J.value_shift,
+                                                          r.y - r.x, std2, outline2, suffix_min, eps,
                                                           counters, tile);
 }
 
@@ -1082,7 +1190,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(con
 template <uint32_t MODE, bool PORTABLE_EXP, bool FEW>
 __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     raster_direct_kernel(const RasterJob J, const uint32_t *__restrict__ rects, const uint4 *__restrict__ info,
-                         uint32_t ranks, uint32_t shift, uint2 *__restrict__ pairs, uint32_t max_pairs, float std2,
+                         uint32_t ranks, uint32_t shift, uint32_t *__restrict__ values, uint32_t max_pairs, float std2,
                          float outline2, uint32_t suffix_min, float eps) {
     __shared__ RasterShared S;
     __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;
@@ -1146,10 +1254,10 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     } else {
         uint32_t at = base + before + incl - sum;
         for (uint32_t q = first; q < last; ++q)
-            for (uint32_t m = hits[q]; m; m &= m - 1u) pairs[at++] = make_uint2(tile, info[32u * q + __ffs(m) - 1u].w);
+            for (uint32_t m = hits[q]; m; m &= m - 1u) values[at++] = info[32u * q + __ffs(m) - 1u].w;
     }
     __syncthreads();
-    raster_tile<MODE, PORTABLE_EXP, false, FEW ? 4u : 1u>(S, J, pairs + base, n, std2, outline2, suffix_min, eps, nullptr,
+    raster_tile<MODE, PORTABLE_EXP, false, FEW ? 4u : 1u>(S, J, values + base, 0u, n, std2, outline2, suffix_min, eps, nullptr,
                                                           tile);
 }
 
@@ -1169,8 +1277,10 @@ __global__ void __launch_bounds__(kRasterThreads, 6) raster_views_kernel(const R
     }
     const RasterJob &J = jobs[lo];
     const uint32_t b = blockIdx.x - tile_base[lo], tile = J.order ? J.order[b] : b;
+    if (b == 0 && threadIdx.x == 0) merge_status(J);
     const uint2 r = tile_range(J, tile);
-    raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J, J.pairs + r.x, r.y - r.x, std2, outline2, suffix_min, eps, nullptr,
+    raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J, J.values + ((size_t)r.x << J.value_shift), J.value_shift,
+                                                          r.y - r.x, std2, outline2, suffix_min, eps, nullptr,
                                                tile);
 }
 
@@ -1229,7 +1339,7 @@ static void launch_raster_views_mode(const RasterJob *jobs, const uint32_t *tile
 }
 
 RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, uint32_t W, uint32_t H,
-                     uint32_t pitch, uint32_t max_pairs, void *scratch) {
+                     uint32_t pitch, uint32_t max_pairs, void *scratch, bool segmented) {
     uint32_t max_splats = 0;
     for (uint32_t s = 0; s < nseg; ++s) max_splats += segs[s].max_count;
     const RasterLayout L = raster_layout(scratch, max_splats, W, H, max_pairs);
@@ -1237,7 +1347,9 @@ RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, 
     // Pair values index the model's own splat array (one segment) or the draw-ordered copy.
     J.splats = nseg == 1 ? segs[0].splats : L.sorted;
     J.max_splats = nseg == 1 ? segs[0].max_count : max_splats;
-    J.pairs = L.pairs;
+    const bool compact = L.value_bits && !segmented;  // else the value is a pair's second word
+    J.values = L.items() + (compact ? 0 : 1);
+    J.value_shift = compact ? 0u : 1u;
     J.ranges = L.ranges;
     J.order = L.order;
     J.target = target;
@@ -1247,6 +1359,7 @@ RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, 
     J.tiles_x = L.tiles_x;
     J.ntiles = L.ntiles;
     J.ctrl = L.ctrl;
+    J.sort_ctrl = L.sort_ctrl;
     return J;
 }
 
@@ -1279,73 +1392,61 @@ cudaError_t launch_raster_views(const RasterJob *jobs_dev, const uint32_t *tile_
 }
 
 cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint32_t W,
-                           uint32_t H, uint32_t max_pairs, void *scratch, cudaStream_t st) {
+                                 uint32_t H, uint32_t max_pairs, void *scratch, cudaStream_t st, bool segmented) {
     uint32_t max_splats = 0;
     for (uint32_t s = 0; s < nseg; ++s) max_splats += segs[s].max_count;
     const RasterLayout L = raster_layout(scratch, max_splats, W, H, max_pairs);
     if (L.ntiles == 0) return cudaSuccess;
     // The first segment with splats clears the arena in its bin_count launch; with none, no kernel
     // reads a flag and the arena mark stays.
-    bool any = false;
-    for (uint32_t s = 0; s < nseg; ++s) any = any || segs[s].max_count > 0;
-    const WaitCfg cfg = wait_config();
-    ctrl_init_kernel<<<1, 256, 0, st>>>(L.ctrl, 1, nullptr, any ? L.arena_words : kKeepArena, cfg);
-    count_launches(1);
-    cudaError_t e = sort_pairs_begin(L.sort_ctrl, L.ctrl, st);
-    if (e != cudaSuccess) return e;
-    Ctrl *sort_ctrl = L.sort_ctrl;
-    if (L.counts) {
-        e = cudaMemsetAsync(L.counts, 0, (size_t)L.ntiles * 4, st);
-        if (e != cudaSuccess) return e;
-    }
-    const PassSplit split = tile_split(L.key_bits);
-    // The emit kernel loops over its ranks grid-stride with equal shares per CTA: one resident
-    // wave (at most kEmitBlocks, the per-CTA count area) keeps a second, late wave from
-    // doubling the kernel's span.
-    const size_t emit_smem = L.counts ? (size_t)L.ntiles * 4u : 4u * 256u * 4u;
-    uint32_t emit_wave = L.counts ? resident_ctas(bin_emit_kernel<true>, kBinThreads, emit_smem)
-                                  : resident_ctas(bin_emit_kernel<false>, kBinThreads, emit_smem);
-    if (emit_wave == 0 || emit_wave > kEmitBlocks) emit_wave = kEmitBlocks;
-    uint32_t rank_offset = 0;
-    bool cleared = false;
     prof_mark(kProfBin, true, st);
+    raster_init_kernel<<<1 + (L.counts ? (L.ntiles + 1023) / 1024 : 0), 256, 0, st>>>(
+        L.ctrl, L.sort_ctrl, max_splats ? L.arena_words : kKeepArena, wait_config(), L.counts, L.ntiles);
+    count_launches(1);
+    const PassSplit split = tile_split(L.key_bits);
     const int direct = nseg == 1 ? 1 : 0;
+    uint32_t rank_offset = 0;
     for (uint32_t s = 0; s < nseg; ++s) {
         const RasterSegment &g = segs[s];
         const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
         if (blocks == 0) continue;
-        if (s > 0) {
-            ctrl_init_kernel<<<1, 32, 0, st>>>(L.ctrl, 0, nullptr, kKeepArena, cfg);
-            count_launches(1);
-        }
         // a stored tile record is only for the target the preprocess was given (one model)
         const uint4 *binfo = direct && g.binfo && g.binfo_w == W && g.binfo_h == H ? g.binfo : nullptr;
-        bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(g.splats, binfo, g.sorted_index, g.count, g.max_count,
-                                                         rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y,
-                                                         u.display_mode, u.std_dev * u.std_dev, L.info, L.offsets,
-                                                         L.ctrl, cleared ? nullptr : L.flags, nullptr, 0, nullptr, 0);
-        cleared = true;
-        const uint32_t scan_blocks = (g.max_count + kScanTile - 1) / kScanTile;
-        bin_scan_kernel<<<scan_blocks, 256, 0, st>>>(L.offsets, g.count, g.max_count, L.ctrl, L.flags);
-        const uint32_t eblocks = blocks < emit_wave ? blocks : emit_wave;
-        if (L.counts) {
-            bin_emit_kernel<true><<<eblocks, kBinThreads, emit_smem, st>>>(
-                L.info, L.offsets, g.count, g.max_count, L.pairs, max_pairs, L.tiles_x, L.ntiles, L.ctrl, sort_ctrl,
-                split, L.blockcounts);
-            tile_count_kernel<<<dim3((L.ntiles + 255) / 256, kCountSlices), 256, 0, st>>>(L.blockcounts, eblocks,
-                                                                                         L.ntiles, L.counts);
-            count_launches(1);
-        } else {
-            bin_emit_kernel<false><<<eblocks, kBinThreads, emit_smem, st>>>(
-                L.info, L.offsets, g.count, g.max_count, L.pairs, max_pairs, L.tiles_x, L.ntiles, L.ctrl, sort_ctrl,
-                split, nullptr);
-        }
-        bin_advance_kernel<<<1, 1, 0, st>>>(L.ctrl, g.count, g.max_count, max_pairs);
-        count_launches(4);
+        bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(
+            g.splats, binfo, g.sorted_index, g.count, g.max_count, rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y,
+            u.display_mode, u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
+            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0);
+        count_launches(1);
         rank_offset += g.max_count;
     }
+    // All ranks at once from here on: one segment's live ones, or every segment up to its capacity
+    // (ranks without a splat have no tiles).
+    const uint32_t *count = direct ? segs[0].count : nullptr;
+    if (max_splats) {
+        bin_scan_kernel<<<(max_splats + kScanTile - 1) / kScanTile, 256, 0, st>>>(L.offsets, count, max_splats, max_pairs,
+                                                                                L.ctrl, L.flags);
+        count_launches(1);
+    }
+    // One resident wave at most (and the per-CTA count area): a second, late wave would stretch the
+    // kernel; two CTAs an SM at least, as few splats may cover many tiles.
+    const size_t emit_smem = L.counts ? (size_t)L.ntiles * 4u : 4u * 256u * 4u;
+    const bool compact = L.value_bits && !segmented;
+    auto emit = [&](auto kernel) {
+        uint32_t wave = resident_ctas(kernel, kBinThreads, emit_smem);
+        if (wave == 0 || wave > kEmitBlocks) wave = kEmitBlocks;
+        const uint32_t want = std::max((max_splats + kBinThreads - 1) / kBinThreads, 304u), grid = std::min(want, wave);
+        kernel<<<grid, kBinThreads, emit_smem, st>>>(L.info, L.offsets, count, max_splats, L.pairs, max_pairs, L.value_bits,
+                                                     L.tiles_x, L.ntiles, L.ctrl, L.sort_ctrl, split, L.blockcounts);
+        return grid;
+    };
     if (L.counts) {
-        tile_scan_kernel<<<1, 1024, 0, st>>>(L.counts, L.ntiles, L.ranges, L.order, sort_ctrl, split);
+        const uint32_t grid = compact ? emit(bin_emit_kernel<true, true>) : emit(bin_emit_kernel<true, false>);
+        tile_count_kernel<<<dim3((L.ntiles + 255) / 256, kCountSlices), 256, 0, st>>>(L.blockcounts, grid, L.ntiles,
+                                                                                     L.counts);
+        tile_scan_kernel<<<1, 1024, 0, st>>>(L.counts, L.ntiles, L.ranges, L.order, L.sort_ctrl, split);
+        count_launches(3);
+    } else {
+        emit(bin_emit_kernel<false, false>);
         count_launches(1);
     }
     prof_mark(kProfBin, false, st);
@@ -1411,12 +1512,14 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
     if (e != cudaSuccess) return e;
     prof_mark(kProfTileSort, true, st);
     // counting path: tile_scan wrote the digit offsets already scanned; else the emit's counts
-    e = launch_sort_pairs(L.pairs, max_pairs, &L.ctrl->count, L.key_bits, L.sort_ctrl, L.sort_flags, L.sort_alt, st,
-                          L.counts != nullptr);
+    if (L.value_bits)
+        e = launch_sort_items(L.items(), L.low(max_pairs), reinterpret_cast<uint32_t *>(L.sort_alt), max_pairs,
+                              &L.ctrl->count, L.key_bits, L.value_bits, L.sort_ctrl, L.sort_flags, st);
+    else
+        e = launch_sort_pairs(L.pairs, max_pairs, &L.ctrl->count, L.key_bits, L.sort_ctrl, L.sort_flags, L.sort_alt, st,
+                              L.counts != nullptr);
     prof_mark(kProfTileSort, false, st);
     if (e != cudaSuccess) return e;
-    merge_status_kernel<<<1, 1, 0, st>>>(L.ctrl, L.sort_ctrl);
-    count_launches(1);
     return launch_binning_ranges(segs, nseg, W, H, max_pairs, scratch, st);
 }
 
@@ -1435,7 +1538,7 @@ static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32
                                uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
     const bool few = tiles_at_once <= kFewTiles;
     auto go = [&](auto kernel) {
-        kernel<<<J.ntiles, kRasterThreads, 0, st>>>(J, L.offsets, L.info, ranks, shift, L.pairs, max_pairs, std2, outline2,
+        kernel<<<J.ntiles, kRasterThreads, 0, st>>>(J, L.offsets, L.info, ranks, shift, L.items(), max_pairs, std2, outline2,
                                                     t.suffix_min, t.eps);
     };
     if (exact) few ? go(raster_direct_kernel<MODE, true, true>) : go(raster_direct_kernel<MODE, true, false>);

@@ -31,8 +31,8 @@ constexpr uint32_t kSortCtasPerSm = 2;
 constexpr size_t kSortDynSmem = (size_t)kTileKeys * sizeof(uint2);
 static_assert(kTileKeys % GS_SORT_BLOCK_KVS == 0, "a pass block covers whole blocks of the reference");
 
-__global__ void ctrl_init_kernel(Ctrl *ctrl, int mode, Ctrl *owner, uint32_t arena_words, WaitCfg cfg) {
-    ctrl_reset(ctrl, mode, owner ? owner : ctrl, arena_words, cfg);
+__global__ void ctrl_init_kernel(Ctrl *ctrl, uint32_t arena_words, WaitCfg cfg) {
+    ctrl_reset(ctrl, ctrl, arena_words, cfg);
 }
 
 __device__ __forceinline__ uint32_t load_count(const uint32_t *count, uint32_t max_count) {
@@ -65,6 +65,24 @@ __device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t *tmp, u
     *total = tmp[WARPS - 1];
     __syncthreads();
     return before + x - v;
+}
+
+// The lanes of the warp whose digit d (below 2^bits, bits <= 8) equals the caller's: one ballot a digit
+// bit.  Ballots of bits above the digit, zero in every lane, change nothing; up to bit 5 they cost less
+// than asking.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, uint32_t bits) {
+    uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t b = 0; b < 8; ++b) {
+        if (b >= 6 && b >= bits) break;
+        uint32_t bal;
+        asm volatile("{\n\t.reg .pred p;\n\tand.b32 %0, %1, %2;\n\tsetp.ne.u32 p, %0, 0;\n\t"
+                     "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
+                     : "=r"(bal)
+                     : "r"(d), "r"(1u << b));
+        peers &= bal;
+    }
+    return peers;
 }
 
 // Global digit histograms of all passes in one read of the keys (four keys per thread and
@@ -257,22 +275,9 @@ __device__ __forceinline__ void sort_pass_block(
 #pragma unroll
     for (uint32_t i = 0; i < kSortRows; ++i) {
         const uint32_t d = (k[i] >> shift) & dmask;
-        uint32_t peers = 0xFFFFFFFFu;
-        if constexpr (MATCH) {
-            peers = __match_any_sync(0xFFFFFFFFu, d);
-        } else {
-#pragma unroll
-            for (uint32_t b = 0; b < 8; ++b) {
-                // bits above the digit are zero in every key: a ballot of them changes nothing, and
-                // up to bit 5 it costs less than asking
-                if (b >= 6 && b >= digit_bits) break;
-                uint32_t bal;
-                asm volatile("{\n\t.reg .pred p;\n\tand.b32 %0, %1, %2;\n\tsetp.ne.u32 p, %0, 0;\n\t"
-                             "vote.sync.ballot.b32 %0, p, 0xffffffff;\n\t@!p not.b32 %0, %0;\n\t}"
-                             : "=r"(bal) : "r"(d), "r"(1u << b));
-                peers &= bal;
-            }
-        }
+        uint32_t peers;
+        if constexpr (MATCH) peers = __match_any_sync(0xFFFFFFFFu, d);
+        else peers = digit_peers(d, digit_bits);
         const uint32_t rank = __popc(peers & lt);
         const uint32_t pre = s_whist[warp][d];
         __syncwarp();
@@ -359,6 +364,120 @@ __device__ __forceinline__ void sort_pass_block(
         for (uint32_t i = 0; i < kSortRows; ++i) put(tid + i * kSortThreads, s_kv[tid + i * kSortThreads]);
     } else {
         for (uint32_t j = tid; j < valid; j += kSortThreads) put(j, s_kv[j]);
+    }
+}
+
+// ---- tile sort on compact items ---------------------------------------------------------------
+// A pair whose tile id has its low digit taken away fits one word: high digit above the value.  The
+// emission writes that word and the low digit as a byte; the first pass sorts words by the bytes, and
+// as its output is grouped by the low digit, nobody needs it again; the second sorts by the words' high
+// digit and writes the values alone, all that the rasteriser reads of a pair.  5 + 4 + 4 + 4 bytes a
+// pair instead of 8 each time, half the registers and shared memory of a pair block (three CTAs an
+// SM), and no key to decode twice.
+constexpr uint32_t kItemCtasPerSm = 3;
+template <bool FIRST>
+constexpr size_t kItemDynSmem = kTileKeys * sizeof(uint32_t) + (FIRST ? kTileKeys : 0);
+
+template <bool FIRST>
+__global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
+    tile_pass_kernel(const uint32_t *__restrict__ in, const uint8_t *__restrict__ low, uint32_t *__restrict__ out,
+                     const uint32_t *count, uint32_t max_count, uint32_t hoff, uint32_t value_bits,
+                     uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags) {
+    extern __shared__ __align__(16) uint8_t item_smem[];
+    uint32_t *s_item = reinterpret_cast<uint32_t *>(item_smem);
+    uint8_t *s_low = item_smem + kTileKeys * sizeof(uint32_t);  // FIRST: the digit of each reordered item
+    __shared__ uint32_t s_whist[kSortWarps][256];
+    __shared__ uint32_t s_start[256];
+    __shared__ uint32_t s_gbase[256];
+    __shared__ uint32_t s_tmp[kSortWarps];
+    __shared__ uint32_t s_epoch, s_limit, s_stall;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t n = load_count(count, max_count), tile = blockIdx.x;  // arrives while the counters are cleared
+    if (tid == 0) {
+        s_epoch = *(volatile uint32_t *)&ctrl->epoch;
+        s_limit = ctrl->spin_limit;
+        s_stall = ctrl->stall_tile;
+    }
+    for (uint32_t k = tid; k < kSortWarps * 256; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
+    const uint32_t ntiles = (n + kTileKeys - 1) / kTileKeys;
+    if (tile >= ntiles) return;
+    __syncthreads();
+    const uint32_t epoch = s_epoch, dmask = (1u << digit_bits) - 1u;
+    const uint32_t base = tile * kTileKeys + warp * (32u * kSortRows);
+
+    uint32_t k[kSortRows], r[kSortRows];  // the item; its rank among the warp's of its digit (FIRST: | digit << 16)
+#pragma unroll
+    for (uint32_t i = 0; i < kSortRows; ++i) {
+        const uint32_t pos = base + i * 32u + lane;
+        const bool ok = pos < n;  // padding sorts last, in the largest digit
+        k[i] = ok ? in[pos] : 0xFFFFFFFFu;
+        if constexpr (FIRST) r[i] = ok ? low[pos] : dmask;
+    }
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (uint32_t i = 0; i < kSortRows; ++i) {
+        const uint32_t d = FIRST ? r[i] : (k[i] >> value_bits) & dmask;
+        const uint32_t peers = digit_peers(d, digit_bits);
+        const uint32_t rank = __popc(peers & lt);
+        const uint32_t pre = s_whist[warp][d];
+        __syncwarp();
+        if (rank == 0) s_whist[warp][d] = pre + __popc(peers);
+        __syncwarp();
+        r[i] = pre + rank + (FIRST ? d << 16 : 0u);
+    }
+    __syncthreads();
+
+    // As sort_pass_block: thread d < 256 owns digit d.
+    const uint32_t d = tid;
+    const bool owner = d < 256u, live = d <= dmask;
+    uint32_t total = 0;
+    if (owner) {
+#pragma unroll
+        for (uint32_t w = 0; w < kSortWarps; ++w) {
+            const uint32_t c = s_whist[w][d];
+            s_whist[w][d] = total;
+            total += c;
+        }
+    }
+    const uint32_t invalid = (tile == ntiles - 1) ? ntiles * kTileKeys - n : 0u;
+    const uint32_t pub = (d == dmask) ? total - invalid : total;
+    const uint32_t fstride = dmask + 1u;
+    uint64_t *f = flags + (size_t)tile * fstride + d;
+    if (live) publish_flag(f, tile, s_stall, pack_flag(epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, pub));
+    uint32_t blk_total;
+    const uint32_t start = block_scan_excl<kSortWarps>(total, s_tmp, &blk_total);
+    const uint32_t goff = live ? (&ctrl->hist[0][0])[hoff + d] : 0u;  // exclusive digit offsets
+    uint32_t prefix = 0;
+    if (tile > 0 && live) {
+        prefix = look_back_digit(flags + d, tile, epoch, &ctrl->status, fstride, s_limit);
+        publish_flag(f, tile, s_stall, pack_flag(epoch, kFlagPrefix, prefix + pub));
+    }
+    if (owner) {
+        s_start[d] = start;
+        s_gbase[d] = goff + prefix - start;
+    }
+    __syncthreads();
+    // The block's own counts place its kTileKeys items (padding included), one to a place.
+#pragma unroll
+    for (uint32_t i = 0; i < kSortRows; ++i) {
+        const uint32_t dd = FIRST ? r[i] >> 16 : (k[i] >> value_bits) & dmask;
+        const uint32_t at = s_start[dd] + s_whist[warp][dd] + (FIRST ? r[i] & 0xFFFFu : r[i]);
+        s_item[at] = k[i];
+        if constexpr (FIRST) s_low[at] = (uint8_t)dd;
+    }
+    __syncthreads();
+    const uint32_t valid = min(kTileKeys, n - tile * kTileKeys), vmask = (1u << value_bits) - 1u;
+    auto put = [&](uint32_t j) {
+        const uint32_t item = s_item[j];
+        const uint32_t dd = FIRST ? s_low[j] : (item >> value_bits) & dmask;
+        const uint32_t o = s_gbase[dd] + j;
+        if (o < n) out[o] = FIRST ? item : item & vmask;  // false only where a look-back timed out (status set)
+    };
+    if (valid == kTileKeys) {
+#pragma unroll 5
+        for (uint32_t i = 0; i < kSortRows; ++i) put(tid + i * kSortThreads);
+    } else {
+        for (uint32_t j = tid; j < valid; j += kSortThreads) put(j);
     }
 }
 
@@ -572,6 +691,10 @@ static cudaError_t ensure_sort_smem() {
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortDynSmem);
         if (e != cudaSuccess) return e;
     }
+    e = cudaFuncSetAttribute(tile_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemDynSmem<true>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(tile_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemDynSmem<false>);
+    if (e != cudaSuccess) return e;
     ready.fetch_or(bit, std::memory_order_acq_rel);
     return cudaSuccess;
 }
@@ -651,14 +774,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 #pragma unroll
             for (uint32_t i = 0; i < ROWS; ++i) {
                 const uint32_t d = (k[i] >> shift) & dmask;
-                uint32_t peers = 0xFFFFFFFFu;
-#pragma unroll
-                for (uint32_t b = 0; b < 8; ++b) {
-                    if (b >= bits) break;
-                    const uint32_t bit = (d >> b) & 1u;
-                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, bit);
-                    peers &= bit ? bal : ~bal;
-                }
+                const uint32_t peers = digit_peers(d, bits);
                 const uint32_t rank = __popc(peers & lt);
                 const uint32_t pre = S.whist[warp][d];
                 __syncwarp();
@@ -827,7 +943,7 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     const PassSplit sp = even_split_max(key_bits, db);
     const SortLayout L = sort_layout(scratch, max_count, sp);
     // With no pairs no kernel reads the flags, and none clears them: the arena mark stays.
-    ctrl_init_kernel<<<1, 256, 0, st>>>(L.ctrl, 1, nullptr, max_count ? (uint32_t)L.flag_words : kKeepArena,
+    ctrl_init_kernel<<<1, 256, 0, st>>>(L.ctrl, max_count ? (uint32_t)L.flag_words : kKeepArena,
                                         wait_config());
     count_launches(1);
     if (max_count == 0) return cudaGetLastError();
@@ -865,12 +981,6 @@ cudaError_t launch_sort_segments(const SortSegment *segs_dev, const uint32_t *bl
     return cudaGetLastError();
 }
 
-cudaError_t sort_pairs_begin(Ctrl *ctrl, Ctrl *owner, cudaStream_t st) {
-    ctrl_init_kernel<<<1, 256, 0, st>>>(ctrl, 1, owner, kKeepArena, wait_config());
-    count_launches(1);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *count, uint32_t key_bits, Ctrl *ctrl,
                               uint64_t *flags, uint2 *alt, cudaStream_t st, bool hist_scanned) {
     const PassSplit split = tile_split(key_bits);
@@ -895,6 +1005,21 @@ cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *c
         copy_packed_kernel<<<grid_for(max_count), 256, 0, st>>>(src, data, count, max_count);
         count_launches(1);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sort_items(uint32_t *items, const uint8_t *low, uint32_t *alt, uint32_t max_count, const uint32_t *count,
+                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st) {
+    const PassSplit split = tile_split(key_bits);
+    if (max_count == 0) return cudaSuccess;
+    if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
+    const uint32_t ntiles = (uint32_t)sort_tiles(max_count);
+    tile_pass_kernel<true><<<ntiles, kSortThreads, kItemDynSmem<true>, st>>>(items, low, alt, count, max_count, 0, value_bits,
+                                                                           split.bits[0], ctrl, flags);
+    tile_pass_kernel<false><<<ntiles, kSortThreads, kItemDynSmem<false>, st>>>(
+        alt, nullptr, items, count, max_count, hist_stride(2), value_bits, split.bits[1], ctrl,
+        flags + ((size_t)ntiles << split.bits[0]));
+    count_launches(2);
     return cudaGetLastError();
 }
 
