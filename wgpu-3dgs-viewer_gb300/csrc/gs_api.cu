@@ -341,6 +341,16 @@ void count_launches(uint32_t n) {
 
 bool prof_counting() { return g_prof_on && g_prof_count; }
 
+bool frame_launch_overlaps(cudaStream_t st) {
+    if (t_capturing) return false;
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return c == cudaStreamCaptureStatusNone;
+}
+
 // Look-back configuration of every launch (spin limit in the low word, stalled tile in the high).
 namespace {
 std::atomic<uint64_t> g_wait_cfg{((uint64_t)kNoStall << 32) | kSpinLimit};

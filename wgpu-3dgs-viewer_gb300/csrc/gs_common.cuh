@@ -122,6 +122,12 @@ __device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena) 
     if (b < hi && blockIdx.x == 0 && threadIdx.x == 0) arena[b] = 0ull;
 }
 
+// Start of a kernel launched by launch_frame_kernel (a plain launch passes through).
+__device__ __forceinline__ void frame_kernel_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // L2 prefetch hint for a byte range (no data returned): 16-byte aligned address, size a
 // nonzero multiple of 16.
 __device__ __forceinline__ void prefetch_l2_bulk(const void *src, uint32_t bytes) {

@@ -474,10 +474,11 @@ constexpr uint32_t kPrefetchTiles = 152 * 4;
 
 // Records [first, first + cnt) into shared rows: FP32 records by one bulk copy on the mbarrier
 // (phase 0, initialised by the caller before a __syncthreads), half records by 16-byte cp.async
-// chunks into padded rows.  Returns with the rows visible to every thread of the CTA.
+// chunks into padded rows.  stage_start() puts them on their way (and asks L2 for the records of a later
+// tile), stage_finish() returns with the rows visible to every thread of the CTA.
 template <uint32_t FMT>
-__device__ __forceinline__ void stage_records(uint4 *s_rec, uint64_t *s_bar, const uint8_t *records, uint32_t first,
-                                              uint32_t cnt, uint32_t *status, uint32_t prefetch_n = 0) {
+__device__ __forceinline__ void stage_start(uint4 *s_rec, uint64_t *s_bar, const uint8_t *records, uint32_t first,
+                                            uint32_t cnt, uint32_t prefetch_n = 0) {
     constexpr uint32_t REC = (FMT == GS_FORMAT_FP32) ? 224u : 128u;
     constexpr uint32_t C16 = REC / 16;
     constexpr uint32_t ROW16 = (FMT == GS_FORMAT_FP32) ? C16 : C16 + 1;
@@ -486,12 +487,8 @@ __device__ __forceinline__ void stage_records(uint4 *s_rec, uint64_t *s_bar, con
         if (tid == 0) {
             mbar_expect_tx(s_bar, cnt * REC);
             bulk_g2s(s_rec, records + (size_t)first * REC, cnt * REC, s_bar);
-            if (prefetch_n > 0) prefetch_l2_bulk(records + (size_t)(first + kPrefetchTiles * kPreThreads) * REC, prefetch_n * REC);
         }
-        if (!mbar_wait(s_bar, 0)) atomicOr(status, kStatusTimeout);
     } else {
-        if (tid == 0 && prefetch_n > 0)
-            prefetch_l2_bulk(records + (size_t)(first + kPrefetchTiles * kPreThreads) * REC, prefetch_n * REC);
         // consecutive threads copy consecutive 16-byte chunks (coalesced); chunk q of the CTA
         // is chunk q % C16 of record q / C16
         const uint4 *src = reinterpret_cast<const uint4 *>(records + (size_t)first * REC);
@@ -504,6 +501,16 @@ __device__ __forceinline__ void stage_records(uint4 *s_rec, uint64_t *s_bar, con
                 cp_async16(&s_rec[r * ROW16 + (q - r * C16)], src + q);
             }
         }
+    }
+    if (tid == 0 && prefetch_n > 0)
+        prefetch_l2_bulk(records + (size_t)(first + kPrefetchTiles * kPreThreads) * REC, prefetch_n * REC);
+}
+
+template <uint32_t FMT>
+__device__ __forceinline__ void stage_finish(uint64_t *s_bar, uint32_t *status) {
+    if constexpr (FMT == GS_FORMAT_FP32) {
+        if (!mbar_wait(s_bar, 0)) atomicOr(status, kStatusTimeout);
+    } else {
         cp_async_wait_all();
         __syncthreads();
     }
@@ -520,9 +527,21 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
     constexpr uint32_t ROW16 = BULK ? C16 : C16 + 1;
     __shared__ __align__(16) uint4 s_rec[kPreThreads * ROW16];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ uint32_t s_tile, s_epoch, s_base, s_limit, s_stall, s_warp[kPreThreads / 32];
+    __shared__ uint32_t s_epoch, s_base, s_limit, s_stall, s_warp[kPreThreads / 32];
     __shared__ __align__(16) gs_frame_uniforms s_u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t tile = blockIdx.x;  // look-back predecessors are lower, earlier-dispatched CTAs
+    const uint32_t first = tile * kPreThreads;
+    const uint32_t cnt = min(kPreThreads, P.n - first);
+    const uint32_t ahead = tile + kPrefetchTiles;  // records of that tile: [ahead·128, +pcnt)
+    const uint32_t pcnt = ahead < P.ntiles ? min(kPreThreads, P.n - ahead * kPreThreads) : 0u;
+    if (BULK) {
+        if (tid == 0) mbar_init(&s_bar, 1);
+        __syncthreads();
+    }
+    // The records were in place before the control block's reset, the kernel before this one, started.
+    stage_start<FMT>(s_rec, &s_bar, P.records, first, cnt, pcnt);
+    frame_kernel_enter();
     if constexpr (DEV_UNIFORMS) {
         const uint32_t *src = reinterpret_cast<const uint32_t *>(P.u_dev);
         for (uint32_t i = tid; i < sizeof(gs_frame_uniforms) / 4; i += kPreThreads)
@@ -534,16 +553,10 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
         s_epoch = *(volatile uint32_t *)&P.ctrl->epoch;
         s_limit = P.ctrl->spin_limit;
         s_stall = P.ctrl->stall_tile;
-        s_tile = blockIdx.x;  // look-back predecessors are lower, earlier-dispatched CTAs
-        if (BULK) mbar_init(&s_bar, 1);
     }
     __syncthreads();
-    const uint32_t tile = s_tile, epoch = s_epoch;
-    const uint32_t first = tile * kPreThreads;
-    const uint32_t cnt = min(kPreThreads, P.n - first);
-    const uint32_t ahead = tile + kPrefetchTiles;  // records of that tile: [ahead·128, +pcnt)
-    const uint32_t pcnt = ahead < P.ntiles ? min(kPreThreads, P.n - ahead * kPreThreads) : 0u;
-    stage_records<FMT>(s_rec, &s_bar, P.records, first, cnt, &P.ctrl->status, pcnt);
+    const uint32_t epoch = s_epoch;
+    stage_finish<FMT>(&s_bar, &P.ctrl->status);
 
     const uint32_t i = first + tid;
     bool vis = false;
@@ -654,7 +667,8 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_views_kernel(const __g
     const uint32_t tile = s_tile;
     const uint32_t first = tile * kPreThreads;
     const uint32_t cnt = min(kPreThreads, P.n - first);
-    stage_records<FMT>(s_rec, &s_bar, P.records, first, cnt, &P.group->status);
+    stage_start<FMT>(s_rec, &s_bar, P.records, first, cnt);
+    stage_finish<FMT>(&s_bar, &P.group->status);
 
     const uint32_t i = first + tid;
     const bool sel = tid < cnt && gaussian_selected(P.selection, P.invert, i);
@@ -841,7 +855,8 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
                               const gs_frame_uniforms *u_dev, uint4 *binfo) {
     Ctrl *ctrl = reinterpret_cast<Ctrl *>(scratch);
     uint64_t *flags = reinterpret_cast<uint64_t *>((uint8_t *)scratch + align_up(sizeof(Ctrl), 256));
-    ctrl_init_kernel<<<1, 256, 0, st>>>(ctrl, kKeepArena, wait_config());
+    const bool overlap = frame_launch_overlaps(st);
+    launch_frame_kernel(ctrl_init_kernel, 1, 256, 0, st, overlap, ctrl, kKeepArena, wait_config());
     count_launches(1);
     if (n == 0) {
         preprocess_empty_kernel<<<1, 1, 0, st>>>(indirect, dispatch, ctrl);
@@ -873,25 +888,25 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
     if (u_dev) {
         switch (format) {
             case GS_FORMAT_FP32:
-                preprocess_kernel<GS_FORMAT_FP32, true><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_FP32, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
             case GS_FORMAT_HALF_SH_FP16:
-                preprocess_kernel<GS_FORMAT_HALF_SH_FP16, true><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_FP16, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
             default:
-                preprocess_kernel<GS_FORMAT_HALF_SH_BF16, true><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_BF16, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
         }
     } else {
         switch (format) {
             case GS_FORMAT_FP32:
-                preprocess_kernel<GS_FORMAT_FP32, false><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_FP32, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
             case GS_FORMAT_HALF_SH_FP16:
-                preprocess_kernel<GS_FORMAT_HALF_SH_FP16, false><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_FP16, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
             default:
-                preprocess_kernel<GS_FORMAT_HALF_SH_BF16, false><<<P.ntiles, kPreThreads, 0, st>>>(P);
+                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_BF16, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
                 break;
         }
     }

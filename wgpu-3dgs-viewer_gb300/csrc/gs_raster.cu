@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *__restrict__ info,
     uint32_t *__restrict__ counts, const Ctrl *owner, uint64_t *arena, uint32_t *__restrict__ rects,
     uint32_t rect_shift, Ctrl *reset, uint32_t arena_words) {
+    frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
     if (reset && blockIdx.x == 0 && threadIdx.x == 0) ctrl_reset_flagless(reset, arena_words);
     const uint32_t n = count ? min(*count, max_count) : max_count;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(256) bin_scan_kernel(uint32_t *__restrict__ da
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_tile, s_epoch, s_prefix, s_limit, s_stall;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    frame_kernel_enter();
     if (tid == 0) {
         s_epoch = *(volatile uint32_t *)&ctrl->epoch;
         s_limit = ctrl->spin_limit;
@@ -349,11 +351,12 @@ __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
     extern __shared__ uint32_t s_bins[];
     const uint32_t nbins = COUNTS ? ntiles : 4u * 256u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    for (uint32_t i = tid; i < nbins; i += kBinThreads) s_bins[i] = 0u;
+    frame_kernel_enter();
     const uint32_t n = count ? min(*count, max_count) : max_count;
     const uint32_t total = ctrl->total;
     // a scan that gave up leaves offsets nothing can be found by (status already set): emit nothing
     const bool sound = !(*(volatile uint32_t *)&ctrl->status & kStatusTimeout);
-    for (uint32_t i = tid; i < nbins; i += kBinThreads) s_bins[i] = 0u;
     __syncthreads();
     uint32_t *items = reinterpret_cast<uint32_t *>(pairs);
     uint8_t *low = reinterpret_cast<uint8_t *>(pairs) + (size_t)max_pairs * 4u;
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
 // other CTAs.
 __global__ void __launch_bounds__(256) raster_init_kernel(Ctrl *ctrl, Ctrl *sort_ctrl, uint32_t arena_words, WaitCfg cfg,
                                                           uint32_t *counts, uint32_t ntiles) {
+    frame_kernel_enter();
     if (blockIdx.x == 0) {
         ctrl_reset(ctrl, ctrl, arena_words, cfg);
         ctrl_reset(sort_ctrl, ctrl, kKeepArena, cfg);
@@ -491,6 +495,7 @@ constexpr uint32_t kCountSlices = 16;
 
 __global__ void __launch_bounds__(256) tile_count_kernel(const uint32_t *__restrict__ blockcounts, uint32_t nblocks,
                                                          uint32_t ntiles, uint32_t *__restrict__ counts) {
+    frame_kernel_enter();
     const uint32_t t = blockIdx.x * 256u + threadIdx.x;
     if (t >= ntiles) return;
     const uint32_t per = (nblocks + kCountSlices - 1) / kCountSlices;
@@ -531,6 +536,7 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restr
     __shared__ uint32_t s_w[32], s_low[1024], s_lw[10], s_cls[96];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = lanemask_lt();
     if (tid < 96u) s_cls[tid] = 0u;
+    frame_kernel_enter();
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) {
         const uint32_t t = tid + 1024u * j;
@@ -650,6 +656,7 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restr
 // consecutive pairs with two 16-byte loads.
 __global__ void tile_ranges_kernel(const uint2 *__restrict__ pairs, const Ctrl *ctrl, uint2 *ranges,
                                    uint32_t ntiles) {
+    frame_kernel_enter();
     const uint32_t n = ctrl->count;
     const uint32_t stride = gridDim.x * blockDim.x * 4u;
     for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) * 4u; base < n; base += stride) {
@@ -1174,6 +1181,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(con
                                                                 uint32_t suffix_min, float eps,
                                                                 unsigned long long *counters) {
     __shared__ RasterShared S;
+    frame_kernel_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) merge_status(J);
     const uint32_t tile = J.order ? J.order[blockIdx.x] : blockIdx.x;
     const uint2 r = tile_range(J, tile);
@@ -1200,6 +1208,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     const uint32_t tx = tile % J.tiles_x, ty = tile / J.tiles_x, words = (ranks + 31u) / 32u;
     const uint32_t here = pack_rect(tx, ty, tx, ty, shift);
     constexpr uint32_t STEP = kRasterThreads / 32u;
+    frame_kernel_enter();
     for (uint32_t q0 = warp; q0 < words; q0 += 8u * STEP) {
         uint32_t r[8];
 #pragma unroll
@@ -1269,6 +1278,7 @@ __global__ void __launch_bounds__(kRasterThreads, 6) raster_views_kernel(const R
                                                                       uint32_t nviews, float std2, float outline2,
                                                                       uint32_t suffix_min, float eps) {
     __shared__ RasterShared S;
+    frame_kernel_enter();
     uint32_t lo = 0, hi = nviews - 1;
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
@@ -1299,8 +1309,8 @@ cudaError_t raster_counters(unsigned long long out[4], bool reset) {
 template <uint32_t MODE, bool EXACT, bool COUNT, bool FEW>
 static void launch_raster_tiles(const RasterJob &J, float std2, float outline2, cudaStream_t st, const Tuning &t,
                                 unsigned long long *counts) {
-    raster_kernel<MODE, EXACT, COUNT, FEW><<<J.ntiles, kRasterThreads, 0, st>>>(J, std2, outline2, t.suffix_min, t.eps,
-                                                                                counts);
+    launch_frame_kernel(raster_kernel<MODE, EXACT, COUNT, FEW>, J.ntiles, kRasterThreads, 0, st, frame_launch_overlaps(st), J,
+                        std2, outline2, t.suffix_min, t.eps, counts);
 }
 
 // Grids of up to four resident waves of the FEW kernel take it: 1456 tiles (1.4M splats at 892x401)
@@ -1400,8 +1410,9 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
     // The first segment with splats clears the arena in its bin_count launch; with none, no kernel
     // reads a flag and the arena mark stays.
     prof_mark(kProfBin, true, st);
-    raster_init_kernel<<<1 + (L.counts ? (L.ntiles + 1023) / 1024 : 0), 256, 0, st>>>(
-        L.ctrl, L.sort_ctrl, max_splats ? L.arena_words : kKeepArena, wait_config(), L.counts, L.ntiles);
+    const bool overlap = frame_launch_overlaps(st);
+    launch_frame_kernel(raster_init_kernel, 1 + (L.counts ? (L.ntiles + 1023) / 1024 : 0), 256, 0, st, overlap, L.ctrl,
+                        L.sort_ctrl, max_splats ? L.arena_words : kKeepArena, wait_config(), L.counts, L.ntiles);
     count_launches(1);
     const PassSplit split = tile_split(L.key_bits);
     const int direct = nseg == 1 ? 1 : 0;
@@ -1412,10 +1423,10 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         if (blocks == 0) continue;
         // a stored tile record is only for the target the preprocess was given (one model)
         const uint4 *binfo = direct && g.binfo && g.binfo_w == W && g.binfo_h == H ? g.binfo : nullptr;
-        bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(
-            g.splats, binfo, g.sorted_index, g.count, g.max_count, rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y,
-            u.display_mode, u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
-            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0);
+        launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
+                            g.max_count, rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y, u.display_mode,
+                            u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
+                            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0);
         count_launches(1);
         rank_offset += g.max_count;
     }
@@ -1423,8 +1434,8 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
     // (ranks without a splat have no tiles).
     const uint32_t *count = direct ? segs[0].count : nullptr;
     if (max_splats) {
-        bin_scan_kernel<<<(max_splats + kScanTile - 1) / kScanTile, 256, 0, st>>>(L.offsets, count, max_splats, max_pairs,
-                                                                                L.ctrl, L.flags);
+        launch_frame_kernel(bin_scan_kernel, (max_splats + kScanTile - 1) / kScanTile, 256, 0, st, overlap, L.offsets, count,
+                            max_splats, max_pairs, L.ctrl, L.flags);
         count_launches(1);
     }
     // One resident wave at most (and the per-CTA count area): a second, late wave would stretch the
@@ -1435,15 +1446,15 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         uint32_t wave = resident_ctas(kernel, kBinThreads, emit_smem);
         if (wave == 0 || wave > kEmitBlocks) wave = kEmitBlocks;
         const uint32_t want = std::max((max_splats + kBinThreads - 1) / kBinThreads, 304u), grid = std::min(want, wave);
-        kernel<<<grid, kBinThreads, emit_smem, st>>>(L.info, L.offsets, count, max_splats, L.pairs, max_pairs, L.value_bits,
-                                                     L.tiles_x, L.ntiles, L.ctrl, L.sort_ctrl, split, L.blockcounts);
+        launch_frame_kernel(kernel, grid, kBinThreads, emit_smem, st, overlap, L.info, L.offsets, count, max_splats, L.pairs,
+                            max_pairs, L.value_bits, L.tiles_x, L.ntiles, L.ctrl, L.sort_ctrl, split, L.blockcounts);
         return grid;
     };
     if (L.counts) {
         const uint32_t grid = compact ? emit(bin_emit_kernel<true, true>) : emit(bin_emit_kernel<true, false>);
-        tile_count_kernel<<<dim3((L.ntiles + 255) / 256, kCountSlices), 256, 0, st>>>(L.blockcounts, grid, L.ntiles,
-                                                                                     L.counts);
-        tile_scan_kernel<<<1, 1024, 0, st>>>(L.counts, L.ntiles, L.ranges, L.order, L.sort_ctrl, split);
+        launch_frame_kernel(tile_count_kernel, dim3((L.ntiles + 255) / 256, kCountSlices), 256, 0, st, overlap, L.blockcounts,
+                            grid, L.ntiles, L.counts);
+        launch_frame_kernel(tile_scan_kernel, 1, 1024, 0, st, overlap, L.counts, L.ntiles, L.ranges, L.order, L.sort_ctrl, split);
         count_launches(3);
     } else {
         emit(bin_emit_kernel<false, false>);
@@ -1495,7 +1506,8 @@ cudaError_t launch_binning_ranges(const RasterSegment *segs, uint32_t nseg, uint
         uint32_t rblocks = (max_pairs + 255) / 256;
         if (rblocks > 152 * 8) rblocks = 152 * 8;
         if (rblocks == 0) rblocks = 1;
-        tile_ranges_kernel<<<rblocks, 256, 0, st>>>(L.pairs, L.ctrl, L.ranges, L.ntiles);
+        launch_frame_kernel(tile_ranges_kernel, rblocks, 256, 0, st, frame_launch_overlaps(st), L.pairs, L.ctrl, L.ranges,
+                            L.ntiles);
         prof_mark(kProfRanges, false, st);
         count_launches(1);
     }
@@ -1538,8 +1550,8 @@ static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32
                                uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
     const bool few = tiles_at_once <= kFewTiles;
     auto go = [&](auto kernel) {
-        kernel<<<J.ntiles, kRasterThreads, 0, st>>>(J, L.offsets, L.info, ranks, shift, L.items(), max_pairs, std2, outline2,
-                                                    t.suffix_min, t.eps);
+        launch_frame_kernel(kernel, J.ntiles, kRasterThreads, 0, st, frame_launch_overlaps(st), J, L.offsets, L.info, ranks,
+                            shift, L.items(), max_pairs, std2, outline2, t.suffix_min, t.eps);
     };
     if (exact) few ? go(raster_direct_kernel<MODE, true, true>) : go(raster_direct_kernel<MODE, true, false>);
     else few ? go(raster_direct_kernel<MODE, false, true>) : go(raster_direct_kernel<MODE, false, false>);
@@ -1561,11 +1573,10 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
         const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
         if (blocks == 0) continue;
         const uint4 *binfo = direct && g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
-        bin_count_kernel<<<blocks, kBinThreads, 0, st>>>(g.splats, binfo, g.sorted_index, g.count, g.max_count, rank_offset,
-                                                         L.sorted, direct, L.tiles_x, L.tiles_y, u.display_mode, std2,
-                                                         L.info + rank_offset, nullptr, nullptr, nullptr,
-                                                         L.offsets + rank_offset, shift, started ? nullptr : L.ctrl,
-                                                         L.arena_words);
+        launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
+                            g.sorted_index, g.count, g.max_count, rank_offset, L.sorted, direct, L.tiles_x, L.tiles_y,
+                            u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
+                            shift, started ? nullptr : L.ctrl, L.arena_words);
         count_launches(1);
         started = true;
         rank_offset += g.max_count;

@@ -32,6 +32,7 @@ constexpr size_t kSortDynSmem = (size_t)kTileKeys * sizeof(uint2);
 static_assert(kTileKeys % GS_SORT_BLOCK_KVS == 0, "a pass block covers whole blocks of the reference");
 
 __global__ void ctrl_init_kernel(Ctrl *ctrl, uint32_t arena_words, WaitCfg cfg) {
+    frame_kernel_enter();
     ctrl_reset(ctrl, ctrl, arena_words, cfg);
 }
 
@@ -119,8 +120,9 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t *__restri
     __shared__ uint32_t h[1024];
     const uint32_t npasses = sp.n, hs = hist_stride(sp.n);
     uint32_t *gh = &ctrl->hist[0][0];
-    arena_clear(ctrl, arena);
     for (uint32_t k = threadIdx.x; k < 1024; k += blockDim.x) h[k] = 0u;
+    frame_kernel_enter();
+    arena_clear(ctrl, arena);
     __syncthreads();
     const uint32_t n = load_count(count, max_count);
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -239,14 +241,15 @@ __device__ __forceinline__ void sort_pass_block(
     __shared__ uint32_t s_tmp[kSortWarps];
     __shared__ uint32_t s_epoch, s_limit, s_stall;
 
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t n = load_count(count, max_count), tile = block;  // arrives while the counters are cleared
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = block;
+    for (uint32_t k = tid; k < kSortWarps * 256; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
+    frame_kernel_enter();
+    const uint32_t n = load_count(count, max_count);
     if (tid == 0) {
         s_epoch = *(volatile uint32_t *)&ctrl->epoch;
         s_limit = ctrl->spin_limit;
         s_stall = ctrl->stall_tile;
     }
-    for (uint32_t k = tid; k < kSortWarps * 256; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
     // The grid covers the capacity: CTAs past the pairs there are (half of a tile sort's) leave here.
     const uint32_t ntiles = (n + kTileKeys - 1) / kTileKeys;
     if (tile >= ntiles) return;
@@ -391,14 +394,15 @@ __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
     __shared__ uint32_t s_gbase[256];
     __shared__ uint32_t s_tmp[kSortWarps];
     __shared__ uint32_t s_epoch, s_limit, s_stall;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t n = load_count(count, max_count), tile = blockIdx.x;  // arrives while the counters are cleared
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
+    for (uint32_t k = tid; k < kSortWarps * 256; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
+    frame_kernel_enter();
+    const uint32_t n = load_count(count, max_count);
     if (tid == 0) {
         s_epoch = *(volatile uint32_t *)&ctrl->epoch;
         s_limit = ctrl->spin_limit;
         s_stall = ctrl->stall_tile;
     }
-    for (uint32_t k = tid; k < kSortWarps * 256; k += kSortThreads) (&s_whist[0][0])[k] = 0u;
     const uint32_t ntiles = (n + kTileKeys - 1) / kTileKeys;
     if (tile >= ntiles) return;
     __syncthreads();
@@ -520,6 +524,7 @@ __global__ void merge_segments_status_kernel(const SortSegment *segs, uint32_t n
 
 __global__ void unpack_pairs_kernel(const uint2 *src, uint32_t *kd, uint32_t *vd, const uint32_t *count,
                                     uint32_t max_count) {
+    frame_kernel_enter();
     const uint32_t n = load_count(count, max_count);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint2 kv = src[i];
@@ -529,6 +534,7 @@ __global__ void unpack_pairs_kernel(const uint2 *src, uint32_t *kd, uint32_t *vd
 }
 
 __global__ void copy_packed_kernel(const uint2 *src, uint2 *dst, const uint32_t *count, uint32_t max_count) {
+    frame_kernel_enter();
     const uint32_t n = load_count(count, max_count);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
 }
@@ -645,20 +651,21 @@ template <bool MATCH, bool MATCH_LAST>
 static void launch_sort_passes(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
                                const PassSplit &sp, const SortLayout &L, cudaStream_t st) {
     const uint32_t npasses = sp.n, hs = hist_stride(sp.n);
+    const bool overlap = frame_launch_overlaps(st);
     uint64_t *f = L.flags;
     if (npasses == 1) {
-        sort_pass_kernel<false, true, MATCH><<<L.ntiles, kSortThreads, kSortDynSmem, st>>>(
+        launch_frame_kernel(sort_pass_kernel<false, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
             keys, vals, nullptr, nullptr, nullptr, L.alt_a, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f, 1u);
-        unpack_pairs_kernel<<<grid_for(max_count), 256, 0, st>>>(L.alt_a, keys, vals, count, max_count);
+        launch_frame_kernel(unpack_pairs_kernel, grid_for(max_count), 256, 0, st, overlap, L.alt_a, keys, vals, count, max_count);
         count_launches(2);
         return;
     }
     uint2 *src = L.alt_a, *dst = L.alt_b;
-    sort_pass_kernel<false, true, MATCH><<<L.ntiles, kSortThreads, kSortDynSmem, st>>>(
+    launch_frame_kernel(sort_pass_kernel<false, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
         keys, vals, nullptr, nullptr, nullptr, src, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f, 1u);
     f += (size_t)L.ntiles << sp.bits[0];
     for (uint32_t p = 1; p + 1 < npasses; ++p) {
-        sort_pass_kernel<true, true, MATCH><<<L.ntiles, kSortThreads, kSortDynSmem, st>>>(
+        launch_frame_kernel(sort_pass_kernel<true, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
             nullptr, nullptr, src, nullptr, nullptr, dst, count, max_count, p * hs, sp.shift[p], sp.bits[p], L.ctrl, f,
             1u);
         f += (size_t)L.ntiles << sp.bits[p];
@@ -666,7 +673,7 @@ static void launch_sort_passes(uint32_t *keys, uint32_t *vals, uint32_t max_coun
         src = dst;
         dst = t;
     }
-    sort_pass_kernel<true, false, MATCH || MATCH_LAST><<<L.ntiles, kSortThreads, kSortDynSmem, st>>>(
+    launch_frame_kernel(sort_pass_kernel<true, false, MATCH || MATCH_LAST>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
         nullptr, nullptr, src, keys, vals, nullptr, count, max_count, (npasses - 1) * hs, sp.shift[npasses - 1],
         sp.bits[npasses - 1], L.ctrl, f, 1u);
     count_launches(npasses);
@@ -752,6 +759,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     ClusterShared<ROWS> &S = *reinterpret_cast<ClusterShared<ROWS> *>(cluster_smem);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, lt = lanemask_lt();
     const uint32_t me = cluster_rank(), ctas = cluster_size();
+    frame_kernel_enter();
     if (me == 0 && tid == 0) ctrl->status = 0u;  // of the call; no flag is waited for here
     const uint32_t n = load_count(count, max_count);
     const bool some = me * K < n;  // this CTA holds pairs
@@ -892,17 +900,19 @@ static bool launch_cluster_rows(uint32_t *keys, uint32_t *vals, uint32_t max_cou
     constexpr uint32_t K = kClusterThreads * ROWS;
     const uint32_t ctas = (max_count + K - 1) / K;
     if (ctas == 0 || ctas > cluster_ctas_supported<ROWS>()) return false;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = ctas;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(kClusterThreads);
     cfg.dynamicSmemBytes = sizeof(ClusterShared<ROWS>);
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = frame_launch_overlaps(st) ? 2 : 1;
     *err = cudaLaunchKernelEx(&cfg, sort_cluster_kernel<ROWS>, keys, vals, count, max_count, sp, ctrl);
     count_launches(1);
     return true;
@@ -942,8 +952,9 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
                                                              : tn.sort_digit_bits;
     const PassSplit sp = even_split_max(key_bits, db);
     const SortLayout L = sort_layout(scratch, max_count, sp);
+    const bool overlap = frame_launch_overlaps(st);
     // With no pairs no kernel reads the flags, and none clears them: the arena mark stays.
-    ctrl_init_kernel<<<1, 256, 0, st>>>(L.ctrl, max_count ? (uint32_t)L.flag_words : kKeepArena,
+    launch_frame_kernel(ctrl_init_kernel, 1, 256, 0, st, overlap, L.ctrl, max_count ? (uint32_t)L.flag_words : kKeepArena,
                                         wait_config());
     count_launches(1);
     if (max_count == 0) return cudaGetLastError();
@@ -951,7 +962,7 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     uint32_t hist_blocks = (max_count + 256 * 4 * 4 - 1) / (256 * 4 * 4);
     if (hist_blocks > 152 * 8) hist_blocks = 152 * 8;
     if (tn.hist_blocks) hist_blocks = tn.hist_blocks < 152 * 8 ? tn.hist_blocks : 152 * 8;
-    sort_hist_kernel<<<hist_blocks, 256, 0, st>>>(keys, vals, count, max_count, sp, L.ctrl, L.flags);
+    launch_frame_kernel(sort_hist_kernel, hist_blocks, 256, 0, st, overlap, keys, vals, count, max_count, sp, L.ctrl, L.flags);
     count_launches(1);
     // Keys of kDepthKeyBits are the render path's float depth keys (1 - ndc.z).
     if (tn.sort_match)
@@ -987,10 +998,11 @@ cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *c
     if (max_count == 0) return cudaSuccess;
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const uint32_t ntiles = (uint32_t)sort_tiles(max_count);
+    const bool overlap = frame_launch_overlaps(st);
     uint2 *src = data, *dst = alt;
     uint64_t *f = flags;
     for (uint32_t p = 0; p < split.n; ++p) {
-        sort_pass_kernel<true, true, false><<<ntiles, kSortThreads, kSortDynSmem, st>>>(nullptr, nullptr, src, nullptr, nullptr, dst,
+        launch_frame_kernel(sort_pass_kernel<true, true, false>, ntiles, kSortThreads, kSortDynSmem, st, overlap, nullptr, nullptr, src, nullptr, nullptr, dst,
                                                                             count, max_count, p * hist_stride(split.n),
                                                                             split.shift[p],
                                                                             split.bits[p], ctrl, f,
@@ -1002,7 +1014,7 @@ cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *c
     }
     count_launches(split.n);
     if (split.n & 1u) {
-        copy_packed_kernel<<<grid_for(max_count), 256, 0, st>>>(src, data, count, max_count);
+        launch_frame_kernel(copy_packed_kernel, grid_for(max_count), 256, 0, st, overlap, src, data, count, max_count);
         count_launches(1);
     }
     return cudaGetLastError();
@@ -1014,9 +1026,10 @@ cudaError_t launch_sort_items(uint32_t *items, const uint8_t *low, uint32_t *alt
     if (max_count == 0) return cudaSuccess;
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const uint32_t ntiles = (uint32_t)sort_tiles(max_count);
-    tile_pass_kernel<true><<<ntiles, kSortThreads, kItemDynSmem<true>, st>>>(items, low, alt, count, max_count, 0, value_bits,
+    const bool overlap = frame_launch_overlaps(st);
+    launch_frame_kernel(tile_pass_kernel<true>, ntiles, kSortThreads, kItemDynSmem<true>, st, overlap, items, low, alt, count, max_count, 0, value_bits,
                                                                            split.bits[0], ctrl, flags);
-    tile_pass_kernel<false><<<ntiles, kSortThreads, kItemDynSmem<false>, st>>>(
+    launch_frame_kernel(tile_pass_kernel<false>, ntiles, kSortThreads, kItemDynSmem<false>, st, overlap, 
         alt, nullptr, items, count, max_count, hist_stride(2), value_bits, split.bits[1], ctrl,
         flags + ((size_t)ntiles << split.bits[0]));
     count_launches(2);
