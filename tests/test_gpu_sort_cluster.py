@@ -1,4 +1,4 @@
-"""The sorter at the sizes where it changes between one cluster (1, 2, 4 or 8 rows a thread, 1 to 16
+"""The sorter at the sizes where it changes between one cluster (1, 2 or 4 rows a thread, 1 to 16
 CTAs) and the pass kernels, with device-side counts below the capacity, keys of all ones (the padding's
 value) and ties, against a stable sort: equal bits."""
 import numpy as np

@@ -1316,7 +1316,7 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
                 if (vs != cs) err = cudaStreamWaitEvent(vs, b->chunk_events[c], 0);
                 if (err == cudaSuccess)
                     err = launch_sort((uint32_t *)v.depths.ptr, (uint32_t *)v.indices.ptr, ms[i]->n, ind + 1, kDepthKeyBits,
-                                      v.sort_scratch.ptr, vs, kProfDepthSort, &b->tuning, n > 1);
+                                      v.sort_scratch.ptr, vs, kProfDepthSort, &b->tuning);
                 if (err == cudaSuccess) {
                     const RasterSegment seg{(const gs_splat *)v.splats.ptr, (const uint32_t *)v.indices.ptr, ind + 1,
                                             ms[i]->n};

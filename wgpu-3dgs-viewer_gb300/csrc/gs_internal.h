@@ -120,10 +120,9 @@ constexpr uint32_t kDepthKeyBits = 30;
 // Passes of a sort at most (32-bit keys in 6-bit digits).
 constexpr uint32_t kMaxPasses = 6;
 size_t sort_scratch_bytes(uint32_t max_count, uint32_t key_bits);
-// overlapped: other views' work runs beside this sort (a batch).
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
                         uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage = kProfDepthSort,
-                        const Tuning *tuning = nullptr, bool overlapped = false);
+                        const Tuning *tuning = nullptr);
 
 // Digits of the packed-pair sort: the key's bits spread evenly over the fewest passes of at
 // most 8 bits (13 bits -> 7 + 6), pass p taking bits [shift[p], shift[p] + bits[p]).

@@ -88,9 +88,9 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, uint32_t bits) {
 
 // Global digit histograms of all passes in one read of the keys (four keys per thread and
 // iteration, 16-byte loads when the keys are 16-byte aligned).  Low digits are counted with plain
-// shared atomics; for the top digit the warp counts the digit of lane 0 with one ballot (the high
-// digits of float depth keys are nearly constant, and same-address shared atomics would
-// serialise) and the other keys with plain shared atomics.
+// shared atomics; for the top digit the warp counts the digit of its first lane with one ballot, then
+// that of the first lane left, (the high digits of float depth keys take few values, and same-address
+// shared atomics would serialise) and the other keys with plain shared atomics.
 __device__ __forceinline__ void hist_add(uint32_t *h, uint32_t k, bool valid, const PassSplit &sp, uint32_t hs,
                                          uint32_t lane) {
     // unrolled over the fixed maximum so every field of the split is read at a constant offset
@@ -102,10 +102,17 @@ __device__ __forceinline__ void hist_add(uint32_t *h, uint32_t k, bool valid, co
             if (valid) atomicAdd(&h[p * hs + d], 1u);
             continue;
         }
-        const uint32_t d0 = __shfl_sync(0xFFFFFFFFu, d, 0);
-        const uint32_t same = __ballot_sync(0xFFFFFFFFu, valid && d == d0);
-        if (lane == 0 && same) atomicAdd(&h[p * hs + d0], (uint32_t)__popc(same));
-        if (valid && d != d0) atomicAdd(&h[p * hs + d], 1u);
+        bool left = valid;
+#pragma unroll
+        for (uint32_t t = 0; t < 2; ++t) {
+            const uint32_t todo = __ballot_sync(0xFFFFFFFFu, left);
+            if (!todo) break;
+            const uint32_t leader = __ffs(todo) - 1u, dl = __shfl_sync(0xFFFFFFFFu, d, leader);
+            const uint32_t same = __ballot_sync(0xFFFFFFFFu, left && d == dl);
+            if (lane == leader) atomicAdd(&h[p * hs + dl], (uint32_t)__popc(same));
+            left = left && d != dl;
+        }
+        if (left) atomicAdd(&h[p * hs + d], 1u);
     }
 }
 
@@ -113,34 +120,33 @@ __device__ __forceinline__ void hist_add(uint32_t *h, uint32_t k, bool valid, co
 // which are the arena's only readers, run after this kernel).
 // With `vals`, each CTA also asks L2 for the values of the keys it reads, which the first pass
 // reads next (the keys themselves arrive in L2 through this kernel's reads).
-__global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t *__restrict__ keys,
-                                                        const uint32_t *__restrict__ vals, const uint32_t *count,
-                                                        uint32_t max_count, const PassSplit sp, Ctrl *ctrl,
-                                                        uint64_t *arena) {
+// Bound by its chain of steps at middle sizes and by the shared atomics at large ones: 400k, 2M and 6M
+// keys 12.2, 17.4 and 31 us with 256 threads a CTA, four waits for keys in a row and the passes' scans one
+// after another; 8.5, 13.6 and 28 with four times the threads, the next keys on their way and a warp a scan.
+constexpr uint32_t kHistThreads = 1024;
+constexpr uint32_t kHistCtas = 152 * 2;  // resident at once
+__global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(const uint32_t *__restrict__ keys,
+                                                                 const uint32_t *__restrict__ vals,
+                                                                 const uint32_t *count, uint32_t max_count,
+                                                                 const PassSplit sp, Ctrl *ctrl, uint64_t *arena) {
     __shared__ uint32_t h[1024];
     const uint32_t npasses = sp.n, hs = hist_stride(sp.n);
     uint32_t *gh = &ctrl->hist[0][0];
-    for (uint32_t k = threadIdx.x; k < 1024; k += blockDim.x) h[k] = 0u;
+    h[threadIdx.x] = 0u;
     frame_kernel_enter();
     arena_clear(ctrl, arena);
     __syncthreads();
     const uint32_t n = load_count(count, max_count);
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const bool vec = ((uintptr_t)keys & 15u) == 0;
     // Whole warps iterate together (bounds padded to the warp) so the ballots see 32 lanes.
     const uint32_t n4 = (n + 3u) / 4u;
     const uint32_t nr = (n4 + 31u) & ~31u;
     const bool pf = vals && ((uintptr_t)vals & 15u) == 0;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nr; q += stride) {
+    auto load = [&](uint32_t q, uint32_t k[4]) {
         const uint32_t i0 = q * 4u;
-        if (pf && threadIdx.x == 0 && i0 < n) {
-            // this CTA's 4 x blockDim keys of the iteration start at i0 (a multiple of 16 bytes)
-            const uint32_t bytes = min(4u * 4u * blockDim.x, (n - i0) * 4u) & ~15u;
-            if (bytes) prefetch_l2_bulk(vals + i0, bytes);
-        }
-        uint32_t k[4];
-        if (vec && i0 + 4u <= n) {
+        if (vec && q < nr && i0 + 4u <= n) {
             const uint4 v = *reinterpret_cast<const uint4 *>(keys + i0);
             k[0] = v.x;
             k[1] = v.y;
@@ -148,30 +154,55 @@ __global__ void __launch_bounds__(256) sort_hist_kernel(const uint32_t *__restri
             k[3] = v.w;
         } else {
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) k[j] = i0 + j < n ? keys[i0 + j] : 0u;
+            for (uint32_t j = 0; j < 4; ++j) k[j] = q < nr && i0 + j < n ? keys[i0 + j] : 0u;
         }
+    };
+    uint32_t k[4];
+    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    load(q, k);
+    for (; q < nr; q += stride) {
+        const uint32_t i0 = q * 4u;
+        if (pf && threadIdx.x == 0 && i0 < n) {
+            // this CTA's 4 x blockDim keys of the iteration start at i0 (a multiple of 16 bytes)
+            const uint32_t bytes = min(4u * 4u * blockDim.x, (n - i0) * 4u) & ~15u;
+            if (bytes) prefetch_l2_bulk(vals + i0, bytes);
+        }
+        uint32_t next[4];
+        load(q + stride, next);  // under way while this iteration's keys are counted
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j) hist_add(h, k[j], i0 + j < n, sp, hs, lane);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) k[j] = next[j];
     }
     __syncthreads();
-    for (uint32_t p = 0; p < npasses; ++p) {
-        const uint32_t v = threadIdx.x < (1u << sp.bits[p]) ? h[p * hs + threadIdx.x] : 0u;
-        if (v) atomicAdd(&gh[p * hs + threadIdx.x], v);
-    }
+    if (const uint32_t v = h[threadIdx.x]) atomicAdd(&gh[threadIdx.x], v);  // the same places in both
     // The last CTA to finish turns the histograms into exclusive digit offsets, once for every
-    // block of every pass.
-    __shared__ uint32_t s_last, s_tmp[8];
+    // block of every pass: a warp a pass.
+    __shared__ uint32_t s_last;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(&ctrl->ticket[7], 1u) == gridDim.x - 1 ? 1u : 0u;
     __syncthreads();
-    if (s_last) {
+    if (s_last && warp < npasses) {
         __threadfence();
-        for (uint32_t p = 0; p < npasses; ++p) {
-            uint32_t total;
-            const bool live = threadIdx.x < (1u << sp.bits[p]);
-            const uint32_t off = block_scan_excl<8>(live ? __ldcg(&gh[p * hs + threadIdx.x]) : 0u, s_tmp, &total);
-            if (live) gh[p * hs + threadIdx.x] = off;
+        const uint32_t digits = 1u << sp.bits[warp];
+        uint32_t v[8], sum = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            v[j] = lane * 8u + j < digits ? __ldcg(&gh[warp * hs + lane * 8u + j]) : 0u;
+            sum += v[j];
+        }
+        uint32_t run = sum;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, run, o);
+            if (lane >= o) run += y;
+        }
+        run -= sum;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (lane * 8u + j < digits) gh[warp * hs + lane * 8u + j] = run;
+            run += v[j];
         }
     }
 }
@@ -707,7 +738,7 @@ static cudaError_t ensure_sort_smem() {
 }
 
 // ---- small sorts: every pass in one launch of one cluster --------------------------------------
-// Up to kClusterMaxPairs pairs are sorted by a single thread-block cluster: CTA c holds positions
+// Up to 65,536 pairs (16 CTAs of 4 rows) are sorted by a single thread-block cluster: CTA c holds positions
 // [c K, (c + 1) K) in registers (K = 1024 ROWS), each pass ranks them as sort_pass_block does, the
 // CTAs exchange their digit counts through distributed shared memory, and every pair goes straight
 // to its place in the shared memory of the CTA that owns it.  Two cluster barriers a pass take the
@@ -919,29 +950,24 @@ static bool launch_cluster_rows(uint32_t *keys, uint32_t *vals, uint32_t max_cou
 }
 
 // The fewest rows that fit: fewer rows a thread and more CTAs are faster throughout (16384 pairs: 24.5,
-// 25.0, 29.2 and 41.4 us at 1, 2, 4 and 8 rows).  Against the histogram and pass kernels: 5,000 pairs 63.9 ->
-// 18.8 us, 30,000 72.9 -> 29.1, 65,536 74.2 -> 37.3, 131,072 72.3 -> 58.2; at 12 rows (196,608 pairs) they
-// are the faster ones, 78.0 against 80.3.
-// Eight rows take an SM's whole register file for most of a frame's sort, which is a loss where other
-// views could run beside it (`overlapped`; 10 views of 93k: 554 -> 582 us a batch with them).
+// 25.0 and 29.2 us at 1, 2 and 4 rows).  Against the histogram and pass kernels, with the launches of
+// either overlapped: 40,000 pairs 29.0 us, 39.9; 65,536 pairs 32.4, 43.4; with 8 rows 70,000 pairs would
+// take 45.1, 43.0 and 131,072 pairs 51.2, 45.4.
 static bool launch_sort_cluster(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
-                                uint32_t key_bits, bool overlapped, Ctrl *ctrl, cudaStream_t st, cudaError_t *err) {
+                                uint32_t key_bits, Ctrl *ctrl, cudaStream_t st, cudaError_t *err) {
     const PassSplit sp = even_split(key_bits);
     return launch_cluster_rows<1>(keys, vals, max_count, count, sp, ctrl, st, err) ||
            launch_cluster_rows<2>(keys, vals, max_count, count, sp, ctrl, st, err) ||
-           launch_cluster_rows<4>(keys, vals, max_count, count, sp, ctrl, st, err) ||
-           (!overlapped && launch_cluster_rows<8>(keys, vals, max_count, count, sp, ctrl, st, err));
+           launch_cluster_rows<4>(keys, vals, max_count, count, sp, ctrl, st, err);
 }
 
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
-                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning,
-                        bool overlapped) {
+                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning) {
     // One cluster where the pairs fit (the bounded-wait hook stalls look-backs, which it has none of).
     if (wait_config().stall_tile == kNoStall) {
         cudaError_t e = cudaSuccess;
         prof_mark(prof_stage, true, st);
-        const bool done = launch_sort_cluster(keys, vals, max_count, count, key_bits, overlapped,
-                                              reinterpret_cast<Ctrl *>(scratch), st, &e);
+        const bool done = launch_sort_cluster(keys, vals, max_count, count, key_bits, reinterpret_cast<Ctrl *>(scratch), st, &e);
         if (done) prof_mark(prof_stage, false, st);
         if (done) return e == cudaSuccess ? cudaGetLastError() : e;
     }
@@ -959,10 +985,11 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     count_launches(1);
     if (max_count == 0) return cudaGetLastError();
     prof_mark(prof_stage, true, st);
-    uint32_t hist_blocks = (max_count + 256 * 4 * 4 - 1) / (256 * 4 * 4);
-    if (hist_blocks > 152 * 8) hist_blocks = 152 * 8;
+    // four keys a thread, up to one resident wave
+    uint32_t hist_blocks = (max_count + kHistThreads * 4 - 1) / (kHistThreads * 4);
+    if (hist_blocks > kHistCtas) hist_blocks = kHistCtas;
     if (tn.hist_blocks) hist_blocks = tn.hist_blocks < 152 * 8 ? tn.hist_blocks : 152 * 8;
-    launch_frame_kernel(sort_hist_kernel, hist_blocks, 256, 0, st, overlap, keys, vals, count, max_count, sp, L.ctrl, L.flags);
+    launch_frame_kernel(sort_hist_kernel, hist_blocks, kHistThreads, 0, st, overlap, keys, vals, count, max_count, sp, L.ctrl, L.flags);
     count_launches(1);
     // Keys of kDepthKeyBits are the render path's float depth keys (1 - ndc.z).
     if (tn.sort_match)
