@@ -217,20 +217,19 @@ struct Model {
         return GS_OK;
     }
 
-    // Preprocess + depth sort of this model for one frame.  `tiles`: the preprocess also stores
-    // each visible splat's tiles for the viewport (binfo), which the binning of a one-model view
-    // gathers instead of the whole splat.
-    gs_status enqueue(const gs_frame_uniforms &u, cudaStream_t st, bool tiles = false) {
+    // Preprocess + depth sort of this model for one frame, its splats written to `out`.  The preprocess
+    // also stores each visible splat's tiles for the viewport (binfo), which the binning gathers
+    // instead of the whole splat.
+    gs_status enqueue(const gs_frame_uniforms &u, gs_splat *out, cudaStream_t st) {
         uint4 *bi = nullptr;
-        if (tiles && n) {
+        if (n) {
             GS_CUDA(binfo.ensure((size_t)n * sizeof(uint4)));
             bi = reinterpret_cast<uint4 *>(binfo.ptr);
         }
         cudaError_t e = launch_preprocess(u, records.ptr, format, n,
                                           has_selection ? (const uint32_t *)selection.ptr : nullptr, invert,
                                           indirect(), indirect() + 4, (uint32_t *)indices.ptr, (float *)depths.ptr,
-                                          gs_depth_capacity(n), (gs_splat *)splats.ptr, pre_scratch.ptr, st, nullptr,
-                                          bi);
+                                          gs_depth_capacity(n), out, pre_scratch.ptr, st, bi);
         if (e != cudaSuccess) return cuda_fail(e, "preprocess launch");
         e = launch_sort((uint32_t *)depths.ptr, (uint32_t *)indices.ptr, n, indirect() + 1, kDepthKeyBits,
                         sort_scratch.ptr, st);
@@ -660,7 +659,7 @@ gs_status viewer_render_locked(gs_viewer *v, uint8_t *target, uint32_t w, uint32
     gs_frame_uniforms u;
     s = gs_frame_uniforms_build(&v->frame.camera, &v->model.model, &v->frame.gt, w, h, &u);
     if (s != GS_OK) return s;
-    s = v->model.enqueue(u, st, true);
+    s = v->model.enqueue(u, (gs_splat *)v->model.splats.ptr, st);
     if (s != GS_OK) return s;
     RasterSegment seg{(const gs_splat *)v->model.splats.ptr, (const uint32_t *)v->model.indices.ptr,
                       v->model.indirect() + 1, v->model.n};
@@ -883,12 +882,22 @@ gs_status multi_render_locked(gs_multi_viewer *v, const std::vector<std::string>
     if (s != GS_OK) return s;
     std::vector<RasterSegment> segs;
     gs_frame_uniforms u{};
+    // Several models' splats go side by side into the raster scratch, one model's into its own buffer.
+    const bool pooled = ms.size() > 1;
+    gs_splat *pool = pooled ? raster_splat_pool(v->frame.raster_scratch.ptr, (uint32_t)total, w, h, v->frame.max_pairs) : nullptr;
     for (Model *m : ms) {
         s = gs_frame_uniforms_build(&v->frame.camera, &m->model, &v->frame.gt, w, h, &u);
         if (s != GS_OK) return s;
-        s = m->enqueue(u, st);
+        gs_splat *out = pooled ? pool : (gs_splat *)m->splats.ptr;
+        s = m->enqueue(u, out, st);
         if (s != GS_OK) return s;
-        segs.push_back(RasterSegment{(const gs_splat *)m->splats.ptr, (const uint32_t *)m->indices.ptr, m->indirect() + 1, m->n});
+        RasterSegment seg{out, (const uint32_t *)m->indices.ptr, m->indirect() + 1, m->n};
+        seg.binfo = reinterpret_cast<const uint4 *>(m->binfo.ptr);
+        seg.binfo_w = w;
+        seg.binfo_h = h;
+        seg.pooled = pooled;
+        segs.push_back(seg);
+        pool += pooled ? m->n : 0;
     }
     if (ms.empty()) {
         gs_model_transform_pod identity{};
@@ -1769,7 +1778,7 @@ gs_status server_launch(gs_server *sv, ServerReq &r, ServerSlot &sl) {
                                             m->has_selection ? (const uint32_t *)m->selection.ptr : nullptr, m->invert,
                                             ind, ind + 4, (uint32_t *)v.indices.ptr, (float *)v.depths.ptr,
                                             gs_depth_capacity(m->n), (gs_splat *)v.splats.ptr, v.pre_scratch.ptr,
-                                            sl.stream, nullptr, reinterpret_cast<uint4 *>(v.binfo.ptr));
+                                            sl.stream, reinterpret_cast<uint4 *>(v.binfo.ptr));
     if (e != cudaSuccess) return cuda_fail(e, "server launch");
     return server_finish(sv, r, sl, target, pitch, u, true);
 }

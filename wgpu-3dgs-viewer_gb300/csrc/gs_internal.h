@@ -68,7 +68,7 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
                               uint32_t n, const uint32_t *selection, int invert, uint32_t *indirect,
                               uint32_t *dispatch, uint32_t *indices, float *depths,
                               uint32_t depth_cap, gs_splat *splats, void *scratch, cudaStream_t st,
-                              const gs_frame_uniforms *u_dev = nullptr, uint4 *binfo = nullptr);
+                              uint4 *binfo = nullptr);
 
 // Several views of one model in one launch (records read once).  A view's scratch is the one
 // launch_preprocess takes for that model; `group` is a zeroed Ctrl-sized block for the launch.
@@ -190,7 +190,13 @@ struct RasterSegment {
     // binfo_h target (indexed by Gaussian index); used when the binning's target matches.
     const uint4 *binfo = nullptr;
     uint32_t binfo_w = 0, binfo_h = 0;
+    // One of several segments, its splats being the raster scratch's own (raster_splat_pool) from the
+    // segment's first rank on: pair values point there, and nothing is copied into draw order.
+    bool pooled = false;
 };
+// Where in the raster scratch the segments of a call can keep their splats (max_splats of them, all
+// segments' capacities one after another).
+gs_splat *raster_splat_pool(void *scratch, uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 size_t raster_scratch_bytes(uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 // exact_exp: 1 = the portable exp (bit-identical with the CPU oracle), 0 = the SFU exp.
 // tiles_at_once: tiles of all views that are rendered side by side with this one (0: it is alone).

@@ -23,7 +23,7 @@ constexpr uint32_t kPreThreads = 128;
 
 struct PreParams {
     gs_frame_uniforms u;
-    const gs_frame_uniforms *u_dev;  // when set (graph-captured batches), uniforms are read here
+    float kx, ky;  // clip_scale of the view
     const uint8_t *records;
     uint32_t n;
     uint32_t ntiles;
@@ -79,6 +79,14 @@ __device__ __forceinline__ float clamp01(float v) { return v > 0.0f ? (v < 1.0f 
 __device__ __forceinline__ float len2(float x, float y) { return sqrtf(x * x + y * y); }
 __device__ __forceinline__ bool cull(float x, float y, float z) {
     return !(x >= -1.0f && y >= -1.0f && z >= 0.0f && x <= 1.0f && y <= 1.0f && z <= 1.0f);
+}
+
+// c / 255 rounded to nearest, c = 0..255, without a division: the quotient from RN(1/255) and one
+// correction by the exact remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Equal to the division for all 256 values (checked exhaustively).
+__device__ __forceinline__ float unorm8(uint32_t c) {
+    const float x = (float)c, r = 1.0f / 255.0f, q = x * r;
+    return fmaf(fmaf(-q, 255.0f, x), r, q);
 }
 
 // Record staged in a padded shared-memory row (16-byte chunks), with the fields every visible
@@ -265,7 +273,7 @@ __device__ __forceinline__ void view_color(const gs_frame_uniforms &u, const Rec
     float res[3];
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch)
-        res[ch] = u.no_sh0 ? 0.5f : (float)((g.color >> (8 * ch)) & 0xFFu) / 255.0f;
+        res[ch] = u.no_sh0 ? 0.5f : unorm8((g.color >> (8 * ch)) & 0xFFu);
     if (u.sh_deg >= 1) {
         float s1[9];
         sh_load<FMT, 0, 9>(g.row, s1);
@@ -316,7 +324,7 @@ __device__ __forceinline__ void view_color(const gs_frame_uniforms &u, const Rec
     }
 #pragma unroll
     for (int ch = 0; ch < 3; ++ch) rgba[ch] = res[ch] > 0.0f ? res[ch] : 0.0f;
-    rgba[3] = (float)((g.color >> 24) & 0xFFu) / 255.0f;
+    rgba[3] = unorm8(g.color >> 24);
 }
 
 // ---- per Gaussian and view -------------------------------------------------------------------
@@ -353,10 +361,14 @@ __device__ __forceinline__ bool gaussian_visible(const gs_frame_uniforms &u, con
     return vis;
 }
 
-// Per-instance vertex work (render.wesl:75-130): the splat record of a visible Gaussian.
+// Pixels per unit of a quad axis, the same for all splats of a view: two divisions that no thread repeats.
+__host__ __device__ __forceinline__ float clip_scale(float viewport, float size) { return (0.5f * viewport) / size; }
+
+// Per-instance vertex work (render.wesl:75-130): the splat record of a visible Gaussian (kx, ky:
+// clip_scale of the view's width and height).
 // With `binfo`, also the splat's tiles for a tiles_x x tiles_y grid, as the binning works them out.
 template <uint32_t FMT>
-__device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, const Rec &g, Proj &pr, gs_splat *out,
+__device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, float kx, float ky, const Rec &g, Proj &pr, gs_splat *out,
                                             uint4 *binfo = nullptr, uint32_t tiles_x = 0, uint32_t tiles_y = 0) {
     float rgba[4];
     view_color<FMT>(u, g, pr.world, rgba);
@@ -388,8 +400,6 @@ __device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, const Re
     } else {
         if (!pr.have_axes) cov2d_axes(u, g.cov3d, p4, u.std_dev_scaled, pr.axes);
         const float *axes = pr.axes;
-        const float kx = (0.5f * W) / u.size[0];
-        const float ky = (0.5f * H) / u.size[1];
         const float a00 = axes[0] * kx, a01 = axes[2] * kx;
         const float a10 = -axes[1] * ky, a11 = -axes[3] * ky;
         const float det = a00 * a11 - a01 * a10;
@@ -516,7 +526,7 @@ __device__ __forceinline__ void stage_finish(uint64_t *s_bar, uint32_t *status) 
     }
 }
 
-template <uint32_t FMT, bool DEV_UNIFORMS>
+template <uint32_t FMT>
 __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_constant__ PreParams P) {
     constexpr uint32_t REC = (FMT == GS_FORMAT_FP32) ? 224u : 128u;
     constexpr uint32_t C16 = REC / 16;  // 16-byte chunks per record
@@ -528,7 +538,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
     __shared__ __align__(16) uint4 s_rec[kPreThreads * ROW16];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ uint32_t s_epoch, s_base, s_limit, s_stall, s_warp[kPreThreads / 32];
-    __shared__ __align__(16) gs_frame_uniforms s_u;
+    const gs_frame_uniforms &u = P.u;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t tile = blockIdx.x;  // look-back predecessors are lower, earlier-dispatched CTAs
     const uint32_t first = tile * kPreThreads;
@@ -542,13 +552,6 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
     // The records were in place before the control block's reset, the kernel before this one, started.
     stage_start<FMT>(s_rec, &s_bar, P.records, first, cnt, pcnt);
     frame_kernel_enter();
-    if constexpr (DEV_UNIFORMS) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(P.u_dev);
-        for (uint32_t i = tid; i < sizeof(gs_frame_uniforms) / 4; i += kPreThreads)
-            reinterpret_cast<uint32_t *>(&s_u)[i] = src[i];
-    }
-    const gs_frame_uniforms &u = DEV_UNIFORMS ? s_u : P.u;
-
     if (tid == 0) {
         s_epoch = *(volatile uint32_t *)&P.ctrl->epoch;
         s_limit = P.ctrl->spin_limit;
@@ -586,7 +589,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
 
     // ---- per-instance vertex work (render.wesl:75-130), written at the Gaussian's index ----
     if (vis && P.splats)
-        write_splat<FMT>(u, g, pr, P.splats + i, P.binfo ? P.binfo + i : nullptr, P.tiles_x, P.tiles_y);
+        write_splat<FMT>(u, P.kx, P.ky, g, pr, P.splats + i, P.binfo ? P.binfo + i : nullptr, P.tiles_x, P.tiles_y);
 
     // ---- global offset: warp 0 looks back over the predecessors' published counts ----
     __syncthreads();
@@ -648,6 +651,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_views_kernel(const __g
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ __align__(16) gs_frame_uniforms s_u;
     __shared__ float s_key[kPreMaxViews][kPreThreads];
+    __shared__ float s_k[2];
     __shared__ uint32_t s_bal[kPreMaxViews][NW];
     __shared__ uint32_t s_base[kPreMaxViews];
     __shared__ uint32_t s_epoch[kPreMaxViews];
@@ -679,6 +683,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_views_kernel(const __g
         const PreView &V = P.views[v];
         for (uint32_t k = tid; k < sizeof(gs_frame_uniforms) / 4; k += kPreThreads)
             reinterpret_cast<uint32_t *>(&s_u)[k] = reinterpret_cast<const uint32_t *>(V.u)[k];
+        if (tid < 2) s_k[tid] = clip_scale(V.u->viewport[tid], V.u->size[tid]);
         __syncthreads();
         bool vis = false;
         float key = 0.0f;
@@ -687,7 +692,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_views_kernel(const __g
         const uint32_t bal = __ballot_sync(0xFFFFFFFFu, vis);
         if (lane == 0) s_bal[v][warp] = bal;
         s_key[v][tid] = key;
-        if (vis && V.splats) write_splat<FMT>(s_u, g, pr, V.splats + i);
+        if (vis && V.splats) write_splat<FMT>(s_u, s_k[0], s_k[1], g, pr, V.splats + i);
         __syncthreads();  // s_bal[v] complete; s_u free for the next view
         if (tid == 0) {
             uint32_t total = 0;
@@ -852,7 +857,7 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
                               uint32_t n, const uint32_t *selection, int invert, uint32_t *indirect,
                               uint32_t *dispatch, uint32_t *indices, float *depths,
                               uint32_t depth_cap, gs_splat *splats, void *scratch, cudaStream_t st,
-                              const gs_frame_uniforms *u_dev, uint4 *binfo) {
+                              uint4 *binfo) {
     Ctrl *ctrl = reinterpret_cast<Ctrl *>(scratch);
     uint64_t *flags = reinterpret_cast<uint64_t *>((uint8_t *)scratch + align_up(sizeof(Ctrl), 256));
     const bool overlap = frame_launch_overlaps(st);
@@ -865,7 +870,8 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
     }
     PreParams P;
     P.u = u;
-    P.u_dev = u_dev;
+    P.kx = clip_scale(u.viewport[0], u.size[0]);
+    P.ky = clip_scale(u.viewport[1], u.size[1]);
     P.records = reinterpret_cast<const uint8_t *>(records);
     P.n = n;
     P.ntiles = (n + kPreThreads - 1) / kPreThreads;
@@ -877,38 +883,23 @@ cudaError_t launch_preprocess(const gs_frame_uniforms &u, const void *records, u
     P.depths = depths;
     P.depth_cap = depth_cap;
     P.splats = splats;
-    // the tile records need the viewport on the host (graph-captured uniforms are not read here)
-    P.binfo = u_dev ? nullptr : binfo;
+    P.binfo = binfo;
     P.tiles_x = ((uint32_t)u.viewport[0] + GS_TILE - 1) / GS_TILE;
     P.tiles_y = ((uint32_t)u.viewport[1] + GS_TILE - 1) / GS_TILE;
     P.ctrl = ctrl;
     P.flags = flags;
     prof_mark(kProfPreprocess, true, st);
     count_launches(1);
-    if (u_dev) {
-        switch (format) {
-            case GS_FORMAT_FP32:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_FP32, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-            case GS_FORMAT_HALF_SH_FP16:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_FP16, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-            default:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_BF16, true>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-        }
-    } else {
-        switch (format) {
-            case GS_FORMAT_FP32:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_FP32, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-            case GS_FORMAT_HALF_SH_FP16:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_FP16, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-            default:
-                launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_BF16, false>, P.ntiles, kPreThreads, 0, st, overlap, P);
-                break;
-        }
+    switch (format) {
+        case GS_FORMAT_FP32:
+            launch_frame_kernel(preprocess_kernel<GS_FORMAT_FP32>, P.ntiles, kPreThreads, 0, st, overlap, P);
+            break;
+        case GS_FORMAT_HALF_SH_FP16:
+            launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_FP16>, P.ntiles, kPreThreads, 0, st, overlap, P);
+            break;
+        default:
+            launch_frame_kernel(preprocess_kernel<GS_FORMAT_HALF_SH_BF16>, P.ntiles, kPreThreads, 0, st, overlap, P);
+            break;
     }
     prof_mark(kProfPreprocess, false, st);
     return cudaGetLastError();
