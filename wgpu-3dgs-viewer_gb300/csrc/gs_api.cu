@@ -1357,7 +1357,7 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
                 uint32_t *ind = reinterpret_cast<uint32_t *>(v.control.ptr);
                 const RasterSegment seg{(const gs_splat *)v.splats.ptr, (const uint32_t *)v.indices.ptr, ind + 1, ms[i]->n};
                 err = launch_binning_ranges(&seg, 1, views[i].width, views[i].height, v.max_pairs, v.raster_scratch.ptr,
-                                            b->capture);
+                                            b->capture, true);
             }
         }
         if (err == cudaSuccess && b->tuning.raster_grid)

@@ -137,10 +137,10 @@ PassSplit even_split_max(uint32_t key_bits, uint32_t max_digit);
 // 1024 / n words a pass beyond (enough for the narrower digits that more passes use).
 __host__ __device__ inline uint32_t hist_stride(uint32_t npasses) { return npasses <= 4 ? 256u : 1024u / npasses; }
 
-// Packed (uint2 {key, value}) in-place sort for internal pair lists whose digit histograms
-// (split by tile_split) the producer accumulated into the control block `ctrl`: as counts, or (hist_scanned) already as exclusive digit offsets.  Its
-// look-back flags (sort_pairs_flag_words of them) lie in the flag arena of the area whose
-// control block `owner` is; `alt` holds max_count pairs.
+// Packed (uint2 {key, value}) in-place sort for internal pair lists whose producer left the exclusive
+// digit offsets (split by tile_split) in the control block `ctrl`.  Its look-back flags
+// (sort_pairs_flag_words of them) lie in the flag arena of the area whose control block `owner` is;
+// `alt` holds max_count pairs.
 size_t sort_pairs_flag_words(uint32_t max_count, uint32_t key_bits);
 // The split of a tile-pair sort (producers of its digit histograms must use the same one).
 PassSplit tile_split(uint32_t key_bits);
@@ -152,7 +152,6 @@ struct SortSegment {
     const uint32_t *count;      // device pair count
     uint32_t max_count;
     uint32_t shift[2], bits[2]; // tile_split of the view's tile-id bits
-    uint32_t hist_scanned;      // digit histograms already exclusive offsets
     Ctrl *ctrl;                 // the view's tile-sort control block
     Ctrl *owner;                // the view's raster control block (its status takes the sort's)
     uint64_t *flags[2];         // look-back flags of each pass
@@ -164,13 +163,15 @@ uint32_t sort_pairs_blocks(uint32_t max_count);
 cudaError_t launch_sort_segments(const SortSegment *segs_dev, const uint32_t *block_base_dev, uint32_t nseg,
                                  uint32_t total_blocks, cudaStream_t st);
 cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *count, uint32_t key_bits, Ctrl *ctrl,
-                              uint64_t *flags, uint2 *alt, cudaStream_t st, bool hist_scanned);
+                              uint64_t *flags, uint2 *alt, cudaStream_t st);
 
 // The tile sort on compact items, in two passes (key_bits <= 16): items hold the tile's high digit
 // (tile >> tile_split.bits[0]) above value_bits bits of value, `low` the low digits; the digit offsets
-// in `ctrl` are exclusive.  The sorted values end up in `items`.
+// in `ctrl` are exclusive.  The sorted values end up in `items`.  With tile_counts (zeroed, one for each of
+// the target's target_tiles tiles) each tile's pairs are counted.
 cudaError_t launch_sort_items(uint32_t *items, const uint8_t *low, uint32_t *alt, uint32_t max_count, const uint32_t *count,
-                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st);
+                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st,
+                              uint32_t *tile_counts, uint32_t target_tiles);
 
 // ---- K3 binning + K4 raster (gs_raster.cu) ----
 // The only frame uniforms binning and rasterisation read: camera, model and SH fields never
@@ -234,10 +235,10 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
 SortSegment tile_sort_segment(const RasterSegment *segs, uint32_t nseg, uint32_t width, uint32_t height,
                               uint32_t max_pairs, void *scratch);
 bool tile_sort_segmentable(uint32_t width, uint32_t height);
-// After the view's tile sort: tile ranges from the sorted pairs where the target has more tiles
-// than the counting path covers (nothing otherwise).
+// After the view's tile sort: tile ranges where the target has more tiles than the counting path covers
+// (nothing otherwise), from the tile counts or (segmented, as in raster_job) from the sorted pairs.
 cudaError_t launch_binning_ranges(const RasterSegment *segs, uint32_t nseg, uint32_t width, uint32_t height,
-                                  uint32_t max_pairs, void *scratch, cudaStream_t st);
+                                  uint32_t max_pairs, void *scratch, cudaStream_t st, bool segmented = false);
 // Binning, tile sort and tile ranges of one view (everything launch_raster does before the
 // rasteriser itself).
 cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint32_t width,

@@ -38,7 +38,8 @@ struct RasterLayout {
     uint32_t *offsets;   // per draw rank: tile count, then its exclusive scan
     uint2 *pairs;        // (tile, value), capacity max_pairs
     uint2 *ranges;       // per tile [start, end)
-    uint32_t *counts;    // per tile pair count (counting path; null above kCountTiles tiles)
+    uint32_t *counts;    // per tile pair count
+    bool counting;       // the emission counts them (up to kCountTiles tiles)
     uint32_t *blockcounts;  // per emit CTA and tile pair count (counting path)
     uint32_t *order;     // tiles by descending pair count: the rasteriser's launch order (counting path)
     uint2 *sort_alt;     // the tile sort's ping-pong buffer, capacity max_pairs
@@ -50,7 +51,7 @@ struct RasterLayout {
 
 // Up to kCountTiles tiles (1080p has 8160), the emit kernel counts pairs per tile in shared
 // memory; the per-tile counts give the tile-sort histograms and, scanned, the tile ranges.
-// Larger targets count per digit instead and find the ranges in the sorted pairs.
+// Larger targets count per digit instead, and the tile sort's second pass counts per tile.
 constexpr uint32_t kCountTiles = 8192;
 constexpr uint32_t kEmitBlocks = 152 * 8;
 
@@ -114,19 +115,20 @@ static RasterLayout raster_layout(void *scratch, uint32_t max_splats, uint32_t w
     p += align_up((size_t)max_pairs * 8, 256);
     L.ranges = reinterpret_cast<uint2 *>(p);
     p += align_up((size_t)L.ntiles * sizeof(uint2), 256);
-    L.counts = L.blockcounts = L.order = nullptr;
-    if (L.ntiles <= kCountTiles) {
-        L.counts = reinterpret_cast<uint32_t *>(p);
-        p += align_up((size_t)L.ntiles * 4, 256);
+    L.counts = reinterpret_cast<uint32_t *>(p);
+    p += align_up((size_t)L.ntiles * 4, 256);
+    L.counting = L.ntiles <= kCountTiles;
+    L.blockcounts = L.order = nullptr;
+    if (L.counting) {
         L.order = reinterpret_cast<uint32_t *>(p);
         p += align_up((size_t)L.ntiles * 4, 256);
         L.blockcounts = reinterpret_cast<uint32_t *>(p);
         p += align_up((size_t)kEmitBlocks * L.ntiles * 4, 256);
     }
     L.sort_alt = reinterpret_cast<uint2 *>(p);
-    // The counting path's tiles take two digits; their high digit leaves 26 bits or more for a value.
+    // Up to 65,536 tiles take two digits, whose high one leaves 24 bits or more for a value.
     const uint32_t bits = bits_for(max_splats);
-    L.value_bits = L.counts && bits < 32 && tile_split(L.key_bits).bits[1] + bits <= 32 ? bits : 0u;
+    L.value_bits = L.key_bits <= 16 && bits < 32 && tile_split(L.key_bits).bits[1] + bits <= 32 ? bits : 0u;
     return L;
 }
 
@@ -137,9 +139,8 @@ size_t raster_scratch_bytes(uint32_t max_splats, uint32_t w, uint32_t h, uint32_
     return 2 * align_up(sizeof(Ctrl), 256) + align_up(arena * sizeof(uint64_t), 256) +
            align_up((size_t)max_splats * sizeof(gs_splat), 256) + align_up((size_t)max_splats * 16, 256) +
            align_up((size_t)max_splats * 4 + 16, 256) + align_up((size_t)max_pairs * 8, 256) +
-           align_up((size_t)tiles * sizeof(uint2), 256) +
-           (tiles <= kCountTiles ? 2 * align_up((size_t)tiles * 4, 256) +
-                                       align_up((size_t)kEmitBlocks * tiles * 4, 256)
+           align_up((size_t)tiles * sizeof(uint2), 256) + align_up((size_t)tiles * 4, 256) +
+           (tiles <= kCountTiles ? align_up((size_t)tiles * 4, 256) + align_up((size_t)kEmitBlocks * tiles * 4, 256)
                                  : 0) +
            align_up((size_t)max_pairs * 8, 256);
 }
@@ -338,21 +339,31 @@ __device__ __forceinline__ uint32_t kept_tile_place(uint32_t m, uint32_t w, uint
 // a close-up cover thousands of tiles each and lie next to one another in draw order (400k splats at
 // 1366x768 from inside the scene: 97 us by ranks, 16 by pairs).  It finds its first rank by a 32-way
 // search of the offsets, then goes through windows of 32 ranks: pair r of a window goes to lane r mod
-// 32, which finds its splat by binary search over the warp's exclusive count prefix and its tile from
-// the pair's place in the splat's rectangle (its kept tiles skip the dropped corners).  Stores are
-// consecutive.  Also accumulates the tile counts (or the tile-key digit histograms of the tile sort) in
+// 32, which finds its splat among the window's in shared memory and its tile from the pair's place in
+// the splat's rectangle (its kept tiles skip the dropped corners).  Stores are consecutive.  Bound by
+// issue: 24.7M pairs took 136 us with the splat found by a binary search of shuffles and its fields by
+// seven more, 126 with an or-reduction and three shared loads; five CTAs an SM, as six (40 registers)
+// spill time into the digit counts of large targets (3M / 4K: 226 us a binning, 237).  Also accumulates the tile counts (or the tile-key digit histograms of the tile sort) in
 // shared memory; each CTA hands its shared bins on once.
 // COUNTS: one counter per tile, else the digit histograms; COMPACT: items and low digits, else pairs.
 constexpr uint32_t kEmitMin = 96;  // pairs of a warp's share at least (its search costs about 3 us)
 
+// A warp's window of 32 ranks.
+struct EmitWindow {
+    uint4 rect[32], at[32];
+    uint8_t nth[32];
+};
+
 template <bool COUNTS, bool COMPACT>
-__global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
+__global__ void __launch_bounds__(kBinThreads, 5) bin_emit_kernel(
     const uint4 *__restrict__ info, const uint32_t *__restrict__ offsets, const uint32_t *count, uint32_t max_count,
     uint2 *__restrict__ pairs, uint32_t max_pairs, uint32_t value_bits, uint32_t tiles_x, uint32_t ntiles, Ctrl *ctrl,
     Ctrl *sort_ctrl, const PassSplit split, uint32_t *__restrict__ blockcounts) {
     extern __shared__ uint32_t s_bins[];
+    __shared__ EmitWindow s_win[kBinThreads / 32];
     const uint32_t nbins = COUNTS ? ntiles : 4u * 256u;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, lt = lanemask_lt(), le = lt | (1u << lane);
+    EmitWindow &win = s_win[tid >> 5];
     for (uint32_t i = tid; i < nbins; i += kBinThreads) s_bins[i] = 0u;
     frame_kernel_enter();
     const uint32_t n = count ? min(*count, max_count) : max_count;
@@ -424,33 +435,31 @@ __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
                 if (lane >= d) incl += y;
             }
             const uint32_t excl = incl - cnt, run = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            // a lane's rectangle: x0 | y0 << 16, width, kept-tile mask, value, 1 / width
+            // The window's splats in shared memory, and its lanes that have pairs in order: pair r of the
+            // run belongs to the last of them that starts at or before r, which a round counts with one
+            // or-reduction of its 32 places' starts.
             const uint32_t iw = in.y & 0xFFFFu;
-            const float inv_w = iw ? 1.0f / (float)iw : 0.0f;
+            const uint32_t some = __ballot_sync(0xFFFFFFFFu, cnt != 0u);
+            __syncwarp();
+            win.rect[lane] = in;  // x0 | y0 << 16, w | h << 16, kept-tile mask, value
+            win.at[lane] = make_uint4(from - excl, off, __float_as_uint(iw ? 1.0f / (float)iw : 0.0f), 0u);
+            if (cnt) win.nth[__popc(some & lt)] = (uint8_t)lane;
+            __syncwarp();
+            uint32_t before = 0;  // lanes of `some` that start ahead of the round
             for (uint32_t r0 = 0; r0 < run; r0 += 32) {
-                const uint32_t r = r0 + lane;
-                // the largest lane whose run starts at or before r (a lane with no pairs shares its
-                // start with the next lane, so the search lands on a lane that has pairs)
-                uint32_t src = 0;
-#pragma unroll
-                for (uint32_t step = 16; step >= 1; step >>= 1) {
-                    const uint32_t e = __shfl_sync(0xFFFFFFFFu, excl, src + step);
-                    if (e <= r) src += step;
-                }
-                const uint32_t sx = __shfl_sync(0xFFFFFFFFu, in.x, src), swh = __shfl_sync(0xFFFFFFFFu, in.y, src);
-                const uint32_t sw = swh & 0xFFFFu;  // in.y: w | h << 16
-                const uint32_t smask = __shfl_sync(0xFFFFFFFFu, in.z, src), sval = __shfl_sync(0xFFFFFFFFu, in.w, src);
-                const float sinv = __shfl_sync(0xFFFFFFFFu, inv_w, src);
-                const uint32_t at = __shfl_sync(0xFFFFFFFFu, from - excl, src) + r;
-                const uint32_t soff = __shfl_sync(0xFFFFFFFFu, off, src);
+                const uint32_t r = r0 + lane, place = excl - r0;
+                const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, cnt && place < 32u ? 1u << place : 0u);
+                const uint32_t src = win.nth[before + __popc(starts & le) - 1u];
+                before += __popc(starts);
                 if (r < run) {
-                    const uint32_t local = at - soff;  // place among the splat's kept tiles
-                    // in.z: tiles kept of a rectangle of at most 16 (bit ty·w + tx); 0 = all of it
-                    const uint32_t pos = smask ? kept_tile_place(smask, sw, swh >> 16, local) : local;
+                    const uint4 rc = win.rect[src], ra = win.at[src];
+                    const uint32_t sw = rc.y & 0xFFFFu, at = ra.x + r, local = at - ra.y;  // place among its kept tiles
+                    // rc.z: tiles kept of a rectangle of at most 16 (bit ty·w + tx); 0 = all of it
+                    const uint32_t pos = rc.z ? kept_tile_place(rc.z, sw, rc.y >> 16, local) : local;
                     // row = floor(pos / w), exact in float: pos < 2^24 and the error of 1/w is
                     // far below the 1/w gap between pos/w and the next integer
-                    const uint32_t ty = (uint32_t)(((float)pos + 0.5f) * sinv), tx = pos - ty * sw;
-                    emit(((sx >> 16) + ty) * tiles_x + (sx & 0xFFFFu) + tx, sval, at);
+                    const uint32_t ty = (uint32_t)(((float)pos + 0.5f) * __uint_as_float(ra.z)), tx = pos - ty * sw;
+                    emit(((rc.x >> 16) + ty) * tiles_x + (rc.x & 0xFFFFu) + tx, rc.w, at);
                 }
             }
             if (!more) break;
@@ -475,6 +484,85 @@ __global__ void __launch_bounds__(kBinThreads) bin_emit_kernel(
             const uint32_t v = s_bins[p * 256u + tid];
             if (v) atomicAdd(&sort_ctrl->hist[p][tid], v);
         }
+        // the last CTA to finish turns the digit histograms into exclusive offsets, a warp a pass
+        __shared__ uint32_t s_last;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(&sort_ctrl->ticket[7], 1u) == gridDim.x - 1u ? 1u : 0u;
+        __syncthreads();
+        const uint32_t p = tid >> 5;
+        if (s_last && p < split.n) {
+            __threadfence();
+            uint32_t v[8], sum = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) sum += v[j] = __ldcg(&sort_ctrl->hist[p][lane * 8u + j]);
+            uint32_t run = sum;
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, run, d);
+                if (lane >= d) run += y;
+            }
+            run -= sum;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                sort_ctrl->hist[p][lane * 8u + j] = run;
+                run += v[j];
+            }
+        }
+    }
+}
+
+// [start, end) of every tile from its pair count where the target has too many tiles for
+// tile_scan_kernel: one CTA, 8192 tiles at a time (4K: 4 rounds, 17 us; 52 us finding the ends in the
+// sorted pairs).
+__global__ void __launch_bounds__(1024) tile_starts_kernel(const uint32_t *__restrict__ counts, uint32_t ntiles,
+                                                           uint2 *__restrict__ ranges) {
+    __shared__ __align__(16) uint32_t s_v[8192 + 4];
+    __shared__ uint32_t s_w[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    frame_kernel_enter();
+    uint32_t before = 0;
+    for (uint32_t t0 = 0; t0 < ntiles; t0 += 8192u) {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t t = tid + 1024u * j;
+            s_v[t] = t0 + t < ntiles ? counts[t0 + t] : 0u;
+        }
+        __syncthreads();
+        uint4 a = *reinterpret_cast<const uint4 *>(&s_v[8u * tid]), b = *reinterpret_cast<const uint4 *>(&s_v[8u * tid + 4u]);
+        const uint32_t sum = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+        uint32_t inc = sum;
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o) inc += x;
+        }
+        if (lane == 31) s_w[warp] = inc;
+        __syncthreads();
+        uint32_t run = before + inc - sum, all = 0;
+        for (uint32_t w = 0; w < 32; ++w) {
+            const uint32_t x = s_w[w];
+            if (w < warp) run += x;
+            all += x;
+        }
+        const uint32_t c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t first[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            first[j] = run;
+            run += c[j];
+        }
+        *reinterpret_cast<uint4 *>(&s_v[8u * tid]) = make_uint4(first[0], first[1], first[2], first[3]);
+        *reinterpret_cast<uint4 *>(&s_v[8u * tid + 4u]) = make_uint4(first[4], first[5], first[6], first[7]);
+        before += all;
+        if (tid == 0) s_v[8192] = before;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t t = tid + 1024u * j;
+            if (t0 + t < ntiles) ranges[t0 + t] = make_uint2(s_v[t], s_v[t + 1]);
+        }
+        __syncthreads();
     }
 }
 
@@ -1420,7 +1508,7 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
     // reads a flag and the arena mark stays.
     prof_mark(kProfBin, true, st);
     const bool overlap = frame_launch_overlaps(st);
-    launch_frame_kernel(raster_init_kernel, 1 + (L.counts ? (L.ntiles + 1023) / 1024 : 0), 256, 0, st, overlap, L.ctrl,
+    launch_frame_kernel(raster_init_kernel, 1 + (L.ntiles + 1023) / 1024, 256, 0, st, overlap, L.ctrl,
                         L.sort_ctrl, max_splats ? L.arena_words : kKeepArena, wait_config(), L.counts, L.ntiles);
     count_launches(1);
     const PassSplit split = tile_split(L.key_bits);
@@ -1448,7 +1536,7 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
     }
     // One resident wave at most (and the per-CTA count area): a second, late wave would stretch the
     // kernel; two CTAs an SM at least, as few splats may cover many tiles.
-    const size_t emit_smem = L.counts ? (size_t)L.ntiles * 4u : 4u * 256u * 4u;
+    const size_t emit_smem = L.counting ? (size_t)L.ntiles * 4u : 4u * 256u * 4u;
     const bool compact = L.value_bits && !segmented;
     auto emit = [&](auto kernel) {
         uint32_t wave = resident_ctas(kernel, kBinThreads, emit_smem);
@@ -1458,14 +1546,14 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
                             max_pairs, L.value_bits, L.tiles_x, L.ntiles, L.ctrl, L.sort_ctrl, split, L.blockcounts);
         return grid;
     };
-    if (L.counts) {
+    if (L.counting) {
         const uint32_t grid = compact ? emit(bin_emit_kernel<true, true>) : emit(bin_emit_kernel<true, false>);
         launch_frame_kernel(tile_count_kernel, dim3((L.ntiles + 255) / 256, kCountSlices), 256, 0, st, overlap, L.blockcounts,
                             grid, L.ntiles, L.counts);
         launch_frame_kernel(tile_scan_kernel, 1, 1024, 0, st, overlap, L.counts, L.ntiles, L.ranges, L.order, L.sort_ctrl, split);
         count_launches(3);
     } else {
-        emit(bin_emit_kernel<false, false>);
+        compact ? emit(bin_emit_kernel<false, true>) : emit(bin_emit_kernel<false, false>);
         count_launches(1);
     }
     prof_mark(kProfBin, false, st);
@@ -1488,7 +1576,6 @@ SortSegment tile_sort_segment(const RasterSegment *segs, uint32_t nseg, uint32_t
         S.shift[p] = split.shift[p];
         S.bits[p] = split.bits[p];
     }
-    S.hist_scanned = L.counts ? 1u : 0u;
     S.ctrl = L.sort_ctrl;
     S.owner = L.ctrl;
     S.flags[0] = L.sort_flags;
@@ -1502,23 +1589,25 @@ bool tile_sort_segmentable(uint32_t W, uint32_t H) {
 }
 
 cudaError_t launch_binning_ranges(const RasterSegment *segs, uint32_t nseg, uint32_t W, uint32_t H, uint32_t max_pairs,
-                                  void *scratch, cudaStream_t st) {
+                                  void *scratch, cudaStream_t st, bool segmented) {
     uint32_t max_splats = 0;
     for (uint32_t s = 0; s < nseg; ++s) max_splats += segs[s].max_count;
     const RasterLayout L = raster_layout(scratch, max_splats, W, H, max_pairs);
-    cudaError_t e = cudaSuccess;
-    if (L.ntiles > 0 && !L.counts) {  // more tiles than the counting path covers: ranges from the sorted pairs
-        prof_mark(kProfRanges, true, st);
-        e = cudaMemsetAsync(L.ranges, 0, (size_t)L.ntiles * sizeof(uint2), st);
+    if (L.ntiles == 0 || L.counting) return cudaSuccess;
+    prof_mark(kProfRanges, true, st);
+    if (L.value_bits && !segmented) {
+        launch_frame_kernel(tile_starts_kernel, 1, 1024, 0, st, frame_launch_overlaps(st), L.counts, L.ntiles, L.ranges);
+    } else {
+        const cudaError_t e = cudaMemsetAsync(L.ranges, 0, (size_t)L.ntiles * sizeof(uint2), st);
         if (e != cudaSuccess) return e;
         uint32_t rblocks = (max_pairs + 255) / 256;
         if (rblocks > 152 * 8) rblocks = 152 * 8;
         if (rblocks == 0) rblocks = 1;
         launch_frame_kernel(tile_ranges_kernel, rblocks, 256, 0, st, frame_launch_overlaps(st), L.pairs, L.ctrl, L.ranges,
                             L.ntiles);
-        prof_mark(kProfRanges, false, st);
-        count_launches(1);
     }
+    prof_mark(kProfRanges, false, st);
+    count_launches(1);
     return cudaGetLastError();
 }
 
@@ -1531,13 +1620,12 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
     cudaError_t e = launch_binning_front(segs, nseg, u, W, H, max_pairs, scratch, st);
     if (e != cudaSuccess) return e;
     prof_mark(kProfTileSort, true, st);
-    // counting path: tile_scan wrote the digit offsets already scanned; else the emit's counts
     if (L.value_bits)
         e = launch_sort_items(L.items(), L.low(max_pairs), reinterpret_cast<uint32_t *>(L.sort_alt), max_pairs,
-                              &L.ctrl->count, L.key_bits, L.value_bits, L.sort_ctrl, L.sort_flags, st);
+                              &L.ctrl->count, L.key_bits, L.value_bits, L.sort_ctrl, L.sort_flags, st,
+                              L.counting ? nullptr : L.counts, L.ntiles);
     else
-        e = launch_sort_pairs(L.pairs, max_pairs, &L.ctrl->count, L.key_bits, L.sort_ctrl, L.sort_flags, L.sort_alt, st,
-                              L.counts != nullptr);
+        e = launch_sort_pairs(L.pairs, max_pairs, &L.ctrl->count, L.key_bits, L.sort_ctrl, L.sort_flags, L.sort_alt, st);
     prof_mark(kProfTileSort, false, st);
     if (e != cudaSuccess) return e;
     return launch_binning_ranges(segs, nseg, W, H, max_pairs, scratch, st);

@@ -14,6 +14,7 @@
 // can be enqueued (or graph-captured) without a host round trip.
 #include <atomic>
 #include <mutex>
+#include <utility>
 
 #include "gs300.h"
 #include "gs_internal.h"
@@ -263,8 +264,7 @@ template <bool IN_PACKED, bool OUT_PACKED, bool MATCH>
 __device__ __forceinline__ void sort_pass_block(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
-    uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags,
-    uint32_t hist_scanned, uint32_t block) {
+    uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags, uint32_t block) {
     extern __shared__ uint2 s_kv[];  // kTileKeys pairs (dynamic)
     __shared__ uint32_t s_whist[kSortWarps][256];
     __shared__ uint32_t s_start[256];
@@ -344,13 +344,11 @@ __device__ __forceinline__ void sort_pass_block(
     uint64_t *f = flags + (size_t)tile * fstride + d;
     if (live) publish_flag(f, tile, s_stall, pack_flag(epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, pub));
 
-    uint32_t blk_total, hist_total;
+    uint32_t blk_total;
     const uint32_t start = block_scan_excl<kSortWarps>(total, s_tmp, &blk_total);
-    // the digit's first place in the output: the histograms hold exclusive offsets already
-    // when their producer scanned them (hist_scanned is uniform over the grid)
-    // (pass histogram at flat offset hoff; digits above dmask hold no key)
-    const uint32_t hv = live ? (&ctrl->hist[0][0])[hoff + d] : 0u;
-    const uint32_t goff = hist_scanned ? hv : block_scan_excl<kSortWarps>(hv, s_tmp, &hist_total);
+    // the digit's first place in the output: the histograms' producer left exclusive offsets (pass
+    // histogram at flat offset hoff; digits above dmask hold no key)
+    const uint32_t goff = live ? (&ctrl->hist[0][0])[hoff + d] : 0u;
     uint32_t prefix = 0;
     if (tile > 0 && live) {
         prefix = look_back_digit(flags + d, tile, epoch, &ctrl->status, fstride, s_limit);
@@ -407,16 +405,20 @@ __device__ __forceinline__ void sort_pass_block(
 // as its output is grouped by the low digit, nobody needs it again; the second sorts by the words' high
 // digit and writes the values alone, all that the rasteriser reads of a pair.  5 + 4 + 4 + 4 bytes a
 // pair instead of 8 each time, half the registers and shared memory of a pair block (three CTAs an
-// SM), and no key to decode twice.
+// SM), and no key to decode twice (6M / 1080p: 278 us as pairs, 228).
+// TALLY (second pass): also counts each tile's pairs, which the emission does not for targets of many
+// tiles.  A block's items have the low digit of the first pass's run they lie in, mostly one for the
+// whole block, whose digit counts are then its tiles' counts.
 constexpr uint32_t kItemCtasPerSm = 3;
 template <bool FIRST>
 constexpr size_t kItemDynSmem = kTileKeys * sizeof(uint32_t) + (FIRST ? kTileKeys : 0);
 
-template <bool FIRST>
+template <bool FIRST, bool TALLY>
 __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
     tile_pass_kernel(const uint32_t *__restrict__ in, const uint8_t *__restrict__ low, uint32_t *__restrict__ out,
                      const uint32_t *count, uint32_t max_count, uint32_t hoff, uint32_t value_bits,
-                     uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags) {
+                     uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags, uint32_t low_bits,
+                     uint32_t *__restrict__ tile_counts, uint32_t target_tiles) {
     extern __shared__ __align__(16) uint8_t item_smem[];
     uint32_t *s_item = reinterpret_cast<uint32_t *>(item_smem);
     uint8_t *s_low = item_smem + kTileKeys * sizeof(uint32_t);  // FIRST: the digit of each reordered item
@@ -479,6 +481,34 @@ __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
     const uint32_t fstride = dmask + 1u;
     uint64_t *f = flags + (size_t)tile * fstride + d;
     if (live) publish_flag(f, tile, s_stall, pack_flag(epoch, tile == 0 ? kFlagPrefix : kFlagAggregate, pub));
+    if constexpr (TALLY) {
+        __shared__ uint32_t s_run[256];  // first places of the low digits' runs
+        const uint32_t lows = 1u << low_bits, at0 = tile * kTileKeys, at1 = min(n, at0 + kTileKeys) - 1u;
+        const uint32_t run = tid < lows ? ctrl->hist[0][tid] : 0xFFFFFFFFu;
+        if (tid < 256u) s_run[tid] = run;
+        // the last run that starts at or before a place holds it
+        const uint32_t lo0 = max(1, __syncthreads_count(run <= at0)) - 1u, lo1 = max(1, __syncthreads_count(run <= at1)) - 1u;
+        auto tally = [&](uint32_t high, uint32_t lo, uint32_t c) {
+            const uint32_t t = (high << low_bits) | lo;
+            if (t < target_tiles) atomicAdd(&tile_counts[t], c);
+            else atomicOr(&ctrl->status, kStatusBounds);  // pairs of an emission that gave up
+        };
+        if (lo0 == lo1) {
+            if (live && pub) tally(d, lo0, pub);
+        } else {
+            for (uint32_t i = 0; i < kSortRows; ++i) {
+                const uint32_t pos = base + i * 32u + lane;
+                if (pos >= n) break;
+                uint32_t lo = lo0, hi = lo1;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1u) >> 1;
+                    if (s_run[mid] <= pos) lo = mid;
+                    else hi = mid - 1u;
+                }
+                tally((in[pos] >> value_bits) & dmask, lo, 1u);
+            }
+        }
+    }
     uint32_t blk_total;
     const uint32_t start = block_scan_excl<kSortWarps>(total, s_tmp, &blk_total);
     const uint32_t goff = live ? (&ctrl->hist[0][0])[hoff + d] : 0u;  // exclusive digit offsets
@@ -520,11 +550,10 @@ template <bool IN_PACKED, bool OUT_PACKED, bool MATCH>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_pass_kernel(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
-    uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags,
-    uint32_t hist_scanned) {
+    uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags) {
     // look-back predecessors are lower, earlier-dispatched CTAs
     sort_pass_block<IN_PACKED, OUT_PACKED, MATCH>(kin, vin, pin, kout, vout, pout, count, max_count, hoff, shift,
-                                                  digit_bits, ctrl, flags, hist_scanned, blockIdx.x);
+                                                  digit_bits, ctrl, flags, blockIdx.x);
 }
 
 // One pass of many independent packed pair sorts in a single launch (a segmented sort): segment v
@@ -544,8 +573,7 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm)
     const uint2 *in = pass ? S.alt : S.data;
     uint2 *out = pass ? S.data : S.alt;
     sort_pass_block<true, true, false>(nullptr, nullptr, in, nullptr, nullptr, out, S.count, S.max_count,
-                                       pass * hist_stride(2), S.shift[pass], S.bits[pass], S.ctrl, S.flags[pass],
-                                       S.hist_scanned, blockIdx.x - block_base[lo]);
+                                       pass * hist_stride(2), S.shift[pass], S.bits[pass], S.ctrl, S.flags[pass], blockIdx.x - block_base[lo]);
 }
 
 // Each segment's sort status into the control block of the area it belongs to.
@@ -686,19 +714,18 @@ static void launch_sort_passes(uint32_t *keys, uint32_t *vals, uint32_t max_coun
     uint64_t *f = L.flags;
     if (npasses == 1) {
         launch_frame_kernel(sort_pass_kernel<false, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
-            keys, vals, nullptr, nullptr, nullptr, L.alt_a, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f, 1u);
+            keys, vals, nullptr, nullptr, nullptr, L.alt_a, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f);
         launch_frame_kernel(unpack_pairs_kernel, grid_for(max_count), 256, 0, st, overlap, L.alt_a, keys, vals, count, max_count);
         count_launches(2);
         return;
     }
     uint2 *src = L.alt_a, *dst = L.alt_b;
     launch_frame_kernel(sort_pass_kernel<false, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
-        keys, vals, nullptr, nullptr, nullptr, src, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f, 1u);
+        keys, vals, nullptr, nullptr, nullptr, src, count, max_count, 0, sp.shift[0], sp.bits[0], L.ctrl, f);
     f += (size_t)L.ntiles << sp.bits[0];
     for (uint32_t p = 1; p + 1 < npasses; ++p) {
         launch_frame_kernel(sort_pass_kernel<true, true, MATCH>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
-            nullptr, nullptr, src, nullptr, nullptr, dst, count, max_count, p * hs, sp.shift[p], sp.bits[p], L.ctrl, f,
-            1u);
+            nullptr, nullptr, src, nullptr, nullptr, dst, count, max_count, p * hs, sp.shift[p], sp.bits[p], L.ctrl, f);
         f += (size_t)L.ntiles << sp.bits[p];
         uint2 *t = src;
         src = dst;
@@ -706,7 +733,7 @@ static void launch_sort_passes(uint32_t *keys, uint32_t *vals, uint32_t max_coun
     }
     launch_frame_kernel(sort_pass_kernel<true, false, MATCH || MATCH_LAST>, L.ntiles, kSortThreads, kSortDynSmem, st, overlap, 
         nullptr, nullptr, src, keys, vals, nullptr, count, max_count, (npasses - 1) * hs, sp.shift[npasses - 1],
-        sp.bits[npasses - 1], L.ctrl, f, 1u);
+        sp.bits[npasses - 1], L.ctrl, f);
     count_launches(npasses);
 }
 
@@ -729,10 +756,15 @@ static cudaError_t ensure_sort_smem() {
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortDynSmem);
         if (e != cudaSuccess) return e;
     }
-    e = cudaFuncSetAttribute(tile_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemDynSmem<true>);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(tile_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemDynSmem<false>);
-    if (e != cudaSuccess) return e;
+    const std::pair<const void *, size_t> items[] = {
+        {(const void *)tile_pass_kernel<true, false>, kItemDynSmem<true>},
+        {(const void *)tile_pass_kernel<false, false>, kItemDynSmem<false>},
+        {(const void *)tile_pass_kernel<false, true>, kItemDynSmem<false>},
+    };
+    for (const auto &f : items) {
+        e = cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.second);
+        if (e != cudaSuccess) return e;
+    }
     ready.fetch_or(bit, std::memory_order_acq_rel);
     return cudaSuccess;
 }
@@ -1020,7 +1052,7 @@ cudaError_t launch_sort_segments(const SortSegment *segs_dev, const uint32_t *bl
 }
 
 cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *count, uint32_t key_bits, Ctrl *ctrl,
-                              uint64_t *flags, uint2 *alt, cudaStream_t st, bool hist_scanned) {
+                              uint64_t *flags, uint2 *alt, cudaStream_t st) {
     const PassSplit split = tile_split(key_bits);
     if (max_count == 0) return cudaSuccess;
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
@@ -1032,8 +1064,7 @@ cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *c
         launch_frame_kernel(sort_pass_kernel<true, true, false>, ntiles, kSortThreads, kSortDynSmem, st, overlap, nullptr, nullptr, src, nullptr, nullptr, dst,
                                                                             count, max_count, p * hist_stride(split.n),
                                                                             split.shift[p],
-                                                                            split.bits[p], ctrl, f,
-                                                                            hist_scanned ? 1u : 0u);
+                                                                            split.bits[p], ctrl, f);
         f += (size_t)ntiles << split.bits[p];
         uint2 *t = src;
         src = dst;
@@ -1048,17 +1079,19 @@ cudaError_t launch_sort_pairs(uint2 *data, uint32_t max_count, const uint32_t *c
 }
 
 cudaError_t launch_sort_items(uint32_t *items, const uint8_t *low, uint32_t *alt, uint32_t max_count, const uint32_t *count,
-                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st) {
+                              uint32_t key_bits, uint32_t value_bits, Ctrl *ctrl, uint64_t *flags, cudaStream_t st,
+                              uint32_t *tile_counts, uint32_t target_tiles) {
     const PassSplit split = tile_split(key_bits);
     if (max_count == 0) return cudaSuccess;
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const uint32_t ntiles = (uint32_t)sort_tiles(max_count);
     const bool overlap = frame_launch_overlaps(st);
-    launch_frame_kernel(tile_pass_kernel<true>, ntiles, kSortThreads, kItemDynSmem<true>, st, overlap, items, low, alt, count, max_count, 0, value_bits,
-                                                                           split.bits[0], ctrl, flags);
-    launch_frame_kernel(tile_pass_kernel<false>, ntiles, kSortThreads, kItemDynSmem<false>, st, overlap, 
-        alt, nullptr, items, count, max_count, hist_stride(2), value_bits, split.bits[1], ctrl,
-        flags + ((size_t)ntiles << split.bits[0]));
+    uint64_t *flags1 = flags + ((size_t)ntiles << split.bits[0]);
+    launch_frame_kernel(tile_pass_kernel<true, false>, ntiles, kSortThreads, kItemDynSmem<true>, st, overlap, items, low, alt,
+                        count, max_count, 0, value_bits, split.bits[0], ctrl, flags, 0, nullptr, 0);
+    launch_frame_kernel(tile_counts ? tile_pass_kernel<false, true> : tile_pass_kernel<false, false>, ntiles, kSortThreads,
+                        kItemDynSmem<false>, st, overlap, alt, nullptr, items, count, max_count, hist_stride(2), value_bits,
+                        split.bits[1], ctrl, flags1, split.bits[0], tile_counts, target_tiles);
     count_launches(2);
     return cudaGetLastError();
 }
