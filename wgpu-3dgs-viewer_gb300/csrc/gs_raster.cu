@@ -8,8 +8,8 @@
 //     counts (block scan + decoupled look-back) and emits (tile, value) pairs; a stable radix sort
 //     by tile then groups the values per tile with draw order kept inside each tile.  Frames of few
 //     splats and tiles skip the scan, the pairs and their sort (raster_direct_kernel).
-//   * K4 runs one CTA per tile; each thread owns one pixel and walks the tile's splats in
-//     draw order (far to near), staged 256 at a time in shared memory.  For every fragment
+//   * K4 runs one CTA per tile; each thread owns one or two pixels and walks the tile's splats in
+//     draw order (far to near), staged a chunk at a time in shared memory.  For every fragment
 //     it evaluates the interpolated quad offset q, the discard test, the alpha of the display
 //     mode, and blends with the 8-bit re-quantisation a Rgba8Unorm attachment performs after
 //     every fragment: d' = round(d·(1-α) + s·α) in units of 1/255.
@@ -17,6 +17,7 @@
 // fragment box and are never visited; skipping them leaves every pixel bit-identical.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "gs_internal.h"
 
@@ -25,7 +26,7 @@ namespace gs {
 constexpr uint32_t kBinThreads = 256;
 constexpr uint32_t kRasterThreads = 256;
 // A warp's pixel block is 8x4 pixels: its pixel centres span 7 x 3 pixels.
-constexpr float kBlockSpanX = 7.0f, kBlockSpanY = 3.0f;
+constexpr float kBlockSpanX = 7.0f;
 
 struct RasterLayout {
     Ctrl *ctrl;          // raster control block: owns the area's epoch counter and flag arena
@@ -343,7 +344,8 @@ __device__ __forceinline__ uint32_t kept_tile_place(uint32_t m, uint32_t w, uint
 // the splat's rectangle (its kept tiles skip the dropped corners).  Stores are consecutive.  Bound by
 // issue: 24.7M pairs took 136 us with the splat found by a binary search of shuffles and its fields by
 // seven more, 126 with an or-reduction and three shared loads; five CTAs an SM, as six (40 registers)
-// spill time into the digit counts of large targets (3M / 4K: 226 us a binning, 237).  Also accumulates the tile counts (or the tile-key digit histograms of the tile sort) in
+// spill time into the digit counts of large targets (3M / 4K: 226 us a binning, 237).
+// Also accumulates the tile counts (or the tile-key digit histograms of the tile sort) in
 // shared memory; each CTA hands its shared bins on once.
 // COUNTS: one counter per tile, else the digit histograms; COMPACT: items and low digits, else pairs.
 constexpr uint32_t kEmitMin = 96;  // pairs of a warp's share at least (its search costs about 3 us)
@@ -818,18 +820,39 @@ __device__ __forceinline__ bool fragment(const float4 a, const float4 b, float p
 // BlendState::ALPHA_BLENDING onto an 8-bit channel, in units of 1/255: round(d·(1-α) + s·α).
 __device__ __forceinline__ float blend8(float d, float om, float s_alpha) { return rintf(fmaf(d, om, s_alpha)); }
 
+// PX: pixels a thread (see raster_tile); a chunk has an entry per thread.
+template <uint32_t PX>
 struct RasterShared {
-    float4 raw[kRasterThreads * 3];  // the next chunk's splats, thread t's own at 3t
-    float4 a[kRasterThreads];        // cx, cy, r² limit, alpha
-    float4 b[kRasterThreads];        // q (or the point half sides)
-    float4 c[kRasterThreads];        // s255.rgb
-    float4 box[kRasterThreads];      // fragment box in pixel-centre coordinates
-    float2 inv[kRasterThreads];      // 1 / |Q·(7, 0)|², 1 / |Q·(0, 3)|² (the block edges in quad space)
-    uint8_t list[kRasterThreads / 32][kRasterThreads];
+    static constexpr uint32_t T = kRasterThreads / PX;
+    float4 raw[T * 3];  // the next chunk's splats, thread t's own at 3t
+    float4 a[T];        // cx, cy, r² limit, alpha
+    float4 b[T];        // q (or the point half sides)
+    float4 box[T];      // fragment box in pixel-centre coordinates
+    float2 inv[T];      // 1 / |Q·(7, 0)|², 1 / |Q·(0, 4 PX - 1)|² (the block edges in quad space)
     uint32_t kmin;
 };
 
-// The tile's list entries, a chunk of 256 at a time, one entry per thread.  The splats of the
+struct RasterShared1 : RasterShared<1> {
+    static constexpr uint32_t PX = 1;
+    float4 c[T];  // s255.rgb
+    uint8_t list[T / 32][T];
+};
+
+// Two pixels a thread: what the blending reads, each value twice for the packed arithmetic; entry T
+// is one that no pixel meets.  The lists hold byte offsets into these arrays.
+struct RasterShared2 : RasterShared<2> {
+    static constexpr uint32_t PX = 2;
+    float4 centre[T + 1];   // -cx, -cx, -cy, -cy
+    float4 qx[T + 1];       // the first row of q: x, x, y, y
+    float4 qy[T + 1];       // the second
+    float4 la[T + 1];       // r² limit, alpha, s255.r twice
+    float4 gb[T + 1];       // s255.g twice, s255.b twice
+    alignas(8) uint32_t list[T / 32][T + 2];
+};
+template <uint32_t PX>
+using RasterSharedOf = typename std::conditional<PX == 1, RasterShared1, RasterShared2>::type;
+
+// The tile's list entries, a chunk at a time, one entry per thread.  The splats of the
 // chunk after the staged one are in flight (cp.async into the thread's own part of `raw`) and the
 // pair of the chunk after that is in a register, so neither of the two dependent global loads of
 // an entry is waited for while the warps blend.
@@ -843,7 +866,8 @@ struct ChunkSource {
         return threadIdx.x < cnt ? values[(size_t)(base + threadIdx.x) << value_shift] : 0xFFFFFFFFu;
     }
 
-    __device__ __forceinline__ void fetch(RasterShared &S, uint32_t k) const {
+    template <class Shared>
+    __device__ __forceinline__ void fetch(Shared &S, uint32_t k) const {
         float4 *dst = S.raw + 3u * threadIdx.x;
         if (k < max_splats) {  // pair values come from the tile sort; else no entry, or a timeout
             const float4 *src = reinterpret_cast<const float4 *>(splats + k);
@@ -857,15 +881,15 @@ struct ChunkSource {
     }
 
     // Start a walk: [base, base + cnt) goes into flight, [next, next + next_cnt) is the chunk after.
-    __device__ __forceinline__ void begin(RasterShared &S, uint32_t base, uint32_t cnt, uint32_t next,
-                                          uint32_t next_cnt) {
+    template <class Shared>
+    __device__ __forceinline__ void begin(Shared &S, uint32_t base, uint32_t cnt, uint32_t next, uint32_t next_cnt) {
         fetch(S, pair_value(base, cnt));
         value = pair_value(next, next_cnt);
     }
 
     // A splat into the thread's staged entry.
-    template <uint32_t MODE>
-    static __device__ __forceinline__ void put(RasterShared &S, const float4 a, const float4 b, const float4 c,
+    template <uint32_t MODE, class Shared>
+    static __device__ __forceinline__ void put(Shared &S, const float4 a, const float4 b, const float4 c,
                                                float std2) {
         const uint32_t tid = threadIdx.x;
         // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
@@ -873,19 +897,28 @@ struct ChunkSource {
             (MODE == GS_DISPLAY_SPLAT) ? splat_r2_bound(c.w, splat_colour_reach(c.x, c.y, c.z), std2) : std2;
         S.a[tid] = make_float4(a.x, a.y, lim, c.w);
         S.b[tid] = b;
-        S.c[tid] = c;
+        if constexpr (Shared::PX == 1) {
+            S.c[tid] = c;
+        } else {
+            S.centre[tid] = make_float4(-a.x, -a.x, -a.y, -a.y);
+            S.qx[tid] = make_float4(b.x, b.x, b.y, b.y);
+            S.qy[tid] = make_float4(b.z, b.z, b.w, b.w);
+            S.la[tid] = make_float4(lim, c.w, c.x, c.x);
+            S.gb[tid] = make_float4(c.y, c.y, c.z, c.z);
+        }
         S.box[tid] = make_float4(a.x - a.z, a.x + a.z, a.y - a.w, a.y + a.w);
         if constexpr (MODE != GS_DISPLAY_POINT) {
             const float e1x = b.x * kBlockSpanX, e1y = b.z * kBlockSpanX;
-            const float e2x = b.y * kBlockSpanY, e2y = b.w * kBlockSpanY;
+            constexpr float span = 4.0f * Shared::PX - 1.0f;
+            const float e2x = b.y * span, e2y = b.w * span;
             S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
         }
     }
 
     // Stage the chunk in flight (cnt entries), then put the next one (if more) in flight and read the
     // pairs [after, after + after_cnt).  The caller puts a barrier on either side.
-    template <uint32_t MODE>
-    __device__ __forceinline__ void stage(RasterShared &S, uint32_t cnt, float std2, bool more, uint32_t after,
+    template <uint32_t MODE, class Shared>
+    __device__ __forceinline__ void stage(Shared &S, uint32_t cnt, float std2, bool more, uint32_t after,
                                           uint32_t after_cnt) {
         const float4 *raw = S.raw + 3u * threadIdx.x;
         cp_async_wait_all();
@@ -897,8 +930,8 @@ struct ChunkSource {
     }
 
     // Stage a list that is one chunk, straight from memory.
-    template <uint32_t MODE>
-    __device__ __forceinline__ void stage_only(RasterShared &S, uint32_t n, float std2) const {
+    template <uint32_t MODE, class Shared>
+    __device__ __forceinline__ void stage_only(Shared &S, uint32_t n, float std2) const {
         if (threadIdx.x >= n) return;
         const uint32_t k = pair_value(0, n);
         float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
@@ -927,6 +960,7 @@ __device__ __forceinline__ bool seg_within(float ux, float uy, float ex, float e
     return px * px + py * py <= lim;
 }
 
+template <uint32_t PX>
 __device__ __forceinline__ bool ellipse_meets_block(const float4 a, const float4 q, const float2 inv, float bx0,
                                                     float bx1, float by0, float by1) {
     const bool inx = a.x >= bx0 && a.x <= bx1, iny = a.y >= by0 && a.y <= by1;
@@ -935,7 +969,8 @@ __device__ __forceinline__ bool ellipse_meets_block(const float4 a, const float4
     const float dx = bx0 - a.x, dy = by0 - a.y;
     const float ux = q.x * dx + q.y * dy, uy = q.z * dx + q.w * dy;  // corner (bx0, by0)
     const float e1x = q.x * kBlockSpanX, e1y = q.z * kBlockSpanX;   // along x, 7 px
-    const float e2x = q.y * kBlockSpanY, e2y = q.w * kBlockSpanY;   // along y, 3 px
+    constexpr float span = 4.0f * PX - 1.0f;
+    const float e2x = q.y * span, e2y = q.w * span;                 // along y, 3 or 7 px
     bool m = false;
     if (!inx) {  // left edge (c left of the block) or right edge
         const bool left = a.x < bx0;
@@ -950,8 +985,8 @@ __device__ __forceinline__ bool ellipse_meets_block(const float4 a, const float4
 
 // The calling warp's list of staged entries from jmin on whose fragments can reach its pixel block, in
 // draw order: the fragment box, then (splat and ellipse modes) the ellipse itself must meet the block.
-template <uint32_t MODE>
-__device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t jmin, uint32_t cnt, float bx0, float bx1,
+template <uint32_t MODE, class Shared>
+__device__ __forceinline__ uint32_t compact_chunk(Shared &S, uint32_t jmin, uint32_t cnt, float bx0, float bx1,
                                                   float by0, float by1) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
@@ -962,11 +997,19 @@ __device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t jmin
         if (j >= jmin && j < cnt) {
             const float4 box = S.box[j];
             hit = !(box.y < bx0 || box.x > bx1 || box.w < by0 || box.z > by1);
-            if (MODE != GS_DISPLAY_POINT && hit) hit = ellipse_meets_block(S.a[j], S.b[j], S.inv[j], bx0, bx1, by0, by1);
+            if (MODE != GS_DISPLAY_POINT && hit)
+                hit = ellipse_meets_block<Shared::PX>(S.a[j], S.b[j], S.inv[j], bx0, bx1, by0, by1);
         }
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit);
-        if (hit) S.list[warp][nl + __popc(m & lt)] = (uint8_t)j;
+        if constexpr (Shared::PX == 1) {
+            if (hit) S.list[warp][nl + __popc(m & lt)] = (uint8_t)j;
+        } else {
+            if (hit) S.list[warp][nl + __popc(m & lt)] = j * 16u;
+        }
         nl += __popc(m);
+    }
+    if constexpr (Shared::PX == 2) {
+        if (lane == 0) S.list[warp][nl] = Shared::T * 16u;  // an even list
     }
     __syncwarp();
     return nl;
@@ -974,7 +1017,41 @@ __device__ __forceinline__ uint32_t compact_chunk(RasterShared &S, uint32_t jmin
 
 // A pixel of a warp's block whose transmittance stands for its quarter of the block.
 __device__ __forceinline__ float sample_x(uint32_t q) { return (q & 1u) ? 6.0f : 1.0f; }
-__device__ __forceinline__ float sample_y(uint32_t q) { return (q & 2u) ? 3.0f : 0.0f; }
+template <uint32_t PX>
+__device__ __forceinline__ float sample_y(uint32_t q) { return PX == 1 ? ((q & 2u) ? 3.0f : 0.0f) : ((q & 2u) ? 6.0f : 1.0f); }
+
+// Two floats in one instruction, each half rounded as the scalar instruction does.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "add.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+// rintf of both halves: by the conversion unit, or by two packed additions (exact for |a| < 2^22; a
+// blended channel lies in [0, 255]).
+__device__ __forceinline__ float2 rint2_convert(float2 a) { return make_float2(rintf(a.x), rintf(a.y)); }
+__device__ __forceinline__ float2 rint2_add(float2 a) {
+    constexpr float big = 12582912.0f;  // 1.5 * 2^23: a float's last bit there is worth one
+    return add2(add2(a, make_float2(big, big)), make_float2(-big, -big));
+}
 
 // Blends the warp's list entries [0, nl) onto the pixel (d), and with BOTH onto the upper bound (h)
 // as well, for lanes with `on`.  UNROLL 1: one entry after another, skipping what the fragment test
@@ -982,7 +1059,7 @@ __device__ __forceinline__ float sample_y(uint32_t q) { return (q & 2u) ? 3.0f :
 // blends with alpha 0, which leaves the pixel as it is; more instructions, but the warp waits for one
 // chain of loads, exp and test where it waited for four.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, bool BOTH, uint32_t UNROLL>
-__device__ __forceinline__ void blend_list(const RasterShared &S, uint32_t nl, bool on, float pxc, float pyc,
+__device__ __forceinline__ void blend_list(const RasterShared1 &S, uint32_t nl, bool on, float pxc, float pyc,
                                            float outline2, float d[3], float h[3], uint32_t &n_eval, uint32_t &n_alpha,
                                            uint32_t &n_blend) {
     const uint32_t warp = threadIdx.x >> 5;
@@ -1024,18 +1101,82 @@ __device__ __forceinline__ void blend_list(const RasterShared &S, uint32_t nl, b
     }
 }
 
-// Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats: three
-// quarters of it (768 by default: 668, 408 and 1962 us at 6M / 1080p, 1M / 1080p and 3M / 4K, against
-// 683, 412, 2084 at 1024 and 669, 425, 1937 at 512).  Ellipses end sooner, as outlines are opaque and
-// interiors keep their full alpha: a quarter (256: the frame of 700k at 1600x900 387 us, against 388
-// at 384, 414 at 768 and 392 at 128).
-constexpr float kWalkCourse = 0.9f;
-template <uint32_t MODE>
-__device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
-    return MODE == GS_DISPLAY_ELLIPSE ? suffix_min / 4u : suffix_min - suffix_min / 4u;
+// blend_list for two pixels a thread, (pc.x, pc.y) and (pc.x, pc.z), in packed arithmetic: the list's
+// entries two at a time, missed ones blended with alpha 0.  A pixel with a NaN coordinate misses all.
+// Bound: the FMA pipe (65 % busy at 1M / 1080p), issue (66 %) and the shared-memory pipe (64 %).
+// The rounding is split between the units: all by conversion keeps the conversion unit busy 79 % of
+// the time (582 us at 6M / 1080p), all by additions takes 505, two channels of three 489, and two of
+// three with both bounds but one of three without 486.  Four entries at a time take 495 us, one 590 (by
+// conversion), a test whether any lane hits 589 (by conversion).
+template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, bool BOTH>
+__device__ __forceinline__ void blend_list2(const RasterShared2 &S, uint32_t nl, const float3 pc, float outline2,
+                                            float2 d[3], float2 h[3], uint32_t &n_eval, uint32_t &n_alpha, uint32_t &n_blend) {
+    const uint32_t warp = threadIdx.x >> 5;
+    const float2 px = make_float2(pc.x, pc.x), py = make_float2(pc.y, pc.z);
+    auto at = [](const float4 *array, uint32_t offset) {
+        return *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(array) + offset);
+    };
+    auto one = [&](uint32_t offset) {
+        const float4 m = at(S.centre, offset), qx = at(S.qx, offset), qy = at(S.qy, offset), la = at(S.la, offset),
+                     gb = at(S.gb, offset);
+        const float2 dx = add2(px, make_float2(m.x, m.y)), dy = add2(py, make_float2(m.z, m.w));
+        const float2 ux = fma2(make_float2(qx.x, qx.y), dx, mul2(make_float2(qx.z, qx.w), dy));
+        const float2 uy = fma2(make_float2(qy.x, qy.y), dx, mul2(make_float2(qy.z, qy.w), dy));
+        const float2 r2 = fma2(ux, ux, mul2(uy, uy));
+        float2 v;
+        if constexpr (MODE == GS_DISPLAY_SPLAT && !PORTABLE_EXP) {
+            const float2 x = mul2(r2, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v.x) : "f"(x.x));
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v.y) : "f"(x.y));
+            v.x = __fmul_rn(la.y, v.x);
+            v.y = __fmul_rn(la.y, v.y);
+        } else {
+            const float4 a = make_float4(0.0f, 0.0f, la.x, la.y);
+            v = make_float2(fragment_alpha<MODE, PORTABLE_EXP>(a, r2.x, outline2),
+                            fragment_alpha<MODE, PORTABLE_EXP>(a, r2.y, outline2));
+        }
+        const bool hit0 = r2.x <= la.x, hit1 = r2.y <= la.x;
+        if (COUNT) {
+            n_eval += (pc.y == pc.y) + (pc.z == pc.z);
+            n_alpha += hit0 + hit1, n_blend += (hit0 + hit1) * (BOTH ? 2 : 1);
+        }
+        const float2 al = make_float2(hit0 ? v.x : 0.0f, hit1 ? v.y : 0.0f);
+        const float2 om = fma2(al, make_float2(-1.0f, -1.0f), make_float2(1.0f, 1.0f));
+        const float2 s[3] = {mul2(make_float2(la.z, la.w), al), mul2(make_float2(gb.x, gb.y), al),
+                             mul2(make_float2(gb.z, gb.w), al)};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const bool add = q < (BOTH ? 2 : 1);
+            d[q] = fma2(d[q], om, s[q]);
+            d[q] = add ? rint2_add(d[q]) : rint2_convert(d[q]);
+            if (BOTH) {
+                h[q] = fma2(h[q], om, s[q]);
+                h[q] = add ? rint2_add(h[q]) : rint2_convert(h[q]);
+            }
+        }
+    };
+    for (uint32_t i = 0; i < nl; i += 2) {
+        const uint2 j = *reinterpret_cast<const uint2 *>(&S.list[warp][i]);
+        one(j.x);
+        one(j.y);
+    }
 }
 
-// K4.  One CTA per 16x16 tile; each warp owns an 8x4 pixel block, each thread one pixel.
+// Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats, a pixel
+// a thread: three quarters of it (13.5k at 237x133 48 us a frame at 768, 52 at 384).  Two pixels a
+// thread walk half as many samples: nine sixteenths (576 by default: 477, 321, 1340 and 232 us at 6M /
+// 1080p, 1M / 1080p, 3M / 4K and 400k / 1366x768, against 486, 320, 1413, 246 at 768 and 480, 330, 1320,
+// 229 at 384).  Ellipses end sooner, as outlines are opaque and interiors keep their full alpha: a
+// quarter (256: the frame of 700k at 1600x900 387 us, against 388 at 384, 414 at 768 and 392 at 128).
+constexpr float kWalkCourse = 0.9f;
+template <uint32_t MODE, uint32_t PX>
+__device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
+    if (MODE == GS_DISPLAY_ELLIPSE) return suffix_min / 4u;
+    return PX == 2 ? suffix_min / 2u + suffix_min / 16u : suffix_min - suffix_min / 4u;
+}
+
+// K4.  One CTA per 16x16 tile; each warp owns an 8x4 pixel block, each thread one pixel, or an 8x8
+// block, each thread two pixels of a column (PX; 128 threads a tile, chunks of 128 entries).
 // Points are opaque: each pixel takes the nearest point that covers it, found front to back.
 // Short tile lists are blended back to front in one pass.  Long ones use an exact early-out:
 //   A. walk the list front to back (nearest first) until the transmittance of four sample pixels
@@ -1048,28 +1189,50 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 //      value, which is exact).
 // Every pixel therefore ends bit-identical to the full back-to-front pass.
 //
-// Bound: instruction issue (no memory system near its limit), so time follows the warp iterations
-// of the list loops and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K:
-// 935, 514 and 2614 us with a walk A of every pixel over compacted lists and each chunk's loads
-// waited for; 635, 396 and 1882 us with the sampled walk, the loads a chunk ahead and the SFU exp
-// without denormal handling.  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
-template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL>
+// Bound: the arithmetic of the list loops (no memory system near its limit), so time follows the warp
+// iterations and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K: 935, 514 and
+// 2614 us with a walk A of every pixel over compacted lists and each chunk's loads waited for; 629,
+// 392 and 1864 us with the sampled walk, the loads a chunk ahead and the SFU exp without denormal
+// handling; 477, 321 and 1340 us with two pixels a thread, which share the list, the loads and, in
+// packed instructions, the arithmetic (64 registers, 8 CTAs an SM; 7, 9 and 10 CTAs take 497, 496 and
+// 506 us where 8 take 489).  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
+template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL, class Shared>
 __device__ __forceinline__ void raster_tile(
-    RasterShared &S, const RasterJob &J, const uint32_t *__restrict__ list, uint32_t list_shift, uint32_t n, float std2, float outline2,
-    uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
+    Shared &S, const RasterJob &J, const uint32_t *__restrict__ list, uint32_t list_shift, uint32_t n, float std2,
+    float outline2, uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
     // Work tallies of the counting variant (profiling only): fragment evaluations, alphas,
     // channel-triple blends and transmittance updates.
     uint32_t n_eval = 0, n_alpha = 0, n_blend = 0, n_trans = 0;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t W = J.W, H = J.H, tx = tile % J.tiles_x, ty = tile / J.tiles_x;
-    const uint32_t wx0 = tx * GS_TILE + (warp & 1u) * 8u, wy0 = ty * GS_TILE + (warp >> 1) * 4u;
+    constexpr uint32_t PX = Shared::PX;
+    const uint32_t wx0 = tx * GS_TILE + (warp & 1u) * 8u, wy0 = ty * GS_TILE + (warp >> 1) * 4u * PX;
     const uint32_t px = wx0 + (lane & 7u), py = wy0 + (lane >> 3);
     const float pxc = (float)px + 0.5f, pyc = (float)py + 0.5f;
     const float bx0 = (float)wx0 + 0.5f, bx1 = (float)wx0 + 7.5f;
-    const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 3.5f;
-    float d[3] = {0.0f, 0.0f, 0.0f};
+    const float by0 = (float)wy0 + 0.5f, by1 = (float)wy0 + 4.0f * PX - 0.5f;
+    // the thread's pixels: (px, py) and, with two, (px, py + 4)
+    using Value = typename std::conditional<PX == 1, float, float2>::type;
+    Value d[3] = {}, h[3] = {};
+    // blends the list onto the pixels whose `on` is set
+    auto blend = [&](auto both, uint32_t nl, const bool *on) {
+        if constexpr (PX == 1) {
+            blend_list<MODE, PORTABLE_EXP, COUNT, decltype(both)::value, UNROLL>(S, nl, on[0], pxc, pyc, outline2, d, h, n_eval,
+                                                                                 n_alpha, n_blend);
+        } else {
+            const float none = __int_as_float(0x7FC00000);
+            const float3 pc = make_float3(pxc, on[0] ? pyc : none, on[1] ? pyc + 4.0f : none);
+            blend_list2<MODE, PORTABLE_EXP, COUNT, decltype(both)::value>(S, nl, pc, outline2, d, h, n_eval, n_alpha, n_blend);
+        }
+    };
+    if constexpr (PX == 2) {
+        if (tid == 0) {  // the entry that fills up a list: read after the first barrier
+            S.centre[Shared::T] = S.qx[Shared::T] = S.qy[Shared::T] = S.gb[Shared::T] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            S.la[Shared::T] = make_float4(-1.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
     ChunkSource src{J.splats, list, list_shift, J.max_splats, 0u};
-    constexpr uint32_t C = kRasterThreads;
+    constexpr uint32_t C = Shared::T;
     // the chunk before list position `end` (for walks from the end of the list)
     auto below = [](uint32_t end) { return end > C ? end - C : 0u; };
 
@@ -1093,7 +1256,7 @@ __device__ __forceinline__ void raster_tile(
         };
         if (n <= C) {
             if (n > 0) {
-                src.stage_only<MODE>(S, n, std2);
+                src.template stage_only<MODE>(S, n, std2);
                 __syncthreads();
                 nearest(n);
             }
@@ -1101,7 +1264,7 @@ __device__ __forceinline__ void raster_tile(
             uint32_t base = n - C;
             src.begin(S, base, C, below(base), base - below(base));
             for (uint32_t end = n; end > 0;) {
-                src.stage<MODE>(S, end - base, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+                src.template stage<MODE>(S, end - base, std2, base > 0, below(below(base)), below(base) - below(below(base)));
                 __syncthreads();
                 if (__any_sync(0xFFFFFFFFu, !found)) nearest(end - base);
                 if (__syncthreads_and(found)) break;
@@ -1109,133 +1272,152 @@ __device__ __forceinline__ void raster_tile(
                 base = below(end);
             }
         }
-    } else if (n <= C && n < early_out_min<MODE>(suffix_min)) {
-        if (n > 0) {
-            src.stage_only<MODE>(S, n, std2);
-            __syncthreads();
-            const uint32_t nl = compact_chunk<MODE>(S, 0, n, bx0, bx1, by0, by1);
-            blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, true, pxc, pyc, outline2, d, d, n_eval, n_alpha,
-                                                                 n_blend);
-        }
-    } else if (n < early_out_min<MODE>(suffix_min)) {
-        src.begin(S, 0, C, C, min(C, n - C));
-        for (uint32_t base = 0; base < n; base += C) {
-            const uint32_t cnt = min(C, n - base), after = base + 2u * C;
-            src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
-            __syncthreads();
-            const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
-            blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, true, pxc, pyc, outline2, d, d, n_eval, n_alpha,
-                                                                 n_blend);
-            __syncthreads();
-        }
     } else {
-        // ---- A: front-to-back transmittance of the samples to find the start position k ----
-        uint32_t k = 0;
-        {
-            const float sxc = bx0 + sample_x(lane & 3u), syc = by0 + sample_y(lane & 3u);
-            float T = 1.0f;  // this lane's share of its sample's transmittance
-            bool found = false;
-            uint32_t base = below(n), cnt = n - base;
-            src.begin(S, base, cnt, below(base), base - below(base));
-            for (uint32_t end = n; end > 0;) {
-                src.stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
-                __syncthreads();
-                for (int top = (int)cnt; top > 0 && !found; top -= 32) {
+        bool all_on[PX];
 #pragma unroll
-                    for (int it = 0; it < 4; ++it) {
-                        const int j = top - 1 - it * 8 - (int)(lane >> 2);
-                        float al;
-                        if (COUNT && j >= 0) ++n_eval;
-                        if (j >= 0 && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], sxc, syc, outline2, &al)) {
-                            if (COUNT) ++n_alpha, ++n_trans;
-                            // an ellipse's outline is opaque where the sample lies, not where the
-                            // block's other pixels do
-                            if (MODE == GS_DISPLAY_ELLIPSE) al = S.a[j].w;
-                            T = __fmul_rn(T, __fsub_rn(1.0f, al));
+        for (uint32_t p = 0; p < PX; ++p) all_on[p] = true;
+        if (n <= C && n < early_out_min<MODE, PX>(suffix_min)) {
+            if (n > 0) {
+                src.template stage_only<MODE>(S, n, std2);
+                __syncthreads();
+                const uint32_t nl = compact_chunk<MODE>(S, 0, n, bx0, bx1, by0, by1);
+                blend(std::false_type(), nl, all_on);
+            }
+        } else if (n < early_out_min<MODE, PX>(suffix_min)) {
+            src.begin(S, 0, C, C, min(C, n - C));
+            for (uint32_t base = 0; base < n; base += C) {
+                const uint32_t cnt = min(C, n - base), after = base + 2u * C;
+                src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
+                __syncthreads();
+                const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
+                blend(std::false_type(), nl, all_on);
+                __syncthreads();
+            }
+        } else {
+            // ---- A: front-to-back transmittance of the samples to find the start position k ----
+            uint32_t k = 0;
+            {
+                const float sxc = bx0 + sample_x(lane & 3u), syc = by0 + sample_y<PX>(lane & 3u);
+                float T = 1.0f;  // this lane's share of its sample's transmittance
+                bool found = false;
+                uint32_t base = below(n), cnt = n - base;
+                src.begin(S, base, cnt, below(base), base - below(base));
+                for (uint32_t end = n; end > 0;) {
+                    src.template stage<MODE>(S, cnt, std2, base > 0, below(below(base)), below(base) - below(below(base)));
+                    __syncthreads();
+                    for (int top = (int)cnt; top > 0 && !found; top -= 32) {
+#pragma unroll
+                        for (int it = 0; it < 4; ++it) {
+                            const int j = top - 1 - it * 8 - (int)(lane >> 2);
+                            float al;
+                            if (COUNT && j >= 0) ++n_eval;
+                            if (j >= 0 && fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], sxc, syc, outline2, &al)) {
+                                if (COUNT) ++n_alpha, ++n_trans;
+                                // an ellipse's outline is opaque where the sample lies, not where the
+                                // block's other pixels do
+                                if (MODE == GS_DISPLAY_ELLIPSE) al = S.a[j].w;
+                                T = __fmul_rn(T, __fsub_rn(1.0f, al));
+                            }
+                        }
+                        float t = T;  // the product over the sample's eight lanes
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
+                        if (__all_sync(0xFFFFFFFFu, t < eps)) {
+                            found = true;
+                            k = base + (uint32_t)max(top - 32, 0);
                         }
                     }
-                    float t = T;  // the product over the sample's eight lanes
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
-                    if (__all_sync(0xFFFFFFFFu, t < eps)) {
-                        found = true;
-                        k = base + (uint32_t)max(top - 32, 0);
+                    // A walk that will end in the far part of the list saves nothing: B costs more per
+                    // entry than one blend of the whole list.  T falls about evenly per entry, so from a
+                    // quarter of the list on it must be on course for eps (to the power kWalkCourse of
+                    // the share walked).
+                    if (!found && 4u * (n - base) >= n) {
+                        float t = T;
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
+                        t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
+                        const float course = __powf(eps, kWalkCourse * (float)(n - base) / (float)n);
+                        found = __any_sync(0xFFFFFFFFu, !(t < course));  // k = 0
+                    }
+                    if (__syncthreads_and(found)) break;
+                    end = base;
+                    base = below(end);
+                    cnt = end - base;
+                }
+            }
+            // ---- B: bounded back-to-front passes from k (the same for all pixels of a warp) ----
+            bool active[PX];
+#pragma unroll
+            for (uint32_t p = 0; p < PX; ++p) active[p] = true;
+            auto any_active = [&]() { return active[0] || active[PX - 1]; };
+            auto met = [&](uint32_t p) {
+                if constexpr (PX == 1) return d[0] == h[0] && d[1] == h[1] && d[2] == h[2];
+                else return p == 0 ? d[0].x == h[0].x && d[1].x == h[1].x && d[2].x == h[2].x
+                                   : d[0].y == h[0].y && d[1].y == h[1].y && d[2].y == h[2].y;
+            };
+            for (;;) {
+                if (tid == 0) S.kmin = 0xFFFFFFFFu;
+                __syncthreads();
+                const uint32_t wmin = __reduce_min_sync(0xFFFFFFFFu, any_active() ? k : 0xFFFFFFFFu);
+                if (lane == 0 && wmin != 0xFFFFFFFFu) atomicMin(&S.kmin, wmin);
+                __syncthreads();
+                const uint32_t kmin = S.kmin;
+                if (kmin == 0xFFFFFFFFu) break;
+                const float top = (k == 0) ? 0.0f : 255.0f;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    if constexpr (PX == 1) {
+                        if (active[0]) d[q] = 0.0f, h[q] = top;
+                    } else {
+                        if (active[0]) d[q].x = 0.0f, h[q].x = top;
+                        if (active[1]) d[q].y = 0.0f, h[q].y = top;
                     }
                 }
-                // A walk that will end in the far part of the list saves nothing: B costs more per
-                // entry than one blend of the whole list.  T falls about evenly per entry, so from a
-                // quarter of the list on it must be on course for eps (to the power kWalkCourse of
-                // the share walked).
-                if (!found && 4u * (n - base) >= n) {
-                    float t = T;
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 4);
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 8);
-                    t *= __shfl_xor_sync(0xFFFFFFFFu, t, 16);
-                    const float course = __powf(eps, kWalkCourse * (float)(n - base) / (float)n);
-                    found = __any_sync(0xFFFFFFFFu, !(t < course));  // k = 0
-                }
-                if (__syncthreads_and(found)) break;
-                end = base;
-                base = below(end);
-                cnt = end - base;
-            }
-        }
-        // ---- B: bounded back-to-front passes from k (the same for all pixels of a warp) ----
-        bool active = true;
-        float h[3] = {0.0f, 0.0f, 0.0f};
-        auto met = [&]() { return d[0] == h[0] && d[1] == h[1] && d[2] == h[2]; };
-        for (;;) {
-            if (tid == 0) S.kmin = 0xFFFFFFFFu;
-            __syncthreads();
-            const uint32_t wmin = __reduce_min_sync(0xFFFFFFFFu, active ? k : 0xFFFFFFFFu);
-            if (lane == 0 && wmin != 0xFFFFFFFFu) atomicMin(&S.kmin, wmin);
-            __syncthreads();
-            const uint32_t kmin = S.kmin;
-            if (kmin == 0xFFFFFFFFu) break;
-            if (active) {
-                d[0] = d[1] = d[2] = 0.0f;
-                h[0] = h[1] = h[2] = (k == 0) ? 0.0f : 255.0f;
-            }
-            const uint32_t start = kmin / C * C;
-            src.begin(S, start, min(C, n - start), start + C, start + C < n ? min(C, n - start - C) : 0u);
-            for (uint32_t base = start; base < n; base += C) {
-                const uint32_t cnt = min(C, n - base), after = base + 2u * C;
-                __syncthreads();
-                src.stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
-                __syncthreads();
-                // wmin is the warp's k: a warp whose suffix starts past this chunk skips it
-                if (wmin < base + C) {
-                    const uint32_t nl = compact_chunk<MODE>(S, wmin > base ? wmin - base : 0u, cnt, bx0, bx1, by0, by1);
-                    // Bounds that have met stay equal (same inputs, same operations), so once
-                    // every started lane of the warp has met, one chain per channel suffices.
-                    if (__all_sync(0xFFFFFFFFu, !active || met())) {
-                        blend_list<MODE, PORTABLE_EXP, COUNT, false, UNROLL>(S, nl, active, pxc, pyc, outline2, d, h,
-                                                                             n_eval, n_alpha, n_blend);
-                        if (active) {
+                const uint32_t start = kmin / C * C;
+                src.begin(S, start, min(C, n - start), start + C, start + C < n ? min(C, n - start - C) : 0u);
+                for (uint32_t base = start; base < n; base += C) {
+                    const uint32_t cnt = min(C, n - base), after = base + 2u * C;
+                    __syncthreads();
+                    src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
+                    __syncthreads();
+                    // wmin is the warp's k: a warp whose suffix starts past this chunk skips it
+                    if (wmin < base + C) {
+                        const uint32_t nl = compact_chunk<MODE>(S, wmin > base ? wmin - base : 0u, cnt, bx0, bx1, by0, by1);
+                        // Bounds that have met stay equal (same inputs, same operations), so once
+                        // every started lane of the warp has met, one chain per channel suffices.
+                        if (__all_sync(0xFFFFFFFFu, (!active[0] || met(0)) && (!active[PX - 1] || met(PX - 1)))) {
+                            blend(std::false_type(), nl, active);
+                            // (a pixel that is not active has met before: its bounds are equal as well)
 #pragma unroll
                             for (int q = 0; q < 3; ++q) h[q] = d[q];
+                        } else {
+                            blend(std::true_type(), nl, active);
                         }
-                    } else {
-                        blend_list<MODE, PORTABLE_EXP, COUNT, true, UNROLL>(S, nl, active, pxc, pyc, outline2, d, h,
-                                                                            n_eval, n_alpha, n_blend);
                     }
                 }
-            }
-            __syncthreads();
-            if (active) {
-                if (met()) {
-                    active = false;
-                } else {
-                    const uint32_t suffix = n - k;
-                    k = k > suffix ? k - suffix : 0u;
+                __syncthreads();
+                if (any_active()) {
+                    active[0] = active[0] && !met(0);
+                    if (PX == 2) active[PX - 1] = active[PX - 1] && !met(PX - 1);
+                    if (any_active()) {
+                        const uint32_t suffix = n - k;
+                        k = k > suffix ? k - suffix : 0u;
+                    }
                 }
             }
         }
     }
-    if (px < W && py < H) {
-        const uint32_t rgba = (uint32_t)d[0] | ((uint32_t)d[1] << 8) | ((uint32_t)d[2] << 16) | 0xFF000000u;
-        *reinterpret_cast<uint32_t *>(J.target + (size_t)py * J.pitch + (size_t)px * 4u) = rgba;
+    auto store = [&](uint32_t y, float r, float g, float b) {
+        if (px < W && y < H)
+            *reinterpret_cast<uint32_t *>(J.target + (size_t)y * J.pitch + (size_t)px * 4u) =
+                (uint32_t)r | ((uint32_t)g << 8) | ((uint32_t)b << 16) | 0xFF000000u;
+    };
+    if constexpr (PX == 1) {
+        store(py, d[0], d[1], d[2]);
+    } else {
+        store(py, d[0].x, d[1].x, d[2].x);
+        store(py + 4u, d[0].y, d[1].y, d[2].y);
     }
     if constexpr (COUNT) {
         const uint32_t v[4] = {n_eval, n_alpha, n_blend, n_trans};
@@ -1266,11 +1448,19 @@ __device__ __forceinline__ uint2 tile_range(const RasterJob &J, uint32_t tile) {
 // FEW: a grid of few tiles (at most kFewTiles), whose time is that of its longest lists, not of the
 // instructions of all: blend_list four entries at a time, in up to 64 registers a thread (4 CTAs an SM;
 // 3 and 5 CTAs take 48 and 55 us for 100k at 640x360, and 4 CTAs 49 us, against 70 us without FEW).
+// Pixels a thread: two in packed arithmetic where the instructions count, one for points (a thread
+// stops at its first hit) and for grids of few tiles.
+template <uint32_t MODE, bool FEW>
+constexpr uint32_t kPixels = FEW || MODE == GS_DISPLAY_POINT ? 1u : 2u;
+template <uint32_t MODE, bool FEW>
+constexpr uint32_t kTileThreads = kRasterThreads / kPixels<MODE, FEW>;
+template <uint32_t MODE, bool FEW>
+constexpr uint32_t kTileCtas = kPixels<MODE, FEW> == 2 ? 8u : FEW ? 4u : 6u;
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, bool FEW>
-__global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6) raster_kernel(const RasterJob J, float std2, float outline2,
-                                                                uint32_t suffix_min, float eps,
-                                                                unsigned long long *counters) {
-    __shared__ RasterShared S;
+__global__ void __launch_bounds__(kTileThreads<MODE, FEW>, kTileCtas<MODE, FEW>)
+    raster_kernel(const RasterJob J, float std2, float outline2, uint32_t suffix_min, float eps,
+                  unsigned long long *counters) {
+    __shared__ RasterSharedOf<kPixels<MODE, FEW>> S;
     frame_kernel_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) merge_status(J);
     const uint32_t tile = J.order ? J.order[blockIdx.x] : blockIdx.x;
@@ -1290,7 +1480,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     raster_direct_kernel(const RasterJob J, const uint32_t *__restrict__ rects, const uint4 *__restrict__ info,
                          uint32_t ranks, uint32_t shift, uint32_t *__restrict__ values, uint32_t max_pairs, float std2,
                          float outline2, uint32_t suffix_min, float eps) {
-    __shared__ RasterShared S;
+    __shared__ RasterShared1 S;
     __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;
     uint32_t *hits = reinterpret_cast<uint32_t *>(S.raw);  // bit r of word q: rank 32 q + r holds the tile
     static_assert(sizeof(S.raw) * 8 >= kDirectMaxRanks, "a bit per rank");
@@ -1363,11 +1553,10 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
 // One grid over the tiles of several views (a batch): CTA b rasterises tile b - tile_base[v] of
 // the view v with tile_base[v] <= b < tile_base[v + 1].
 template <uint32_t MODE, bool PORTABLE_EXP>
-__global__ void __launch_bounds__(kRasterThreads, 6) raster_views_kernel(const RasterJob *__restrict__ jobs,
-                                                                      const uint32_t *__restrict__ tile_base,
-                                                                      uint32_t nviews, float std2, float outline2,
-                                                                      uint32_t suffix_min, float eps) {
-    __shared__ RasterShared S;
+__global__ void __launch_bounds__(kTileThreads<MODE, false>, kTileCtas<MODE, false>)
+    raster_views_kernel(const RasterJob *__restrict__ jobs, const uint32_t *__restrict__ tile_base, uint32_t nviews,
+                        float std2, float outline2, uint32_t suffix_min, float eps) {
+    __shared__ RasterSharedOf<kPixels<MODE, false>> S;
     frame_kernel_enter();
     uint32_t lo = 0, hi = nviews - 1;
     while (lo < hi) {
@@ -1399,8 +1588,8 @@ cudaError_t raster_counters(unsigned long long out[4], bool reset) {
 template <uint32_t MODE, bool EXACT, bool COUNT, bool FEW>
 static void launch_raster_tiles(const RasterJob &J, float std2, float outline2, cudaStream_t st, const Tuning &t,
                                 unsigned long long *counts) {
-    launch_frame_kernel(raster_kernel<MODE, EXACT, COUNT, FEW>, J.ntiles, kRasterThreads, 0, st, frame_launch_overlaps(st), J,
-                        std2, outline2, t.suffix_min, t.eps, counts);
+    launch_frame_kernel(raster_kernel<MODE, EXACT, COUNT, FEW>, J.ntiles, kTileThreads<MODE, FEW>, 0, st,
+                        frame_launch_overlaps(st), J, std2, outline2, t.suffix_min, t.eps, counts);
 }
 
 // Grids of up to four resident waves of the FEW kernel take it: 1456 tiles (1.4M splats at 892x401)
@@ -1430,12 +1619,8 @@ template <uint32_t MODE>
 static void launch_raster_views_mode(const RasterJob *jobs, const uint32_t *tile_base, uint32_t nviews,
                                      uint32_t total_tiles, float std2, float outline2, int exact, cudaStream_t st,
                                      const Tuning &t) {
-    if (exact)
-        raster_views_kernel<MODE, true><<<total_tiles, kRasterThreads, 0, st>>>(jobs, tile_base, nviews, std2,
-                                                                                 outline2, t.suffix_min, t.eps);
-    else
-        raster_views_kernel<MODE, false><<<total_tiles, kRasterThreads, 0, st>>>(jobs, tile_base, nviews, std2,
-                                                                                  outline2, t.suffix_min, t.eps);
+    const auto kernel = exact ? raster_views_kernel<MODE, true> : raster_views_kernel<MODE, false>;
+    kernel<<<total_tiles, kTileThreads<MODE, false>, 0, st>>>(jobs, tile_base, nviews, std2, outline2, t.suffix_min, t.eps);
 }
 
 gs_splat *raster_splat_pool(void *scratch, uint32_t max_splats, uint32_t W, uint32_t H, uint32_t max_pairs) {
