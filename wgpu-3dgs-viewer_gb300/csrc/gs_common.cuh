@@ -320,15 +320,17 @@ struct TileCull {
 
     // Tile whose first pixel centre is (x0, y0).  Only box edges facing the centre can hold
     // the point nearest to it, and a linear map keeps which side of an edge a point lies on.
+    // At most one edge of each direction faces the centre: two edge tests, not four, in a warp
+    // whose splats lie on different sides.
     __device__ __forceinline__ bool meets(float x0, float y0) const {
         const float x1 = x0 + (float)(GS_TILE - 1), y1 = y0 + (float)(GS_TILE - 1);
         const float dx = x0 - cx, dy = y0 - cy;
         const float ux = q0 * dx + q1 * dy, uy = q2 * dx + q3 * dy;  // corner (x0, y0)
-        if (cx < x0 && edge(ux, uy, e2x, e2y, i2)) return true;                  // left edge
-        if (cx > x1 && edge(ux + e1x, uy + e1y, e2x, e2y, i2)) return true;      // right edge
-        if (cy < y0 && edge(ux, uy, e1x, e1y, i1)) return true;                  // top edge
-        if (cy > y1 && edge(ux + e2x, uy + e2y, e1x, e1y, i1)) return true;      // bottom edge
-        return cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1;                     // centre inside
+        const bool left = cx < x0, right = cx > x1, top = cy < y0, bottom = cy > y1;
+        bool m = cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1;  // centre inside
+        if (left || right) m = edge(left ? ux : ux + e1x, left ? uy : uy + e1y, e2x, e2y, i2);
+        if (!m && (top || bottom)) m = edge(top ? ux : ux + e2x, top ? uy : uy + e2y, e1x, e1y, i1);
+        return m;
     }
 };
 

@@ -331,12 +331,15 @@ __device__ __forceinline__ void view_color(const gs_frame_uniforms &u, const Rec
 // Projection state of one Gaussian in one view, carried from the cull to the splat record.
 struct Proj {
     float nx, ny, world[4], axes[4];
-    bool have_axes;
 };
 
 // `main` (preprocess.wesl:60-106): NDC cull, then the bound cull along the major axis for
-// centres outside the frustum.  Returns visibility; *key = 1 - ndc.z.
-__device__ __forceinline__ bool gaussian_visible(const gs_frame_uniforms &u, const Rec &g, Proj &pr, float *key) {
+// centres outside the frustum.  Returns visibility; *key = 1 - ndc.z.  With `splats`, the axes of every
+// Gaussian that a splat record of the display mode needs them for: worked out in one place, as most
+// warps hold centres on both sides of the frustum (6M: 358 us a preprocess with the cull's axes apart
+// from the splats', 342 so).
+__device__ __forceinline__ bool gaussian_visible(const gs_frame_uniforms &u, const Rec &g, Proj &pr, float *key,
+                                                 bool splats) {
     const float p4[4] = {g.pos[0], g.pos[1], g.pos[2], 1.0f};
     float clip[4];
     mat4_vec(u.model, p4, pr.world);
@@ -344,11 +347,11 @@ __device__ __forceinline__ bool gaussian_visible(const gs_frame_uniforms &u, con
     pr.nx = clip[0] / clip[3];
     pr.ny = clip[1] / clip[3];
     const float nz = clip[2] / clip[3];
-    pr.have_axes = false;
     bool vis = true;
-    if (cull(pr.nx, pr.ny, nz)) {
+    const bool outside = cull(pr.nx, pr.ny, nz);
+    if (outside || (splats && u.display_mode != GS_DISPLAY_POINT))
         cov2d_axes(u, g.cov3d, p4, u.std_dev_scaled, pr.axes);
-        pr.have_axes = true;
+    if (outside) {
         const float mx = pr.axes[0] * u.std_dev / u.size[0];
         const float my = pr.axes[1] * u.std_dev / u.size[1];
         const float mlen = len2(mx, my);
@@ -368,7 +371,7 @@ __host__ __device__ __forceinline__ float clip_scale(float viewport, float size)
 // clip_scale of the view's width and height).
 // With `binfo`, also the splat's tiles for a tiles_x x tiles_y grid, as the binning works them out.
 template <uint32_t FMT>
-__device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, float kx, float ky, const Rec &g, Proj &pr, gs_splat *out,
+__device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, float kx, float ky, const Rec &g, const Proj &pr, gs_splat *out,
                                             uint4 *binfo = nullptr, uint32_t tiles_x = 0, uint32_t tiles_y = 0) {
     float rgba[4];
     view_color<FMT>(u, g, pr.world, rgba);
@@ -398,7 +401,6 @@ __device__ __forceinline__ void write_splat(const gs_frame_uniforms &u, float kx
             ey = -1.0f;
         }
     } else {
-        if (!pr.have_axes) cov2d_axes(u, g.cov3d, p4, u.std_dev_scaled, pr.axes);
         const float *axes = pr.axes;
         const float a00 = axes[0] * kx, a01 = axes[2] * kx;
         const float a10 = -axes[1] * ky, a11 = -axes[3] * ky;
@@ -568,7 +570,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(const __grid_co
     Rec g;
     if (tid < cnt && gaussian_selected(P.selection, P.invert, i)) {
         g = load_rec<FMT>(s_rec + tid * ROW16);
-        vis = gaussian_visible(u, g, pr, &key);
+        vis = gaussian_visible(u, g, pr, &key, P.splats != nullptr);
     }
 
     // ---- order-preserving compaction: ballot + block scan; the CTA's count is published now
@@ -688,7 +690,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_views_kernel(const __g
         bool vis = false;
         float key = 0.0f;
         Proj pr;
-        if (sel) vis = gaussian_visible(s_u, g, pr, &key);
+        if (sel) vis = gaussian_visible(s_u, g, pr, &key, V.splats != nullptr);
         const uint32_t bal = __ballot_sync(0xFFFFFFFFu, vis);
         if (lane == 0) s_bal[v][warp] = bal;
         s_key[v][tid] = key;
