@@ -14,6 +14,7 @@
 #include <condition_variable>
 #include <deque>
 #include <map>
+#include <set>
 #include <thread>
 #include <unordered_map>
 #include <mutex>
@@ -217,22 +218,31 @@ struct Model {
         return GS_OK;
     }
 
-    // Preprocess + depth sort of this model for one frame, its splats written to `out`.  The preprocess
-    // also stores each visible splat's tiles for the viewport (binfo), which the binning gathers
-    // instead of the whole splat.
-    gs_status enqueue(const gs_frame_uniforms &u, gs_splat *out, cudaStream_t st) {
+    // The preprocess of this model for one frame, its splats written to `out`; also stores each visible
+    // splat's tiles for the viewport (binfo), which the binning gathers instead of the whole splat.
+    gs_status enqueue_preprocess(const gs_frame_uniforms &u, gs_splat *out, cudaStream_t st) {
         uint4 *bi = nullptr;
         if (n) {
             GS_CUDA(binfo.ensure((size_t)n * sizeof(uint4)));
             bi = reinterpret_cast<uint4 *>(binfo.ptr);
         }
-        cudaError_t e = launch_preprocess(u, records.ptr, format, n,
+        const cudaError_t e = launch_preprocess(u, records.ptr, format, n,
                                           has_selection ? (const uint32_t *)selection.ptr : nullptr, invert,
                                           indirect(), indirect() + 4, (uint32_t *)indices.ptr, (float *)depths.ptr,
                                           gs_depth_capacity(n), out, pre_scratch.ptr, st, bi);
         if (e != cudaSuccess) return cuda_fail(e, "preprocess launch");
-        e = launch_sort((uint32_t *)depths.ptr, (uint32_t *)indices.ptr, n, indirect() + 1, kDepthKeyBits,
-                        sort_scratch.ptr, st);
+        return GS_OK;
+    }
+
+    DepthSort depth_sort() {
+        return {(uint32_t *)depths.ptr, (uint32_t *)indices.ptr, indirect() + 1, n, sort_scratch.ptr};
+    }
+
+    // Preprocess + depth sort.
+    gs_status enqueue(const gs_frame_uniforms &u, gs_splat *out, cudaStream_t st) {
+        if (const gs_status s = enqueue_preprocess(u, out, st); s != GS_OK) return s;
+        const DepthSort d = depth_sort();
+        const cudaError_t e = launch_depth_sorts(&d, 1, st);
         if (e != cudaSuccess) return cuda_fail(e, "sort launch");
         return GS_OK;
     }
@@ -885,11 +895,16 @@ gs_status multi_render_locked(gs_multi_viewer *v, const std::vector<std::string>
     // Several models' splats go side by side into the raster scratch, one model's into its own buffer.
     const bool pooled = ms.size() > 1;
     gs_splat *pool = pooled ? raster_splat_pool(v->frame.raster_scratch.ptr, (uint32_t)total, w, h, v->frame.max_pairs) : nullptr;
+    // The models' sorts go together after all preprocesses, unless a model is drawn twice: its second
+    // preprocess would write the buffers of the first one's sort.
+    const bool together = std::set<Model *>(ms.begin(), ms.end()).size() == ms.size();
+    std::vector<DepthSort> sorts;
     for (Model *m : ms) {
         s = gs_frame_uniforms_build(&v->frame.camera, &m->model, &v->frame.gt, w, h, &u);
         if (s != GS_OK) return s;
         gs_splat *out = pooled ? pool : (gs_splat *)m->splats.ptr;
-        s = m->enqueue(u, out, st);
+        s = together ? m->enqueue_preprocess(u, out, st) : m->enqueue(u, out, st);
+        if (together) sorts.push_back(m->depth_sort());
         if (s != GS_OK) return s;
         RasterSegment seg{out, (const uint32_t *)m->indices.ptr, m->indirect() + 1, m->n};
         seg.binfo = reinterpret_cast<const uint4 *>(m->binfo.ptr);
@@ -906,8 +921,10 @@ gs_status multi_render_locked(gs_multi_viewer *v, const std::vector<std::string>
         s = gs_frame_uniforms_build(&v->frame.camera, &identity, &v->frame.gt, w, h, &u);
         if (s != GS_OK) return s;
     }
+    cudaError_t e = launch_depth_sorts(sorts.data(), (uint32_t)sorts.size(), st);
+    if (e != cudaSuccess) return cuda_fail(e, "sort launch");
     // Binning and raster read only std dev and display mode (RasterMode), which all models share.
-    const cudaError_t e = launch_raster(segs.data(), (uint32_t)segs.size(), raster_mode(u), target, w, h, pitch, v->frame.max_pairs,
+    e = launch_raster(segs.data(), (uint32_t)segs.size(), raster_mode(u), target, w, h, pitch, v->frame.max_pairs,
                                         v->frame.raster_scratch.ptr, v->frame.exact_exp, st);
     if (e != cudaSuccess) return cuda_fail(e, "raster launch");
     v->last_keys = keys;

@@ -108,18 +108,20 @@ __device__ __forceinline__ void ctrl_reset_flagless(Ctrl *ctrl, uint32_t arena_w
 }
 
 // The arena words this call must clear (set by the owner's reset), cleared by every CTA
-// of a grid that runs before any look-back of the call (grid-stride, 16-byte stores).
-__device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena) {
+// of a grid (or of the `blocks` CTAs that serve the area) that runs before any look-back of the call
+// (grid-stride, 16-byte stores).
+__device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena, uint32_t block = blockIdx.x,
+                                            uint32_t blocks = gridDim.x) {
     const uint32_t lo = owner->clear_lo, hi = owner->clear_hi;
     if (lo >= hi) return;
-    const uint32_t stride = gridDim.x * blockDim.x;
+    const uint32_t stride = blocks * blockDim.x;
     uint32_t a = (lo + 1u) & ~1u;  // first even word
     if (a > hi) a = hi;
-    if (lo < a && blockIdx.x == 0 && threadIdx.x == 0) arena[lo] = 0ull;
+    if (lo < a && block == 0 && threadIdx.x == 0) arena[lo] = 0ull;
     const uint32_t b = a + ((hi - a) & ~1u);
-    for (uint32_t w = a + 2u * (blockIdx.x * blockDim.x + threadIdx.x); w < b; w += 2u * stride)
+    for (uint32_t w = a + 2u * (block * blockDim.x + threadIdx.x); w < b; w += 2u * stride)
         *reinterpret_cast<ulonglong2 *>(arena + w) = make_ulonglong2(0ull, 0ull);
-    if (b < hi && blockIdx.x == 0 && threadIdx.x == 0) arena[b] = 0ull;
+    if (b < hi && block == 0 && threadIdx.x == 0) arena[b] = 0ull;
 }
 
 // Start of a kernel launched by launch_frame_kernel (a plain launch passes through).

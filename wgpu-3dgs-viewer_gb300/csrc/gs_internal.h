@@ -124,6 +124,16 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
                         uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage = kProfDepthSort,
                         const Tuning *tuning = nullptr);
 
+// Several independent sorts by kDepthKeyBits, each with its own buffers and scratch, in the launches of
+// one where they are large.
+struct DepthSort {
+    uint32_t *keys, *vals;
+    const uint32_t *count;
+    uint32_t max_count;
+    void *scratch;
+};
+cudaError_t launch_depth_sorts(const DepthSort *sorts, uint32_t n, cudaStream_t st);
+
 // Digits of the packed-pair sort: the key's bits spread evenly over the fewest passes of at
 // most 8 bits (13 bits -> 7 + 6), pass p taking bits [shift[p], shift[p] + bits[p]).
 struct PassSplit {
