@@ -1320,6 +1320,8 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
             GS_CUDA(b->sort_base_dev.ensure((size_t)(n + 1) * 4));
             GS_CUDA(cudaMemcpy(b->sort_base_dev.ptr, sort_base.data(), (size_t)(n + 1) * 4, cudaMemcpyHostToDevice));
         }
+        uint64_t keys_at_once = 0;
+        for (const Model *m : ms) keys_at_once += m->n;
         GS_CUDA(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal));
         t_capturing = true;
         t_captured_launches = 0;
@@ -1342,7 +1344,7 @@ gs_status batch_render_locked(gs_batch *b, const gs_batch_view *views, uint32_t 
                 if (vs != cs) err = cudaStreamWaitEvent(vs, b->chunk_events[c], 0);
                 if (err == cudaSuccess)
                     err = launch_sort((uint32_t *)v.depths.ptr, (uint32_t *)v.indices.ptr, ms[i]->n, ind + 1, kDepthKeyBits,
-                                      v.sort_scratch.ptr, vs, kProfDepthSort, &b->tuning);
+                                      v.sort_scratch.ptr, vs, kProfDepthSort, &b->tuning, keys_at_once);
                 if (err == cudaSuccess) {
                     const RasterSegment seg{(const gs_splat *)v.splats.ptr, (const uint32_t *)v.indices.ptr, ind + 1,
                                             ms[i]->n};

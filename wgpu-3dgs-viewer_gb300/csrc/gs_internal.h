@@ -122,7 +122,7 @@ constexpr uint32_t kMaxPasses = 6;
 size_t sort_scratch_bytes(uint32_t max_count, uint32_t key_bits);
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
                         uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage = kProfDepthSort,
-                        const Tuning *tuning = nullptr);
+                        const Tuning *tuning = nullptr, uint64_t keys_at_once = 0);
 
 // Several independent sorts by kDepthKeyBits, each with its own buffers and scratch, in the launches of
 // one where they are large.

@@ -269,12 +269,13 @@ __device__ __forceinline__ uint32_t look_back_digit(const uint64_t *flags, uint3
 // per warp, ranks by it.
 // The pass of one block (`block`: the look-back tile; lower blocks are lower, earlier-dispatched
 // CTAs of the same launch).
-template <bool IN_PACKED, bool OUT_PACKED, bool MATCH>
+template <bool IN_PACKED, bool OUT_PACKED, bool MATCH, uint32_t ROWS = kSortRows>
 __device__ __forceinline__ void sort_pass_block(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
     uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags, uint32_t block) {
-    extern __shared__ uint2 s_kv[];  // kTileKeys pairs (dynamic)
+    constexpr uint32_t KEYS = kSortThreads * ROWS;
+    extern __shared__ uint2 s_kv[];  // KEYS pairs (dynamic)
     __shared__ uint32_t s_whist[kSortWarps][256];
     __shared__ uint32_t s_start[256];
     __shared__ uint32_t s_gbase[256];
@@ -291,17 +292,17 @@ __device__ __forceinline__ void sort_pass_block(
         s_stall = ctrl->stall_tile;
     }
     // The grid covers the capacity: CTAs past the pairs there are (half of a tile sort's) leave here.
-    const uint32_t ntiles = (n + kTileKeys - 1) / kTileKeys;
+    const uint32_t ntiles = (n + KEYS - 1) / KEYS;
     if (tile >= ntiles) return;
     __syncthreads();
     const uint32_t epoch = s_epoch;
     const uint32_t dmask = (1u << digit_bits) - 1u;  // bits above the key width are ignored
-    const uint32_t base = tile * kTileKeys + warp * (32u * kSortRows);
+    const uint32_t base = tile * KEYS + warp * (32u * ROWS);
 
-    uint32_t k[kSortRows], r[kSortRows];
-    uint32_t v[IN_PACKED ? kSortRows : 1];
+    uint32_t k[ROWS], r[ROWS];
+    uint32_t v[IN_PACKED ? ROWS : 1];
 #pragma unroll
-    for (uint32_t i = 0; i < kSortRows; ++i) {
+    for (uint32_t i = 0; i < ROWS; ++i) {
         const uint32_t pos = base + i * 32u + lane;
         const bool ok = pos < n;
         if constexpr (IN_PACKED) {
@@ -316,7 +317,7 @@ __device__ __forceinline__ void sort_pass_block(
     // ballot per live digit bit).
     const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (uint32_t i = 0; i < kSortRows; ++i) {
+    for (uint32_t i = 0; i < ROWS; ++i) {
         const uint32_t d = (k[i] >> shift) & dmask;
         uint32_t peers;
         if constexpr (MATCH) peers = __match_any_sync(0xFFFFFFFFu, d);
@@ -343,7 +344,7 @@ __device__ __forceinline__ void sort_pass_block(
         }
     }
     const uint32_t total = run;
-    const uint32_t invalid = (tile == ntiles - 1) ? ntiles * kTileKeys - n : 0u;
+    const uint32_t invalid = (tile == ntiles - 1) ? ntiles * KEYS - n : 0u;
     // Padding keys (all ones) rank last, in the largest digit.
     const uint32_t pub = (d == dmask) ? total - invalid : total;
     // Digits above dmask hold no key (padding keys sit in digit dmask), so only live digits
@@ -370,17 +371,17 @@ __device__ __forceinline__ void sort_pass_block(
     }
     __syncthreads();
 
-    // The block's own counts place its kTileKeys keys (padding included), one to a place.
+    // The block's own counts place its KEYS keys (padding included), one to a place.
     if constexpr (IN_PACKED) {
 #pragma unroll
-        for (uint32_t i = 0; i < kSortRows; ++i) {
+        for (uint32_t i = 0; i < ROWS; ++i) {
             const uint32_t dd = (k[i] >> shift) & dmask;
             s_kv[s_start[dd] + s_whist[warp][dd] + r[i]] = make_uint2(k[i], v[i]);
         }
     } else {
         // Values are read only now, after ranking, which keeps them out of registers above.
 #pragma unroll
-        for (uint32_t i = 0; i < kSortRows; ++i) {
+        for (uint32_t i = 0; i < ROWS; ++i) {
             const uint32_t pos = base + i * 32u + lane;
             const uint32_t vv = pos < n ? vin[pos] : 0u;
             const uint32_t dd = (k[i] >> shift) & dmask;
@@ -388,7 +389,7 @@ __device__ __forceinline__ void sort_pass_block(
         }
     }
     __syncthreads();
-    const uint32_t valid = min(kTileKeys, n - tile * kTileKeys);
+    const uint32_t valid = min(KEYS, n - tile * KEYS);
     auto put = [&](uint32_t j, const uint2 kv) {
         const uint32_t o = s_gbase[(kv.x >> shift) & dmask] + j;
         if (o < n) {  // always true unless a look-back timed out (status already set)
@@ -400,9 +401,9 @@ __device__ __forceinline__ void sort_pass_block(
             }
         }
     };
-    if (valid == kTileKeys) {
+    if (valid == KEYS) {
 #pragma unroll 5
-        for (uint32_t i = 0; i < kSortRows; ++i) put(tid + i * kSortThreads, s_kv[tid + i * kSortThreads]);
+        for (uint32_t i = 0; i < ROWS; ++i) put(tid + i * kSortThreads, s_kv[tid + i * kSortThreads]);
     } else {
         for (uint32_t j = tid; j < valid; j += kSortThreads) put(j, s_kv[j]);
     }
@@ -555,13 +556,13 @@ __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
     }
 }
 
-template <bool IN_PACKED, bool OUT_PACKED, bool MATCH>
+template <bool IN_PACKED, bool OUT_PACKED, bool MATCH, uint32_t ROWS = kSortRows>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_pass_kernel(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
     uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags) {
     // look-back predecessors are lower, earlier-dispatched CTAs
-    sort_pass_block<IN_PACKED, OUT_PACKED, MATCH>(kin, vin, pin, kout, vout, pout, count, max_count, hoff, shift,
+    sort_pass_block<IN_PACKED, OUT_PACKED, MATCH, ROWS>(kin, vin, pin, kout, vout, pout, count, max_count, hoff, shift,
                                                   digit_bits, ctrl, flags, blockIdx.x);
 }
 
@@ -702,15 +703,15 @@ PassSplit even_split_max(uint32_t key_bits, uint32_t max_digit) {
 // Digit widths the split-array sort can be run with (Tuning::sort_digit_bits).
 constexpr uint32_t kMinDigitBits = 6, kMaxDigitBits = 8;
 
-static size_t sort_tiles(uint32_t max_count) {
-    size_t t = (max_count + kTileKeys - 1) / kTileKeys;
+static size_t sort_tiles(uint32_t max_count, uint32_t rows = kSortRows) {
+    const size_t keys = (size_t)kSortThreads * rows, t = (max_count + keys - 1) / keys;
     return t ? t : 1;
 }
 
 // Look-back flags of a sort: per pass, one word per block and live digit ([tiles][2^bits]).
-size_t sort_flag_words(uint32_t max_count, const PassSplit &sp) {
+static size_t sort_flag_words(uint32_t max_count, const PassSplit &sp, uint32_t rows = kSortRows) {
     size_t w = 0;
-    for (uint32_t p = 0; p < sp.n; ++p) w += sort_tiles(max_count) << sp.bits[p];
+    for (uint32_t p = 0; p < sp.n; ++p) w += sort_tiles(max_count, rows) << sp.bits[p];
     return w;
 }
 
@@ -724,15 +725,16 @@ struct SortLayout {
 
 // Scratch: control block | flag arena (look-back flags of every pass) | packed buffer A | packed
 // buffer B (split sorts of 3+ passes only).  The control block and the arena start at offsets no
-// call size moves; the buffers after the arena follow its size.
-static SortLayout sort_layout(void *scratch, uint32_t max_count, const PassSplit &sp) {
+// call size moves; the buffers after the arena follow its size.  A sort in small blocks has no buffer B: its
+// longer arena (768 or 1024 words for 2048 keys) ends in that buffer's 8 bytes a key.
+static SortLayout sort_layout(void *scratch, uint32_t max_count, const PassSplit &sp, uint32_t rows = kSortRows) {
     SortLayout L;
     uint8_t *p = reinterpret_cast<uint8_t *>(scratch);
-    L.ntiles = (uint32_t)sort_tiles(max_count);
+    L.ntiles = (uint32_t)sort_tiles(max_count, rows);
     L.ctrl = reinterpret_cast<Ctrl *>(p);
     p += align_up(sizeof(Ctrl), 256);
     L.flags = reinterpret_cast<uint64_t *>(p);
-    L.flag_words = sort_flag_words(max_count, sp);
+    L.flag_words = sort_flag_words(max_count, sp, rows);
     p += align_up(L.flag_words * sizeof(uint64_t), 256);
     L.alt_a = reinterpret_cast<uint2 *>(p);
     p += align_up((size_t)max_count * 8, 256);
@@ -794,6 +796,27 @@ static void launch_sort_passes(uint32_t *keys, uint32_t *vals, uint32_t max_coun
     count_launches(npasses);
 }
 
+// Passes of a small sort, an even number: from the split arrays to A and back, ROWS rows a block.
+template <bool MATCH_LAST, uint32_t ROWS>
+static void launch_small_passes(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
+                                const PassSplit &sp, const SortLayout &L, cudaStream_t st) {
+    const uint32_t hs = hist_stride(sp.n);
+    const size_t smem = (size_t)kSortThreads * ROWS * sizeof(uint2);
+    const bool overlap = frame_launch_overlaps(st);
+    uint64_t *f = L.flags;
+    for (uint32_t p = 0; p < sp.n; ++p) {
+        auto go = [&](auto kernel) {
+            launch_frame_kernel(kernel, L.ntiles, kSortThreads, smem, st, overlap, keys, vals, L.alt_a, keys, vals, L.alt_a,
+                                count, max_count, p * hs, sp.shift[p], sp.bits[p], L.ctrl, f);
+        };
+        if (p % 2 == 0) go(sort_pass_kernel<false, true, false, ROWS>);
+        else if (p + 1 < sp.n) go(sort_pass_kernel<true, false, false, ROWS>);
+        else go(sort_pass_kernel<true, false, MATCH_LAST, ROWS>);
+        f += (size_t)L.ntiles << sp.bits[p];
+    }
+    count_launches(sp.n);
+}
+
 // The pass kernels take kSortDynSmem of dynamic shared memory, above the default 48 KB a launch
 // may ask for: allow it once per device, before the first launch there.
 static cudaError_t ensure_sort_smem() {
@@ -808,6 +831,8 @@ static cudaError_t ensure_sort_smem() {
         (const void *)sort_pass_kernel<true, false, false>, (const void *)sort_pass_kernel<false, true, true>,
         (const void *)sort_pass_kernel<true, true, true>,   (const void *)sort_pass_kernel<true, false, true>,
         (const void *)sort_segments_kernel,
+        (const void *)sort_pass_kernel<false, true, false, 8>, (const void *)sort_pass_kernel<true, false, false, 8>,
+        (const void *)sort_pass_kernel<true, false, true, 8>,
         (const void *)sort_pass_group_kernel<false, true, false>, (const void *)sort_pass_group_kernel<true, true, false>,
         (const void *)sort_pass_group_kernel<true, false, true>,
     };
@@ -1063,8 +1088,21 @@ static uint32_t hist_grid(uint32_t max_count, const Tuning &tn) {
     return std::min((max_count + kHistThreads * 4 - 1) / (kHistThreads * 4), kHistCtas);
 }
 
+// Rows of a pass block.  A block of 15 rows keeps one SM's issue slots busy for about 4.5 us, so sorts that
+// leave SMs without a block take fewer rows: up to 96 blocks of 4 (70,000 pairs 42.5 -> 31.3 us, 131,072
+// 44.5 -> 34.4, 200,000 46.5 -> 38.8, 38.4 with 8 rows), up to 400 blocks of 8 (400,000 50.4 -> 44.9, 1M
+// 75.7 -> 64.5, 1.4M 86.2 -> 77.0; 2M 91.4 -> 100).  2 rows are slower throughout, 6 in between.  Sorts that
+// run at the same time (a batch's views) fill the SMs together, so the keys of all of them count.
+constexpr uint32_t kRows4Keys = 96 * 4 * kSortThreads, kRows8Keys = 400 * 8 * kSortThreads;
+static uint32_t sort_rows(uint64_t keys_at_once, const PassSplit &sp, const Tuning &tn) {
+    // an even number of passes, which ends in the split arrays without a second packed buffer
+    if (sp.n % 2 != 0 || tn.sort_match) return kSortRows;
+    return keys_at_once <= kRows4Keys ? 4u : keys_at_once <= kRows8Keys ? 8u : kSortRows;
+}
+
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
-                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning) {
+                        uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage, const Tuning *tuning,
+                        uint64_t keys_at_once) {
     // One cluster where the pairs fit (the bounded-wait hook stalls look-backs, which it has none of).
     if (wait_config().stall_tile == kNoStall) {
         cudaError_t e = cudaSuccess;
@@ -1076,7 +1114,8 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const Tuning tn = tuning ? *tuning : default_tuning();
     const PassSplit sp = pass_split(key_bits, tn);
-    const SortLayout L = sort_layout(scratch, max_count, sp);
+    const uint32_t rows = sort_rows(std::max<uint64_t>(keys_at_once, max_count), sp, tn);
+    const SortLayout L = sort_layout(scratch, max_count, sp, rows);
     const bool overlap = frame_launch_overlaps(st);
     // With no pairs no kernel reads the flags, and none clears them: the arena mark stays.
     launch_frame_kernel(ctrl_init_kernel, 1, 256, 0, st, overlap, L.ctrl, max_count ? (uint32_t)L.flag_words : kKeepArena,
@@ -1088,7 +1127,13 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     launch_frame_kernel(sort_hist_kernel, hist_blocks, kHistThreads, 0, st, overlap, keys, vals, count, max_count, sp, L.ctrl, L.flags);
     count_launches(1);
     // Keys of kDepthKeyBits are the render path's float depth keys (1 - ndc.z).
-    if (tn.sort_match)
+    if (rows == 4)
+        key_bits == kDepthKeyBits ? launch_small_passes<true, 4>(keys, vals, max_count, count, sp, L, st)
+                                  : launch_small_passes<false, 4>(keys, vals, max_count, count, sp, L, st);
+    else if (rows == 8)
+        key_bits == kDepthKeyBits ? launch_small_passes<true, 8>(keys, vals, max_count, count, sp, L, st)
+                                  : launch_small_passes<false, 8>(keys, vals, max_count, count, sp, L, st);
+    else if (tn.sort_match)
         launch_sort_passes<true, true>(keys, vals, max_count, count, sp, L, st);
     else if (key_bits == kDepthKeyBits)
         launch_sort_passes<false, true>(keys, vals, max_count, count, sp, L, st);
