@@ -39,3 +39,31 @@ def test_block_sizes_in_turn(gs, cuda):
     for i, n in enumerate([100_000, 1_700_000, 150_000, 400_000, 30_000, 1_600_000, 100_000, 1_650_000]):
         for key_bits in (30, 32):
             _check(gs, cuda, n, n - 7 * i, key_bits, scratch, nbytes, seed=i)
+
+
+@pytest.mark.parametrize("key_bits", [9, 12, 13, 16, 30, 32])
+@pytest.mark.parametrize("n", [65_537, 196_608, 1_000_001])
+def test_smallest_accepted_scratch(gs, cuda, n, key_bits):
+    """With the fewest bytes of scratch that the entry point accepts, nothing beyond them is written."""
+    full = gs.RadixSorter.scratch_bytes(n)
+    keys = cuda.zeros(n, dtype=cuda.int32, device="cuda")
+    count = cuda.zeros(1, dtype=cuda.int32, device="cuda")
+    scratch = cuda.zeros(full + 65_536, dtype=cuda.uint8, device="cuda")
+
+    def accepted(nbytes):
+        try:
+            gs.RadixSorter.sort(keys, keys.clone(), n, scratch, nbytes, count=count, key_bits=key_bits)
+        except gs.GsError:
+            return False
+        return True
+
+    lo, hi = 0, full  # refused, accepted
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if accepted(mid) else (mid, hi)
+    cuda.cuda.synchronize()
+    scratch[hi:] = 0xA5
+    scratch[:hi] = 0
+    for live in (n, n // 3):
+        _check(gs, cuda, n, live, key_bits, scratch, hi, seed=n + key_bits)
+    assert bool((scratch[hi:] == 0xA5).all())

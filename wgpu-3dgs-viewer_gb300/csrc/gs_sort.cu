@@ -1093,11 +1093,16 @@ static uint32_t hist_grid(uint32_t max_count, const Tuning &tn) {
 // 44.5 -> 34.4, 200,000 46.5 -> 38.8, 38.4 with 8 rows), up to 400 blocks of 8 (400,000 50.4 -> 44.9, 1M
 // 75.7 -> 64.5, 1.4M 86.2 -> 77.0; 2M 91.4 -> 100).  2 rows are slower throughout, 6 in between.  Sorts that
 // run at the same time (a batch's views) fill the SMs together, so the keys of all of them count.
+// Never more scratch than sort_scratch_bytes asks for: sorts of 9 to 12 key bits have one packed buffer
+// there, which leaves a longer arena no room.
 constexpr uint32_t kRows4Keys = 96 * 4 * kSortThreads, kRows8Keys = 400 * 8 * kSortThreads;
-static uint32_t sort_rows(uint64_t keys_at_once, const PassSplit &sp, const Tuning &tn) {
+static uint32_t sort_rows(uint32_t max_count, uint64_t keys_at_once, uint32_t key_bits, const PassSplit &sp, const Tuning &tn) {
     // an even number of passes, which ends in the split arrays without a second packed buffer
     if (sp.n % 2 != 0 || tn.sort_match) return kSortRows;
-    return keys_at_once <= kRows4Keys ? 4u : keys_at_once <= kRows8Keys ? 8u : kSortRows;
+    const uint32_t rows = keys_at_once <= kRows4Keys ? 4u : keys_at_once <= kRows8Keys ? 8u : kSortRows;
+    const size_t bytes = align_up(sizeof(Ctrl), 256) + align_up(sort_flag_words(max_count, sp, rows) * sizeof(uint64_t), 256) +
+                         align_up((size_t)max_count * 8, 256);
+    return bytes <= sort_scratch_bytes(max_count, key_bits) ? rows : kSortRows;
 }
 
 cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
@@ -1114,7 +1119,7 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
     if (cudaError_t e = ensure_sort_smem(); e != cudaSuccess) return e;
     const Tuning tn = tuning ? *tuning : default_tuning();
     const PassSplit sp = pass_split(key_bits, tn);
-    const uint32_t rows = sort_rows(std::max<uint64_t>(keys_at_once, max_count), sp, tn);
+    const uint32_t rows = sort_rows(max_count, std::max<uint64_t>(keys_at_once, max_count), key_bits, sp, tn);
     const SortLayout L = sort_layout(scratch, max_count, sp, rows);
     const bool overlap = frame_launch_overlaps(st);
     // With no pairs no kernel reads the flags, and none clears them: the arena mark stays.
