@@ -860,6 +860,7 @@ def main():
     P = statistics.mean(pairs)
     N = args.n
     hbm_peak, sm_max_mhz, peak_kind = measured_peaks()
+    compact = ((W + 15) // 16) * ((H + 15) // 16) <= 65536
     algo = {
         # records read once + key, index, splat record and 16-byte tile record written per visible
         # Gaussian
@@ -867,10 +868,12 @@ def main():
         # key histogram read + 4 passes of (key, index) read and written
         "depth_sort": 68.0 * V,
         # per rank: sorted index and tile record read, rectangle record and tile count written, the
-        # count scanned in place, rectangle and offset read by the emit; (tile, value) pairs written
-        "bin": V * (4 + 16 + 16 + 4 + 8 + 16 + 4) + 8.0 * P,
-        # 2 passes over (tile, value) pairs (digit histograms come from the per-tile counts)
-        "tile_sort": 32.0 * P,
+        # count scanned in place, rectangle and offset read by the emit; pair items (a word and a
+        # byte; whole 8-byte pairs above 65,536 tiles) written
+        "bin": V * (4 + 16 + 16 + 4 + 8 + 16 + 4) + (5.0 if compact else 8.0) * P,
+        # 2 passes over the items (digit histograms come from the per-tile counts): 5 + 4 bytes, then
+        # 4 + 4
+        "tile_sort": (17.0 if compact else 32.0) * P,
         "ranges": 4.0 * P,
         # pair ranks + splat records read per pair, frame written
         "raster": P * (4 + SPLAT_BYTES) + 4.0 * W * H,
@@ -882,7 +885,7 @@ def main():
         avg = tot_ms / n
         stages[s] = {"ms": avg, "launches": n, "algo_bytes": algo[s], "gbs": algo[s] / (avg / 1000.0) / 1e9,
                      "frac_hbm": algo[s] / (avg / 1000.0) / 1e9 / hbm_peak}
-    # The rasteriser is bound by FP32 issue, not HBM: its work is counted (evaluations of a
+    # The rasteriser is bound by FP32 arithmetic, not HBM: its work is counted (evaluations of a
     # pixel-splat pair, fragment alphas, channel-triple blends, transmittance updates) and
     # weighted by the FP32 FLOPs each step takes (11, 2, 16, 2; an FMA counts 2).
     sms = torch.cuda.get_device_properties(local).multi_processor_count
@@ -921,7 +924,7 @@ def main():
             "issue_frac": ras_issue[0] if ras_issue else None,
             "issue_source": f"{ras_issue[2]} (workload {ras_issue[1]})" if ras_issue else None,
             "issue_note": "instructions issued / SM issue peak (ncu sm__inst_issued.avg.pct_of_peak_sustained_active): "
-            "the kernel is issue-bound, so this, not the FP32 FLOP fraction, is its distance to the hardware limit",
+            "its instructions are packed arithmetic, shared loads, tests and rounding, few of them FLOPs",
         }
     else:
         roofline = {

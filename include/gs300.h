@@ -368,8 +368,9 @@ gs_status gs_batch_synchronize(gs_batch *batch, gs_stream stream);
 
 /* Launch choices of a batch that change its speed, never its frames. */
 typedef struct gs_tuning {
-    uint32_t suffix_min;       /* raster: tile lists of at least 3/4 of this many splats (1/4 of it in
-                                  ellipse frames) take the exact early-out (>= 1) */
+    uint32_t suffix_min;       /* raster: tile lists of at least 9/16 of this many splats (3/4 of it in
+                                  targets of few tiles, 1/4 in ellipse frames) take the exact
+                                  early-out (>= 1) */
     float eps;                 /* raster: transmittance ending the front-to-back walk, (0, 0.5] */
     uint32_t views_per_launch; /* views of one model sharing a preprocess launch, 1..16 */
     uint32_t streams;          /* streams the captured graph fans out over, 1..16 */
