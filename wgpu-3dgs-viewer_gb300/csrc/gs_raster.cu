@@ -892,9 +892,10 @@ struct ChunkSource {
         value = pair_value(next, next_cnt);
     }
 
-    // A splat into the thread's staged entry.
+    // A splat into the thread's staged entry.  True for a colour or an alpha out of its range (only a
+    // caller's own splats can have one): blend_list's arithmetic is for those within.
     template <uint32_t MODE, class Shared>
-    static __device__ __forceinline__ void put(Shared &S, const float4 a, const float4 b, const float4 c,
+    static __device__ __forceinline__ bool put(Shared &S, const float4 a, const float4 b, const float4 c,
                                                float std2) {
         const uint32_t tid = threadIdx.x;
         // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
@@ -918,26 +919,28 @@ struct ChunkSource {
             const float e2x = b.y * span, e2y = b.w * span;
             S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
         }
+        return !(splat_colour_reach(c.x, c.y, c.z) <= 255.0f && c.w >= 0.0f && c.w <= 1.0f && (c.x + c.y) + c.z <= 765.0f);
     }
 
     // Stage the chunk in flight (cnt entries), then put the next one (if more) in flight and read the
     // pairs [after, after + after_cnt).  The caller puts a barrier on either side.
     template <uint32_t MODE, class Shared>
-    __device__ __forceinline__ void stage(Shared &S, uint32_t cnt, float std2, bool more, uint32_t after,
+    __device__ __forceinline__ bool stage(Shared &S, uint32_t cnt, float std2, bool more, uint32_t after,
                                           uint32_t after_cnt) {
         const float4 *raw = S.raw + 3u * threadIdx.x;
         cp_async_wait_all();
-        if (threadIdx.x < cnt) put<MODE>(S, raw[0], raw[1], raw[2], std2);
+        const bool odd = threadIdx.x < cnt && put<MODE>(S, raw[0], raw[1], raw[2], std2);
         if (more) {
             fetch(S, value);
             value = pair_value(after, after_cnt);
         }
+        return odd;
     }
 
     // Stage a list that is one chunk, straight from memory.
     template <uint32_t MODE, class Shared>
-    __device__ __forceinline__ void stage_only(Shared &S, uint32_t n, float std2) const {
-        if (threadIdx.x >= n) return;
+    __device__ __forceinline__ bool stage_only(Shared &S, uint32_t n, float std2) const {
+        if (threadIdx.x >= n) return false;
         const uint32_t k = pair_value(0, n);
         float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
         if (k < max_splats) {
@@ -946,7 +949,7 @@ struct ChunkSource {
             b = __ldg(s + 1);
             c = __ldg(s + 2);
         }
-        put<MODE>(S, a, b, c, std2);
+        return put<MODE>(S, a, b, c, std2);
     }
 };
 
@@ -1168,6 +1171,41 @@ __device__ __forceinline__ void blend_list2(const RasterShared2 &S, uint32_t nl,
     }
 }
 
+// blend_list2 for lists with a colour or an alpha out of its range, whose product with alpha 0 may be NaN
+// and whose blend the additions may not round: one entry and pixel at a time, misses passed by.
+struct PairState {
+    float2 d[3], h[3];
+};
+template <uint32_t MODE, bool PORTABLE_EXP, bool BOTH>
+__device__ __noinline__ PairState blend_list2_odd(const RasterShared2 &S, uint32_t nl, float3 pc, float outline2, PairState P) {
+    const uint32_t warp = threadIdx.x >> 5;
+    for (uint32_t i = 0; i < nl; ++i) {
+        const uint32_t j = S.list[warp][i] / 16u;
+        const float4 la = S.la[j], gb = S.gb[j];
+        const float c[3] = {la.z, gb.x, gb.z};
+        float al;
+        if (fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pc.x, pc.y, outline2, &al)) {
+            const float om = __fsub_rn(1.0f, al);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float s = __fmul_rn(c[q], al);
+                P.d[q].x = blend8(P.d[q].x, om, s);
+                if (BOTH) P.h[q].x = blend8(P.h[q].x, om, s);
+            }
+        }
+        if (fragment<MODE, PORTABLE_EXP>(S.a[j], S.b[j], pc.x, pc.z, outline2, &al)) {
+            const float om = __fsub_rn(1.0f, al);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float s = __fmul_rn(c[q], al);
+                P.d[q].y = blend8(P.d[q].y, om, s);
+                if (BOTH) P.h[q].y = blend8(P.h[q].y, om, s);
+            }
+        }
+    }
+    return P;
+}
+
 // Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats, a pixel
 // a thread: three quarters of it (13.5k at 237x133 48 us a frame at 768, 52 at 384).  Two pixels a
 // thread walk half as many samples: nine sixteenths (576 by default: 477, 321, 1340 and 232 us at 6M /
@@ -1220,14 +1258,26 @@ __device__ __forceinline__ void raster_tile(
     // the thread's pixels: (px, py) and, with two, (px, py + 4)
     using Value = typename std::conditional<PX == 1, float, float2>::type;
     Value d[3] = {}, h[3] = {};
+    bool odd = false;  // a chunk staged so far had a colour or an alpha out of its range
     // blends the list onto the pixels whose `on` is set
     auto blend = [&](auto both, uint32_t nl, const bool *on) {
         if constexpr (PX == 1) {
-            blend_list<MODE, PORTABLE_EXP, COUNT, decltype(both)::value, UNROLL>(S, nl, on[0], pxc, pyc, outline2, d, h, n_eval,
-                                                                                 n_alpha, n_blend);
+            if (UNROLL > 1 && odd)
+                blend_list<MODE, PORTABLE_EXP, COUNT, decltype(both)::value, 1>(S, nl, on[0], pxc, pyc, outline2, d, h,
+                                                                                n_eval, n_alpha, n_blend);
+            else
+                blend_list<MODE, PORTABLE_EXP, COUNT, decltype(both)::value, UNROLL>(S, nl, on[0], pxc, pyc, outline2, d, h,
+                                                                                     n_eval, n_alpha, n_blend);
         } else {
             const float none = __int_as_float(0x7FC00000);
             const float3 pc = make_float3(pxc, on[0] ? pyc : none, on[1] ? pyc + 4.0f : none);
+            if (odd) {
+                PairState P{{d[0], d[1], d[2]}, {h[0], h[1], h[2]}};
+                P = blend_list2_odd<MODE, PORTABLE_EXP, decltype(both)::value>(S, nl, pc, outline2, P);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) d[q] = P.d[q], h[q] = P.h[q];
+                return;
+            }
             blend_list2<MODE, PORTABLE_EXP, COUNT, decltype(both)::value>(S, nl, pc, outline2, d, h, n_eval, n_alpha, n_blend);
         }
     };
@@ -1284,8 +1334,7 @@ __device__ __forceinline__ void raster_tile(
         for (uint32_t p = 0; p < PX; ++p) all_on[p] = true;
         if (n <= C && n < early_out_min<MODE, PX>(suffix_min)) {
             if (n > 0) {
-                src.template stage_only<MODE>(S, n, std2);
-                __syncthreads();
+                odd = __syncthreads_or(src.template stage_only<MODE>(S, n, std2));
                 const uint32_t nl = compact_chunk<MODE>(S, 0, n, bx0, bx1, by0, by1);
                 blend(std::false_type(), nl, all_on);
             }
@@ -1293,8 +1342,8 @@ __device__ __forceinline__ void raster_tile(
             src.begin(S, 0, C, C, min(C, n - C));
             for (uint32_t base = 0; base < n; base += C) {
                 const uint32_t cnt = min(C, n - base), after = base + 2u * C;
-                src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
-                __syncthreads();
+                odd |= __syncthreads_or(
+                    src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u));
                 const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
                 blend(std::false_type(), nl, all_on);
                 __syncthreads();
@@ -1385,8 +1434,8 @@ __device__ __forceinline__ void raster_tile(
                 for (uint32_t base = start; base < n; base += C) {
                     const uint32_t cnt = min(C, n - base), after = base + 2u * C;
                     __syncthreads();
-                    src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
-                    __syncthreads();
+                    odd |= __syncthreads_or(
+                        src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u));
                     // wmin is the warp's k: a warp whose suffix starts past this chunk skips it
                     if (wmin < base + C) {
                         const uint32_t nl = compact_chunk<MODE>(S, wmin > base ? wmin - base : 0u, cnt, bx0, bx1, by0, by1);
@@ -1404,8 +1453,9 @@ __device__ __forceinline__ void raster_tile(
                 }
                 __syncthreads();
                 if (any_active()) {
-                    active[0] = active[0] && !met(0);
-                    if (PX == 2) active[PX - 1] = active[PX - 1] && !met(PX - 1);
+                    // a pass over the whole list is exact, and the last: NaN would never meet itself
+                    active[0] = active[0] && k > 0 && !met(0);
+                    if (PX == 2) active[PX - 1] = active[PX - 1] && k > 0 && !met(PX - 1);
                     if (any_active()) {
                         const uint32_t suffix = n - k;
                         k = k > suffix ? k - suffix : 0u;
