@@ -893,7 +893,8 @@ struct ChunkSource {
     }
 
     // A splat into the thread's staged entry.  True for a colour or an alpha out of its range (only a
-    // caller's own splats can have one): blend_list's arithmetic is for those within.
+    // caller's own splats can have one): blend_list's arithmetic is for those within.  The test takes 478
+    // -> 482 us at 6M / 1080p.
     template <uint32_t MODE, class Shared>
     static __device__ __forceinline__ bool put(Shared &S, const float4 a, const float4 b, const float4 c,
                                                float std2) {
@@ -1237,7 +1238,7 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // iterations and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K: 935, 514 and
 // 2614 us with a walk A of every pixel over compacted lists and each chunk's loads waited for; 629,
 // 392 and 1864 us with the sampled walk, the loads a chunk ahead and the SFU exp without denormal
-// handling; 477, 321 and 1340 us with two pixels a thread, which share the list, the loads and, in
+// handling; 482, 323 and 1355 us with two pixels a thread, which share the list, the loads and, in
 // packed instructions, the arithmetic (64 registers, 8 CTAs an SM; 7, 9 and 10 CTAs take 497, 496 and
 // 506 us where 8 take 489).  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL, class Shared>
