@@ -885,9 +885,12 @@ struct ChunkSource {
         }
     }
 
-    // Start a walk: [base, base + cnt) goes into flight, [next, next + next_cnt) is the chunk after.
+    // Start a walk: [base, base + cnt) goes into flight, [next, next + next_cnt) is the chunk after.  A walk
+    // that ended early left a chunk in flight, whose copies nothing orders with new ones to the same
+    // places: they are waited for first.
     template <class Shared>
     __device__ __forceinline__ void begin(Shared &S, uint32_t base, uint32_t cnt, uint32_t next, uint32_t next_cnt) {
+        cp_async_wait_all();
         fetch(S, pair_value(base, cnt));
         value = pair_value(next, next_cnt);
     }
@@ -1328,6 +1331,7 @@ __device__ __forceinline__ void raster_tile(
                 end = base;
                 base = below(end);
             }
+            cp_async_wait_all();  // of a walk that ended early
         }
     } else {
         bool all_on[PX];
