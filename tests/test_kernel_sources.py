@@ -36,3 +36,18 @@ def test_no_copy_is_in_flight_when_a_walk_begins_or_a_tile_ends():
         assert min(w for w in waits if w >= 0) < rest.index("store(")
     points = _block(tile, tile.index("if constexpr (MODE == GS_DISPLAY_POINT)"))
     assert points.rindex("cp_async_wait_all();") > points.rindex("break;")
+
+
+# Tables that the host uploads before the launch: no kernel of a frame writes them.
+HOST_TABLES = {"jobs", "tile_base", "segs", "block_base"}
+
+
+def test_overlapped_kernels_read_what_their_predecessors_write_by_plain_loads():
+    """A kernel that starts while its predecessor still runs may not hold that one's output for constant:
+    no __restrict__ pointer and no read-only load, in the kernels or the functions they are made of."""
+    for name in ("gs_raster.cu", "gs_sort.cu", "gs_preprocess.cu"):
+        src = _source(name)
+        assert "frame_kernel_enter();" in src
+        assert not re.search(r"\b__(ldg|ldcs|ldca|ldlu)\(|ld\.global\.nc", src), name
+        names = set(re.findall(r"__restrict__\s+(\w+)", src))
+        assert names <= HOST_TABLES, (name, names - HOST_TABLES)

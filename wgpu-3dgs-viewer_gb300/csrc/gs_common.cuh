@@ -124,7 +124,11 @@ __device__ __forceinline__ void arena_clear(const Ctrl *owner, uint64_t *arena, 
     if (b < hi && block == 0 && threadIdx.x == 0) arena[b] = 0ull;
 }
 
-// Start of a kernel launched by launch_frame_kernel (a plain launch passes through).
+// Start of a kernel launched by launch_frame_kernel (a plain launch passes through).  The kernel may have
+// started while the one before it still wrote, so what that one writes is not constant for this
+// kernel's life: it is read through plain pointers.  A __restrict__ pointer or __ldg would let the
+// compiler read it by a path that assumes so, or ahead of the wait.  What no kernel of a frame
+// writes (records, selections, tables the host uploaded) may be read in any way.
 __device__ __forceinline__ void frame_kernel_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -182,10 +182,10 @@ __device__ __forceinline__ bool rect_may_hold(uint32_t rect, uint32_t tile) {
 // gets its rectangle in one word, an empty one where there is no splat or no tile is kept; the first
 // segment's launch (reset non-null) starts the call's control block.
 __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
-    const gs_splat *__restrict__ splats, const uint4 *__restrict__ binfo, const uint32_t *__restrict__ sorted_index,
-    const uint32_t *count, uint32_t max_count, uint32_t base, gs_splat *__restrict__ sorted_out, int several,
-    uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *__restrict__ info,
-    uint32_t *__restrict__ counts, const Ctrl *owner, uint64_t *arena, uint32_t *__restrict__ rects,
+    const gs_splat *splats, const uint4 *binfo, const uint32_t *sorted_index,
+    const uint32_t *count, uint32_t max_count, uint32_t base, gs_splat *sorted_out, int several,
+    uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
+    uint32_t *counts, const Ctrl *owner, uint64_t *arena, uint32_t *rects,
     uint32_t rect_shift, Ctrl *reset, uint32_t arena_words) {
     frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
         } else {
             // all three 16-byte parts in one round trip (the colour bounds the corner-tile test)
             const float4 *src = reinterpret_cast<const float4 *>(splats + gi);
-            const float4 a = __ldg(src);
-            const float4 q = __ldg(src + 1);
-            const float4 c = __ldg(src + 2);
+            const float4 a = src[0];
+            const float4 q = src[1];
+            const float4 c = src[2];
             if (sorted_out) {
                 float4 *dst = reinterpret_cast<float4 *>(sorted_out + base + k);
                 dst[0] = a;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
 // the last tile records the pairs wanted and kept, and a list overflow.
-__global__ void __launch_bounds__(256) bin_scan_kernel(uint32_t *__restrict__ data, const uint32_t *count,
+__global__ void __launch_bounds__(256) bin_scan_kernel(uint32_t *data, const uint32_t *count,
                                                        uint32_t max_count, uint32_t max_pairs, Ctrl *ctrl,
                                                        uint64_t *flags) {
     __shared__ uint32_t s_warp[8];
@@ -358,9 +358,9 @@ struct EmitWindow {
 
 template <bool COUNTS, bool COMPACT>
 __global__ void __launch_bounds__(kBinThreads, 5) bin_emit_kernel(
-    const uint4 *__restrict__ info, const uint32_t *__restrict__ offsets, const uint32_t *count, uint32_t max_count,
-    uint2 *__restrict__ pairs, uint32_t max_pairs, uint32_t value_bits, uint32_t tiles_x, uint32_t ntiles, Ctrl *ctrl,
-    Ctrl *sort_ctrl, const PassSplit split, uint32_t *__restrict__ blockcounts) {
+    const uint4 *info, const uint32_t *offsets, const uint32_t *count, uint32_t max_count,
+    uint2 *pairs, uint32_t max_pairs, uint32_t value_bits, uint32_t tiles_x, uint32_t ntiles, Ctrl *ctrl,
+    Ctrl *sort_ctrl, const PassSplit split, uint32_t *blockcounts) {
     extern __shared__ uint32_t s_bins[];
     __shared__ EmitWindow s_win[kBinThreads / 32];
     const uint32_t nbins = COUNTS ? ntiles : 4u * 256u;
@@ -517,8 +517,8 @@ __global__ void __launch_bounds__(kBinThreads, 5) bin_emit_kernel(
 // [start, end) of every tile from its pair count where the target has too many tiles for
 // tile_scan_kernel: one CTA, 8192 tiles at a time (4K: 4 rounds, 17 us; 52 us finding the ends in the
 // sorted pairs).
-__global__ void __launch_bounds__(1024) tile_starts_kernel(const uint32_t *__restrict__ counts, uint32_t ntiles,
-                                                           uint2 *__restrict__ ranges) {
+__global__ void __launch_bounds__(1024) tile_starts_kernel(const uint32_t *counts, uint32_t ntiles,
+                                                           uint2 *ranges) {
     __shared__ __align__(16) uint32_t s_v[8192 + 4];
     __shared__ uint32_t s_w[32];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -585,8 +585,8 @@ __global__ void __launch_bounds__(256) raster_init_kernel(Ctrl *ctrl, Ctrl *sort
 // counts.  blockIdx.y takes a slice of the emit CTAs, so the sum runs wide, not long.
 constexpr uint32_t kCountSlices = 16;
 
-__global__ void __launch_bounds__(256) tile_count_kernel(const uint32_t *__restrict__ blockcounts, uint32_t nblocks,
-                                                         uint32_t ntiles, uint32_t *__restrict__ counts) {
+__global__ void __launch_bounds__(256) tile_count_kernel(const uint32_t *blockcounts, uint32_t nblocks,
+                                                         uint32_t ntiles, uint32_t *counts) {
     frame_kernel_enter();
     const uint32_t t = blockIdx.x * 256u + threadIdx.x;
     if (t >= ntiles) return;
@@ -621,8 +621,8 @@ __device__ __forceinline__ uint32_t order_class(uint32_t c) {
 // with strided accesses, an atomic per tile and digit and a serial walk over the classes).
 constexpr uint32_t kScanTilesMax = 8192;
 static_assert(kCountTiles <= kScanTilesMax, "8 tiles a thread");
-__global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restrict__ counts, uint32_t ntiles,
-                                                         uint2 *__restrict__ ranges, uint32_t *__restrict__ order,
+__global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *counts, uint32_t ntiles,
+                                                         uint2 *ranges, uint32_t *order,
                                                          Ctrl *sort_ctrl, const PassSplit split) {
     __shared__ __align__(16) uint32_t s_v[kScanTilesMax + 4];
     __shared__ uint32_t s_w[32], s_low[1024], s_lw[10], s_cls[96];
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(const uint32_t *__restr
 
 // [start, end) of every tile's run in the tile-sorted pairs; each thread checks four
 // consecutive pairs with two 16-byte loads.
-__global__ void tile_ranges_kernel(const uint2 *__restrict__ pairs, const Ctrl *ctrl, uint2 *ranges,
+__global__ void tile_ranges_kernel(const uint2 *pairs, const Ctrl *ctrl, uint2 *ranges,
                                    uint32_t ntiles) {
     frame_kernel_enter();
     const uint32_t n = ctrl->count;
@@ -862,8 +862,8 @@ using RasterSharedOf = typename std::conditional<PX == 1, RasterShared1, RasterS
 // pair of the chunk after that is in a register, so neither of the two dependent global loads of
 // an entry is waited for while the warps blend.
 struct ChunkSource {
-    const gs_splat *__restrict__ splats;
-    const uint32_t *__restrict__ values;  // the tile's own list (RasterJob::values)
+    const gs_splat *splats;
+    const uint32_t *values;  // the tile's own list (RasterJob::values)
     uint32_t value_shift, max_splats;
     uint32_t value;  // pair value of the chunk after the one in flight
 
@@ -949,9 +949,9 @@ struct ChunkSource {
         float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
         if (k < max_splats) {
             const float4 *s = reinterpret_cast<const float4 *>(splats + k);
-            a = __ldg(s);
-            b = __ldg(s + 1);
-            c = __ldg(s + 2);
+            a = s[0];
+            b = s[1];
+            c = s[2];
         }
         return put<MODE>(S, a, b, c, std2);
     }
@@ -1246,7 +1246,7 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // 506 us where 8 take 489).  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL, class Shared>
 __device__ __forceinline__ void raster_tile(
-    Shared &S, const RasterJob &J, const uint32_t *__restrict__ list, uint32_t list_shift, uint32_t n, float std2,
+    Shared &S, const RasterJob &J, const uint32_t *list, uint32_t list_shift, uint32_t n, float std2,
     float outline2, uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
     // Work tallies of the counting variant (profiling only): fragment evaluations, alphas,
     // channel-triple blends and transmittance updates.
@@ -1538,8 +1538,8 @@ __global__ void __launch_bounds__(kTileThreads<MODE, FEW>, kTileCtas<MODE, FEW>)
 // words 102 us), the lists by the latency of a thread's few tile records.
 template <uint32_t MODE, bool PORTABLE_EXP, bool FEW>
 __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
-    raster_direct_kernel(const RasterJob J, const uint32_t *__restrict__ rects, const uint4 *__restrict__ info,
-                         uint32_t ranks, uint32_t shift, uint32_t *__restrict__ values, uint32_t max_pairs, float std2,
+    raster_direct_kernel(const RasterJob J, const uint32_t *rects, const uint4 *info,
+                         uint32_t ranks, uint32_t shift, uint32_t *values, uint32_t max_pairs, float std2,
                          float outline2, uint32_t suffix_min, float eps) {
     __shared__ RasterShared1 S;
     __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;

@@ -128,7 +128,7 @@ __device__ __forceinline__ void hist_add(uint32_t *h, uint32_t k, bool valid, co
 constexpr uint32_t kHistThreads = 1024;
 constexpr uint32_t kHistCtas = 152 * 2;  // resident at once
 // CTA `block` of the `blocks` that count one sort's keys.
-__device__ __forceinline__ void sort_hist_block(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
+__device__ __forceinline__ void sort_hist_block(const uint32_t *keys, const uint32_t *vals,
                                                 const uint32_t *count, uint32_t max_count, const PassSplit &sp,
                                                 Ctrl *ctrl, uint64_t *arena, uint32_t block, uint32_t blocks) {
     __shared__ uint32_t h[1024];
@@ -209,8 +209,8 @@ __device__ __forceinline__ void sort_hist_block(const uint32_t *__restrict__ key
     }
 }
 
-__global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(const uint32_t *__restrict__ keys,
-                                                                 const uint32_t *__restrict__ vals,
+__global__ void __launch_bounds__(kHistThreads) sort_hist_kernel(const uint32_t *keys,
+                                                                 const uint32_t *vals,
                                                                  const uint32_t *count, uint32_t max_count,
                                                                  const __grid_constant__ PassSplit sp, Ctrl *ctrl,
                                                                  uint64_t *arena) {
@@ -271,8 +271,8 @@ __device__ __forceinline__ uint32_t look_back_digit(const uint64_t *flags, uint3
 // CTAs of the same launch).
 template <bool IN_PACKED, bool OUT_PACKED, bool MATCH, uint32_t ROWS = kSortRows>
 __device__ __forceinline__ void sort_pass_block(
-    const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
-    uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
+    const uint32_t *kin, const uint32_t *vin, const uint2 *pin,
+    uint32_t *kout, uint32_t *vout, uint2 *pout, const uint32_t *count,
     uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags, uint32_t block) {
     constexpr uint32_t KEYS = kSortThreads * ROWS;
     extern __shared__ uint2 s_kv[];  // KEYS pairs (dynamic)
@@ -425,10 +425,10 @@ constexpr size_t kItemDynSmem = kTileKeys * sizeof(uint32_t) + (FIRST ? kTileKey
 
 template <bool FIRST, bool TALLY>
 __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
-    tile_pass_kernel(const uint32_t *__restrict__ in, const uint8_t *__restrict__ low, uint32_t *__restrict__ out,
+    tile_pass_kernel(const uint32_t *in, const uint8_t *low, uint32_t *out,
                      const uint32_t *count, uint32_t max_count, uint32_t hoff, uint32_t value_bits,
                      uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags, uint32_t low_bits,
-                     uint32_t *__restrict__ tile_counts, uint32_t target_tiles) {
+                     uint32_t *tile_counts, uint32_t target_tiles) {
     extern __shared__ __align__(16) uint8_t item_smem[];
     uint32_t *s_item = reinterpret_cast<uint32_t *>(item_smem);
     uint8_t *s_low = item_smem + kTileKeys * sizeof(uint32_t);  // FIRST: the digit of each reordered item
@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(kSortThreads, kItemCtasPerSm)
 
 template <bool IN_PACKED, bool OUT_PACKED, bool MATCH, uint32_t ROWS = kSortRows>
 __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) sort_pass_kernel(
-    const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, const uint2 *__restrict__ pin,
-    uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint2 *__restrict__ pout, const uint32_t *count,
+    const uint32_t *kin, const uint32_t *vin, const uint2 *pin,
+    uint32_t *kout, uint32_t *vout, uint2 *pout, const uint32_t *count,
     uint32_t max_count, uint32_t hoff, uint32_t shift, uint32_t digit_bits, Ctrl *ctrl, uint64_t *flags) {
     // look-back predecessors are lower, earlier-dispatched CTAs
     sort_pass_block<IN_PACKED, OUT_PACKED, MATCH, ROWS>(kin, vin, pin, kout, vout, pout, count, max_count, hoff, shift,
@@ -900,7 +900,7 @@ __device__ __forceinline__ uint32_t remote_smem(const void *p, uint32_t cta) {
 
 template <uint32_t ROWS>
 __global__ void __launch_bounds__(kClusterThreads, 1)
-    sort_cluster_kernel(uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, const uint32_t *count,
+    sort_cluster_kernel(uint32_t *keys, uint32_t *vals, const uint32_t *count,
                         uint32_t max_count, const PassSplit sp, Ctrl *ctrl) {
     constexpr uint32_t K = kClusterThreads * ROWS;
     extern __shared__ __align__(16) uint8_t cluster_smem[];
