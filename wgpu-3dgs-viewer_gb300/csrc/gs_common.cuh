@@ -49,7 +49,8 @@ struct Ctrl {
     uint32_t ticket[8];
     uint32_t count;       // preprocess: V; raster: tile pairs kept
     uint32_t total;       // raster: tile pairs wanted (saturating)
-    uint32_t unused[2];
+    uint32_t colours;     // raster: largest colour_class of the frame's splats
+    uint32_t unused;
     uint32_t serial;      // area owner: last epoch handed out in the area
     uint32_t clean;       // area owner: leading arena words holding only zeros or flag words
     uint32_t clear_lo;    // area owner: arena words [clear_lo, clear_hi) to clear in this call
@@ -91,6 +92,7 @@ __device__ __forceinline__ void ctrl_reset(Ctrl *ctrl, Ctrl *owner, uint32_t are
         for (int k = 0; k < 8; ++k) ctrl->ticket[k] = 0u;
         ctrl->count = 0u;
         ctrl->total = 0u;
+        ctrl->colours = 0u;
         ctrl->spin_limit = cfg.spin_limit;
         ctrl->stall_tile = cfg.stall_tile;
     }

@@ -47,6 +47,8 @@ struct RasterLayout {
     uint32_t tiles_x, tiles_y, ntiles, key_bits;
     uint32_t value_bits;  // compact items (see launch_sort_items): bits of a pair value; 0: whole pairs
     uint32_t *items() const { return reinterpret_cast<uint32_t *>(pairs); }
+    // A direct frame sorts no tiles: a word for each CTA of its tile records in the sort's histograms.
+    uint32_t *blocks() const { return &sort_ctrl->hist[0][0]; }
     uint8_t *low(uint32_t max_pairs) const { return reinterpret_cast<uint8_t *>(pairs) + (size_t)max_pairs * 4; }
 };
 
@@ -58,6 +60,8 @@ constexpr uint32_t kEmitBlocks = 152 * 8;
 
 // Ranks a direct frame can have: a bit each in shared memory (RasterShared::raw).
 constexpr uint32_t kDirectMaxRanks = 3u * 16u * kRasterThreads * 8u;
+// ... and CTAs of tile records, segments rounded up (RasterLayout::blocks).
+constexpr uint32_t kDirectMaxBlocks = sizeof(Ctrl::hist) / sizeof(uint32_t);
 
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = 256 * kScanItems;
@@ -170,6 +174,21 @@ __device__ __forceinline__ bool rect_may_hold(uint32_t rect, uint32_t tile) {
     return (((tile | kRectGuard) - rect) & kRectGuard) == kRectGuard;
 }
 
+// Range of a splat's colour and alpha.  The preprocess writes colours of 0..255 and alphas of 0..1: class 0.
+// A caller's own splats may hold others: class k, 1..kColourClasses, for colours within +-255 2^k, whose
+// blends stay within them too as long as the alpha is in 0..1; kWildColours for the rest and NaN.
+constexpr uint32_t kColourClasses = 12, kWildColours = 15;
+__device__ __forceinline__ uint32_t colour_class(const float4 c) {
+    const bool alpha = c.w >= 0.0f && c.w <= 1.0f;
+    // the sum is for NaN, which the comparisons of the reach pass over
+    if (alpha && splat_colour_reach(c.x, c.y, c.z) <= 255.0f && (c.x + c.y) + c.z <= 765.0f) return 0u;
+    const float reach = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))), sum = (c.x + c.y) + c.z;
+    if (!alpha || sum != sum || !(reach <= 255.0f * (float)(1u << kColourClasses))) return kWildColours;
+    uint32_t k = 1;
+    while (255.0f * (float)(1u << k) < reach) ++k;
+    return k;
+}
+
 // K3a: per draw rank, the splat's tile rectangle, the corner tiles its footprint misses, and
 // its tile count.  With `binfo` (the preprocess having stored each visible splat's tiles) the rank
 // gathers that 16-byte record; otherwise it gathers the 48-byte splat and works the tiles out here.
@@ -180,50 +199,61 @@ __device__ __forceinline__ bool rect_may_hold(uint32_t rect, uint32_t tile) {
 // clear, before the scan and the tile sort read any flag.
 // With `rects` (and no counts) the ranks are scanned by raster_direct_kernel up to the capacity: each
 // gets its rectangle in one word, an empty one where there is no splat or no tile is kept; the first
-// segment's launch (reset non-null) starts the call's control block.
+// segment's launch (reset non-null) starts the call's control block.  The splats' colour_class goes to the
+// owner, or with `rects` each CTA's to its word of `blocks` (tile records stand for class 0).
 __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     const gs_splat *splats, const uint4 *binfo, const uint32_t *sorted_index,
     const uint32_t *count, uint32_t max_count, uint32_t base, gs_splat *sorted_out, int several,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
-    uint32_t *counts, const Ctrl *owner, uint64_t *arena, uint32_t *rects,
-    uint32_t rect_shift, Ctrl *reset, uint32_t arena_words) {
+    uint32_t *counts, Ctrl *owner, uint64_t *arena, uint32_t *rects,
+    uint32_t rect_shift, Ctrl *reset, uint32_t arena_words, uint32_t *blocks) {
+    __shared__ uint32_t s_class;
+    if (threadIdx.x == 0) s_class = 0u;
+    __syncthreads();
     frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
     if (reset && blockIdx.x == 0 && threadIdx.x == 0) ctrl_reset_flagless(reset, arena_words);
     const uint32_t n = count ? min(*count, max_count) : max_count;
     const uint32_t k = blockIdx.x * kBinThreads + threadIdx.x;
-    if (k >= n) {
-        if (k >= max_count) return;
-        if (rects) rects[k] = kEmptyRect;
-        else if (several) counts[k] = 0u;  // several models: the scan covers every segment's capacity
+    uint4 t = make_uint4(0u, 0u, 0u, 0u);  // x0 | y0 << 16, w | h << 16, mask, count
+    uint32_t colours = 0;
+    if (k < n) {
+        // Indices come from the depth sort; the bound check only matters if that sort timed out.
+        const uint32_t gi = sorted_index[k];
+        if (gi < max_count) {
+            if (binfo) {
+                t = binfo[gi];
+            } else {
+                // all three 16-byte parts in one round trip (the colour bounds the corner-tile test)
+                const float4 *src = reinterpret_cast<const float4 *>(splats + gi);
+                const float4 a = src[0];
+                const float4 q = src[1];
+                const float4 c = src[2];
+                if (sorted_out) {
+                    float4 *dst = reinterpret_cast<float4 *>(sorted_out + base + k);
+                    dst[0] = a;
+                    dst[1] = q;
+                    dst[2] = c;
+                }
+                t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
+                if (t.w) colours = colour_class(c);
+            }
+        }
+        info[k] = make_uint4(t.x, t.y, t.z, base + (sorted_out ? k : gi));
+    }
+    if (!rects) {
+        if (k < n) counts[k] = t.w;
+        else if (k < max_count && several) counts[k] = 0u;  // the scan covers every segment's capacity
+        if (colours) atomicMax(&owner->colours, colours);
         return;
     }
-    // Indices come from the depth sort; the bound check only matters if that sort timed out.
-    const uint32_t gi = sorted_index[k];
-    uint4 t = make_uint4(0u, 0u, 0u, 0u);  // x0 | y0 << 16, w | h << 16, mask, count
-    if (gi < max_count) {
-        if (binfo) {
-            t = binfo[gi];
-        } else {
-            // all three 16-byte parts in one round trip (the colour bounds the corner-tile test)
-            const float4 *src = reinterpret_cast<const float4 *>(splats + gi);
-            const float4 a = src[0];
-            const float4 q = src[1];
-            const float4 c = src[2];
-            if (sorted_out) {
-                float4 *dst = reinterpret_cast<float4 *>(sorted_out + base + k);
-                dst[0] = a;
-                dst[1] = q;
-                dst[2] = c;
-            }
-            t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
-        }
-    }
-    if (counts) counts[k] = t.w;
-    else rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
-                                    (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
-                        : kEmptyRect;
-    info[k] = make_uint4(t.x, t.y, t.z, base + (sorted_out ? k : gi));
+    if (k < max_count)
+        rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
+                                   (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
+                       : kEmptyRect;
+    if (colours) atomicMax(&s_class, colours);
+    __syncthreads();
+    if (threadIdx.x == 0) blocks[blockIdx.x] = s_class;
 }
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
@@ -895,11 +925,9 @@ struct ChunkSource {
         value = pair_value(next, next_cnt);
     }
 
-    // A splat into the thread's staged entry.  True for a colour or an alpha out of its range (only a
-    // caller's own splats can have one): blend_list's arithmetic is for those within.  The test takes 478
-    // -> 482 us at 6M / 1080p.
+    // A splat into the thread's staged entry.
     template <uint32_t MODE, class Shared>
-    static __device__ __forceinline__ bool put(Shared &S, const float4 a, const float4 b, const float4 c,
+    static __device__ __forceinline__ void put(Shared &S, const float4 a, const float4 b, const float4 c,
                                                float std2) {
         const uint32_t tid = threadIdx.x;
         // Fragments beyond the r² limit cannot change the pixel (see splat_r2_bound).
@@ -923,28 +951,26 @@ struct ChunkSource {
             const float e2x = b.y * span, e2y = b.w * span;
             S.inv[tid] = make_float2(__frcp_rn(e1x * e1x + e1y * e1y), __frcp_rn(e2x * e2x + e2y * e2y));
         }
-        return !(splat_colour_reach(c.x, c.y, c.z) <= 255.0f && c.w >= 0.0f && c.w <= 1.0f && (c.x + c.y) + c.z <= 765.0f);
     }
 
     // Stage the chunk in flight (cnt entries), then put the next one (if more) in flight and read the
     // pairs [after, after + after_cnt).  The caller puts a barrier on either side.
     template <uint32_t MODE, class Shared>
-    __device__ __forceinline__ bool stage(Shared &S, uint32_t cnt, float std2, bool more, uint32_t after,
+    __device__ __forceinline__ void stage(Shared &S, uint32_t cnt, float std2, bool more, uint32_t after,
                                           uint32_t after_cnt) {
         const float4 *raw = S.raw + 3u * threadIdx.x;
         cp_async_wait_all();
-        const bool odd = threadIdx.x < cnt && put<MODE>(S, raw[0], raw[1], raw[2], std2);
+        if (threadIdx.x < cnt) put<MODE>(S, raw[0], raw[1], raw[2], std2);
         if (more) {
             fetch(S, value);
             value = pair_value(after, after_cnt);
         }
-        return odd;
     }
 
     // Stage a list that is one chunk, straight from memory.
     template <uint32_t MODE, class Shared>
-    __device__ __forceinline__ bool stage_only(Shared &S, uint32_t n, float std2) const {
-        if (threadIdx.x >= n) return false;
+    __device__ __forceinline__ void stage_only(Shared &S, uint32_t n, float std2) const {
+        if (threadIdx.x >= n) return;
         const uint32_t k = pair_value(0, n);
         float4 a = make_float4(0.0f, 0.0f, -1.0f, -1.0f), b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = b;
         if (k < max_splats) {
@@ -953,7 +979,7 @@ struct ChunkSource {
             b = s[1];
             c = s[2];
         }
-        return put<MODE>(S, a, b, c, std2);
+        put<MODE>(S, a, b, c, std2);
     }
 };
 
@@ -1175,13 +1201,13 @@ __device__ __forceinline__ void blend_list2(const RasterShared2 &S, uint32_t nl,
     }
 }
 
-// blend_list2 for lists with a colour or an alpha out of its range, whose product with alpha 0 may be NaN
-// and whose blend the additions may not round: one entry and pixel at a time, misses passed by.
+// blend_list2 for frames of kWildColours, whose products with alpha 0 may be NaN and whose blends the
+// additions may not round: one entry and pixel at a time, misses passed by.
 struct PairState {
     float2 d[3], h[3];
 };
 template <uint32_t MODE, bool PORTABLE_EXP, bool BOTH>
-__device__ __noinline__ PairState blend_list2_odd(const RasterShared2 &S, uint32_t nl, float3 pc, float outline2, PairState P) {
+__device__ __noinline__ PairState blend_list2_wild(const RasterShared2 &S, uint32_t nl, float3 pc, float outline2, PairState P) {
     const uint32_t warp = threadIdx.x >> 5;
     for (uint32_t i = 0; i < nl; ++i) {
         const uint32_t j = S.list[warp][i] / 16u;
@@ -1232,7 +1258,9 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 //      samples at a time: k only says where to start, so no pixel's own walk is needed;
 //   B. blend positions k.. back to front twice, from destination 0 and from 255.  The blend
 //      with 8-bit rounding is monotone in the destination, so the two results bound the
-//      result of every history before k; when they meet, that is the exact pixel.  A pixel
+//      result of every history before k; when they meet, that is the exact pixel.  (Colours of
+//      class k leave histories within +-255 2^k, from which the two start then; wild colours
+//      leave none that is bounded, and their lists are blended in one pass.)  A pixel
 //      whose bounds do not meet restarts B from k - (n - k) (k = 0 starts from the cleared
 //      value, which is exact).
 // Every pixel therefore ends bit-identical to the full back-to-front pass.
@@ -1247,7 +1275,7 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL, class Shared>
 __device__ __forceinline__ void raster_tile(
     Shared &S, const RasterJob &J, const uint32_t *list, uint32_t list_shift, uint32_t n, float std2,
-    float outline2, uint32_t suffix_min, float eps, unsigned long long *counters, uint32_t tile) {
+    float outline2, uint32_t suffix_min, float eps, uint32_t colours, unsigned long long *counters, uint32_t tile) {
     // Work tallies of the counting variant (profiling only): fragment evaluations, alphas,
     // channel-triple blends and transmittance updates.
     uint32_t n_eval = 0, n_alpha = 0, n_blend = 0, n_trans = 0;
@@ -1262,11 +1290,12 @@ __device__ __forceinline__ void raster_tile(
     // the thread's pixels: (px, py) and, with two, (px, py + 4)
     using Value = typename std::conditional<PX == 1, float, float2>::type;
     Value d[3] = {}, h[3] = {};
-    bool odd = false;  // a chunk staged so far had a colour or an alpha out of its range
+    const bool wild = colours > kColourClasses;
+    const uint32_t early = wild ? 0xFFFFFFFFu : early_out_min<MODE, PX>(suffix_min);
     // blends the list onto the pixels whose `on` is set
     auto blend = [&](auto both, uint32_t nl, const bool *on) {
         if constexpr (PX == 1) {
-            if (UNROLL > 1 && odd)
+            if (UNROLL > 1 && wild)
                 blend_list<MODE, PORTABLE_EXP, COUNT, decltype(both)::value, 1>(S, nl, on[0], pxc, pyc, outline2, d, h,
                                                                                 n_eval, n_alpha, n_blend);
             else
@@ -1275,9 +1304,9 @@ __device__ __forceinline__ void raster_tile(
         } else {
             const float none = __int_as_float(0x7FC00000);
             const float3 pc = make_float3(pxc, on[0] ? pyc : none, on[1] ? pyc + 4.0f : none);
-            if (odd) {
+            if (wild) {
                 PairState P{{d[0], d[1], d[2]}, {h[0], h[1], h[2]}};
-                P = blend_list2_odd<MODE, PORTABLE_EXP, decltype(both)::value>(S, nl, pc, outline2, P);
+                P = blend_list2_wild<MODE, PORTABLE_EXP, decltype(both)::value>(S, nl, pc, outline2, P);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) d[q] = P.d[q], h[q] = P.h[q];
                 return;
@@ -1337,18 +1366,19 @@ __device__ __forceinline__ void raster_tile(
         bool all_on[PX];
 #pragma unroll
         for (uint32_t p = 0; p < PX; ++p) all_on[p] = true;
-        if (n <= C && n < early_out_min<MODE, PX>(suffix_min)) {
+        if (n <= C && n < early) {
             if (n > 0) {
-                odd = __syncthreads_or(src.template stage_only<MODE>(S, n, std2));
+                src.template stage_only<MODE>(S, n, std2);
+                __syncthreads();
                 const uint32_t nl = compact_chunk<MODE>(S, 0, n, bx0, bx1, by0, by1);
                 blend(std::false_type(), nl, all_on);
             }
-        } else if (n < early_out_min<MODE, PX>(suffix_min)) {
+        } else if (n < early) {
             src.begin(S, 0, C, C, min(C, n - C));
             for (uint32_t base = 0; base < n; base += C) {
                 const uint32_t cnt = min(C, n - base), after = base + 2u * C;
-                odd |= __syncthreads_or(
-                    src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u));
+                src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
+                __syncthreads();
                 const uint32_t nl = compact_chunk<MODE>(S, 0, cnt, bx0, bx1, by0, by1);
                 blend(std::false_type(), nl, all_on);
                 __syncthreads();
@@ -1424,14 +1454,14 @@ __device__ __forceinline__ void raster_tile(
                 __syncthreads();
                 const uint32_t kmin = S.kmin;
                 if (kmin == 0xFFFFFFFFu) break;
-                const float top = (k == 0) ? 0.0f : 255.0f;
+                const float top = (k == 0) ? 0.0f : 255.0f * (float)(1u << colours), low = colours ? -top : 0.0f;
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
                     if constexpr (PX == 1) {
-                        if (active[0]) d[q] = 0.0f, h[q] = top;
+                        if (active[0]) d[q] = low, h[q] = top;
                     } else {
-                        if (active[0]) d[q].x = 0.0f, h[q].x = top;
-                        if (active[1]) d[q].y = 0.0f, h[q].y = top;
+                        if (active[0]) d[q].x = low, h[q].x = top;
+                        if (active[1]) d[q].y = low, h[q].y = top;
                     }
                 }
                 const uint32_t start = kmin / C * C;
@@ -1439,8 +1469,8 @@ __device__ __forceinline__ void raster_tile(
                 for (uint32_t base = start; base < n; base += C) {
                     const uint32_t cnt = min(C, n - base), after = base + 2u * C;
                     __syncthreads();
-                    odd |= __syncthreads_or(
-                        src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u));
+                    src.template stage<MODE>(S, cnt, std2, base + C < n, after, after < n ? min(C, n - after) : 0u);
+                    __syncthreads();
                     // wmin is the warp's k: a warp whose suffix starts past this chunk skips it
                     if (wmin < base + C) {
                         const uint32_t nl = compact_chunk<MODE>(S, wmin > base ? wmin - base : 0u, cnt, bx0, bx1, by0, by1);
@@ -1458,7 +1488,7 @@ __device__ __forceinline__ void raster_tile(
                 }
                 __syncthreads();
                 if (any_active()) {
-                    // a pass over the whole list is exact, and the last: NaN would never meet itself
+                    // a pass over the whole list is exact, and the last
                     active[0] = active[0] && k > 0 && !met(0);
                     if (PX == 2) active[PX - 1] = active[PX - 1] && k > 0 && !met(PX - 1);
                     if (any_active()) {
@@ -1527,7 +1557,7 @@ __global__ void __launch_bounds__(kTileThreads<MODE, FEW>, kTileCtas<MODE, FEW>)
     const uint32_t tile = J.order ? J.order[blockIdx.x] : blockIdx.x;
     const uint2 r = tile_range(J, tile);
     raster_tile<MODE, PORTABLE_EXP, COUNT, FEW ? 4u : 1u>(S, J, J.values + ((size_t)r.x << J.value_shift), J.value_shift,
-                                                          r.y - r.x, std2, outline2, suffix_min, eps,
+                                                          r.y - r.x, std2, outline2, suffix_min, eps, J.ctrl->colours,
                                                           counters, tile);
 }
 
@@ -1540,9 +1570,9 @@ template <uint32_t MODE, bool PORTABLE_EXP, bool FEW>
 __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     raster_direct_kernel(const RasterJob J, const uint32_t *rects, const uint4 *info,
                          uint32_t ranks, uint32_t shift, uint32_t *values, uint32_t max_pairs, float std2,
-                         float outline2, uint32_t suffix_min, float eps) {
+                         float outline2, uint32_t suffix_min, float eps, const uint32_t *blocks, uint32_t nblocks) {
     __shared__ RasterShared1 S;
-    __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;
+    __shared__ uint32_t s_warp[kRasterThreads / 32], s_class[kRasterThreads / 32], s_base;
     uint32_t *hits = reinterpret_cast<uint32_t *>(S.raw);  // bit r of word q: rank 32 q + r holds the tile
     static_assert(sizeof(S.raw) * 8 >= kDirectMaxRanks, "a bit per rank");
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
@@ -1550,6 +1580,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     const uint32_t here = pack_rect(tx, ty, tx, ty, shift);
     constexpr uint32_t STEP = kRasterThreads / 32u;
     frame_kernel_enter();
+    uint32_t colours = tid < nblocks ? blocks[tid] : 0u;  // waited for after the scan
     for (uint32_t q0 = warp; q0 < words; q0 += 8u * STEP) {
         uint32_t r[8];
 #pragma unroll
@@ -1588,12 +1619,16 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
         if (lane >= o) incl += y;
     }
     if (lane == 31) s_warp[warp] = incl;
+    for (uint32_t b = tid + kRasterThreads; b < nblocks; b += kRasterThreads) colours = max(colours, blocks[b]);
+    colours = __reduce_max_sync(0xFFFFFFFFu, colours);
+    if (lane == 0) s_class[warp] = colours;
     __syncthreads();
     uint32_t before = 0, n = 0;
 #pragma unroll
     for (uint32_t w = 0; w < kRasterThreads / 32u; ++w) {
         if (w < warp) before += s_warp[w];
         n += s_warp[w];
+        colours = max(colours, s_class[w]);
     }
     if (tid == 0) s_base = n ? atomicAdd(&J.ctrl->total, n) : 0u;
     __syncthreads();
@@ -1607,8 +1642,8 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
             for (uint32_t m = hits[q]; m; m &= m - 1u) values[at++] = info[32u * q + __ffs(m) - 1u].w;
     }
     __syncthreads();
-    raster_tile<MODE, PORTABLE_EXP, false, FEW ? 4u : 1u>(S, J, values + base, 0u, n, std2, outline2, suffix_min, eps, nullptr,
-                                                          tile);
+    raster_tile<MODE, PORTABLE_EXP, false, FEW ? 4u : 1u>(S, J, values + base, 0u, n, std2, outline2, suffix_min, eps, colours,
+                                                          nullptr, tile);
 }
 
 // One grid over the tiles of several views (a batch): CTA b rasterises tile b - tile_base[v] of
@@ -1630,8 +1665,8 @@ __global__ void __launch_bounds__(kTileThreads<MODE, false>, kTileCtas<MODE, fal
     if (b == 0 && threadIdx.x == 0) merge_status(J);
     const uint2 r = tile_range(J, tile);
     raster_tile<MODE, PORTABLE_EXP, false, 1u>(S, J, J.values + ((size_t)r.x << J.value_shift), J.value_shift,
-                                                          r.y - r.x, std2, outline2, suffix_min, eps, nullptr,
-                                               tile);
+                                                          r.y - r.x, std2, outline2, suffix_min, eps, J.ctrl->colours,
+                                               nullptr, tile);
 }
 
 // Work tallies of the counting raster variant (profiling only).
@@ -1768,7 +1803,7 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
                             g.max_count, rank_offset, indexed(g, nseg) ? nullptr : L.sorted, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
                             u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
-                            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0);
+                            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0, nullptr);
         count_launches(1);
         rank_offset += g.max_count;
     }
@@ -1883,17 +1918,18 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
 // (8.8e7): 128 -> 125; 68.4k x 1400 (9.6e7): 157 -> 167; 28.6k x 5292 (1.5e8): 135 -> 161.  Views of a
 // batch overlap, so the tiles of all of them count (10 views of 11.6k, 4e8 so counted: 234 -> 440).
 constexpr uint64_t kDirectWork = 60'000'000;
-static bool direct_raster(uint32_t ranks, uint32_t tiles_at_once) {
-    return ranks > 0 && ranks <= kDirectMaxRanks && (uint64_t)ranks * tiles_at_once <= kDirectWork;
+static bool direct_raster(uint32_t ranks, uint32_t blocks, uint32_t tiles_at_once) {
+    return ranks > 0 && ranks <= kDirectMaxRanks && blocks <= kDirectMaxBlocks &&
+           (uint64_t)ranks * tiles_at_once <= kDirectWork;
 }
 
 template <uint32_t MODE>
-static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift,
+static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift, uint32_t nblocks,
                                uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
     const bool few = tiles_at_once <= kFewTiles;
     auto go = [&](auto kernel) {
         launch_frame_kernel(kernel, J.ntiles, kRasterThreads, 0, st, frame_launch_overlaps(st), J, L.offsets, L.info, ranks,
-                            shift, L.items(), max_pairs, std2, outline2, t.suffix_min, t.eps);
+                            shift, L.items(), max_pairs, std2, outline2, t.suffix_min, t.eps, L.blocks(), nblocks);
     };
     if (exact) few ? go(raster_direct_kernel<MODE, true, true>) : go(raster_direct_kernel<MODE, true, false>);
     else few ? go(raster_direct_kernel<MODE, false, true>) : go(raster_direct_kernel<MODE, false, false>);
@@ -1905,7 +1941,7 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
                                         int exact_exp, cudaStream_t st, const Tuning &tn) {
     const RasterLayout L = raster_layout(scratch, ranks, J.W, J.H, max_pairs);
     const float std2 = u.std_dev * u.std_dev, o = u.std_dev - 0.1f, outline2 = o * o;
-    uint32_t rank_offset = 0, shift = 0;
+    uint32_t rank_offset = 0, shift = 0, nblocks = 0;
     while (((L.tiles_x - 1u) >> shift) > 127u || ((L.tiles_y - 1u) >> shift) > 127u) ++shift;
     bool started = false;
     prof_mark(kProfBin, true, st);
@@ -1917,22 +1953,23 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
         launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
                             g.sorted_index, g.count, g.max_count, rank_offset, indexed(g, nseg) ? nullptr : L.sorted,
                             nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
-                            shift, started ? nullptr : L.ctrl, L.arena_words);
+                            shift, started ? nullptr : L.ctrl, L.arena_words, L.blocks() + nblocks);
         count_launches(1);
         started = true;
         rank_offset += g.max_count;
+        nblocks += blocks;
     }
     prof_mark(kProfBin, false, st);
     prof_mark(kProfRaster, true, st);
     switch (u.display_mode) {
         case GS_DISPLAY_SPLAT:
-            launch_direct_mode<GS_DISPLAY_SPLAT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_SPLAT>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
         case GS_DISPLAY_ELLIPSE:
-            launch_direct_mode<GS_DISPLAY_ELLIPSE>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_ELLIPSE>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
         default:
-            launch_direct_mode<GS_DISPLAY_POINT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_POINT>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
     }
     count_launches(1);
@@ -1947,10 +1984,13 @@ cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const Raster
     const RasterJob J = raster_job(segs, nseg, target, W, H, pitch, max_pairs, scratch);
     if (J.ntiles == 0) return cudaSuccess;
     const uint32_t at_once = tiles_at_once > J.ntiles ? tiles_at_once : J.ntiles;
-    uint32_t ranks = 0;
-    for (uint32_t s = 0; s < nseg; ++s) ranks += segs[s].max_count;
+    uint32_t ranks = 0, blocks = 0;
+    for (uint32_t s = 0; s < nseg; ++s) {
+        ranks += segs[s].max_count;
+        blocks += (segs[s].max_count + kBinThreads - 1) / kBinThreads;
+    }
     // (the counting rasteriser and the bounded-wait hook know the general path only)
-    if (direct_raster(ranks, at_once) && !prof_counting() && wait_config().stall_tile == kNoStall)
+    if (direct_raster(ranks, blocks, at_once) && !prof_counting() && wait_config().stall_tile == kNoStall)
         return launch_raster_direct(segs, nseg, ranks, u, J, max_pairs, scratch, at_once, exact_exp, st, tn);
     cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
     if (e != cudaSuccess) return e;
