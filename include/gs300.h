@@ -210,8 +210,9 @@ size_t gs_rasterize_scratch_bytes(uint32_t max_splats, uint32_t width, uint32_t 
  * splat in the order of sorted_indices[0..V) (V read from `count`), back to front, one
  * 8-bit re-quantisation per fragment as a Rgba8Unorm attachment does.  `splats` is the
  * array gs_preprocess wrote.  `target` is width x height RGBA8 with row pitch
- * `pitch_bytes`.  Returns GS_ERR_CAPACITY (asynchronously, via gs_status_word) when the
- * tile-pair list exceeds `max_pairs`. */
+ * `pitch_bytes`.  Returns GS_ERR_CAPACITY (asynchronously, via gs_scratch_status) when the
+ * tile-pair list exceeds `max_pairs`: the frame then holds the first `max_pairs` pairs in draw
+ * order, a splat's in row-major order of its tiles. */
 gs_status gs_rasterize(const gs_frame_uniforms *uniforms, const gs_splat *splats,
                        const uint32_t *sorted_indices, const uint32_t *count, uint32_t max_splats,
                        uint8_t *target, uint32_t width, uint32_t height, uint32_t pitch_bytes,

@@ -60,8 +60,10 @@ constexpr uint32_t kEmitBlocks = 152 * 8;
 
 // Ranks a direct frame can have: a bit each in shared memory (RasterShared::raw).
 constexpr uint32_t kDirectMaxRanks = 3u * 16u * kRasterThreads * 8u;
-// ... and CTAs of tile records, segments rounded up (RasterLayout::blocks).
+// ... and CTAs of tile records, segments rounded up (RasterLayout::blocks): a word each, the pairs of its
+// ranks (at most kDirectWork) below their colour class.
 constexpr uint32_t kDirectMaxBlocks = sizeof(Ctrl::hist) / sizeof(uint32_t);
+constexpr uint32_t kBlockPairBits = 28;
 
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = 256 * kScanItems;
@@ -200,15 +202,16 @@ __device__ __forceinline__ uint32_t colour_class(const float4 c) {
 // With `rects` (and no counts) the ranks are scanned by raster_direct_kernel up to the capacity: each
 // gets its rectangle in one word, an empty one where there is no splat or no tile is kept; the first
 // segment's launch (reset non-null) starts the call's control block.  The splats' colour_class goes to the
-// owner, or with `rects` each CTA's to its word of `blocks` (tile records stand for class 0).
+// owner, or with `rects` each CTA's to its word of `blocks`, above the CTA's pairs (tile records stand
+// for class 0).
 __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     const gs_splat *splats, const uint4 *binfo, const uint32_t *sorted_index,
     const uint32_t *count, uint32_t max_count, uint32_t base, gs_splat *sorted_out, int several,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
     uint32_t *counts, Ctrl *owner, uint64_t *arena, uint32_t *rects,
     uint32_t rect_shift, Ctrl *reset, uint32_t arena_words, uint32_t *blocks) {
-    __shared__ uint32_t s_class;
-    if (threadIdx.x == 0) s_class = 0u;
+    __shared__ uint32_t s_class, s_pairs;
+    if (threadIdx.x == 0) s_class = s_pairs = 0u;
     __syncthreads();
     frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
@@ -252,8 +255,10 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
                                    (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
                        : kEmptyRect;
     if (colours) atomicMax(&s_class, colours);
+    const uint32_t pairs = __reduce_add_sync(0xFFFFFFFFu, t.w);
+    if ((threadIdx.x & 31u) == 0) atomicAdd(&s_pairs, pairs);
     __syncthreads();
-    if (threadIdx.x == 0) blocks[blockIdx.x] = s_class;
+    if (threadIdx.x == 0) blocks[blockIdx.x] = (s_class << kBlockPairBits) | s_pairs;
 }
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
@@ -1561,6 +1566,47 @@ __global__ void __launch_bounds__(kTileThreads<MODE, FEW>, kTileCtas<MODE, FEW>)
                                                           counters, tile);
 }
 
+// A direct frame whose pairs do not all fit keeps the first max_pairs of them in draw order, a splat's in
+// row-major order of its tiles, as the emission does.  Takes the marks of the ranks past them from
+// `hits`; each thread has its own words [first, last).
+__device__ __noinline__ void direct_cut(uint32_t *hits, const uint32_t *rects, const uint4 *info, uint32_t ranks,
+                                        uint32_t first, uint32_t last, uint32_t tx, uint32_t ty, uint32_t max_pairs,
+                                        uint32_t *s_warp) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    auto pairs_of = [&](uint32_t k, const uint4 in) {
+        return rects[k] == kEmptyRect ? 0u : in.z ? (uint32_t)__popc(in.z) : (in.y & 0xFFFFu) * (in.y >> 16);
+    };
+    const uint32_t k0 = 32u * first, k1 = min(ranks, 32u * last);
+    uint32_t mine = 0;
+    for (uint32_t k = k0; k < k1; ++k) mine += pairs_of(k, info[k]);
+    uint32_t incl = mine;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = incl - mine;
+    for (uint32_t w = 0; w < warp; ++w) before += s_warp[w];
+    __syncthreads();
+    uint32_t room = max_pairs > before ? max_pairs - before : 0u;
+    for (uint32_t k = k0; k < k1; ++k) {
+        const uint4 in = info[k];
+        const uint32_t c = pairs_of(k, in);
+        if (c <= room) {
+            room -= c;
+            continue;
+        }
+        const uint32_t dx = tx - (in.x & 0xFFFFu), dy = ty - (in.x >> 16), w = in.y & 0xFFFFu;
+        if (dx < w && dy < (in.y >> 16)) {  // else not a tile of it at all
+            const uint32_t pos = dy * w + dx, place = in.z ? (uint32_t)__popc(in.z & ((1u << pos) - 1u)) : pos;
+            if (place >= room) hits[k / 32u] &= ~(1u << (k & 31u));
+        }
+        room = 0;
+    }
+}
+
 // A frame of few splats and tiles without the binning's scan, emission and tile sort: each tile's CTA
 // goes through the rectangles of all ranks (draw order), marks those that hold its tile in one bit
 // each, and writes its own list of pairs behind those of the CTAs before it.  The scan is bound by L2
@@ -1572,7 +1618,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
                          uint32_t ranks, uint32_t shift, uint32_t *values, uint32_t max_pairs, float std2,
                          float outline2, uint32_t suffix_min, float eps, const uint32_t *blocks, uint32_t nblocks) {
     __shared__ RasterShared1 S;
-    __shared__ uint32_t s_warp[kRasterThreads / 32], s_class[kRasterThreads / 32], s_base;
+    __shared__ uint32_t s_warp[kRasterThreads / 32], s_class[kRasterThreads / 32], s_pairs[kRasterThreads / 32], s_base;
     uint32_t *hits = reinterpret_cast<uint32_t *>(S.raw);  // bit r of word q: rank 32 q + r holds the tile
     static_assert(sizeof(S.raw) * 8 >= kDirectMaxRanks, "a bit per rank");
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
@@ -1580,7 +1626,7 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     const uint32_t here = pack_rect(tx, ty, tx, ty, shift);
     constexpr uint32_t STEP = kRasterThreads / 32u;
     frame_kernel_enter();
-    uint32_t colours = tid < nblocks ? blocks[tid] : 0u;  // waited for after the scan
+    const uint32_t block = tid < nblocks ? blocks[tid] : 0u;  // waited for after the scan
     for (uint32_t q0 = warp; q0 < words; q0 += 8u * STEP) {
         uint32_t r[8];
 #pragma unroll
@@ -1595,10 +1641,31 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
             if (lane == 0 && q < words) hits[q] = m;
         }
     }
+    // the frame's pairs and colour class, from the tile records' CTAs
+    constexpr uint32_t pair_mask = (1u << kBlockPairBits) - 1u;
+    uint32_t colours = block >> kBlockPairBits, wanted = block & pair_mask;
+    for (uint32_t b = tid + kRasterThreads; b < nblocks; b += kRasterThreads) {
+        colours = max(colours, blocks[b] >> kBlockPairBits);
+        wanted += blocks[b] & pair_mask;
+    }
+    colours = __reduce_max_sync(0xFFFFFFFFu, colours);
+    wanted = __reduce_add_sync(0xFFFFFFFFu, wanted);
+    if (lane == 0) s_class[warp] = colours, s_pairs[warp] = wanted;
     __syncthreads();
+    colours = wanted = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kRasterThreads / 32u; ++w) {
+        colours = max(colours, s_class[w]);
+        wanted += s_pairs[w];
+    }
+    if (tile == 0 && tid == 0) {
+        J.ctrl->total = wanted;
+        if (wanted > max_pairs) atomicOr(&J.ctrl->status, kStatusCapacity);
+    }
     // thread t owns the words [t per, (t + 1) per): their places in the list by a block scan
     const uint32_t per = (words + kRasterThreads - 1u) / kRasterThreads;
     const uint32_t first = min(words, tid * per), last = min(words, first + per);
+    if (wanted > max_pairs) direct_cut(hits, rects, info, ranks, first, last, tx, ty, max_pairs, s_warp);
     uint32_t sum = 0;
     for (uint32_t q = first; q < last; ++q) {
         const uint32_t found = hits[q];
@@ -1619,22 +1686,18 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
         if (lane >= o) incl += y;
     }
     if (lane == 31) s_warp[warp] = incl;
-    for (uint32_t b = tid + kRasterThreads; b < nblocks; b += kRasterThreads) colours = max(colours, blocks[b]);
-    colours = __reduce_max_sync(0xFFFFFFFFu, colours);
-    if (lane == 0) s_class[warp] = colours;
     __syncthreads();
     uint32_t before = 0, n = 0;
 #pragma unroll
     for (uint32_t w = 0; w < kRasterThreads / 32u; ++w) {
         if (w < warp) before += s_warp[w];
         n += s_warp[w];
-        colours = max(colours, s_class[w]);
     }
-    if (tid == 0) s_base = n ? atomicAdd(&J.ctrl->total, n) : 0u;
+    if (tid == 0) s_base = n ? atomicAdd(&J.ctrl->count, n) : 0u;
     __syncthreads();
     uint32_t base = s_base;
-    if (base > max_pairs || n > max_pairs - base) {  // the list is full: reported, the tile stays empty
-        if (tid == 0) atomicOr(&J.ctrl->status, kStatusCapacity);
+    if (base > max_pairs || n > max_pairs - base) {  // the lists hold as many pairs as were counted, or fit
+        if (tid == 0) atomicOr(&J.ctrl->status, kStatusBounds);
         base = n = 0;
     } else {
         uint32_t at = base + before + incl - sum;
@@ -1918,6 +1981,7 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
 // (8.8e7): 128 -> 125; 68.4k x 1400 (9.6e7): 157 -> 167; 28.6k x 5292 (1.5e8): 135 -> 161.  Views of a
 // batch overlap, so the tiles of all of them count (10 views of 11.6k, 4e8 so counted: 234 -> 440).
 constexpr uint64_t kDirectWork = 60'000'000;
+static_assert(kDirectWork < (1u << kBlockPairBits) && kWildColours < (1u << (32u - kBlockPairBits)), "a word a CTA");
 static bool direct_raster(uint32_t ranks, uint32_t blocks, uint32_t tiles_at_once) {
     return ranks > 0 && ranks <= kDirectMaxRanks && blocks <= kDirectMaxBlocks &&
            (uint64_t)ranks * tiles_at_once <= kDirectWork;
