@@ -1772,8 +1772,14 @@ gs_status server_finish(gs_server *sv, ServerReq &r, ServerSlot &sl, uint8_t *ta
             seg.binfo_w = r.w;
             seg.binfo_h = r.h;
         }
+        uint64_t direct_in_flight = 0;  // this request's slot is busy already
+        for (const ServerSlot &o : sv->slots) {
+            if (!o.busy) continue;
+            const ServerReq &q = sv->reqs[o.req];
+            direct_in_flight += direct_raster_work(q.model->n, q.w, q.h);
+        }
         e = launch_raster(&seg, 1, raster_mode(u), target, r.w, r.h, pitch, v.max_pairs, v.raster_scratch.ptr,
-                          sv->mv->frame.exact_exp, sl.stream);
+                          sv->mv->frame.exact_exp, sl.stream, nullptr, 0, direct_in_flight);
     }
     if (e == cudaSuccess && r.out_on_host && r.out)
         e = cudaMemcpyAsync(r.out, target, (size_t)r.w * r.h * 4, cudaMemcpyDeviceToHost, sl.stream);

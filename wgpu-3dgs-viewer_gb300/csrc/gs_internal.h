@@ -211,10 +211,15 @@ gs_splat *raster_splat_pool(void *scratch, uint32_t max_splats, uint32_t width, 
 size_t raster_scratch_bytes(uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 // exact_exp: 1 = the portable exp (bit-identical with the CPU oracle), 0 = the SFU exp.
 // tiles_at_once: tiles of all views that are rendered side by side with this one (0: it is alone).
+// direct_in_flight: direct_raster_work() of all frames that overlap on the device with this one, its own
+// included (0: it is alone).
 cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const RasterMode &u,
                           uint8_t *target, uint32_t width, uint32_t height, uint32_t pitch,
                           uint32_t max_pairs, void *scratch, int exact_exp, cudaStream_t st,
-                          const Tuning *tuning = nullptr, uint32_t tiles_at_once = 0);
+                          const Tuning *tuning = nullptr, uint32_t tiles_at_once = 0, uint64_t direct_in_flight = 0);
+// Ranks x tiles of a one-segment frame that can be rendered without a pair list and its sort; 0 where
+// it cannot.
+uint64_t direct_raster_work(uint32_t max_splats, uint32_t width, uint32_t height);
 // Scratch control block of a raster call (status, pair counts).
 const Ctrl *raster_ctrl(const void *scratch);
 

@@ -1987,6 +1987,17 @@ static bool direct_raster(uint32_t ranks, uint32_t blocks, uint32_t tiles_at_onc
            (uint64_t)ranks * tiles_at_once <= kDirectWork;
 }
 
+// Frames of separate requests that overlap share the L2 that their scans are bound by: their work
+// together is limited too.  Eight served at once, frames/s direct and binned: 12k x 920 tiles (8.8e7
+// together) 31,200 and 27,000; 30k x 920 (2.2e8) 24,300 and 24,100; 8k x 3600 (2.3e8) 26,100 and 24,300;
+// 16.6k x 3600 (4.8e8) 16,400 and 23,200; 65k x 920 (4.8e8) 13,700 and 20,100.
+constexpr uint64_t kDirectWorkInFlight = 240'000'000;
+
+uint64_t direct_raster_work(uint32_t max_splats, uint32_t W, uint32_t H) {
+    const uint32_t tiles = ((W + GS_TILE - 1) / GS_TILE) * ((H + GS_TILE - 1) / GS_TILE);
+    return direct_raster(max_splats, (max_splats + kBinThreads - 1) / kBinThreads, tiles) ? (uint64_t)max_splats * tiles : 0;
+}
+
 template <uint32_t MODE>
 static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift, uint32_t nblocks,
                                uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
@@ -2043,7 +2054,7 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
 
 cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const RasterMode &u, uint8_t *target,
                           uint32_t W, uint32_t H, uint32_t pitch, uint32_t max_pairs, void *scratch, int exact_exp,
-                          cudaStream_t st, const Tuning *tuning, uint32_t tiles_at_once) {
+                          cudaStream_t st, const Tuning *tuning, uint32_t tiles_at_once, uint64_t direct_in_flight) {
     const Tuning tn = tuning ? *tuning : default_tuning();
     const RasterJob J = raster_job(segs, nseg, target, W, H, pitch, max_pairs, scratch);
     if (J.ntiles == 0) return cudaSuccess;
@@ -2054,7 +2065,7 @@ cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const Raster
         blocks += (segs[s].max_count + kBinThreads - 1) / kBinThreads;
     }
     // (the counting rasteriser and the bounded-wait hook know the general path only)
-    if (direct_raster(ranks, blocks, at_once) && !prof_counting() && wait_config().stall_tile == kNoStall)
+    if (direct_raster(ranks, blocks, at_once) && direct_in_flight <= kDirectWorkInFlight && !prof_counting() && wait_config().stall_tile == kNoStall)
         return launch_raster_direct(segs, nseg, ranks, u, J, max_pairs, scratch, at_once, exact_exp, st, tn);
     cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
     if (e != cudaSuccess) return e;
