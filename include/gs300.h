@@ -367,7 +367,8 @@ gs_status gs_batch_render(gs_batch *batch, const gs_batch_view *views, uint32_t 
 /* Wait, check every view's device status, regrow overflowed tile-pair lists and re-render. */
 gs_status gs_batch_synchronize(gs_batch *batch, gs_stream stream);
 
-/* Launch choices of a batch that change its speed, never its frames. */
+/* Launch choices of a batch that change its speed, never its frames.  The depth sort's three are for views of
+ * more than 65,536 Gaussians; smaller ones are sorted in one launch that has no such choice. */
 typedef struct gs_tuning {
     uint32_t suffix_min;       /* raster: tile lists of at least 9/16 of this many splats (3/4 of it in
                                   targets of few tiles, 1/4 in ellipse frames) take the exact

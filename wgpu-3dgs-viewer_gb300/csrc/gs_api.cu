@@ -1602,11 +1602,14 @@ gs_status gs_batch_autotune(gs_batch *b, const gs_batch_view *views, uint32_t n,
     const uint32_t vpl_c[] = {1, 4, 8, 16};
     const uint32_t streams_c[] = {4, 8, 16};
     const uint32_t match_c[] = {0, 1};
-    const uint32_t hist_c[] = {0, 304, 608};
+    const uint32_t hist_c[] = {0, 76, 152};  // a quarter and half of the CTAs that are resident at once
     const uint32_t digit_c[] = {6, 7, 8};
     const uint32_t grid_c[] = {0, 1};
+    bool pass_sorts = false;  // a view's depth sort has passes for the sort knobs to choose
+    for (uint32_t i = 0; i < n && s == GS_OK; ++i) pass_sorts = pass_sorts || !sort_in_cluster(b->slots[i].model->n);
     for (uint32_t round = 0; round < rounds && s == GS_OK; ++round) {
         for (int knob = 0; knob < 8 && s == GS_OK; ++knob) {
+            if (knob >= 4 && knob <= 6 && !pass_sorts) continue;
             const size_t nc = knob == 0   ? 4
                               : knob == 1 ? 2
                               : knob == 2 ? 4

@@ -124,6 +124,10 @@ cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t max_count, cons
                         uint32_t key_bits, void *scratch, cudaStream_t st, int prof_stage = kProfDepthSort,
                         const Tuning *tuning = nullptr, uint64_t keys_at_once = 0);
 
+// Whether launch_sort takes one launch of one cluster for it: the sort knobs of the tuning (match, histogram
+// blocks, digit bits) then choose nothing.
+bool sort_in_cluster(uint32_t max_count);
+
 // Several independent sorts by kDepthKeyBits, each with its own buffers and scratch, in the launches of
 // one where they are large.
 struct DepthSort {

@@ -1041,13 +1041,22 @@ static uint32_t cluster_ctas_supported() {
     return best;
 }
 
+// Whether a sort goes to one cluster, where the tuning's sort knobs have nothing to choose.
+template <uint32_t ROWS>
+static bool cluster_holds(uint32_t max_count) {
+    return max_count > 0 && (max_count - 1) / (kClusterThreads * ROWS) < cluster_ctas_supported<ROWS>();
+}
+bool sort_in_cluster(uint32_t max_count) {
+    return cluster_holds<1>(max_count) || cluster_holds<2>(max_count) || cluster_holds<4>(max_count);
+}
+
 // Launches the sort on one cluster where `max_count` fits ROWS rows; false: not this size.
 template <uint32_t ROWS>
 static bool launch_cluster_rows(uint32_t *keys, uint32_t *vals, uint32_t max_count, const uint32_t *count,
                                 const PassSplit &sp, Ctrl *ctrl, cudaStream_t st, cudaError_t *err) {
     constexpr uint32_t K = kClusterThreads * ROWS;
+    if (!cluster_holds<ROWS>(max_count)) return false;
     const uint32_t ctas = (max_count + K - 1) / K;
-    if (ctas == 0 || ctas > cluster_ctas_supported<ROWS>()) return false;
     cudaLaunchAttribute attr[2] = {};
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
@@ -1165,7 +1174,8 @@ static cudaError_t launch_sort_group(const SortGroup &G, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Sorts of more pairs than a cluster holds go together, up to kSortGroup at a time.
+// Sorts of more pairs than a cluster holds go together, up to kSortGroup at a time (with sort_match, which
+// the grouped passes have no variant for, one by one).
 cudaError_t launch_depth_sorts(const DepthSort *sorts, uint32_t n, cudaStream_t st) {
     SortGroup G{};
     const Tuning tn = default_tuning();
@@ -1185,7 +1195,7 @@ cudaError_t launch_depth_sorts(const DepthSort *sorts, uint32_t n, cudaStream_t 
     for (uint32_t i = 0; i < n; ++i) {
         const DepthSort &s = sorts[i];
         cudaError_t e = cudaSuccess;
-        if (s.max_count <= kClusterMaxPairs) {
+        if (s.max_count <= kClusterMaxPairs || tn.sort_match) {
             e = launch_sort(s.keys, s.vals, s.max_count, s.count, kDepthKeyBits, s.scratch, st);
         } else {
             const SortLayout L = sort_layout(s.scratch, s.max_count, G.sp);
