@@ -210,11 +210,17 @@ struct Model {
         GS_CUDA(cudaMemset(control.ptr, 0, 64));
         GS_CUDA(indices.ensure((size_t)n * 4));
         GS_CUDA(depths.ensure((size_t)gs_depth_capacity(n) * 4));
-        GS_CUDA(splats.ensure((size_t)n * sizeof(gs_splat)));
         GS_CUDA(pre_scratch.ensure(preprocess_scratch_bytes(n)));
         GS_CUDA(cudaMemset(pre_scratch.ptr, 0, pre_scratch.bytes));
         GS_CUDA(sort_scratch.ensure(sort_scratch_bytes(n, kDepthKeyBits)));
         GS_CUDA(cudaMemset(sort_scratch.ptr, 0, sort_scratch.bytes));
+        return GS_OK;
+    }
+
+    // The model's own splats.  Frames of several models keep theirs in the raster scratch, so a model has none
+    // until it is drawn alone.
+    gs_status ensure_splats() {
+        GS_CUDA(splats.ensure((size_t)n * sizeof(gs_splat)));
         return GS_OK;
     }
 
@@ -694,7 +700,8 @@ extern "C" {
 gs_status gs_viewer_create(const void *host_records, uint32_t count, uint32_t format, gs_viewer **out) {
     if (!out) return fail(GS_ERR_INVALID_ARG, "out is NULL");
     gs_viewer *v = new gs_viewer();
-    const gs_status s = v->model.create(host_records, count, format);
+    gs_status s = v->model.create(host_records, count, format);
+    if (s == GS_OK) s = v->model.ensure_splats();
     if (s != GS_OK) {
         delete v;
         return s;
@@ -707,7 +714,8 @@ gs_status gs_viewer_create(const void *host_records, uint32_t count, uint32_t fo
 gs_status gs_viewer_create_from_ply(const void *ply_bytes, size_t len, uint32_t format, gs_viewer **out) {
     if (!out || !ply_bytes) return fail(GS_ERR_INVALID_ARG, "NULL argument");
     gs_viewer *v = new gs_viewer();
-    const gs_status s = v->model.create_from_ply(ply_bytes, len, format);
+    gs_status s = v->model.create_from_ply(ply_bytes, len, format);
+    if (s == GS_OK) s = v->model.ensure_splats();
     if (s != GS_OK) {
         delete v;
         return s;
@@ -894,6 +902,7 @@ gs_status multi_render_locked(gs_multi_viewer *v, const std::vector<std::string>
     gs_frame_uniforms u{};
     // Several models' splats go side by side into the raster scratch, one model's into its own buffer.
     const bool pooled = ms.size() > 1;
+    if (ms.size() == 1 && (s = ms[0]->ensure_splats()) != GS_OK) return s;
     gs_splat *pool = pooled ? raster_splat_pool(v->frame.raster_scratch.ptr, (uint32_t)total, w, h, v->frame.max_pairs) : nullptr;
     // The models' sorts go together after all preprocesses, unless a model is drawn twice: its second
     // preprocess would write the buffers of the first one's sort.
