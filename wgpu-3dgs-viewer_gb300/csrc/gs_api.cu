@@ -919,7 +919,6 @@ gs_status multi_render_locked(gs_multi_viewer *v, const std::vector<std::string>
         seg.binfo = reinterpret_cast<const uint4 *>(m->binfo.ptr);
         seg.binfo_w = w;
         seg.binfo_h = h;
-        seg.pooled = pooled;
         segs.push_back(seg);
         pool += pooled ? m->n : 0;
     }

@@ -205,12 +205,9 @@ struct RasterSegment {
     // binfo_h target (indexed by Gaussian index); used when the binning's target matches.
     const uint4 *binfo = nullptr;
     uint32_t binfo_w = 0, binfo_h = 0;
-    // One of several segments, its splats being the raster scratch's own (raster_splat_pool) from the
-    // segment's first rank on: pair values point there, and nothing is copied into draw order.
-    bool pooled = false;
 };
-// Where in the raster scratch the segments of a call can keep their splats (max_splats of them, all
-// segments' capacities one after another).
+// Where in the raster scratch the splats of a call of several segments lie (max_splats of them, all segments'
+// capacities one after another).
 gs_splat *raster_splat_pool(void *scratch, uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 size_t raster_scratch_bytes(uint32_t max_splats, uint32_t width, uint32_t height, uint32_t max_pairs);
 // exact_exp: 1 = the portable exp (bit-identical with the CPU oracle), 0 = the SFU exp.

@@ -34,7 +34,7 @@ struct RasterLayout {
     uint64_t *flags;     // flag arena, first part: scan look-back flags
     uint64_t *sort_flags;  // flag arena, second part: tile-sort look-back flags
     uint32_t arena_words;  // words of the flag arena (both parts)
-    gs_splat *sorted;    // several models: their splats side by side, or copied into draw order, capacity max_splats
+    gs_splat *splats;    // several models: their splats side by side, capacity max_splats
     uint4 *info;         // per draw rank: tile rectangle, kept-tile mask, pair value
     uint32_t *offsets;   // per draw rank: tile count, then its exclusive scan
     uint2 *pairs;        // (tile, value), capacity max_pairs
@@ -112,7 +112,7 @@ static RasterLayout raster_layout(void *scratch, uint32_t max_splats, uint32_t w
     L.sort_flags = L.flags + scan_words;
     L.arena_words = (uint32_t)arena;
     p += align_up(arena * sizeof(uint64_t), 256);
-    L.sorted = reinterpret_cast<gs_splat *>(p);
+    L.splats = reinterpret_cast<gs_splat *>(p);
     p += align_up((size_t)max_splats * sizeof(gs_splat), 256);
     L.info = reinterpret_cast<uint4 *>(p);
     p += align_up((size_t)max_splats * 16, 256);
@@ -194,9 +194,8 @@ __device__ __forceinline__ uint32_t colour_class(const float4 c) {
 // K3a: per draw rank, the splat's tile rectangle, the corner tiles its footprint misses, and
 // its tile count.  With `binfo` (the preprocess having stored each visible splat's tiles) the rank
 // gathers that 16-byte record; otherwise it gathers the 48-byte splat and works the tiles out here.
-// The pair value is the splat's index from `base` on, or with `sorted_out` (several models whose splats
-// lie apart) its rank from `base` on, the splat being copied there.  Four models of 6M splats: 174 us
-// copying, 70 us with their splats side by side.
+// The pair value is the splat's index from `base` on (several models: in their common array.  Four models of
+// 6M splats: 174 us a binning with the splats copied into draw order, 70 us with them side by side).
 // The first segment's launch (arena non-null) also clears the flag-arena words the call must
 // clear, before the scan and the tile sort read any flag.
 // With `rects` (and no counts) the ranks are scanned by raster_direct_kernel up to the capacity: each
@@ -206,7 +205,7 @@ __device__ __forceinline__ uint32_t colour_class(const float4 c) {
 // for class 0).
 __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
     const gs_splat *splats, const uint4 *binfo, const uint32_t *sorted_index,
-    const uint32_t *count, uint32_t max_count, uint32_t base, gs_splat *sorted_out, int several,
+    const uint32_t *count, uint32_t max_count, uint32_t base, int several,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
     uint32_t *counts, Ctrl *owner, uint64_t *arena, uint32_t *rects,
     uint32_t rect_shift, Ctrl *reset, uint32_t arena_words, uint32_t *blocks) {
@@ -232,17 +231,11 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
                 const float4 a = src[0];
                 const float4 q = src[1];
                 const float4 c = src[2];
-                if (sorted_out) {
-                    float4 *dst = reinterpret_cast<float4 *>(sorted_out + base + k);
-                    dst[0] = a;
-                    dst[1] = q;
-                    dst[2] = c;
-                }
                 t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
                 if (t.w) colours = colour_class(c);
             }
         }
-        info[k] = make_uint4(t.x, t.y, t.z, base + (sorted_out ? k : gi));
+        info[k] = make_uint4(t.x, t.y, t.z, base + gi);
     }
     if (!rects) {
         if (k < n) counts[k] = t.w;
@@ -1783,11 +1776,8 @@ static void launch_raster_views_mode(const RasterJob *jobs, const uint32_t *tile
 }
 
 gs_splat *raster_splat_pool(void *scratch, uint32_t max_splats, uint32_t W, uint32_t H, uint32_t max_pairs) {
-    return raster_layout(scratch, max_splats, W, H, max_pairs).sorted;
+    return raster_layout(scratch, max_splats, W, H, max_pairs).splats;
 }
-
-// Whether a segment's pair values are splat indices (else its splats are copied into draw order).
-static bool indexed(const RasterSegment &g, uint32_t nseg) { return nseg == 1 || g.pooled; }
 
 RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, uint32_t W, uint32_t H,
                      uint32_t pitch, uint32_t max_pairs, void *scratch, bool segmented) {
@@ -1795,8 +1785,8 @@ RasterJob raster_job(const RasterSegment *segs, uint32_t nseg, uint8_t *target, 
     for (uint32_t s = 0; s < nseg; ++s) max_splats += segs[s].max_count;
     const RasterLayout L = raster_layout(scratch, max_splats, W, H, max_pairs);
     RasterJob J;
-    // Pair values index the model's own splat array (one segment), the pool or the draw-ordered copy.
-    J.splats = nseg == 1 ? segs[0].splats : L.sorted;
+    // Pair values index the model's own splat array (one segment) or the common one.
+    J.splats = nseg == 1 ? segs[0].splats : L.splats;
     J.max_splats = nseg == 1 ? segs[0].max_count : max_splats;
     const bool compact = L.value_bits && !segmented;  // else the value is a pair's second word
     J.values = L.items() + (compact ? 0 : 1);
@@ -1862,9 +1852,9 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
         if (blocks == 0) continue;
         // a stored tile record is only for the target the preprocess was given
-        const uint4 *binfo = indexed(g, nseg) && g.binfo && g.binfo_w == W && g.binfo_h == H ? g.binfo : nullptr;
+        const uint4 *binfo = g.binfo && g.binfo_w == W && g.binfo_h == H ? g.binfo : nullptr;
         launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
-                            g.max_count, rank_offset, indexed(g, nseg) ? nullptr : L.sorted, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
+                            g.max_count, rank_offset, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
                             u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
                             rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0, nullptr);
         count_launches(1);
@@ -2024,10 +2014,10 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
         const RasterSegment &g = segs[s];
         const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
         if (blocks == 0) continue;
-        const uint4 *binfo = indexed(g, nseg) && g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
+        const uint4 *binfo = g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
         launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
-                            g.sorted_index, g.count, g.max_count, rank_offset, indexed(g, nseg) ? nullptr : L.sorted,
-                            nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
+                            g.sorted_index, g.count, g.max_count, rank_offset, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y,
+                            u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
                             shift, started ? nullptr : L.ctrl, L.arena_words, L.blocks() + nblocks);
         count_launches(1);
         started = true;
