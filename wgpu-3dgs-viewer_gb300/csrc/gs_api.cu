@@ -629,7 +629,8 @@ gs_status gs_rasterize(const gs_frame_uniforms *u, const gs_splat *splats, const
     if (splats && !aligned(splats, 16)) return fail(GS_ERR_INVALID_ARG, "splats must be 16-byte aligned");
     if (!scratch || scratch_bytes < raster_scratch_bytes(max_splats, w, h, max_pairs))
         return fail(GS_ERR_INVALID_ARG, "scratch smaller than gs_rasterize_scratch_bytes");
-    const RasterSegment seg{splats, sorted, count, max_splats};
+    RasterSegment seg{splats, sorted, count, max_splats};
+    seg.foreign = true;
     const int exact = getenv("GS300_EXACT_EXP") ? 1 : 0;
     const cudaError_t e = launch_raster(&seg, 1, raster_mode(*u), target, w, h, pitch, max_pairs, scratch, exact, (cudaStream_t)stream);
     return e == cudaSuccess ? GS_OK : cuda_fail(e, "gs_rasterize");

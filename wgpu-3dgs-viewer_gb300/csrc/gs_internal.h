@@ -205,6 +205,7 @@ struct RasterSegment {
     // binfo_h target (indexed by Gaussian index); used when the binning's target matches.
     const uint4 *binfo = nullptr;
     uint32_t binfo_w = 0, binfo_h = 0;
+    bool foreign = false;  // the splats may be a caller's own: colours and alphas of any value
 };
 // Where in the raster scratch the splats of a call of several segments lie (max_splats of them, all segments'
 // capacities one after another).

@@ -180,15 +180,19 @@ __device__ __forceinline__ bool rect_may_hold(uint32_t rect, uint32_t tile) {
 // A caller's own splats may hold others: class k, 1..kColourClasses, for colours within +-255 2^k, whose
 // blends stay within them too as long as the alpha is in 0..1; kWildColours for the rest and NaN.
 constexpr uint32_t kColourClasses = 12, kWildColours = 15;
-__device__ __forceinline__ uint32_t colour_class(const float4 c) {
-    const bool alpha = c.w >= 0.0f && c.w <= 1.0f;
-    // the sum is for NaN, which the comparisons of the reach pass over
-    if (alpha && splat_colour_reach(c.x, c.y, c.z) <= 255.0f && (c.x + c.y) + c.z <= 765.0f) return 0u;
-    const float reach = fmaxf(fabsf(c.x), fmaxf(fabsf(c.y), fabsf(c.z))), sum = (c.x + c.y) + c.z;
-    if (!alpha || sum != sum || !(reach <= 255.0f * (float)(1u << kColourClasses))) return kWildColours;
+__device__ __noinline__ uint32_t colour_class_beyond(float r, float g, float b, float alpha) {
+    const float reach = fmaxf(fabsf(r), fmaxf(fabsf(g), fabsf(b))), sum = (r + g) + b;  // the sum is for NaN
+    if (!(alpha >= 0.0f && alpha <= 1.0f) || sum != sum || !(reach <= 255.0f * (float)(1u << kColourClasses)))
+        return kWildColours;
     uint32_t k = 1;
     while (255.0f * (float)(1u << k) < reach) ++k;
     return k;
+}
+__device__ __forceinline__ uint32_t colour_class(const float4 c) {
+    // as words, floats from 0 on are in order, and below those with a sign and NaN
+    const uint32_t most = max(__float_as_uint(c.x), max(__float_as_uint(c.y), __float_as_uint(c.z)));
+    const bool in = most <= __float_as_uint(255.0f) && __float_as_uint(c.w) <= __float_as_uint(1.0f);
+    return in ? 0u : colour_class_beyond(c.x, c.y, c.z, c.w);
 }
 
 // K3a: per draw rank, the splat's tile rectangle, the corner tiles its footprint misses, and
@@ -198,20 +202,25 @@ __device__ __forceinline__ uint32_t colour_class(const float4 c) {
 // 6M splats: 174 us a binning with the splats copied into draw order, 70 us with them side by side).
 // The first segment's launch (arena non-null) also clears the flag-arena words the call must
 // clear, before the scan and the tile sort read any flag.
-// With `rects` (and no counts) the ranks are scanned by raster_direct_kernel up to the capacity: each
-// gets its rectangle in one word, an empty one where there is no splat or no tile is kept; the first
-// segment's launch (reset non-null) starts the call's control block.  The splats' colour_class goes to the
-// owner, or with `rects` each CTA's to its word of `blocks`, above the CTA's pairs (tile records stand
-// for class 0).
-__global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
+// DIRECT: the ranks are scanned by raster_direct_kernel up to the capacity: each gets its rectangle in one
+// word (`rects`, in place of the count), an empty one where there is no splat or no tile is kept; the first
+// segment's launch (reset non-null) starts the call's control block.
+// The colour_class of `foreign` splats goes to the owner, or (DIRECT) each CTA's to its word of `blocks`,
+// above the CTA's pairs.
+// Bound by the latency of the gather: six CTAs an SM (40 registers) take 249 us a binning of four models of
+// 6M splats, five (45 registers) 255.
+template <bool DIRECT>
+__global__ void __launch_bounds__(kBinThreads, 6) bin_count_kernel(
     const gs_splat *splats, const uint4 *binfo, const uint32_t *sorted_index,
-    const uint32_t *count, uint32_t max_count, uint32_t base, int several,
+    const uint32_t *count, uint32_t max_count, uint32_t base, int several, int foreign,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
     uint32_t *counts, Ctrl *owner, uint64_t *arena, uint32_t *rects,
     uint32_t rect_shift, Ctrl *reset, uint32_t arena_words, uint32_t *blocks) {
     __shared__ uint32_t s_class, s_pairs;
-    if (threadIdx.x == 0) s_class = s_pairs = 0u;
-    __syncthreads();
+    if constexpr (DIRECT) {
+        if (threadIdx.x == 0) s_class = s_pairs = 0u;
+        __syncthreads();
+    }
     frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
     if (reset && blockIdx.x == 0 && threadIdx.x == 0) ctrl_reset_flagless(reset, arena_words);
@@ -232,26 +241,26 @@ __global__ void __launch_bounds__(kBinThreads) bin_count_kernel(
                 const float4 q = src[1];
                 const float4 c = src[2];
                 t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
-                if (t.w) colours = colour_class(c);
+                if (foreign && t.w) colours = colour_class(c);
             }
         }
         info[k] = make_uint4(t.x, t.y, t.z, base + gi);
     }
-    if (!rects) {
+    if constexpr (DIRECT) {
+        if (k < max_count)
+            rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
+                                       (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
+                           : kEmptyRect;
+        if (colours) atomicMax(&s_class, colours);
+        const uint32_t pairs = __reduce_add_sync(0xFFFFFFFFu, t.w);
+        if ((threadIdx.x & 31u) == 0) atomicAdd(&s_pairs, pairs);
+        __syncthreads();
+        if (threadIdx.x == 0) blocks[blockIdx.x] = (s_class << kBlockPairBits) | s_pairs;
+    } else {
         if (k < n) counts[k] = t.w;
         else if (k < max_count && several) counts[k] = 0u;  // the scan covers every segment's capacity
         if (colours) atomicMax(&owner->colours, colours);
-        return;
     }
-    if (k < max_count)
-        rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
-                                   (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
-                       : kEmptyRect;
-    if (colours) atomicMax(&s_class, colours);
-    const uint32_t pairs = __reduce_add_sync(0xFFFFFFFFu, t.w);
-    if ((threadIdx.x & 31u) == 0) atomicAdd(&s_pairs, pairs);
-    __syncthreads();
-    if (threadIdx.x == 0) blocks[blockIdx.x] = (s_class << kBlockPairBits) | s_pairs;
 }
 
 // K3b: exclusive scan of the tile counts in place (decoupled look-back over 4096-count tiles);
@@ -863,6 +872,7 @@ struct RasterShared {
     float4 box[T];      // fragment box in pixel-centre coordinates
     float2 inv[T];      // 1 / |Q·(7, 0)|², 1 / |Q·(0, 4 PX - 1)|² (the block edges in quad space)
     uint32_t kmin;
+    uint32_t colours;   // the frame's colour class
 };
 
 struct RasterShared1 : RasterShared<1> {
@@ -1290,6 +1300,7 @@ __device__ __forceinline__ void raster_tile(
     Value d[3] = {}, h[3] = {};
     const bool wild = colours > kColourClasses;
     const uint32_t early = wild ? 0xFFFFFFFFu : early_out_min<MODE, PX>(suffix_min);
+    if (tid == 0) S.colours = colours;  // read after the first barrier
     // blends the list onto the pixels whose `on` is set
     auto blend = [&](auto both, uint32_t nl, const bool *on) {
         if constexpr (PX == 1) {
@@ -1452,7 +1463,8 @@ __device__ __forceinline__ void raster_tile(
                 __syncthreads();
                 const uint32_t kmin = S.kmin;
                 if (kmin == 0xFFFFFFFFu) break;
-                const float top = (k == 0) ? 0.0f : 255.0f * (float)(1u << colours), low = colours ? -top : 0.0f;
+                const uint32_t range = S.colours;
+                const float top = (k == 0) ? 0.0f : 255.0f * (float)(1u << range), low = range ? -top : 0.0f;
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
                     if constexpr (PX == 1) {
@@ -1853,8 +1865,8 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         if (blocks == 0) continue;
         // a stored tile record is only for the target the preprocess was given
         const uint4 *binfo = g.binfo && g.binfo_w == W && g.binfo_h == H ? g.binfo : nullptr;
-        launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
-                            g.max_count, rank_offset, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
+        launch_frame_kernel(bin_count_kernel<false>, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
+                            g.max_count, rank_offset, nseg > 1 ? 1 : 0, g.foreign ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
                             u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
                             rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0, nullptr);
         count_launches(1);
@@ -2015,8 +2027,8 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
         const uint32_t blocks = (g.max_count + kBinThreads - 1) / kBinThreads;
         if (blocks == 0) continue;
         const uint4 *binfo = g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
-        launch_frame_kernel(bin_count_kernel, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
-                            g.sorted_index, g.count, g.max_count, rank_offset, nseg > 1 ? 1 : 0, L.tiles_x, L.tiles_y,
+        launch_frame_kernel(bin_count_kernel<true>, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
+                            g.sorted_index, g.count, g.max_count, rank_offset, nseg > 1 ? 1 : 0, g.foreign ? 1 : 0, L.tiles_x, L.tiles_y,
                             u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
                             shift, started ? nullptr : L.ctrl, L.arena_words, L.blocks() + nblocks);
         count_launches(1);
