@@ -251,6 +251,18 @@ __device__ __forceinline__ float exp_portable(float x) {
     return __fmul_rn(p, __uint_as_float((uint32_t)(ki + 127) << 23));
 }
 
+// exp(x) on [-9, 0] by the special function unit: e^x = 2^(x log2 e).  The PTX ISA gives ex2.approx.ftz an
+// error of at most 2^-22 of a result in [1, 2); the product below 16 is off by half its last place, 2^-21, at
+// most and by 9 2^-24 through the rounding of log2 e, each worth ln 2 of it in the result: below 2^-20
+// of exp(x) together.
+constexpr float kLog2E = 1.4426950408889634f;
+__device__ __forceinline__ float exp2_sfu(float x) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x));
+    return e;
+}
+__device__ __forceinline__ float exp_sfu(float x) { return exp2_sfu(__fmul_rn(x, kLog2E)); }
+
 // Fragment-bearing r² bound of a splat (see gs_splat.ex).  A fragment of alpha a moves a channel
 // of destination d in [0, 255] by a·(s - d), |s - d| <= m = max over the colour channels of
 // max(s, 255 - s); with a·m <= 0.499 (plus FP32 rounding far below 1e-3) the rounded blend gives

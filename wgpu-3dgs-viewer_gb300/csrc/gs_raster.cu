@@ -813,14 +813,6 @@ __global__ void tile_ranges_kernel(const uint2 *pairs, const Ctrl *ctrl, uint2 *
     }
 }
 
-// exp(x) on [-9, 0] by the SFU: what __expf computes, without its handling of denormal arguments
-// and results (an argument that small flushes to 0, whose exp is the same 1).
-__device__ __forceinline__ float exp_sfu(float x) {
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(x, 1.4426950408889634f)));
-    return e;
-}
-
 // Squared quad offset of the pixel centre (pxc, pyc) from a staged splat, and the alpha there
 // (render.wesl:143-181).
 __device__ __forceinline__ float fragment_r2(const float4 a, const float4 b, float pxc, float pyc) {
@@ -1172,11 +1164,9 @@ __device__ __forceinline__ void blend_list2(const RasterShared2 &S, uint32_t nl,
         const float2 r2 = fma2(ux, ux, mul2(uy, uy));
         float2 v;
         if constexpr (MODE == GS_DISPLAY_SPLAT && !PORTABLE_EXP) {
-            const float2 x = mul2(r2, make_float2(-1.4426950408889634f, -1.4426950408889634f));
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v.x) : "f"(x.x));
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v.y) : "f"(x.y));
-            v.x = __fmul_rn(la.y, v.x);
-            v.y = __fmul_rn(la.y, v.y);
+            const float2 x = mul2(r2, make_float2(-kLog2E, -kLog2E));
+            v.x = __fmul_rn(la.y, exp2_sfu(x.x));
+            v.y = __fmul_rn(la.y, exp2_sfu(x.y));
         } else {
             const float4 a = make_float4(0.0f, 0.0f, la.x, la.y);
             v = make_float2(fragment_alpha<MODE, PORTABLE_EXP>(a, r2.x, outline2),
