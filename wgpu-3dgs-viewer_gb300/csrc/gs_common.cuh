@@ -57,7 +57,12 @@ struct Ctrl {
     uint32_t clear_hi;
     uint32_t spin_limit;  // look-back poll bound of this call
     uint32_t stall_tile;  // testing: look-back tile that never publishes (kNoStall: none)
-    uint32_t pad[4];
+    // raster, direct frames: pairs and largest colour_class of a frame's splats, in two sets by turns.  A frame's
+    // tile records add to the set `direct_next`, which starts at zero; its tiles read it (`direct_now`),
+    // clear the other set and make that the next.
+    uint32_t direct_pairs[2], direct_class[2];
+    uint32_t direct_now, direct_next;
+    uint32_t pad[2];
     uint32_t hist[4][256];  // sort: global digit histograms
 };
 static_assert(sizeof(Ctrl) % 16 == 0, "Ctrl must keep 16-byte alignment of what follows");

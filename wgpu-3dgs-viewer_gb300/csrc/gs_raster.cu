@@ -47,8 +47,6 @@ struct RasterLayout {
     uint32_t tiles_x, tiles_y, ntiles, key_bits;
     uint32_t value_bits;  // compact items (see launch_sort_items): bits of a pair value; 0: whole pairs
     uint32_t *items() const { return reinterpret_cast<uint32_t *>(pairs); }
-    // A direct frame sorts no tiles: a word for each CTA of its tile records in the sort's histograms.
-    uint32_t *blocks() const { return &sort_ctrl->hist[0][0]; }
     uint8_t *low(uint32_t max_pairs) const { return reinterpret_cast<uint8_t *>(pairs) + (size_t)max_pairs * 4; }
 };
 
@@ -60,10 +58,6 @@ constexpr uint32_t kEmitBlocks = 152 * 8;
 
 // Ranks a direct frame can have: a bit each in shared memory (RasterShared::raw).
 constexpr uint32_t kDirectMaxRanks = 3u * 16u * kRasterThreads * 8u;
-// ... and CTAs of tile records, segments rounded up (RasterLayout::blocks): a word each, the pairs of its
-// ranks (at most kDirectWork) below their colour class.
-constexpr uint32_t kDirectMaxBlocks = sizeof(Ctrl::hist) / sizeof(uint32_t);
-constexpr uint32_t kBlockPairBits = 28;
 
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = 256 * kScanItems;
@@ -204,9 +198,9 @@ __device__ __forceinline__ uint32_t colour_class(const float4 c) {
 // clear, before the scan and the tile sort read any flag.
 // DIRECT: the ranks are scanned by raster_direct_kernel up to the capacity: each gets its rectangle in one
 // word (`rects`, in place of the count), an empty one where there is no splat or no tile is kept; the first
-// segment's launch (reset non-null) starts the call's control block.
-// The colour_class of `foreign` splats goes to the owner, or (DIRECT) each CTA's to its word of `blocks`,
-// above the CTA's pairs.
+// segment's launch (reset) starts the call's control block.
+// The largest colour_class of `foreign` splats goes to the owner, for direct frames with the pairs to the frame's
+// set of sums.
 // Bound by the latency of the gather: six CTAs an SM (40 registers) take 249 us a binning of four models of
 // 6M splats, five (45 registers) 255.
 template <bool DIRECT>
@@ -215,15 +209,14 @@ __global__ void __launch_bounds__(kBinThreads, 6) bin_count_kernel(
     const uint32_t *count, uint32_t max_count, uint32_t base, int several, int foreign,
     uint32_t tiles_x, uint32_t tiles_y, uint32_t mode, float std2, uint4 *info,
     uint32_t *counts, Ctrl *owner, uint64_t *arena, uint32_t *rects,
-    uint32_t rect_shift, Ctrl *reset, uint32_t arena_words, uint32_t *blocks) {
-    __shared__ uint32_t s_class, s_pairs;
-    if constexpr (DIRECT) {
-        if (threadIdx.x == 0) s_class = s_pairs = 0u;
-        __syncthreads();
-    }
+    uint32_t rect_shift, int reset, uint32_t arena_words) {
     frame_kernel_enter();
     if (arena) arena_clear(owner, arena);
-    if (reset && blockIdx.x == 0 && threadIdx.x == 0) ctrl_reset_flagless(reset, arena_words);
+    const uint32_t set = DIRECT ? owner->direct_next : 0u;
+    if (DIRECT && reset && blockIdx.x == 0 && threadIdx.x == 0) {
+        ctrl_reset_flagless(owner, arena_words);
+        owner->direct_now = set;
+    }
     const uint32_t n = count ? min(*count, max_count) : max_count;
     const uint32_t k = blockIdx.x * kBinThreads + threadIdx.x;
     uint4 t = make_uint4(0u, 0u, 0u, 0u);  // x0 | y0 << 16, w | h << 16, mask, count
@@ -251,11 +244,9 @@ __global__ void __launch_bounds__(kBinThreads, 6) bin_count_kernel(
             rects[k] = t.w ? pack_rect(t.x & 0xFFFFu, t.x >> 16, (t.x & 0xFFFFu) + (t.y & 0xFFFFu) - 1u,
                                        (t.x >> 16) + (t.y >> 16) - 1u, rect_shift)
                            : kEmptyRect;
-        if (colours) atomicMax(&s_class, colours);
+        if (colours) atomicMax(&owner->direct_class[set], colours);
         const uint32_t pairs = __reduce_add_sync(0xFFFFFFFFu, t.w);
-        if ((threadIdx.x & 31u) == 0) atomicAdd(&s_pairs, pairs);
-        __syncthreads();
-        if (threadIdx.x == 0) blocks[blockIdx.x] = (s_class << kBlockPairBits) | s_pairs;
+        if ((threadIdx.x & 31u) == 0 && pairs) atomicAdd(&owner->direct_pairs[set], pairs);
     } else {
         if (k < n) counts[k] = t.w;
         else if (k < max_count && several) counts[k] = 0u;  // the scan covers every segment's capacity
@@ -1290,7 +1281,7 @@ __device__ __forceinline__ void raster_tile(
     Value d[3] = {}, h[3] = {};
     const bool wild = colours > kColourClasses;
     const uint32_t early = wild ? 0xFFFFFFFFu : early_out_min<MODE, PX>(suffix_min);
-    if (tid == 0) S.colours = colours;  // read after the first barrier
+    if (MODE != GS_DISPLAY_POINT && tid == 0) S.colours = colours;  // read after the first barrier
     // blends the list onto the pixels whose `on` is set
     auto blend = [&](auto both, uint32_t nl, const bool *on) {
         if constexpr (PX == 1) {
@@ -1611,9 +1602,9 @@ template <uint32_t MODE, bool PORTABLE_EXP, bool FEW>
 __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     raster_direct_kernel(const RasterJob J, const uint32_t *rects, const uint4 *info,
                          uint32_t ranks, uint32_t shift, uint32_t *values, uint32_t max_pairs, float std2,
-                         float outline2, uint32_t suffix_min, float eps, const uint32_t *blocks, uint32_t nblocks) {
+                         float outline2, uint32_t suffix_min, float eps) {
     __shared__ RasterShared1 S;
-    __shared__ uint32_t s_warp[kRasterThreads / 32], s_class[kRasterThreads / 32], s_pairs[kRasterThreads / 32], s_base;
+    __shared__ uint32_t s_warp[kRasterThreads / 32], s_base;
     uint32_t *hits = reinterpret_cast<uint32_t *>(S.raw);  // bit r of word q: rank 32 q + r holds the tile
     static_assert(sizeof(S.raw) * 8 >= kDirectMaxRanks, "a bit per rank");
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, tile = blockIdx.x;
@@ -1621,7 +1612,15 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
     const uint32_t here = pack_rect(tx, ty, tx, ty, shift);
     constexpr uint32_t STEP = kRasterThreads / 32u;
     frame_kernel_enter();
-    const uint32_t block = tid < nblocks ? blocks[tid] : 0u;  // waited for after the scan
+    // Both sets' pairs and classes at once, on their way while the ranks are scanned (65k splats at 640x360: 116
+    // us a frame through shared memory, 112 so; points, with registers to spare, 98 so and 92 after the scan).
+    uint4 sums;
+    uint32_t set;
+    auto read_sums = [&]() {
+        sums = *reinterpret_cast<const uint4 *>(J.ctrl->direct_pairs);
+        set = J.ctrl->direct_now;
+    };
+    if constexpr (MODE != GS_DISPLAY_POINT) read_sums();
     for (uint32_t q0 = warp; q0 < words; q0 += 8u * STEP) {
         uint32_t r[8];
 #pragma unroll
@@ -1636,26 +1635,14 @@ __global__ void __launch_bounds__(kRasterThreads, FEW ? 4 : 6)
             if (lane == 0 && q < words) hits[q] = m;
         }
     }
-    // the frame's pairs and colour class, from the tile records' CTAs
-    constexpr uint32_t pair_mask = (1u << kBlockPairBits) - 1u;
-    uint32_t colours = block >> kBlockPairBits, wanted = block & pair_mask;
-    for (uint32_t b = tid + kRasterThreads; b < nblocks; b += kRasterThreads) {
-        colours = max(colours, blocks[b] >> kBlockPairBits);
-        wanted += blocks[b] & pair_mask;
-    }
-    colours = __reduce_max_sync(0xFFFFFFFFu, colours);
-    wanted = __reduce_add_sync(0xFFFFFFFFu, wanted);
-    if (lane == 0) s_class[warp] = colours, s_pairs[warp] = wanted;
+    if constexpr (MODE == GS_DISPLAY_POINT) read_sums();
     __syncthreads();
-    colours = wanted = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kRasterThreads / 32u; ++w) {
-        colours = max(colours, s_class[w]);
-        wanted += s_pairs[w];
-    }
+    const uint32_t wanted = set ? sums.y : sums.x, colours = set ? sums.w : sums.z;
     if (tile == 0 && tid == 0) {
         J.ctrl->total = wanted;
         if (wanted > max_pairs) atomicOr(&J.ctrl->status, kStatusCapacity);
+        J.ctrl->direct_pairs[set ^ 1u] = J.ctrl->direct_class[set ^ 1u] = 0u;
+        J.ctrl->direct_next = set ^ 1u;
     }
     // thread t owns the words [t per, (t + 1) per): their places in the list by a block scan
     const uint32_t per = (words + kRasterThreads - 1u) / kRasterThreads;
@@ -1858,7 +1845,7 @@ cudaError_t launch_binning_front(const RasterSegment *segs, uint32_t nseg, const
         launch_frame_kernel(bin_count_kernel<false>, blocks, kBinThreads, 0, st, overlap, g.splats, binfo, g.sorted_index, g.count,
                             g.max_count, rank_offset, nseg > 1 ? 1 : 0, g.foreign ? 1 : 0, L.tiles_x, L.tiles_y, u.display_mode,
                             u.std_dev * u.std_dev, L.info + rank_offset, L.offsets + rank_offset, L.ctrl,
-                            rank_offset ? nullptr : L.flags, nullptr, 0, nullptr, 0, nullptr);
+                            rank_offset ? nullptr : L.flags, nullptr, 0, 0, 0);
         count_launches(1);
         rank_offset += g.max_count;
     }
@@ -1973,10 +1960,8 @@ cudaError_t launch_binning(const RasterSegment *segs, uint32_t nseg, const Raste
 // (8.8e7): 128 -> 125; 68.4k x 1400 (9.6e7): 157 -> 167; 28.6k x 5292 (1.5e8): 135 -> 161.  Views of a
 // batch overlap, so the tiles of all of them count (10 views of 11.6k, 4e8 so counted: 234 -> 440).
 constexpr uint64_t kDirectWork = 60'000'000;
-static_assert(kDirectWork < (1u << kBlockPairBits) && kWildColours < (1u << (32u - kBlockPairBits)), "a word a CTA");
-static bool direct_raster(uint32_t ranks, uint32_t blocks, uint32_t tiles_at_once) {
-    return ranks > 0 && ranks <= kDirectMaxRanks && blocks <= kDirectMaxBlocks &&
-           (uint64_t)ranks * tiles_at_once <= kDirectWork;
+static bool direct_raster(uint32_t ranks, uint32_t tiles_at_once) {
+    return ranks > 0 && ranks <= kDirectMaxRanks && (uint64_t)ranks * tiles_at_once <= kDirectWork;
 }
 
 // Frames of separate requests that overlap share the L2 that their scans are bound by: their work
@@ -1987,16 +1972,16 @@ constexpr uint64_t kDirectWorkInFlight = 240'000'000;
 
 uint64_t direct_raster_work(uint32_t max_splats, uint32_t W, uint32_t H) {
     const uint32_t tiles = ((W + GS_TILE - 1) / GS_TILE) * ((H + GS_TILE - 1) / GS_TILE);
-    return direct_raster(max_splats, (max_splats + kBinThreads - 1) / kBinThreads, tiles) ? (uint64_t)max_splats * tiles : 0;
+    return direct_raster(max_splats, tiles) ? (uint64_t)max_splats * tiles : 0;
 }
 
 template <uint32_t MODE>
-static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift, uint32_t nblocks,
+static void launch_direct_mode(const RasterJob &J, const RasterLayout &L, uint32_t ranks, uint32_t shift,
                                uint32_t max_pairs, uint32_t tiles_at_once, float std2, float outline2, int exact, cudaStream_t st, const Tuning &t) {
     const bool few = tiles_at_once <= kFewTiles;
     auto go = [&](auto kernel) {
         launch_frame_kernel(kernel, J.ntiles, kRasterThreads, 0, st, frame_launch_overlaps(st), J, L.offsets, L.info, ranks,
-                            shift, L.items(), max_pairs, std2, outline2, t.suffix_min, t.eps, L.blocks(), nblocks);
+                            shift, L.items(), max_pairs, std2, outline2, t.suffix_min, t.eps);
     };
     if (exact) few ? go(raster_direct_kernel<MODE, true, true>) : go(raster_direct_kernel<MODE, true, false>);
     else few ? go(raster_direct_kernel<MODE, false, true>) : go(raster_direct_kernel<MODE, false, false>);
@@ -2008,7 +1993,7 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
                                         int exact_exp, cudaStream_t st, const Tuning &tn) {
     const RasterLayout L = raster_layout(scratch, ranks, J.W, J.H, max_pairs);
     const float std2 = u.std_dev * u.std_dev, o = u.std_dev - 0.1f, outline2 = o * o;
-    uint32_t rank_offset = 0, shift = 0, nblocks = 0;
+    uint32_t rank_offset = 0, shift = 0;
     while (((L.tiles_x - 1u) >> shift) > 127u || ((L.tiles_y - 1u) >> shift) > 127u) ++shift;
     bool started = false;
     prof_mark(kProfBin, true, st);
@@ -2019,24 +2004,23 @@ static cudaError_t launch_raster_direct(const RasterSegment *segs, uint32_t nseg
         const uint4 *binfo = g.binfo && g.binfo_w == J.W && g.binfo_h == J.H ? g.binfo : nullptr;
         launch_frame_kernel(bin_count_kernel<true>, blocks, kBinThreads, 0, st, frame_launch_overlaps(st), g.splats, binfo,
                             g.sorted_index, g.count, g.max_count, rank_offset, nseg > 1 ? 1 : 0, g.foreign ? 1 : 0, L.tiles_x, L.tiles_y,
-                            u.display_mode, std2, L.info + rank_offset, nullptr, nullptr, nullptr, L.offsets + rank_offset,
-                            shift, started ? nullptr : L.ctrl, L.arena_words, L.blocks() + nblocks);
+                            u.display_mode, std2, L.info + rank_offset, nullptr, L.ctrl, nullptr, L.offsets + rank_offset,
+                            shift, started ? 0 : 1, L.arena_words);
         count_launches(1);
         started = true;
         rank_offset += g.max_count;
-        nblocks += blocks;
     }
     prof_mark(kProfBin, false, st);
     prof_mark(kProfRaster, true, st);
     switch (u.display_mode) {
         case GS_DISPLAY_SPLAT:
-            launch_direct_mode<GS_DISPLAY_SPLAT>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_SPLAT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
         case GS_DISPLAY_ELLIPSE:
-            launch_direct_mode<GS_DISPLAY_ELLIPSE>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_ELLIPSE>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
         default:
-            launch_direct_mode<GS_DISPLAY_POINT>(J, L, ranks, shift, nblocks, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
+            launch_direct_mode<GS_DISPLAY_POINT>(J, L, ranks, shift, max_pairs, tiles_at_once, std2, outline2, exact_exp, st, tn);
             break;
     }
     count_launches(1);
@@ -2051,13 +2035,10 @@ cudaError_t launch_raster(const RasterSegment *segs, uint32_t nseg, const Raster
     const RasterJob J = raster_job(segs, nseg, target, W, H, pitch, max_pairs, scratch);
     if (J.ntiles == 0) return cudaSuccess;
     const uint32_t at_once = tiles_at_once > J.ntiles ? tiles_at_once : J.ntiles;
-    uint32_t ranks = 0, blocks = 0;
-    for (uint32_t s = 0; s < nseg; ++s) {
-        ranks += segs[s].max_count;
-        blocks += (segs[s].max_count + kBinThreads - 1) / kBinThreads;
-    }
+    uint32_t ranks = 0;
+    for (uint32_t s = 0; s < nseg; ++s) ranks += segs[s].max_count;
     // (the counting rasteriser and the bounded-wait hook know the general path only)
-    if (direct_raster(ranks, blocks, at_once) && direct_in_flight <= kDirectWorkInFlight && !prof_counting() && wait_config().stall_tile == kNoStall)
+    if (direct_raster(ranks, at_once) && direct_in_flight <= kDirectWorkInFlight && !prof_counting() && wait_config().stall_tile == kNoStall)
         return launch_raster_direct(segs, nseg, ranks, u, J, max_pairs, scratch, at_once, exact_exp, st, tn);
     cudaError_t e = launch_binning(segs, nseg, u, W, H, max_pairs, scratch, st);
     if (e != cudaSuccess) return e;
