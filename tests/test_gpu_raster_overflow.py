@@ -72,3 +72,39 @@ def test_overflowing_direct_frame_is_rendered_again(gs, cuda, oracle, monkeypatc
     u = oracle.frame_uniforms(pod, gs.model_transform_pod(), gt, w, h)
     want, *_ = oracle.render(u, sc, R.FORMAT_FP32, w, h, exp_mode=0, threads=8)
     assert np.array_equal(t.download(), want)
+
+
+def test_direct_frames_by_turns_on_one_scratch(gs, cuda):
+    """Frames that fit, overflow, hold colours out of range or are binned, one after another in the same scratch:
+    each as with a scratch of its own, its pair total too."""
+    w, h, n = 320, 180, 4_000
+    u = uniforms(gs, w, h, k=1, radius=3.0)
+    pipe = StagePipeline(gs, cuda, S.synth_scene(n, seed=10), R.FORMAT_FP32, w, h)
+    pipe.preprocess(u)
+    pipe.sort()
+    beyond = pipe.splats.clone()
+    beyond.view(-1, 12)[::5, 8] = 900.0
+    wild = pipe.splats.clone()
+    wild.view(-1, 12)[::7, 9] = float("nan")
+    spare = 300_000  # capacity that takes a frame to the binned route
+    frames = [(pipe.splats, n, 1 << 20), (beyond, n, 1 << 20), (pipe.splats, n, 700), (pipe.splats, n, 1 << 20), (wild, n, 1 << 20),
+              (pipe.splats, n // 3, 1 << 20), (wild, spare, 1 << 20), (pipe.splats, n, 1 << 20), (beyond, n, 900),
+              (pipe.splats, spare, 700), (pipe.splats, n, 1 << 20), (pipe.splats, 50, 1 << 20)]
+    nb = gs.Renderer.scratch_bytes(spare, w, h, 1 << 20)
+    shared = cuda.zeros(nb, dtype=cuda.uint8, device="cuda")
+
+    def render(k, scratch):
+        splats, cap, pairs = frames[k]
+        full = cuda.zeros(cap * 12, dtype=cuda.float32, device="cuda")
+        full[: min(cap, n) * 12] = splats[: min(cap, n) * 12]
+        order = cuda.arange(cap, dtype=cuda.int32, device="cuda")
+        count = cuda.tensor([min(cap, n)], dtype=cuda.int32, device="cuda")
+        gs.Renderer.render(u, full, order, count, cap, pipe.target, w, h, w * 4, pairs, scratch, nb)
+        cuda.cuda.synchronize()
+        return gs.Renderer.status(scratch) + (pipe.frame().tobytes(),)
+
+    alone = [render(k, cuda.zeros(nb, dtype=cuda.uint8, device="cuda")) for k in range(len(frames))]
+    assert {a[0] for a in alone} == {0, 6}
+    for _ in range(2):
+        for k in range(len(frames)):
+            assert render(k, shared) == alone[k], k
