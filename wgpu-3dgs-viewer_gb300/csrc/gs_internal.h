@@ -37,7 +37,7 @@ __global__ void ctrl_init_kernel(Ctrl *ctrl, uint32_t arena_words, WaitCfg cfg);
 // of frame_kernel_enter() may read what kernels up to k - 1 wrote.  Every kernel launched by
 // launch_frame_kernel() calls it in all threads before it touches memory that others write.
 // It hides a launch's latency and drain behind its neighbours: 5k splats at 320x180 44.2 -> 34.8 us a
-// frame (5 launches), 100k at 640x360 164 -> 141 (12), 1M / 1080p 683 -> 657, 6M 1718 -> 1707.
+// frame, 100k at 640x360 164 -> 141, 1M / 1080p 683 -> 657, 6M 1718 -> 1707.
 // Not while `st` is being captured: in a batch's graph the views' chains overlap one another already
 // (10 views of 93k splats 535 us, 553 with programmatic edges; 8 of 9k 164, 158).
 bool frame_launch_overlaps(cudaStream_t st);

@@ -25,7 +25,7 @@ namespace gs {
 
 constexpr uint32_t kBinThreads = 256;
 constexpr uint32_t kRasterThreads = 256;
-// A warp's pixel block is 8x4 pixels: its pixel centres span 7 x 3 pixels.
+// A warp's pixel block is 8x4 pixels, or 8x8 with two pixels a thread: its pixel centres span 7 x 3 or 7 x 7.
 constexpr float kBlockSpanX = 7.0f;
 
 struct RasterLayout {
@@ -230,11 +230,12 @@ __global__ void __launch_bounds__(kBinThreads, 6) bin_count_kernel(
             } else {
                 // all three 16-byte parts in one round trip (the colour bounds the corner-tile test)
                 const float4 *src = reinterpret_cast<const float4 *>(splats + gi);
-                const float4 a = src[0];
-                const float4 q = src[1];
-                const float4 c = src[2];
+                const float4 a = src[0], q = src[1], c = src[2];
+                // ahead of the tile test: the branch keeps the three loads together (8 views of 6M splats 10.96 ms a
+                // batch with the class found behind the test, 10.78 so)
+                if (foreign) colours = colour_class(c);
                 t = splat_tile_info(a, q, c, tiles_x, tiles_y, mode, std2);
-                if (foreign && t.w) colours = colour_class(c);
+                if (t.w == 0u) colours = 0u;
             }
         }
         info[k] = make_uint4(t.x, t.y, t.z, base + gi);
@@ -975,7 +976,7 @@ struct ChunkSource {
 };
 
 // Whether the fragment ellipse {p : |Q·(p - c)|² <= lim} of a staged splat meets the rectangle
-// of pixel centres [bx0, bx0 + 7] x [by0, by0 + 3] of a warp's block.  With c outside the
+// of pixel centres [bx0, bx1] x [by0, by1] of a warp's block.  With c outside the
 // rectangle, the nearest point of the rectangle in the quadratic norm lies on an edge whose
 // half-plane c violates (moving from it toward c must leave the rectangle); Q maps each edge
 // to a segment in quad space, where the distance from the origin is minimised in closed form.
@@ -1227,10 +1228,10 @@ __device__ __noinline__ PairState blend_list2_wild(const RasterShared2 &S, uint3
 
 // Shortest list that takes the early-out, from the caller's suffix_min (default 1024).  Splats, a pixel
 // a thread: three quarters of it (13.5k at 237x133 48 us a frame at 768, 52 at 384).  Two pixels a
-// thread walk half as many samples: nine sixteenths (576 by default: 477, 321, 1340 and 232 us at 6M /
-// 1080p, 1M / 1080p, 3M / 4K and 400k / 1366x768, against 486, 320, 1413, 246 at 768 and 480, 330, 1320,
-// 229 at 384).  Ellipses end sooner, as outlines are opaque and interiors keep their full alpha: a
-// quarter (256: the frame of 700k at 1600x900 387 us, against 388 at 384, 414 at 768 and 392 at 128).
+// thread walk half as many samples: nine sixteenths (576 by default; compared on one build, 477, 321, 1340
+// and 232 us at 6M / 1080p, 1M / 1080p, 3M / 4K and 400k / 1366x768, against 486, 320, 1413, 246 at 768 and
+// 480, 330, 1320, 229 at 384).  Ellipses end sooner, as outlines are opaque and interiors keep their full
+// alpha: a quarter (256: the frame of 700k at 1600x900 387 us, against 388 at 384, 414 at 768 and 392 at 128).
 constexpr float kWalkCourse = 0.9f;
 template <uint32_t MODE, uint32_t PX>
 __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
@@ -1257,8 +1258,8 @@ __device__ __forceinline__ uint32_t early_out_min(uint32_t suffix_min) {
 // Bound: the arithmetic of the list loops (no memory system near its limit), so time follows the warp
 // iterations and what one of them issues.  Measured at 6M / 1080p, 1M / 1080p and 3M / 4K: 935, 514 and
 // 2614 us with a walk A of every pixel over compacted lists and each chunk's loads waited for; 629,
-// 392 and 1864 us with the sampled walk, the loads a chunk ahead and the SFU exp without denormal
-// handling; 482, 323 and 1355 us with two pixels a thread, which share the list, the loads and, in
+// 392 and 1864 us with the sampled walk, the loads a chunk ahead and exp_sfu; 483, 325 and 1357 us with
+// two pixels a thread, which share the list, the loads and, in
 // packed instructions, the arithmetic (64 registers, 8 CTAs an SM; 7, 9 and 10 CTAs take 497, 496 and
 // 506 us where 8 take 489).  Points (1.5M, 1283x717): 107 us blended like splats, 60 us.
 template <uint32_t MODE, bool PORTABLE_EXP, bool COUNT, uint32_t UNROLL, class Shared>

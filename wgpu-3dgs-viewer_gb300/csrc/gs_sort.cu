@@ -3,7 +3,8 @@
 // Same contract as the reference RadixSorter (src/radix_sorter.rs:56-96,658-669; kernels
 // src/shader/radix_sort.wgsl:78-529): 8-bit digits, least significant first, stable; the
 // reference's 3840-key block stays the unit of the depth buffer's padding.  The GB300 design
-// differs: 7680-key pass blocks; one global-histogram kernel reads the keys once
+// differs: up to 65,536 pairs are sorted by one cluster of CTAs in one launch; larger sorts take pass
+// blocks of 2048, 4096 or 7680 keys; one global-histogram kernel reads the keys once
 // for all passes (its last CTA turns the histograms into exclusive digit offsets); each pass is
 // a single kernel that ranks its block warp by warp (match.any, or one ballot per digit bit, so
 // equal digits keep input order), publishes per-digit counts and resolves the block's global
@@ -22,8 +23,8 @@
 
 namespace gs {
 
-// A pass block is 512 threads x 15 keys = 7680 keys, two of the reference's 3840-key blocks:
-// longer digit runs in the scatter, and two CTAs (32 warps) per SM.  Threads 0..255 own the
+// A full pass block is 512 threads x 15 keys = 7680 keys, two of the reference's 3840-key blocks:
+// longer digit runs in the scatter, and two CTAs (32 warps) per SM (fewer rows: see sort_rows).  Threads 0..255 own the
 // digits in the per-digit phases.  The reordered block (60 KB) lives in dynamic shared memory.
 constexpr uint32_t kSortThreads = 512;
 constexpr uint32_t kSortRows = 15;
