@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "gs_record.h"
@@ -66,6 +67,7 @@ struct Ctrl {
     uint32_t hist[4][256];  // sort: global digit histograms
 };
 static_assert(sizeof(Ctrl) % 16 == 0, "Ctrl must keep 16-byte alignment of what follows");
+static_assert(offsetof(Ctrl, direct_pairs) % 16 == 0, "both sets' pairs and classes are read by one 16-byte load");
 
 // Resets a control block for a new stage call (one CTA): epoch, status, tickets, counters,
 // histograms, wait configuration.  The epoch comes from `owner`, the block holding the area's serial
